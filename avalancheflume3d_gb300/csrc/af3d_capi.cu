@@ -1733,10 +1733,12 @@ extern "C" af3d_status af3d_adjoint(af3d_ctx *c, long steps, long ckpt_every, do
     if (e == cudaSuccess) {
       buf.owned.push_back(base);
       for (size_t k = 0; k < tape.size(); k++) {
-        double *pl = reinterpret_cast<double *>(base + slot * k);
+        // the records first: a slot starts on a 256-byte boundary and a record is 192 bytes, so
+        // they stay on the 64-byte boundaries their vector stores need whatever the clump count
+        tape_rec[k] = reinterpret_cast<NbrRec *>(base + slot * k);
+        double *pl = reinterpret_cast<double *>(tape_rec[k] + m);
         for (int i = 0; i < NPLANES; i++) tape[k].p[i] = i < kAdjPlanes + 3 ? pl + (size_t)i * m : nullptr;
-        tape_rec[k] = reinterpret_cast<NbrRec *>(pl + (size_t)(kAdjPlanes + 3) * m);
-        tape_lists[k].items = reinterpret_cast<unsigned *>(tape_rec[k] + m);
+        tape_lists[k].items = reinterpret_cast<unsigned *>(pl + (size_t)(kAdjPlanes + 3) * m);
         tape_lists[k].cnt = reinterpret_cast<int *>(tape_lists[k].items + (size_t)kListCap * m);
         tape_lists[k].ovf = nullptr;
       }

@@ -318,6 +318,24 @@ def test_ensemble_adjoint_equals_each_flume_alone(af3d):
         lo = hi
 
 
+def test_adjoint_of_odd_clump_counts(af3d):
+    """A flume of 75 clumps alone (every tape slot's arrays then start at odd multiples of their
+    element size) equals the same flume as both halves of an ensemble of 150."""
+    from tests.states import flume_system, wall_state
+    n = 75
+    sys, fun = flume_system(n)
+    pp = wall_state(n, 5, sys)
+    solo = _adjoint(af3d, sys, fun, pp, steps=12, ckpt=5)
+    with af3d.Engine(np.stack([sys, sys]), np.stack([fun, fun])) as eng:
+        eng.import_particles(np.concatenate([pp, pp]))
+        both = eng.adjoint(12, 12)
+    for f in range(2):
+        assert solo["J"] == pytest.approx(both["J"][f], rel=1e-14)
+        for k in ("r0", "v0", "w0", "R0"):
+            want = both[k][f * n:(f + 1) * n]
+            assert np.max(np.abs(solo[k] - want)) <= 1e-12 * np.max(np.abs(want)), (f, k)
+
+
 def test_adjoint_with_overflowed_contact_lists(af3d, base, oracle, tangent):
     """Five clumps piled almost on one spot give a clump more sphere contacts than its item lists
     hold (32), every step: its contacts run by the per-clump walk in the forward pass, and the
