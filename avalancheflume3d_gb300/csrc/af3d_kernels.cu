@@ -222,6 +222,24 @@ __device__ __forceinline__ long bin_axis(double x, double xmin, double inv, long
 
 constexpr double kSmallAngle2 = 9.765625e-04;   // (2^-5)^2
 
+// sin t and cos t of a rotation angle t >= 0 with t2 = t^2 (rounded).  Below 2^-5 rad (a step of
+// 2e-6 s turns a clump by ~1e-4) the Maclaurin series, the first omitted terms below 2^-54 of the
+// sums, with one final rounding each: 6 or 10 FP64 instructions where CUDA's sincos takes ~26
+// (1680 cycles of the FP64 unit, measured).
+__device__ __forceinline__ void sincos_step(double t, double t2, double &sn, double &c) {
+  if (!in_open_range_bits(t2, 0.0, kSmallAngle2)) {
+    sincos(t, &sn, &c);
+    return;
+  }
+  double p = 1.0 / 120.0, q = 1.0 / 24.0;
+  if (!in_open_range_bits(t2, 0.0, 9.5367431640625e-07)) {   // 2^-20
+    p = __fma_rn(t2, __fma_rn(t2, 1.0 / 362880.0, -1.0 / 5040.0), p);
+    q = __fma_rn(t2, __fma_rn(t2, 1.0 / 40320.0, -1.0 / 720.0), q);
+  }
+  sn = __fma_rn(t * t2, __fma_rn(t2, p, -1.0 / 6.0), t);
+  c = __fma_rn(-t2, __fma_rn(-t2, q, 0.5), 1.0);
+}
+
 // init_Verlet.cu:25-148 for one clump that is not removed: r, v, w and the rotation rows move
 // one step with a_i, alpha_i; sp receives the new sphere centres.
 __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, V3 &Rx, V3 &Ry, V3 &Rz, V3 *sp,
@@ -265,7 +283,7 @@ __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, 
       imag = rsqrt(mag2);
       mag = mag2 * imag;
     } else {
-      mag = sqrt(mag2);
+      mag = sqrt_rn(mag2);
     }
     if (mag > 0.0) {
       // Rodrigues rotation about dO/|dO| by |dO| (init_Verlet.cu:63-83)
@@ -275,8 +293,9 @@ __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, 
         u = mk(dO.x * imag, dO.y * imag, dO.z * imag);
         sincos(mag, &sn, &c);
       } else {
-        u = mk(dO.x / mag, dO.y / mag, dO.z / mag);
-        sincos(mag, &sn, &c);   // init_Verlet.cu's cos and sin, from one argument reduction
+        const Divisor by = divisor_of(mag);
+        u = mk(div_by(dO.x, by), div_by(dO.y, by), div_by(dO.z, by));
+        sincos_step(mag, mag2, sn, c);   // init_Verlet.cu's cos and sin
       }
       const double omc = 1.0 - c;
       dRx = mk(omc * u.x * u.x + c, omc * u.x * u.y - sn * u.z, omc * u.x * u.z + sn * u.y);
@@ -309,18 +328,19 @@ __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, 
     in = inv_norm(Tx.z * Tx.z + Ty.z * Ty.z + Tz.z * Tz.z);
     Rx.z = Tx.z * in; Ry.z = Ty.z * in; Rz.z = Tz.z * in;
   } else {
-    double nrm = sqrt(Tx.x * Tx.x + Ty.x * Ty.x + Tz.x * Tz.x);
-    Rx.x = Tx.x / nrm; Ry.x = Ty.x / nrm; Rz.x = Tz.x / nrm;
-    nrm = sqrt(Tx.y * Tx.y + Ty.y * Ty.y + Tz.y * Tz.y);
-    Rx.y = Tx.y / nrm; Ry.y = Ty.y / nrm; Rz.y = Tz.y / nrm;
-    nrm = sqrt(Tx.z * Tx.z + Ty.z * Ty.z + Tz.z * Tz.z);
-    Rx.z = Tx.z / nrm; Ry.z = Ty.z / nrm; Rz.z = Tz.z / nrm;
+    Divisor by = divisor_of(sqrt_rn(Tx.x * Tx.x + Ty.x * Ty.x + Tz.x * Tz.x));
+    Rx.x = div_by(Tx.x, by); Ry.x = div_by(Ty.x, by); Rz.x = div_by(Tz.x, by);
+    by = divisor_of(sqrt_rn(Tx.y * Tx.y + Ty.y * Ty.y + Tz.y * Tz.y));
+    Rx.y = div_by(Tx.y, by); Ry.y = div_by(Ty.y, by); Rz.y = div_by(Tz.y, by);
+    by = divisor_of(sqrt_rn(Tx.z * Tx.z + Ty.z * Ty.z + Tz.z * Tz.z));
+    Rx.z = div_by(Tx.z, by); Ry.z = div_by(Ty.z, by); Rz.z = div_by(Tz.z, by);
   }
   w.x += dt * al.x;
   w.y += dt * al.y;
   w.z += dt * al.z;
   // sphere centres r + (radius/sqrt2) R (+-1,+-1,+-1) (init_Verlet.cu:130-142)
-  const double pos = kFast ? rad * (1.0 / kROOT2) : rad / kROOT2;
+  constexpr Divisor root2 = constant_divisor(kROOT2, 0x3FF6A09E667F3BCCull);
+  const double pos = kFast ? rad * (1.0 / kROOT2) : div_by(rad, root2);
   if (kFast) {
     // the four patterns (a + c, b - c, c - a, -(b + c)) with a = x + y, b = x - y, from the
     // two partial sums r0 + pos c and r0 - pos c: eight operations per row

@@ -51,7 +51,7 @@ cudaError_t measure_dfma(int sms, double *tflops) {
 
 namespace {
 
-// The integer-pipe helpers of af3d_physics.cuh against the hardware instructions they replace:
+// The integer-pipe helpers of af3d_physics.cuh and af3d_intfp64.cuh against the hardware instructions they replace:
 // per element, one bit per helper that disagreed.
 __global__ void k_check_bits(const double *x, int *bad, long n) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -66,6 +66,13 @@ __global__ void k_check_bits(const double *x, int *bad, long n) {
   const double lo = 1.0 - 1.4901161193847656e-08, hi = 1.0 + 1.4901161193847656e-08;
   if (!(v < 0.0) && in_open_range_bits(v, lo, hi) != (fabs(v - 1.0) < 1.4901161193847656e-08)) b |= 32;
   if (!(v < 0.0) && in_open_range_bits(v, 0.0, 9.765625e-04) != (v > 0.0 && v < 9.765625e-04)) b |= 64;
+  // the divisor: the array's mirror element, so that a caller chooses the pairs
+  const double w = x[n - 1 - i];
+  auto differ = [](double p, double q) { return bits_of(p) != bits_of(q) && !(isnan(p) && isnan(q)); };
+  if (differ(sqrt_rn(v), __dsqrt_rn(v))) b |= 128;
+  if (differ(div_rn(v, w), __ddiv_rn(v, w))) b |= 256;
+  const double r = reciprocal(v), want = __ddiv_rn(1.0, v);
+  if (differ(r, want) && llabs((long long)(bits_of(r) - bits_of(want))) > 1) b |= 512;
   bad[i] = b;
 }
 

@@ -27,6 +27,7 @@
 #pragma once
 
 #include "af3d_internal.h"
+#include "af3d_intfp64.cuh"
 
 namespace af3d {
 
@@ -140,8 +141,8 @@ __device__ __forceinline__ bool contact_law_fast(V3 dvvc, V3 n, double comp, dou
   const double vn = dvvc.x * n.x + dvvc.y * n.y + dvvc.z * n.z;
   const V3 vt = mk(dvvc.x - vn * n.x, dvvc.y - vn * n.y, dvvc.z - vn * n.z);
   const double vt2 = vt.x * vt.x + vt.y * vt.y + vt.z * vt.z;
-  const double inv_vt = rsqrt(vt2);          // +inf for vt = 0: the tangential part is then NaN
-  const double vt_mag = vt2 * inv_vt;        // and skipped, as in the exact law
+  double inv_vt;                             // +inf for vt = 0: the tangential part is then skipped,
+  const double vt_mag = sqrt_and_inverse(vt2, inv_vt);   // as in the exact law
   // dvvc . vt / |vt| = |vt| up to the rounding of vt's orthogonality to n, which the exact law
   // also rounds: the fast law takes |vt| itself
   const double vt_sig = vt_mag;
@@ -156,7 +157,7 @@ __device__ __forceinline__ bool contact_law_fast(V3 dvvc, V3 n, double comp, dou
       // af = 0.8 mu N / |vt|, t0 = m / af, af / (1 + (dt / t0)^2) = af m^2 / (m^2 + (dt af)^2)
       const double af = 0.8 * mu * normal * inv_vt;
       const double dta = dt * af;
-      const double a = af * (mass_t * mass_t) / (mass_t * mass_t + dta * dta);
+      const double a = af * (mass_t * mass_t) * reciprocal(mass_t * mass_t + dta * dta);
       f.x += a * vt.x;
       f.y += a * vt.y;
       f.z += a * vt.z;
@@ -178,11 +179,12 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
   vt.x = dvvc.x - vn * n.x;
   vt.y = dvvc.y - vn * n.y;
   vt.z = dvvc.z - vn * n.z;
-  double vt_mag = sqrt(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
+  double vt_mag = sqrt_rn(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
+  const Divisor vt_div = divisor_of(vt_mag);
   V3 tv;
-  tv.x = vt.x / vt_mag;
-  tv.y = vt.y / vt_mag;
-  tv.z = vt.z / vt_mag;
+  tv.x = div_by(vt.x, vt_div);
+  tv.y = div_by(vt.y, vt_div);
+  tv.z = div_by(vt.z, vt_div);
   double vt_sig = dvvc.x * tv.x + dvvc.y * tv.y + dvvc.z * tv.z;
   double normal = km * comp + gm * (-vn);
   if (gate ? (normal <= 0.0) : !(normal > 0.0)) return false;
@@ -191,7 +193,7 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
   f.z = -normal * n.z;
   double xi = dt * vt_sig;
   if (cns_1 * normal < fabs(xi)) xi = 0.0;
-  double xi_dot = xi / dt;
+  double xi_dot = nonzero_bits(xi) ? div_rn(xi, dt) : xi;   // dt > 0
   double fsdt = 1.0e12 * mass_t * xi + 2.0e6 * mass_t * xi_dot;
   if (vt_mag > 0.0) {
     // Coulomb branch:  af = 0.8 mu N / |vt|; t0 = m / af; af /= 1 + (dt/t0)^2; f += af vt.
@@ -200,11 +202,11 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
     // a warp whose lanes take different branches executes three divisions, not seven; every
     // lane still evaluates exactly its own branch's operations.
     const bool coulomb = fabs(fsdt) > mu * normal || (xi0 && xi == 0.0);
-    const double q1 = (coulomb ? 0.8 * mu * normal : fsdt * vt.x) / vt_mag;   // af  | f_x term
-    const double q2 = (coulomb ? mass_t : fsdt * vt.y) / (coulomb ? q1 : vt_mag);   // t0 | f_y
-    const double q3 = (coulomb ? dt : fsdt * vt.z) / (coulomb ? q2 : vt_mag);   // dt/t0 | f_z
+    const double q1 = div_by(coulomb ? 0.8 * mu * normal : fsdt * vt.x, vt_div);   // af  | f_x term
+    const double q2 = div_rn(coulomb ? mass_t : fsdt * vt.y, coulomb ? q1 : vt_mag);   // t0 | f_y
+    const double q3 = div_rn(coulomb ? dt : fsdt * vt.z, coulomb ? q2 : vt_mag);   // dt/t0 | f_z
     if (coulomb) {
-      const double af = q1 / (1.0 + q3 * q3);
+      const double af = div_rn(q1, 1.0 + q3 * q3);
       f.x += af * vt.x;
       f.y += af * vt.y;
       f.z += af * vt.z;
@@ -586,12 +588,13 @@ __device__ __forceinline__ bool pair_input(const V3 &rrl, const V3 &vvl, const V
   }
   double dist;
   if (kFast) {
-    const double inv = rsqrt(dist2);
-    dist = sqrt(dist2);   // correctly rounded: the compression sep - dist is the exact mode's
+    double inv;
+    dist = sqrt_and_inverse(dist2, inv);   // correctly rounded: the compression sep - dist is the exact mode's
     ci.n = mk(d.x * inv, d.y * inv, d.z * inv);
   } else {
-    dist = sqrt(dist2);
-    ci.n = mk(d.x / dist, d.y / dist, d.z / dist);
+    dist = sqrt_rn(dist2);
+    const Divisor by = divisor_of(dist);
+    ci.n = mk(div_by(d.x, by), div_by(d.y, by), div_by(d.z, by));
   }
   ci.rrc = mk(s1.x + rad_1 * ci.n.x, s1.y + rad_1 * ci.n.y, s1.z + rad_1 * ci.n.z);
   V3 vl = point_velocity(vvl, wwl, ci.rrc, rrl);
@@ -647,17 +650,17 @@ __device__ __forceinline__ double signed_zero_product(double a, double b) {
 __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 Ry, V3 Rz, double m,
                                               double adrag0, V3 I, V3 &a, V3 &al, double im, double iI) {
   const double v2 = v.x * v.x + v.y * v.y + v.z * v.z;
-  // fast mode: |v| from the reciprocal square root (the drag term is ~1e-3 of gravity here)
-  double vmag = kFast ? (v2 == 0.0 ? 0.0 : v2 * rsqrt(v2)) : sqrt(v2);   // NaN stays NaN
+  double vmag = sqrt_rn(v2);
   double adrag = adrag0 * vmag;
   if (kFast) {
     a.x = f.x * im - adrag * v.x;
     a.y = f.y * im - adrag * v.y;
     a.z = f.z * im - adrag * v.z - kGRAV;
   } else {
-    a.x = f.x / m - adrag * v.x;
-    a.y = f.y / m - adrag * v.y;
-    a.z = f.z / m - adrag * v.z - kGRAV;
+    const Divisor by = divisor_of(m);
+    a.x = div_by(f.x, by) - adrag * v.x;
+    a.y = div_by(f.y, by) - adrag * v.y;
+    a.z = div_by(f.z, by) - adrag * v.z - kGRAV;
   }
   V3 wb, tb, ab;
   if (kFast && I.x == I.y && I.y == I.z && I.x > 0.0 && isfinite(I.x) && isfinite(w.x) && isfinite(w.y) &&
@@ -686,9 +689,10 @@ __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 
       ab.y = tb.y * iI + signed_zero_product(wb.z, wb.x);
       ab.z = tb.z * iI + signed_zero_product(wb.x, wb.y);
     } else {
-      ab.x = tb.x / I.x + signed_zero_product(wb.y, wb.z);
-      ab.y = tb.y / I.y + signed_zero_product(wb.z, wb.x);
-      ab.z = tb.z / I.z + signed_zero_product(wb.x, wb.y);
+      const Divisor by = divisor_of(I.x);
+      ab.x = div_by(tb.x, by) + signed_zero_product(wb.y, wb.z);
+      ab.y = div_by(tb.y, by) + signed_zero_product(wb.z, wb.x);
+      ab.z = div_by(tb.z, by) + signed_zero_product(wb.x, wb.y);
     }
   } else {
     double Cxy = (I.x - I.y) / I.z;

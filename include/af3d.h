@@ -209,9 +209,11 @@ af3d_status af3d_kernel_launches (af3d_ctx *ctx, long *count);
    DFMA), from a bounded ~0.1 s microbenchmark: the denominator of the FP64 roofline. */
 af3d_status af3d_fp64_peak (double *tflops);
 /* Self-check of the kernels' integer-pipe FP64 helpers (no counterpart in the reference): the
-   conversions to float (to nearest, toward +infinity) and to a 64-bit integer, and the
-   finiteness, non-zero and range tests the kernels take from the bit patterns, against the
-   hardware instructions, for each x[i]; bad[i] gets one bit per helper that disagreed. */
+   conversions to float (to nearest, toward +infinity) and to a 64-bit integer, the
+   finiteness, non-zero and range tests the kernels take from the bit patterns, the correctly
+   rounded square root of x[i] and quotient x[i] / x[n - 1 - i] (equal bits) and the reciprocal
+   of x[i] (within one unit in the last place), against the hardware instructions, for each
+   x[i]; bad[i] gets one bit per helper that disagreed. */
 af3d_status af3d_check_fp64_bits (const double *x, long n, int *bad);
 
 /* ---- adjoint (no counterpart in the reference) --------------------------------------------
