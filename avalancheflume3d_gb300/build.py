@@ -35,6 +35,7 @@ UNITS = [
     ("af3d_adjoint.cu", "af3d_adjoint", ["-fmad=false"]),
     ("af3d_adjoint_rot.cu", "af3d_adjoint_rot", ["-fmad=true"]),
     ("af3d_cells.cu", "af3d_cells", []),
+    ("af3d_near.cu", "af3d_near", ["-Xptxas", "-v"]),
     ("af3d_capi.cu", "af3d_capi", []),
     ("af3d_peaks.cu", "af3d_peaks", []),
 ]

@@ -458,24 +458,6 @@ __device__ __forceinline__ void adj_contacts_lane(long s, const Own &o, const Co
   });
 }
 
-constexpr int kAdjCoopBlock = 64;
-
-// Per-warp shared state of the cooperative reverse: the item lists, every owner's force and
-// torque adjoints, and every owner's contact adjoints (centre, v, w, four spheres) accumulated
-// with shared-memory atomics (a reverse needs no order).
-struct AdjQueue {
-  ItemLists il;
-  double fb[6][32];    // [component][lane]
-  double own[21][32];  // [component][lane]
-};
-
-// Adds v to three components of one lane's column (component stride 32).
-__device__ __forceinline__ void shared_add3(double *p, V3 v) {
-  atomicAdd(p, v.x);
-  atomicAdd(p + 32, v.y);
-  atomicAdd(p + 64, v.z);
-}
-
 // Reverse of finish_Verlet and get_accel for clump s (startup: the start-up pass, which has no
 // finish): out.a/out.al receive the finish terms of this step's a_i, alpha_i, rb the clump's own
 // R1 adjoint; returns the adjoints of the force and torque sums (Fb, Tb) and of the predicted
@@ -572,95 +554,14 @@ __device__ __forceinline__ void add_par(ParamBar &par, const ParamBar &ipar) {
   par.kappa_pw += ipar.kappa_pw; par.gamma_pw += ipar.gamma_pw; par.mu_pw += ipar.mu_pw;
 }
 
-// Reverse of finish_Verlet, get_accel and every contact of one clump (startup: the start-up
-// force pass, which has no finish and whose accelerations become a_i of the first step).
+// Reverse of finish_Verlet, get_accel and every contact of a block's clumps (startup: the start-up
+// force pass, which has no finish and whose accelerations become a_i of the first step), from the
+// item lists the forward pass recorded (ContactLists with cnt).
 // in: adjoint of the next state; out.a/out.al receive the finish terms of this step's a_i and
 // alpha_i; acc receives (atomically) the adjoints of every clump's r1, v1, w1 and spheres;
-// rb receives this clump's own R1 adjoint.  The contacts run warp-cooperatively: the item lists
-// of the forward pass, rebuilt here, 32 items a round, each lane reversing one contact for its
-// owner.
-#ifndef AF3D_ADJ_MINB
-#define AF3D_ADJ_MINB 1
-#endif
-__global__ void __launch_bounds__(kAdjCoopBlock, AF3D_ADJ_MINB) k_adj_forces(Planes P, Planes in, Planes out, Planes acc,
-                                                              Planes rb, DevScalars *d, const int *__restrict__ flume,
-                                                              const NbrRec *__restrict__ nbr,
-                                                              const CullRec *__restrict__ cull,
-                                                              const int *__restrict__ start,
-                                                              const int *__restrict__ order,
-                                                              const float4 *__restrict__ csort, double *param_b,
-                                                              int startup, long n) {
-  __shared__ AdjQueue queues[kAdjCoopBlock / 32];
-  AdjQueue &aq = queues[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
-  const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const bool valid = s < n;
-  const long sv = valid ? s : n - 1;
-  const long wbase = blockIdx.x * (long)blockDim.x + (threadIdx.x & ~31u);
-  ParamBar par = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  const int f = flume[sv];
-  const Consts &c = d->flumes[f].c;
-  const af3d_cell_par g = d->flumes[f].grid;
-  const long long off = d->flumes[f].cell_off;
-  const NbrRec &me = nbr[sv];
-  Own o;
-  o.r = mk(me.rx, me.ry, me.rz);
-  o.v = mk(me.vx, me.vy, me.vz);
-  o.w = mk(me.wx, me.wy, me.wz);
-  for (int k = 0; k < 4; k++) o.s[k] = mk(me.s[3 * k], me.s[3 * k + 1], me.s[3 * k + 2]);
-  o.rad = me.rad; o.msph = me.msph; o.mwall = me.mwall;
-  const bool removed = is_removed(*c.tp, o.r.x, c.side_x);
-  const bool act = valid && !removed;
-  ClumpBar ob;
-  V3 Fb, Tb;
-  adj_head(s, act, valid, startup, o, c, P, in, out, rb, ob, Fb, Tb);
-  aq.fb[0][lane] = Fb.x; aq.fb[1][lane] = Fb.y; aq.fb[2][lane] = Fb.z;
-  aq.fb[3][lane] = Tb.x; aq.fb[4][lane] = Tb.y; aq.fb[5][lane] = Tb.z;
-  for (int k = 0; k < 21; k++) aq.own[k][lane] = 0.0;
-  // the contacts: the forward pass's item lists, reversed 32 a round
-  const bool aval = c.phase == AF3D_PHASE_AVALANCHE;
-  const double B = (double)cull[sv].c.w;
-  bool slow = false;
-  ListCounts lcounts;
-  const int nitems = build_item_lists(aq.il.pl, &aq.il.items[0][lane], 32, wbase, sv, act, aval, o.r, c, g,
-                                      d->flumes[f].gridf, off, nbr, cull, start, order, csort, slow, lcounts);
-  const int total = warp_prefix(nitems, aq.il.base);
-  for (int j0 = 0; j0 < total; j0 += 32) {
-    const int j = j0 + lane;
-    if (j < total) {
-      const int lo = owner_of(aq.il.base, j);
-      const unsigned it = aq.il.items[j - aq.il.base[lo]][lo];
-      const long os = wbase + lo;
-      const int of = flume[os];
-      const Consts &co = of == f ? c : d->flumes[of].c;
-      ItemBar ib;
-      ParamBar ipar = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // this item's; the lane's flume or the owner's
-      const int k = adj_item(nbr[os], it, co, mk(aq.fb[0][lo], aq.fb[1][lo], aq.fb[2][lo]),
-                             mk(aq.fb[3][lo], aq.fb[4][lo], aq.fb[5][lo]), nbr, acc, ib, ipar);
-      if (of == f) add_par(par, ipar);
-      else flush_params(param_b, of, ipar);
-      double *ow = &aq.own[0][lo];
-      shared_add3(ow + 32 * CR, ib.r);
-      shared_add3(ow + 32 * CV, ib.v);
-      shared_add3(ow + 32 * CW, ib.w);
-      shared_add3(ow + 32 * (CS + 3 * k), ib.s);
-    }
-  }
-  __syncwarp();
-  if (act) {
-    if (slow) adj_contacts_lane(s, o, c, g, off, B, Fb, Tb, acc, nbr, cull, start, order, ob, par);
-    auto own3 = [&](int c0) { return mk(aq.own[c0][lane], aq.own[c0 + 1][lane], aq.own[c0 + 2][lane]); };
-    atomic_add3(acc, CR, s, ob.r + own3(CR));
-    atomic_add3(acc, CV, s, ob.v + own3(CV));
-    atomic_add3(acc, CW, s, ob.w + own3(CW));
-    for (int k = 0; k < 4; k++) atomic_add3(acc, CS + 3 * k, s, ob.s[k] + own3(CS + 3 * k));
-  }
-  add_params(param_b, f, par);
-}
-
-// The same reverse from the item lists the forward pass recorded (ContactLists with cnt), pooled
-// over a block of 128 clumps: the block's particle items, then its boundary items, 32 a round per
-// warp, owners' adjoints summed in shared memory (a reverse needs no order).
+// rb receives each clump's own R1 adjoint.  The contacts are pooled over a block of 128 clumps:
+// the block's particle items, then its boundary items, 32 a round per warp, owners' adjoints
+// summed in shared memory (a reverse needs no order).
 constexpr int kAdjListBlock = 128;
 struct AdjBlock {
   double fb[6][kAdjListBlock];
@@ -679,7 +580,7 @@ __global__ void __launch_bounds__(kAdjListBlock, AF3D_ADJ_LMINB) k_adj_forces_l(
                                                                const CullRec *__restrict__ cull,
                                                                const int *__restrict__ start,
                                                                const int *__restrict__ order, ContactLists lists,
-                                                               double *param_b, long n) {
+                                                               double *param_b, int startup, long n) {
   __shared__ AdjBlock ab;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long bbase = blockIdx.x * (long)kAdjListBlock;
@@ -700,7 +601,7 @@ __global__ void __launch_bounds__(kAdjListBlock, AF3D_ADJ_LMINB) k_adj_forces_l(
   const bool act = valid && !removed;
   ClumpBar ob;
   V3 Fb, Tb;
-  adj_head(s, act, valid, 0, o, c, P, in, out, rb, ob, Fb, Tb);
+  adj_head(s, act, valid, startup, o, c, P, in, out, rb, ob, Fb, Tb);
   ab.fb[0][tid] = Fb.x; ab.fb[1][tid] = Fb.y; ab.fb[2][tid] = Fb.z;
   ab.fb[3][tid] = Tb.x; ab.fb[4][tid] = Tb.y; ab.fb[5][tid] = Tb.z;
   for (int k = 0; k < 21; k++) ab.own[k][tid] = 0.0;
@@ -900,22 +801,13 @@ __global__ void k_state_copy(Planes P, Planes tape, int to_tape, long n) {
 
 }  // namespace
 
-void launch_adj_forces(const Launch &L, Planes P, Planes in, Planes out, Planes acc, Planes rb, DevScalars *d,
-                       const int *flume, const NbrRec *nbr, const CullRec *cull, const int *start, const int *order,
-                       const float4 *csort, double *param_b, bool startup) {
-  if (L.n <= 0) return;
-  const unsigned nb = (unsigned)((L.n + kAdjCoopBlock - 1) / kAdjCoopBlock);
-  k_adj_forces<<<nb, kAdjCoopBlock, 0, L.st>>>(P, in, out, acc, rb, d, flume, nbr, cull, start, order, csort, param_b,
-                                               startup ? 1 : 0, L.n);
-}
-
 void launch_adj_forces_lists(const Launch &L, Planes P, Planes in, Planes out, Planes acc, Planes rb, DevScalars *d,
                              const int *flume, const NbrRec *nbr, const CullRec *cull, const int *start,
-                             const int *order, ContactLists lists, double *param_b) {
+                             const int *order, ContactLists lists, double *param_b, bool startup) {
   if (L.n <= 0) return;
   const unsigned nb = (unsigned)((L.n + kAdjListBlock - 1) / kAdjListBlock);
   k_adj_forces_l<<<nb, kAdjListBlock, 0, L.st>>>(P, in, out, acc, rb, d, flume, nbr, cull, start, order, lists,
-                                                 param_b, L.n);
+                                                 param_b, startup ? 1 : 0, L.n);
 }
 
 void launch_adj_objective(const Launch &L, Planes P, DevScalars *d, const int *flume, double *sums, double length) {

@@ -9,6 +9,7 @@
 // Device-side checks raise bits in a status word that af3d_step() and af3d_get_status() read
 // back; nothing calls exit().
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstddef>
@@ -40,18 +41,15 @@ af3d_status fail(af3d_status code, const std::string &msg) {
   } while (0)
 
 constexpr long kRegridEvery = 2000;   // avalanche_hst.cu:470 and :713 (cc % 2000 == 0)
-constexpr long kKernelsPerCellBuild = 5;   // predict/keys, scan, scatter, rank, permute
-constexpr long kKernelsPerForcePass = 1;   // lists and forces in one kernel
+constexpr long kKernelsPerSort = 3;        // scan, scatter, rank
 #ifndef AF3D_HOST_PARTS
 #define AF3D_HOST_PARTS 4
 #endif
 constexpr int kHostParts = AF3D_HOST_PARTS;   // af3d_step_host: parts whose copies overlap the step
-constexpr long kKernelsPerStep = kKernelsPerCellBuild + 1 + kKernelsPerForcePass;   // + time advance
-constexpr long kKernelsPerKeptStep = kKernelsPerStep - 1;    // a step without the permutation
 constexpr long kKernelsPerRegrid = 4;
 // The clumps are moved into (cell, id) order by a permutation of every plane at most this many
 // steps apart (the context's `resort_every`, by default kResortEvery); the steps in between keep
-// the slot order and reach the sorted order through the sort's index array.  Results do not
+// the slot order.  Results do not
 // depend on it (every sum runs in (sph_id, cell, id) order); it bounds how far the slot order
 // may drift from the spatial order.  A long captured graph covers one such period (its first
 // step permutes), so the interval is even (the pointer period of the plane sets is 2).
@@ -65,14 +63,16 @@ struct PtrState {
   int *fl_cur, *fl_alt;
   NbrRec *nbr, *nbr_next;
   CullRec *cull, *cull_next;
+  int *occ, *occ_next;
   bool look;
 };
 
+// One period of resort_every captured steps, the first of which permutes the planes.
 struct StepGraph {
   PtrState start{}, end{};      // before and after the captured steps
-  long steps = 0;
-  bool resort_first = false;    // the first captured step permutes the planes
   bool look_last = false;       // the last captured force pass looks ahead
+  long since_build = 0;         // steps the near lists have served at its end
+  long kernels = 0;
   cudaGraphExec_t exec = nullptr;
 };
 
@@ -139,6 +139,9 @@ struct af3d_ctx {
   // the last step's corrected state.
   bool look = false;
   ContactLists lists{};   // the item lists of the current force pass
+  NearLists near{};       // what may touch within the next steps
+  long since_build = kBuildEvery;   // steps the near lists have served (kBuildEvery: build them anew)
+  const int *built_order = nullptr;   // the slots' place in the sort they were built from (null: in that order)
   Cells cells{};
   DevScalars *d = nullptr;
   DevFlume *flumes = nullptr;
@@ -179,7 +182,7 @@ bool same_planes(const Planes &a, const Planes &b) {
 
 PtrState ptr_state(const af3d_ctx *c) {
   return PtrState{c->cur, c->alt, c->id_cur, c->id_alt, c->fl_cur, c->fl_alt, c->nbr, c->nbr_next, c->cull,
-                  c->cull_next, c->look};
+                  c->cull_next, c->cells.occ, c->cells.occ_next, c->look};
 }
 
 void set_ptr_state(af3d_ctx *c, const PtrState &p) {
@@ -188,14 +191,26 @@ void set_ptr_state(af3d_ctx *c, const PtrState &p) {
   c->fl_cur = p.fl_cur; c->fl_alt = p.fl_alt;
   c->nbr = p.nbr; c->nbr_next = p.nbr_next;
   c->cull = p.cull; c->cull_next = p.cull_next;
+  c->cells.occ = p.occ; c->cells.occ_next = p.occ_next;
   c->look = p.look;
 }
 
 bool same_state(const PtrState &a, const PtrState &b) {
   return same_planes(a.cur, b.cur) && same_planes(a.alt, b.alt) && a.id_cur == b.id_cur &&
          a.id_alt == b.id_alt && a.fl_cur == b.fl_cur && a.fl_alt == b.fl_alt && a.nbr == b.nbr &&
-         a.nbr_next == b.nbr_next && a.cull == b.cull && a.cull_next == b.cull_next && a.look == b.look;
+         a.nbr_next == b.nbr_next && a.cull == b.cull && a.cull_next == b.cull_next && a.occ == b.occ &&
+         a.occ_next == b.occ_next && a.look == b.look;
 }
+
+// The margins of the records and near lists, for the largest clump any flume may hold.
+void set_margins(af3d_ctx *c) {
+  double rmax = 0.0;
+  for (const auto &s : c->sys) rmax = std::max(rmax, s.rmax);
+  c->cur.m = c->alt.m = margins_for(rmax, c->sys[0].dt, kBuildEvery);
+}
+
+// The state, the grid or the slots changed other than by a step: the next step builds its lists.
+void drop_lists(af3d_ctx *c) { c->since_build = kBuildEvery; }
 
 void drop_graphs(af3d_ctx *c) {
   for (auto &g : c->graphs) {
@@ -208,6 +223,9 @@ void drop_graphs(af3d_ctx *c) {
 // device-derived grids are read back first so that they are not overwritten.
 af3d_status push_params(af3d_ctx *c) {
   drop_graphs(c);   // graphs hold the constants of their force launches
+  set_margins(c);
+  c->records_valid = false;   // made with the margins before
+  drop_lists(c);
   std::vector<DevFlume> fl(c->nflumes);
   AF3D_CUDA(cudaMemcpyAsync(fl.data(), c->flumes, sizeof(DevFlume) * c->nflumes, cudaMemcpyDeviceToHost, c->st));
   AF3D_CUDA(cudaStreamSynchronize(c->st));
@@ -244,14 +262,21 @@ af3d_status ensure_buckets(af3d_ctx *c, long ncell_total) {
   cudaFree(c->cells.count);
   cudaFree(c->cells.start);
   cudaFree(c->cells.tile_count);
-  c->cells.count = c->cells.start = c->cells.tile_count = nullptr;
+  cudaFree(c->cells.occ);
+  cudaFree(c->cells.occ_next);
+  c->cells.count = c->cells.start = c->cells.tile_count = c->cells.occ = c->cells.occ_next = nullptr;
   AF3D_CUDA(cudaMalloc(&c->cells.count, sizeof(int) * cap));
   AF3D_CUDA(cudaMalloc(&c->cells.start, sizeof(int) * (cap + 1)));
   AF3D_CUDA(cudaMalloc(&c->cells.tile_count, sizeof(int) * (scan_tiles(cap) + 1)));
+  AF3D_CUDA(cudaMalloc(&c->cells.occ, sizeof(int) * cap));
+  AF3D_CUDA(cudaMalloc(&c->cells.occ_next, sizeof(int) * cap));
+  AF3D_CUDA(cudaMemsetAsync(c->cells.occ, 0, sizeof(int) * cap, c->st));
+  AF3D_CUDA(cudaMemsetAsync(c->cells.occ_next, 0, sizeof(int) * cap, c->st));
   AF3D_CUDA(cudaMemsetAsync(c->cells.count, 0, sizeof(int) * cap, c->st));
   AF3D_CUDA(cudaMemsetAsync(c->cells.tile_count, 0, sizeof(int) * (scan_tiles(cap) + 1), c->st));
   c->cells.cap = cap;
   c->cells_valid = false;
+  drop_lists(c);
   drop_graphs(c);
   return AF3D_OK;
 }
@@ -277,6 +302,7 @@ af3d_status set_grids_device(af3d_ctx *c) {
   AF3D_CUDA(cudaStreamSynchronize(c->st));
   c->have_grid = true;
   c->cells_valid = false;
+  drop_lists(c);
   return AF3D_OK;
 }
 
@@ -300,32 +326,45 @@ af3d_status regrid(af3d_ctx *c) {
   }
   c->have_grid = true;
   c->cells_valid = false;
+  drop_lists(c);
   return pull_params(c);
 }
 
 // clear_cell + clear_ocup + cell_locate: keys (optionally fused with the predictor), counting
 // sort, permutation of every plane into the new order, neighbour records.
 // The predictor and force launchers of the context's FP64 mode (the other kernels have one form).
-void predict_for(af3d_ctx *c, bool predict, bool keys, bool t_prev, bool records = false, long s0 = 0,
-                 long count = -1) {
+// records: also the neighbour records, at the clumps' own slots; counted: for a step that keeps its
+// near lists.
+void predict_for(af3d_ctx *c, bool predict, bool keys, bool t_prev, bool records = false, bool counted = false,
+                 long s0 = 0, long count = -1) {
   NbrRec *nbr = records ? c->nbr : nullptr;
   CullRec *cull = records ? c->cull : nullptr;
-  if (c->fp_mode == AF3D_FP_FAST)
-    fast::launch_predict(c->L(), c->cur, c->d, predict, keys, t_prev, c->cells, c->id_cur, c->fl_cur, nbr, cull,
-                         s0, count);
-  else
-    launch_predict(c->L(), c->cur, c->d, predict, keys, t_prev, c->cells, c->id_cur, c->fl_cur, nbr, cull, s0,
-                   count);
+  auto run = c->fp_mode == AF3D_FP_FAST ? fast::launch_predict : launch_predict;
+  run(c->L(), c->cur, c->d, predict, keys, t_prev, c->cells, c->id_cur, c->fl_cur, c->ntags, c->near, c->built_order,
+      counted, nbr, cull, s0, count);
+  c->launches++;
 }
 
-// order: null when the slots were just permuted into (cell, id) order; out: where the corrected
-// velocities go.
+void sort_for(af3d_ctx *c, bool with_centres) {
+  launch_sort(c->L(), c->d, c->cells, c->id_cur, c->ntags, with_centres ? c->cull : nullptr);
+  c->launches += kKernelsPerSort;
+}
+
+// The near lists from the sort just made (order: null when the slots were permuted into it).
+void build_lists(af3d_ctx *c, const int *order, long s0 = 0, long count = -1) {
+  launch_build_lists(c->L(), c->cur.m, c->d, c->fl_cur, c->cull, c->cells, order, c->id_cur, c->near, s0, count);
+  c->launches++;
+  c->built_order = order;
+  c->since_build = 0;
+}
+
+// out: where the corrected velocities go.  counted: the step kept its lists (its buckets are in
+// cells.occ).  look: run the next step's predictor; next_builds: that step sorts and builds.
 // A single-flume context passes its constants as a kernel parameter (from the host mirrors,
 // which push_params keeps equal to the device table; captured graphs are dropped whenever they
 // change).
-void forces_for(af3d_ctx *c, bool write_ft, const int *order, Planes out, bool warm = false, bool look = false,
-                long s0 = 0, long count = -1) {
-  const float4 *csort = order ? c->cells.csort : nullptr;
+void forces_for(af3d_ctx *c, bool write_ft, Planes out, bool warm = false, bool look = false,
+                bool counted = false, bool next_builds = false, long s0 = 0, long count = -1) {
   Consts kc;
   const Consts *uni = nullptr;
   if (c->nflumes == 1) {
@@ -333,107 +372,130 @@ void forces_for(af3d_ctx *c, bool write_ft, const int *order, Planes out, bool w
     uni = &kc;
   }
   LookAhead la{};
-  if (look) la = LookAhead{c->nbr_next, c->cull_next, c->cells, c->id_cur};
-  if (c->fp_mode == AF3D_FP_FAST)
-    fast::launch_lists_forces(c->L(), c->cur, out, c->d, c->fl_cur, c->nbr, c->cull, c->cells.start, order, csort,
-                              c->lists, write_ft, uni, warm, la, s0, count, c->force_shape);
-  else
-    launch_lists_forces(c->L(), c->cur, out, c->d, c->fl_cur, c->nbr, c->cull, c->cells.start, order, csort,
-                        c->lists, write_ft, uni, warm, la, s0, count, c->force_shape);
+  if (look) la = LookAhead{c->nbr_next, c->cull_next, next_builds};
+  auto run = c->fp_mode == AF3D_FP_FAST ? fast::launch_lists_forces : launch_lists_forces;
+  run(c->L(), c->cur, out, c->d, c->fl_cur, c->nbr, c->cull, c->cells, c->built_order, c->id_cur, c->near, c->lists,
+      c->ntags, write_ft, counted, uni, warm, la, s0, count, c->force_shape);
+  c->launches++;
 }
 
-void enqueue_cell_build(af3d_ctx *c, bool predict, bool t_prev, bool ft = true) {
-  predict_for(c, predict, true, t_prev);
-  launch_sort(c->L(), c->d, c->cells, c->id_cur, c->ntags);
-  launch_permute_records(c->L(), c->cur, c->alt, c->cells.perm, c->id_cur, c->id_alt, c->fl_cur, c->fl_alt,
-                         c->nbr, c->cull, ft);
+// Every plane into the order just sorted, with the records.
+void enqueue_permutation(af3d_ctx *c, bool ft) {
+  launch_permute_records(c->L(), c->cur, c->alt, c->cells.perm, c->cells.key, c->id_cur, c->id_alt, c->fl_cur,
+                         c->fl_alt, c->nbr, c->cull, ft);
+  c->launches++;
   std::swap(c->cur, c->alt);
   std::swap(c->id_cur, c->id_alt);
   std::swap(c->fl_cur, c->fl_alt);
   c->sorted = true;
   c->since_sort = 0;
+  drop_lists(c);
 }
 
-// One fused step: time += dt, init_Verlet + cell build, every force of the phase, get_accel,
-// finish_Verlet, and the acceleration swap.  With `resort` the planes are permuted into the new
-// (cell, id) order; otherwise the predictor writes the records at the clumps' own slots, the
-// force pass reaches the sorted order through cells.perm and corrects the velocities in place.
-// When the previous pass looked ahead (c->look), this step's predictor has already run and the
-// step is the sort and the force pass.  `look`: this step's force pass runs the next step's
-// predictor.
-void enqueue_fused_step(af3d_ctx *c, bool resort, bool write_ft = false, bool look = false) {
-  const bool warm = !resort && c->look;
-  if (!warm) launch_advance_time(c->st, c->d);   // a warm step advances the clock in its sort
-  if (resort) {
+void enqueue_cell_build(af3d_ctx *c, bool predict, bool t_prev, bool ft = true) {
+  predict_for(c, predict, true, t_prev);
+  sort_for(c, false);
+  enqueue_permutation(c, ft);
+}
+
+// What one fused step does: permute the planes (resort), start from the previous pass's look-ahead
+// (warm), sort and build the near lists (build), look ahead itself, to a step that builds.
+struct StepPlan {
+  bool resort, warm, build, look, next_builds;
+};
+
+// look: the next step of the run keeps the slot order and no re-grid comes between.
+StepPlan plan_step(const af3d_ctx *c, bool resort, bool look) {
+  StepPlan p;
+  p.resort = resort;
+  p.warm = !resort && c->look;
+  p.build = resort || c->since_build >= kBuildEvery;
+  p.look = look;
+  p.next_builds = (p.build ? 1 : c->since_build + 1) >= kBuildEvery;
+  return p;
+}
+
+void step_predict(af3d_ctx *c, const StepPlan &p) {
+  if (!p.resort && !p.warm) predict_for(c, true, true, true, true, !p.build);
+}
+
+void step_lists(af3d_ctx *c, const StepPlan &p) {
+  if (p.resort) {
     enqueue_cell_build(c, true, true, false);   // F, T and a_f are rewritten before being read
-    forces_for(c, write_ft, nullptr, c->alt, false, look);
-    swap_velocity_planes(c->cur, c->alt);
-  } else {
-    if (!warm) predict_for(c, true, true, true, true);
-    launch_sort(c->L(), c->d, c->cells, c->id_cur, c->ntags, c->cull, warm);
-    forces_for(c, write_ft, c->cells.perm, c->cur, warm, look);
+    build_lists(c, nullptr);
+  } else if (p.build) {
+    sort_for(c, true);
+    build_lists(c, c->cells.perm);
   }
-  if (look) {
+}
+
+void step_forces(af3d_ctx *c, const StepPlan &p, bool write_ft) {
+  forces_for(c, write_ft, p.resort ? c->alt : c->cur, p.warm, p.look, !p.build, p.next_builds);
+  if (p.resort) swap_velocity_planes(c->cur, c->alt);
+  if (p.look) {
     std::swap(c->nbr, c->nbr_next);
     std::swap(c->cull, c->cull_next);
+    std::swap(c->cells.occ, c->cells.occ_next);
   }
-  c->look = look;
+  c->look = p.look;
+  c->since_build++;
   swap_accel_planes(c->cur);
   swap_accel_planes(c->alt);
-  c->sorted = resort;
+  c->sorted = p.resort;
 }
 
-// Kernels of `len` fused steps, the first one permuting (resort_first) or, with look_first,
-// predicted by the previous pass; every later step is predicted by its previous pass.
-long kernels_of(long len, bool resort_first, bool look_first) {
-  // a predicted step skips the predictor and advances the clock inside its sort
-  const long warm = kKernelsPerKeptStep - 2;
-  const long first = resort_first ? kKernelsPerStep : (look_first ? warm : kKernelsPerKeptStep);
-  return first + (len - 1) * warm;
+// One fused step: time += dt, init_Verlet, the near lists when they are due, every force of the
+// phase, get_accel, finish_Verlet, and the acceleration swap.  With `resort` the planes are
+// permuted into the new (cell, id) order; otherwise the slots stay.  When the previous pass looked
+// ahead (c->look), its last block advanced the clock and this step's predictor has run: unless
+// its lists are due the step is the force pass alone.
+void enqueue_fused_step(af3d_ctx *c, bool resort, bool write_ft = false, bool look = false) {
+  const StepPlan p = plan_step(c, resort, look);
+  if (!p.warm) {
+    launch_advance_time(c->st, c->d);
+    c->launches++;
+  }
+  step_predict(c, p);
+  step_lists(c, p);
+  step_forces(c, p, write_ft);
 }
 
 // launch false: capture (and cache) the graphs m steps would replay without running anything;
 // the caller restores the context's step state afterwards.
 af3d_status run_steps(af3d_ctx *c, long m, bool launch = true) {
   // Captured graphs of resort_every steps (the first one permuting the planes) while that many
-  // steps remain, then of two steps (permuting first only when the last permutation is due); an odd
-  // last step is enqueued directly.  A graph is replayed when the context is in the pointer
-  // state it was captured from, and leaves the context in the state it ended in.  A force pass
-  // looks ahead (runs the next step's predictor) when the next step of the run keeps the slot
-  // order; a permuting step predicts from the planes itself.
-  auto resorts = [&](long since, long left) {   // does the next batch of `left` steps permute first?
-    if (left >= 2) {
-      const long l = left >= c->resort_every ? c->resort_every : 2;
-      return l == c->resort_every || since + l > c->resort_every;
-    }
-    return since + 1 > c->resort_every;
+  // steps remain; the rest are enqueued one by one (mostly one kernel each, so their launches
+  // hide behind the steps before them), permuting when that is due.  A graph is replayed when
+  // the context is in the pointer state it was captured from, and leaves the context in the
+  // state it ended in.  A force pass looks ahead (runs the next step's predictor) when the next
+  // step of the run keeps the slot order; a permuting step predicts from the planes itself.
+  auto resorts = [&](long since, long left) {   // does the next of `left` steps permute?
+    return left >= c->resort_every || since + 1 > c->resort_every;
   };
-  while (m >= 2) {
-    const long len = m >= c->resort_every ? c->resort_every : 2;
-    const bool resort_first = len == c->resort_every || c->since_sort + len > c->resort_every;
-    const long since_after = resort_first ? len - 1 : c->since_sort + len;
-    const bool look_last = m > len && !resorts(since_after, m - len);
-    const bool look_first = c->look;
+  while (m >= c->resort_every) {
+    const long len = c->resort_every;
+    const bool look_last = m > len && !resorts(len - 1, m - len);
+    c->look = false;   // (a pass before a permuting step does not look ahead)
     const PtrState now = ptr_state(c);
     StepGraph *g = nullptr;
     for (auto &cand : c->graphs)
-      if (cand.exec && cand.steps == len && cand.resort_first == resort_first && cand.look_last == look_last &&
-          same_state(cand.start, now))
-        g = &cand;
+      if (cand.exec && cand.look_last == look_last && same_state(cand.start, now)) g = &cand;
     if (!g) {
       g = &c->graphs[c->graph_next];
       c->graph_next = (c->graph_next + 1) % 4;
       if (g->exec) cudaGraphExecDestroy(g->exec);
       *g = StepGraph{};
       g->start = now;
-      g->steps = len;
-      g->resort_first = resort_first;
       g->look_last = look_last;
+      const long launches0 = c->launches;
       cudaGraph_t graph;
       AF3D_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-      for (long i = 0; i < len; i++) enqueue_fused_step(c, i == 0 && resort_first, false, i + 1 < len || look_last);
+      for (long i = 0; i < len; i++) enqueue_fused_step(c, i == 0, false, i + 1 < len || look_last);
       AF3D_CUDA(cudaStreamEndCapture(c->st, &graph));
       g->end = ptr_state(c);
+      g->since_build = c->since_build;
+      g->kernels = c->launches - launches0;
+      c->launches = launches0;
       set_ptr_state(c, now);
       cudaError_t e = cudaGraphInstantiate(&g->exec, graph, 0);
       cudaGraphDestroy(graph);
@@ -442,19 +504,22 @@ af3d_status run_steps(af3d_ctx *c, long m, bool launch = true) {
         return fail(AF3D_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
       }
     }
-    if (launch) AF3D_CUDA(cudaGraphLaunch(g->exec, c->st));
+    if (launch) {
+      AF3D_CUDA(cudaGraphLaunch(g->exec, c->st));
+      c->launches += g->kernels;
+    }
     set_ptr_state(c, g->end);
     c->sorted = false;   // the last captured step keeps the slot order
-    c->since_sort = since_after;
-    if (launch) c->launches += kernels_of(len, resort_first, look_first);
+    c->since_sort = len - 1;
+    c->since_build = g->since_build;
+    c->built_order = len > kBuildEvery ? c->cells.perm : nullptr;
     m -= len;
   }
-  if (m == 1 && launch) {
-    const bool resort = c->since_sort + 1 > c->resort_every;
-    const bool look_first = c->look;
-    enqueue_fused_step(c, resort);
-    c->since_sort = resort ? 0 : c->since_sort + 1;
-    c->launches += kernels_of(1, resort, look_first);
+  for (; launch && m > 0; m--) {
+    const bool resort = resorts(c->since_sort, m);
+    const long since = resort ? 0 : c->since_sort + 1;
+    enqueue_fused_step(c, resort, false, m > 1 && !resorts(since, m - 1));
+    c->since_sort = since;
   }
   return AF3D_OK;
 }
@@ -575,6 +640,11 @@ af3d_status af3d_create_ensemble(int nflumes, const af3d_system_par *sys, const 
   ok = ok && cudaMalloc((void **)&c->nbr_next, sizeof(NbrRec) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->cull_next, sizeof(CullRec) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->lists.items, sizeof(unsigned) * kListCap * n) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&c->near.items, sizeof(unsigned) * kNearCap * n) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&c->near.info, sizeof(int) * n) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&c->near.bnd, sizeof(unsigned) * n) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&c->near.rem, sizeof(float) * n) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&c->near.loose, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->cells.key, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->cells.rank_tmp, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->cells.tmp_slot, sizeof(int) * n) == cudaSuccess;
@@ -591,6 +661,7 @@ af3d_status af3d_create_ensemble(int nflumes, const af3d_system_par *sys, const 
     c->cur.p[k] = c->plane_mem[0] + (size_t)k * n;
     c->alt.p[k] = c->plane_mem[1] + (size_t)k * n;
   }
+  set_margins(c);
   std::vector<int> fid((size_t)n, 0);
   for (int f = 0; f < nflumes; f++)
     for (long i = c->first_id[f]; i < c->first_id[f + 1]; i++) fid[i] = f;
@@ -613,6 +684,7 @@ af3d_status af3d_create_ensemble(int nflumes, const af3d_system_par *sys, const 
   ds.variant = c->variant;
   ds.nflumes = nflumes;
   ds.flumes = c->flumes;
+  ds.all_slow = ds.brute = INT_MAX;
   cudaMemsetAsync(c->plane_mem[0], 0, sizeof(double) * n * NPLANES, c->st);
   cudaMemsetAsync(c->plane_mem[1], 0, sizeof(double) * n * NPLANES, c->st);
   cudaMemcpyAsync(c->flume_of_id, fid.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->st);
@@ -640,7 +712,8 @@ af3d_status af3d_destroy(af3d_ctx *c) {
                   (void *)c->fl_cur, (void *)c->fl_alt, (void *)c->flume_of_id, (void *)c->nbr,
                   (void *)c->cull, (void *)c->lists.items, (void *)c->nbr_next, (void *)c->cull_next, (void *)c->cells.key, (void *)c->cells.rank_tmp, (void *)c->cells.tmp_slot,
                   (void *)c->cells.perm, (void *)c->cells.csort, (void *)c->cells.count, (void *)c->cells.start,
-                  (void *)c->cells.tile_count, (void *)c->d, (void *)c->flumes, (void *)c->d_aos,
+                  (void *)c->cells.tile_count, (void *)c->cells.occ, (void *)c->cells.occ_next, (void *)c->near.items,
+                  (void *)c->near.info, (void *)c->near.bnd, (void *)c->near.rem, (void *)c->near.loose, (void *)c->d, (void *)c->flumes, (void *)c->d_aos,
                   (void *)c->d_acc, (void *)c->d_anga, (void *)c->d_tmp, (void *)c->d_count})
     if (p) cudaFree(p);
   if (c->own_stream && c->st) cudaStreamDestroy(c->st);
@@ -724,6 +797,7 @@ af3d_status enqueue_import(af3d_ctx *c, const af3d_particle *pp, const af3d_vec3
   c->cells_valid = false;
   c->sorted = false;
   c->look = false;
+  drop_lists(c);
   if (!keep_order) {
     c->since_sort = c->resort_every;
     drop_graphs(c);
@@ -825,7 +899,7 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
     AF3D_CUDA(cudaStreamWaitEvent(c->st, c->part_in[parts], 0));
     launch_aos_to_planes(c->L(), c->d_aos, acc_in ? c->d_acc : nullptr, anga_in ? c->d_anga : nullptr,
                          c->flume_of_id, c->cur, c->id_cur, c->fl_cur, false, s0, cnt);
-    predict_for(c, true, true, true, true, s0, cnt);
+    predict_for(c, true, true, true, true, false, s0, cnt);
     parts++;
   }
   c->imported = true;
@@ -834,10 +908,10 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   c->sorted = false;
   c->look = false;
   c->since_sort = c->resort_every;
-  // The rest of the step (a kept-order step of af3d_step): the sort, then the force pass in
-  // kHostParts launches of whole blocks; after each, the part's clumps go to the AoS staging
+  // The rest of the step (a kept-order step of af3d_step): the sort, then the near lists and the
+  // force pass in kHostParts launches of whole blocks; after each, the part's clumps go to the AoS staging
   // buffer and, on the copy stream, to the host while the next part computes.
-  launch_sort(c->L(), c->d, c->cells, c->id_cur, c->ntags, c->cull, false);
+  sort_for(c, true);
   Planes after = c->cur;   // the plane set as the step leaves it (accelerations swapped)
   swap_accel_planes(after);
   const int in_parts = parts;
@@ -845,7 +919,8 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   for (int j = 0; j < kHostParts; j++) {
     const long s0 = out_at[j], cnt = out_at[j + 1] - s0;
     if (cnt <= 0) continue;
-    forces_for(c, false, c->cells.perm, c->cur, false, false, s0, cnt);
+    build_lists(c, c->cells.perm, s0, cnt);
+    forces_for(c, false, c->cur, false, false, false, false, s0, cnt);
     launch_planes_to_aos(c->L(), after, c->id_cur, c->fl_cur, c->d_aos, acc_out ? c->d_acc : nullptr,
                          anga_out ? c->d_anga : nullptr, c->d, s0, cnt);
     AF3D_CUDA(cudaEventRecord(c->part_done[parts], c->st));
@@ -862,7 +937,8 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   }
   swap_accel_planes(c->cur);
   swap_accel_planes(c->alt);
-  c->launches += (kKernelsPerKeptStep - kKernelsPerForcePass - 1) + 2L * in_parts + 2L * parts;
+  c->launches += 1 + in_parts + parts;   // the clock, the conversions
+  drop_lists(c);   // the next import changes the slots or their clumps
   // af3d_step's bookkeeping for one step
   c->time = c->time + c->sys[0].dt;
   const bool do_regrid = c->cc % kRegridEvery == 0;
@@ -1086,9 +1162,11 @@ af3d_status af3d_open_door(af3d_ctx *c) {
 
 af3d_status af3d_init_verlet(af3d_ctx *c) {
   CHECK_STATE(c);
-  launch_predict(c->L(), c->cur, c->d, true, false, false, c->cells, c->id_cur, c->fl_cur);
+  launch_predict(c->L(), c->cur, c->d, true, false, false, c->cells, c->id_cur, c->fl_cur, c->ntags, c->near, nullptr,
+                 false);
   c->launches++;
   c->records_valid = false;
+  drop_lists(c);
   return AF3D_OK;
 }
 
@@ -1118,7 +1196,6 @@ af3d_status af3d_cell_build(af3d_ctx *c) {
   CHECK_STATE(c);
   if (!c->have_grid) return fail(AF3D_ERR_ARG, "no grid");
   enqueue_cell_build(c, false, false);
-  c->launches += kKernelsPerCellBuild;
   c->records_valid = true;
   c->cells_valid = true;
   return AF3D_OK;
@@ -1163,6 +1240,7 @@ af3d_status af3d_finish_verlet(af3d_ctx *c) {
   launch_finish_verlet(c->L(), c->cur, c->d, c->fl_cur);
   c->launches++;
   c->records_valid = false;
+  drop_lists(c);
   return AF3D_OK;
 }
 
@@ -1180,8 +1258,9 @@ af3d_status af3d_forces(af3d_ctx *c) {
   enqueue_cell_build(c, false, false);
   c->cells_valid = true;
   // Corrected velocities go to the dead plane set and are dropped: this pass stops at get_accel.
-  forces_for(c, true, nullptr, c->alt);
-  c->launches += kKernelsPerCellBuild + kKernelsPerForcePass;
+  build_lists(c, nullptr);
+  forces_for(c, true, c->alt);
+  drop_lists(c);
   c->records_valid = true;
   int flags = 0;
   af3d_status s = read_status(c, &flags);
@@ -1223,12 +1302,15 @@ af3d_status af3d_prepare_steps(af3d_ctx *c, long k) {
   // The graphs the next af3d_step(ctx, k) replays up to its first re-grid, captured now (a
   // re-grid may move the cell buffers, so later ones are captured when they come).
   const PtrState p0 = ptr_state(c);
-  const long since0 = c->since_sort;
+  const long since0 = c->since_sort, build0 = c->since_build;
+  const int *order0 = c->built_order;
   const bool sorted0 = c->sorted;
   const long to_regrid = (kRegridEvery - c->cc % kRegridEvery) % kRegridEvery;
   const af3d_status s = run_steps(c, std::min(k, to_regrid + 1), false);
   set_ptr_state(c, p0);
   c->since_sort = since0;
+  c->since_build = build0;
+  c->built_order = order0;
   c->sorted = sorted0;
   return s;
 }
@@ -1375,41 +1457,26 @@ af3d_status af3d_step_profile(af3d_ctx *c, long k, double *ms) {
     // The steps af3d_step runs, one at a time (the planes are permuted when that is due; a pass
     // looks ahead when the next step keeps the slot order and no re-grid comes between).
     const bool resort = c->since_sort + 1 > c->resort_every;
-    const bool warm = !resort && c->look;
     const bool regrid_after = c->cc % kRegridEvery == 0;
     const bool look = i + 1 < k && !regrid_after && !((resort ? 0 : c->since_sort + 1) + 1 > c->resort_every);
+    const StepPlan p = plan_step(c, resort, look);
     AF3D_CUDA(cudaEventRecord(ev[0], c->st));
-    if (!warm) launch_advance_time(c->st, c->d);
+    if (!p.warm) {
+      launch_advance_time(c->st, c->d);
+      c->launches++;
+    }
     AF3D_CUDA(cudaEventRecord(ev[1], c->st));
-    if (!warm) predict_for(c, true, true, true, !resort);
+    if (p.resort) predict_for(c, true, true, true);
+    else step_predict(c, p);
     AF3D_CUDA(cudaEventRecord(ev[2], c->st));
-    launch_sort(c->L(), c->d, c->cells, c->id_cur, c->ntags, resort ? nullptr : c->cull, warm);
+    if (p.build) sort_for(c, !p.resort);
     AF3D_CUDA(cudaEventRecord(ev[3], c->st));
-    if (resort) {
-      launch_permute_records(c->L(), c->cur, c->alt, c->cells.perm, c->id_cur, c->id_alt, c->fl_cur,
-                             c->fl_alt, c->nbr, c->cull, false);
-      std::swap(c->cur, c->alt);
-      std::swap(c->id_cur, c->id_alt);
-      std::swap(c->fl_cur, c->fl_alt);
-    }
+    if (p.resort) enqueue_permutation(c, false);
     AF3D_CUDA(cudaEventRecord(ev[4], c->st));
-    if (resort) {
-      forces_for(c, false, nullptr, c->alt, false, look);
-      swap_velocity_planes(c->cur, c->alt);
-    } else {
-      forces_for(c, false, c->cells.perm, c->cur, warm, look);
-    }
-    if (look) {
-      std::swap(c->nbr, c->nbr_next);
-      std::swap(c->cull, c->cull_next);
-    }
-    c->look = look;
-    swap_accel_planes(c->cur);
-    swap_accel_planes(c->alt);
+    if (p.build) build_lists(c, p.resort ? nullptr : c->cells.perm);
+    step_forces(c, p, false);
     AF3D_CUDA(cudaEventRecord(ev[5], c->st));
-    c->sorted = resort;
     c->since_sort = resort ? 0 : c->since_sort + 1;
-    c->launches += kernels_of(1, resort, warm);
     c->time = c->time + c->sys[0].dt;
     const bool do_regrid = c->cc % kRegridEvery == 0;
     c->cc++;
@@ -1657,15 +1724,17 @@ af3d_status set_device_time(af3d_ctx *c, double t) {
 // the sort, and every force of the phase into F, T and a_f.
 void enqueue_startup_pass(af3d_ctx *c) {
   predict_for(c, false, true, false, true);
-  launch_sort(c->L(), c->d, c->cells, c->id_cur, c->ntags, c->cull);
-  forces_for(c, true, c->cells.perm, c->alt);   // corrected velocities go to the dead set
+  sort_for(c, true);
+  build_lists(c, c->cells.perm);
+  forces_for(c, true, c->alt);   // corrected velocities go to the dead set
+  drop_lists(c);
 }
 
 // This step's cell structure at the recomputed predicted state (records, keys, sort).
 void enqueue_step_cells(af3d_ctx *c) {
   launch_advance_time(c->st, c->d);
   predict_for(c, true, true, true, true);
-  launch_sort(c->L(), c->d, c->cells, c->id_cur, c->ntags, c->cull);
+  sort_for(c, true);
 }
 
 // The plane set with its torque planes replaced by planes 24..26 of a tape slot.
@@ -1750,6 +1819,9 @@ extern "C" af3d_status af3d_adjoint(af3d_ctx *c, long steps, long ckpt_every, do
   double *dsc = nullptr;
   if (e == cudaSuccess) e = cudaMalloc((void **)&dsc, sizeof(double) * (nsc + 3 * (size_t)(steps + 1)));
   if (e == cudaSuccess) buf.owned.push_back(dsc);
+  int *start_cnt = nullptr;   // the start-up pass's list counts
+  if (e == cudaSuccess) e = cudaMalloc((void **)&start_cnt, sizeof(int) * m);
+  if (e == cudaSuccess) buf.owned.push_back(start_cnt);
   if (e != cudaSuccess) return fail(AF3D_ERR_NOMEM, std::string("adjoint buffers: ") + cudaGetErrorString(e));
   double *pgr = dsc + 3 * nf;
   double *t_pair = dsc + nsc;   // [steps + 1][2]: {time, time_prev} during step k
@@ -1861,6 +1933,7 @@ extern "C" af3d_status af3d_adjoint(af3d_ctx *c, long steps, long ckpt_every, do
         for (int q = 0; q < 9; q++) rnext_src.p[R00 + q] = rnext.p[q];
         launch_state_copy(c->L(), c->cur, ckpt[seg], false);
         c->look = false;   // the restored state has not been predicted
+        drop_lists(c);
         AF3D_CUDA(cudaMemcpyAsync(&c->d->time, t_pair + 2 * k0 + 1, sizeof(double), cudaMemcpyDeviceToDevice,
                                   c->st));
         for (long k = k0; k < k1; k++) taped_step(k, k0, k1);
@@ -1887,7 +1960,7 @@ extern "C" af3d_status af3d_adjoint(af3d_ctx *c, long steps, long ckpt_every, do
         }
         AF3D_CUDA(cudaMemsetAsync(acc.p[0], 0, sizeof(double) * kAccPlanes * n, c->st));   // one block
         launch_adj_forces_lists(c->L(), Pk, adjA, adjB, acc, rb, c->d, c->fl_cur, rec, c->cull, c->cells.start,
-                                c->cells.perm, tape_lists[k - k0], pgr);
+                                c->cells.perm, tape_lists[k - k0], pgr, false);
         launch_adj_predict(c->L(), Pk, tape[k - k0], adjA, adjB, acc, rb, c->d, c->fl_cur);
         std::swap(adjA, adjB);
       }
@@ -1896,10 +1969,12 @@ extern "C" af3d_status af3d_adjoint(af3d_ctx *c, long steps, long ckpt_every, do
     launch_state_copy(c->L(), c->cur, state0, false, true);
     s = set_device_time(c, t_init);
     if (s) return s;
+    c->lists.cnt = start_cnt;   // the pass records its lists
     enqueue_startup_pass(c);
     AF3D_CUDA(cudaMemsetAsync(acc.p[0], 0, sizeof(double) * kAccPlanes * n, c->st));
-    launch_adj_forces(c->L(), c->cur, adjA, adjB, acc, rb, c->d, c->fl_cur, c->nbr, c->cull, c->cells.start,
-                      c->cells.perm, c->cells.csort, pgr, true);
+    launch_adj_forces_lists(c->L(), c->cur, adjA, adjB, acc, rb, c->d, c->fl_cur, c->nbr, c->cull, c->cells.start,
+                            c->cells.perm, c->lists, pgr, true);
+    own.restore();
     launch_adj_startup(c->L(), c->cur, adjA, adjB, acc, rb);
     // gradients by clump id
     std::vector<double> h((size_t)kAdjPlanes * n);
@@ -1930,6 +2005,7 @@ extern "C" af3d_status af3d_adjoint(af3d_ctx *c, long steps, long ckpt_every, do
   c->records_valid = false;
   c->cells_valid = false;
   c->look = false;
+  drop_lists(c);
   c->since_sort = c->resort_every;
   c->cc += steps;
   flags = 0;

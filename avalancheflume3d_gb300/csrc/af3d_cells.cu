@@ -10,6 +10,8 @@
 //      makes the final order deterministic and equal to the reference's ascending-id insertion
 //      order (cells.cu:60-109)                 -> perm[new slot] = old slot
 // Integer work only; HBM-bound.
+#include <climits>
+
 #include "af3d_internal.h"
 
 namespace af3d {
@@ -71,14 +73,10 @@ __device__ __forceinline__ long n_buckets(const DevScalars *d, long n) { return 
 
 // Each tile adds the clump counts of the tiles before it (counted at arrival; integer sums are
 // exact in any order), then scans its own buckets.
-// advance: block 0 also performs k_advance_time's time += dt (steps whose predictor ran in the
-// previous force pass start with the sort; nothing before the force pass reads the clock).
+// Lists are built from the sort, so the marks that clumps left since the last ones are void.
 __global__ void k_scan_final(const int *__restrict__ count, const int *__restrict__ tile_count,
-                             int *start, DevScalars *d, bool advance, long n) {
-  if (advance && blockIdx.x == 0 && threadIdx.x == 0) {
-    d->time_prev = d->time;
-    d->time = d->time + d->flumes[0].sys.dt;
-  }
+                             int *start, DevScalars *d, long n) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) d->all_slow = d->brute = INT_MAX;
   const long nb = n_buckets(d, n);
   if (blockIdx.x == 0 && threadIdx.x == 0) start[nb] = (int)n;   // every clump has one bucket
   if (blockIdx.x * (long)kTile >= nb) return;   // a tile past the buckets in use
@@ -135,7 +133,11 @@ __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ star
   int r = 0;
   for (int j = b; j < e; j++) r += id[tmp_slot[j]] < me;
   perm[b + r] = (int)s;
-  if (cull) csort[b + r] = cull[s].c;
+  if (cull) {   // the bound with the clump's allowance
+    float4 c = cull[s].c;
+    c.w += cull[s].allow * (1.0f + 1e-5f);
+    csort[b + r] = c;
+  }
   // cells.cu:96-102: a cell may hold at most ntags - 1 clumps
   if (ntags > 0 && k < ncell3 && r == 0 && (e - b) >= ntags)
     atomicOr(&d->status, 1 << AF3D_ERR_CELL_CAPACITY);
@@ -145,12 +147,11 @@ __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ star
 
 long scan_tiles(long bucket_cap) { return (bucket_cap + kTile - 1) / kTile; }
 
-void launch_sort(const Launch &L, DevScalars *d, Cells c, const long long *id, long ntags, const CullRec *cull,
-                 bool advance) {
+void launch_sort(const Launch &L, DevScalars *d, Cells c, const long long *id, long ntags, const CullRec *cull) {
   // Launch sizes follow the capacity; the kernels read the bucket count in use from the device,
   // so a captured graph stays valid across device-side re-grids.
   const long ntiles = scan_tiles(c.cap);
-  k_scan_final<<<(unsigned)ntiles, kScanThreads, 0, L.st>>>(c.count, c.tile_count, c.start, d, advance, L.n);
+  k_scan_final<<<(unsigned)ntiles, kScanThreads, 0, L.st>>>(c.count, c.tile_count, c.start, d, L.n);
   if (L.n <= 0) return;
   const unsigned g = (unsigned)((L.n + 127) / 128);
   k_scatter<<<g, 128, 0, L.st>>>(c.key, c.rank_tmp, c.start, c.tmp_slot, L.n);

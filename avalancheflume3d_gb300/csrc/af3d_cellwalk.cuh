@@ -16,33 +16,62 @@ __device__ __forceinline__ float d2f(float4 a, float4 b) {
   return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
 }
 
-// 16-bit mask of the sphere pairs of own clump (cull record me) and partner m that the FP32
-// test cannot rule out; bit p = sph_id - 1 = 4 * (partner sphere) + (own sphere).
-__device__ __forceinline__ unsigned pair_mask(const CullRec &me, const CullRec &m) {
-  const float lim = me.c.w + m.c.w;
-  if (d2f(me.c, m.c) > lim * lim * kCullSlack) return 0u;
-  const float rl = me.s[0].w + m.s[0].w;
-  const float r2 = rl * rl * kCullSlack;
+// A clump's own side of the sphere tests: its spheres relative to its first one in units (exact in
+// FP32: below 2^22 units), that sphere's centre and the sphere radius in units.
+struct OwnSpheres {
+  float x[4], y[4], z[4], rad;
+  int cx, cy, cz;
+};
+
+// 2^e, |e| <= 126.
+__device__ __forceinline__ float unit_power(int e) { return __int_as_float((127 + e) << 23); }
+
+// a - b of two coordinates in units, |a - b| < 2^22, as a float (exact): the integer difference
+// placed in the mantissa of 1.5 x 2^23.
+__device__ __forceinline__ float unit_difference(int a, int b) {
+  return __int_as_float(0x4B400000 + (a - b)) - 12582912.0f;
+}
+
+__device__ __forceinline__ OwnSpheres own_spheres(const CullRec &m) {
+  OwnSpheres o;
+  o.rad = __int_as_float(m.s[0].w);
+  o.cx = m.s[0].x; o.cy = m.s[0].y; o.cz = m.s[0].z;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    o.x[k] = unit_difference(m.s[k].x, o.cx);
+    o.y[k] = unit_difference(m.s[k].y, o.cy);
+    o.z[k] = unit_difference(m.s[k].z, o.cz);
+  }
+  return o;
+}
+
+// 16-bit mask of the sphere pairs closer than `margin` units: bit p = sph_id - 1 = 4 * (partner
+// sphere) + (own sphere).  The truncated coordinates leave each difference within 2 units of the
+// exact one (so a distance within 2 sqrt(3)), which the records' radii, inflated by 2 units each,
+// cover; the FP32 squares round by less than the 2^-20 slack.  An infinite radius (kCullMaxUnits)
+// lets every pair pass whatever the differences are.
+__device__ __forceinline__ unsigned sphere_mask(const OwnSpheres &o, const int4 *ms, float margin) {
+  const float r = o.rad + __int_as_float(ms[0].w) + margin;
+  const float r2 = r * r * (1.0f + 9.5367431640625e-07f);
   unsigned mask = 0u;
 #pragma unroll
-  for (int j = 0; j < 4; j++)
+  for (int j = 0; j < 4; j++) {
+    const float px = unit_difference(ms[j].x, o.cx), py = unit_difference(ms[j].y, o.cy),
+                pz = unit_difference(ms[j].z, o.cz);
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (d2f(me.s[k], m.s[j]) <= r2) mask |= 1u << (4 * j + k);
+    for (int k = 0; k < 4; k++) {
+      const float dx = px - o.x[k], dy = py - o.y[k], dz = pz - o.z[k];
+      if (!(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r2)) mask |= 1u << (4 * j + k);
+    }
+  }
   return mask;
 }
 
-// The sixteen sphere tests of pair_mask alone (for partners whose centre test passed).
-__device__ __forceinline__ unsigned sphere_mask(const CullRec &me, const CullRec &m) {
-  const float rl = me.s[0].w + m.s[0].w;
-  const float r2 = rl * rl * kCullSlack;
-  unsigned mask = 0u;
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (d2f(me.s[k], m.s[j]) <= r2) mask |= 1u << (4 * j + k);
-  return mask;
+// The mask of the pairs that may overlap, after the FP32 centre test of the bounding spheres.
+__device__ __forceinline__ unsigned pair_mask(const CullRec &me, const CullRec &m) {
+  const float lim = me.c.w + m.c.w;
+  if (d2f(me.c, m.c) > lim * lim * kCullSlack) return 0u;
+  return sphere_mask(own_spheres(me), m.s, 0.0f);
 }
 
 struct Search {
@@ -165,248 +194,45 @@ __device__ __forceinline__ void for_neighbour_slots_pre(const Search &q, const a
     }
 }
 
-// ---- per-warp item lists (the warp-cooperative contact passes) -----------------------------
-
-constexpr int kLaneItems = kListCap;
 constexpr unsigned kBndItem = 0xFFFFFF00u;   // boundary item: kBndItem | routine << 2 | sphere
 
-// Partners per clump that pass the centre test; a clump with more takes the per-clump walk.  The
-// benchmark states have at most 10 (262,144-clump bed, 524,288-clump polydisperse funnel); the
-// cap sets most of the list phase's shared memory, which the L1 cache shares.
-constexpr int kPassCap = 24;
-constexpr unsigned kSlotMask = 0x3FFFFFFFu;   // pass entry: position or slot | (x offset + 1) << 30
-
-// Per-warp partner lists of the two-stage gather in shared memory, one column per lane
-// ([entry][lane]): a lane's own accesses always fall in its own bank.
-struct PassLists {
-  unsigned pass_t[kPassCap][32];         // partner position, then slot | (cell x offset + 1) << 30
-  unsigned short pass_m[kPassCap][32];   // their 16-bit sphere-pair masks
-  int pbase[33];
-  unsigned short cand[kLaneItems][32];   // candidate sphere pairs in item order: entry << 4 | sph_id-1
-                                         // (0x8000: rejected by the overlap test)
-  int cbase[33];
+// Cell (x, y, z) of bucket `key` of a flume with cell offset `off`; false for a bucket of another
+// flume or of a clump that is not binned.
+struct CellAt {
+  int x, y, z;
 };
-static_assert(((kPassCap - 1) << 4 | 15) < 0x8000, "candidate entries are 15-bit");
-
-// Item lists held in shared memory (the adjoint's cooperative reverse).
-struct ItemLists {
-  unsigned items[kLaneItems][32];
-  int base[33];                          // exclusive prefix of the lanes' item counts
-  PassLists pl;
-};
-
-// Exclusive prefix of `v` over the warp into sh[0..32]; returns the total.
-__device__ __forceinline__ int warp_prefix(int v, int *sh) {
-  const int lane = threadIdx.x & 31;
-  int incl = v;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += u;
-  }
-  sh[lane] = incl - v;
-  const int total = __shfl_sync(0xffffffffu, incl, 31);
-  if (lane == 31) sh[32] = total;
-  __syncwarp();
-  return total;
-}
-
-// The lane whose range [sh[l], sh[l+1]) holds position j (sh: exclusive prefix of 32 counts).
-__device__ __forceinline__ int owner_of(const int *sh, int j) {
-  int lo = 0, hi = 31;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (sh[mid] <= j) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
-// Boundary items of the routines [r0, r1] for one clump (culling record me), appended to the
-// lane's item column `col` (entries `stride` apart); false if the list would overflow.  The FP32
-// gates admit every sphere the routine can touch (and a few more, which the exact test of the
-// force pass then rejects).
-__device__ __forceinline__ bool push_boundary(int r0, int r1, const CullRec &me, const Consts &c, bool door_closed,
-                                              unsigned *col, long stride, int &nitems) {
-  for (int rt = r0; rt <= r1; rt++) {
-    if (!bnd_may_touch_f(rt, me.c, me.c.w, c, door_closed)) continue;
-    for (int ns = 0; ns < 4; ns++) {
-      if (!bnd_may_touch_f(rt, me.s[ns], me.s[ns].w, c, door_closed)) continue;   // one sphere
-      if (nitems == kLaneItems) return false;
-      col[stride * nitems++] = kBndItem | (unsigned)(rt << 2) | (unsigned)ns;
-    }
-  }
+__device__ __forceinline__ bool cell_at(int key, long long off, const GridF &g, CellAt &c) {
+  const int nxy = g.nx * g.ny;
+  const long long lin = (long long)key - off;
+  if (lin < 0 || lin >= (long long)nxy * g.nz) return false;
+  const unsigned l = (unsigned)lin;
+  c.z = (int)(l / (unsigned)nxy);
+  const unsigned r = l - (unsigned)(c.z * nxy);
+  c.y = (int)(r / (unsigned)g.nx);
+  c.x = (int)(r - (unsigned)(c.y * g.nx));
   return true;
 }
 
-// Stage 1 of the gather (per lane): the partners among the 27 neighbour cells whose bounding
-// spheres can touch the clump's (FP32 centre test), the clump itself included.  The three cells of one (jdel, kdel) row are
-// consecutive in the linear cell index, so their members form one slot range split by four
-// start[] values; the nine ranges are walked one after another, two slots a turn with both
-// loads issued together.  Each kept partner is tagged with its cell's x offset (0..2) so that
-// the reference's visiting order (idel, then jdel, kdel, then slot) can be restored.  Returns
-// the number of partners found (which may exceed kPassCap).
-__device__ __forceinline__ int gather_partners(PassLists &pl, long s, float4 mc, const Search &q,
-                                               const af3d_cell_par &g, const int *__restrict__ start,
-                                               const int *__restrict__ order, const float4 *__restrict__ csort,
-                                               const CullRec *__restrict__ cull) {
-  const int lane = threadIdx.x & 31;
-  int npass = 0;
-  // Kept partners are recorded by their position k in the (cell, id) order; stage 2 looks up
-  // their slots (and drops the clump itself) with all lanes busy.
-  auto keep = [&](int k, unsigned tag, float4 pc) {
-    const float lim = mc.w + pc.w;
-    if (d2f(mc, pc) > lim * lim * kCullSlack) return;
-    if (npass < kPassCap) pl.pass_t[npass][lane] = (unsigned)k | (tag << 30);
-    npass++;
-  };
-  const long x0 = q.ci - 1;
+// Visits the slots that the last built cell order holds in the 5 x 5 x 5 cells around `c`.
+template <typename F>
+__device__ __forceinline__ void for_slots_around(const CellAt &c, const GridF &g, long long off,
+                                                 const int *__restrict__ start, const int *__restrict__ order, F &&f) {
+  const int x0 = max(c.x - 2, 0), x1 = min(c.x + 2, g.nx - 1);
 #pragma unroll 1
-  for (int r = 0; r < 9; r++) {
-    const long jn = q.cj + (r / 3 - 1), kn = q.ck + (r % 3 - 1);
-    if (jn < 0 || kn < 0 || jn >= g.ncell.y || kn >= g.ncell.z) continue;
-    const long rb = q.off + g.ncell.x * (jn + g.ncell.y * kn);
-    // boundary e of the row: start of cell x0 + e, clamped into the row (empty cells outside)
-    int b[4];
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      long x = x0 + e;
-      x = x < 0 ? 0 : (x > g.ncell.x ? g.ncell.x : x);
-      b[e] = __ldg(&start[rb + x]);
-    }
-    int k = b[0];
+  for (int z = max(c.z - 2, 0); z <= min(c.z + 2, g.nz - 1); z++)
 #pragma unroll 1
-    for (; k + 1 < b[3]; k += 2) {
-      const float4 p0 = order ? __ldg(&csort[k]) : cull[k].c;
-      const float4 p1 = order ? __ldg(&csort[k + 1]) : cull[k + 1].c;
-      keep(k, 1u + (k >= b[1]) + (k >= b[2]), p0);
-      keep(k + 1, 1u + (k + 1 >= b[1]) + (k + 1 >= b[2]), p1);
+    for (int y = max(c.y - 2, 0); y <= min(c.y + 2, g.ny - 1); y++) {
+      const int *row = start + off + (long long)g.nx * (y + (long long)g.ny * z);
+      const int t1 = __ldg(row + x1 + 1);
+#pragma unroll 1
+      for (int t = __ldg(row + x0); t < t1; t++) f(order ? __ldg(&order[t]) : t);
     }
-    if (k < b[3]) keep(k, 1u + (k >= b[1]) + (k >= b[2]), order ? __ldg(&csort[k]) : cull[k].c);
-  }
-  return npass;
 }
 
-// Every lane's item list of one contact pass, in the reference's order: the boundary routines
-// before the particles (avalanche: hop x3, funnel, fcorners, walls), the particle contacts
-// sph_id-major, the routines after them (avalanche: flume; fill: hop x3).  Boundary items
-// (routine, sphere) for the spheres the routine's 1-Lipschitz gate cannot rule out; particle
-// items (partner slot, sph_id) from a three-stage gather: stage 1 (per lane, gather_partners)
-// keeps the partners whose bounding spheres can touch, stage 2 (whole warp) runs the sixteen
-// FP32 sphere tests of every kept partner, 32 a round, and stage 3 (whole warp) the exact FP64
-// overlap test of every sphere pair the FP32 test could not rule out.  Items go to the lane's column `col`, entries
-// `stride` apart.  All 32 lanes call this; returns the lane's item count, 0 with `slow` set
-// when the lane's lists would overflow.
-// (the counts of a clump's list: `pre` boundary items, then `pair` particle items, then the rest)
+// A clump's list layout: `pre` boundary items, then `pair` particle items, then the rest.
 struct ListCounts {
   int pre, pair;
 };
-
-__device__ __forceinline__ int build_item_lists(PassLists &pl, unsigned *col, long stride, long wbase, long s,
-                                                bool act, bool aval, V3 r, const Consts &c,
-                                                const af3d_cell_par &g, const GridF &gf, long long off,
-                                                const NbrRec *__restrict__ nbr,
-                                                const CullRec *__restrict__ cull, const int *__restrict__ start,
-                                                const int *__restrict__ order, const float4 *__restrict__ csort,
-                                                bool &slow, ListCounts &lc) {
-  const int lane = threadIdx.x & 31;
-  const int pre0 = aval ? R_HOP0 : 1, pre1 = aval ? R_WALLS : 0;         // fill: none before
-  const int post0 = aval ? R_FLUME : R_HOP0, post1 = aval ? R_FLUME : R_HOP2;
-  int nitems = 0;
-  slow = false;
-  lc.pre = lc.pair = 0;
-  const CullRec me = cull[s];
-  const bool door_closed = *c.tp < 0.0;
-  if (act) slow = !push_boundary(pre0, pre1, me, c, door_closed, col, stride, nitems);
-  lc.pre = nitems;
-  int npass = 0;
-  if (act && !slow) {
-    npass = gather_partners(pl, s, me.c, search_centre_f(me.c, r, g, gf, off), g, start, order, csort, cull);
-    if (npass > kPassCap) {
-      slow = true;
-      npass = 0;
-    }
-  }
-  // Stage 2 (whole warp): each kept partner's slot, then its sixteen sphere tests, 32 partners a
-  // round (the clump itself gets an empty mask).
-  const int total_pass = warp_prefix(npass, pl.pbase);
-  for (int j0 = 0; j0 < total_pass; j0 += 32) {
-    const int j = j0 + lane;
-    if (j < total_pass) {
-      const int ow = owner_of(pl.pbase, j), k = j - pl.pbase[ow];
-      const unsigned e = pl.pass_t[k][ow];
-      const int pos = (int)(e & kSlotMask);
-      const int t = order ? __ldg(&order[pos]) : pos;
-      pl.pass_t[k][ow] = (unsigned)t | (e & ~kSlotMask);
-      pl.pass_m[k][ow] = t == wbase + ow ? (unsigned short)0 : (unsigned short)sphere_mask(cull[wbase + ow], cull[t]);
-    }
-  }
-  __syncwarp();
-  // Each lane's candidate sphere pairs in item order: sph_id-major (the order of the sixteen
-  // force_part launches), and within one sph_id in the reference's cell order (x offset, then
-  // row, then slot).  Partners without a candidate sphere pair are dropped first (keeping the
-  // walk order), and only the sph_ids some partner has are visited.
-  int ncand = 0;
-  if (act && !slow) {
-    int m = 0;
-    unsigned any = 0u;
-#pragma unroll 1
-    for (int k = 0; k < npass; k++) {
-      const unsigned mk16 = pl.pass_m[k][lane];
-      if (!mk16) continue;
-      pl.pass_t[m][lane] = pl.pass_t[k][lane];
-      pl.pass_m[m][lane] = (unsigned short)mk16;
-      any |= mk16;
-      m++;
-    }
-#pragma unroll 1
-    while (any && !slow) {
-      const int p = __ffs(any) - 1;
-      any &= any - 1u;
-#pragma unroll 1
-      for (unsigned tag = 1; tag <= 3 && !slow; tag++)
-#pragma unroll 1
-        for (int k = 0; k < m; k++) {
-          if ((pl.pass_t[k][lane] >> 30) != tag || !((pl.pass_m[k][lane] >> p) & 1u)) continue;
-          if (nitems + ncand == kLaneItems) {
-            slow = true;
-            break;
-          }
-          pl.cand[ncand++][lane] = (unsigned short)(((unsigned)k << 4) | (unsigned)p);
-        }
-    }
-    if (slow) ncand = 0;
-  }
-  // Stage 3 (whole warp): the exact FP64 overlap test of every candidate (the test the force
-  // pass would make first), 32 a round, so that the force pass gets only overlapping pairs.
-  const int total_cand = warp_prefix(ncand, pl.cbase);
-  for (int j0 = 0; j0 < total_cand; j0 += 32) {
-    const int j = j0 + lane;
-    if (j < total_cand) {
-      const int ow = owner_of(pl.cbase, j), ci = j - pl.cbase[ow];
-      const unsigned e = pl.cand[ci][ow];
-      const int k = (int)(e >> 4), p = (int)(e & 15u);
-      const NbrRec &mo = nbr[wbase + ow];
-      const V3 s1 = mk(mo.s[3 * (p & 3)], mo.s[3 * (p & 3) + 1], mo.s[3 * (p & 3) + 2]);
-      V3 d;
-      double dist2, sep;
-      if (!spheres_overlap(s1, mo.rad, nbr[pl.pass_t[k][ow] & kSlotMask], p >> 2, d, dist2, sep))
-        pl.cand[ci][ow] = (unsigned short)(e | 0x8000u);
-    }
-  }
-  __syncwarp();
-  if (act && !slow) {
-#pragma unroll 1
-    for (int i = 0; i < ncand; i++) {
-      const unsigned e = pl.cand[i][lane];
-      if (e & 0x8000u) continue;
-      const unsigned t = pl.pass_t[e >> 4][lane] & kSlotMask;
-      col[stride * nitems++] = (t << 4) | (e & 15u);   // (partner slot, sph_id-1)
-    }
-    lc.pair = nitems - lc.pre;
-    slow = !push_boundary(post0, post1, me, c, door_closed, col, stride, nitems);
-  }
-  return slow ? 0 : nitems;
-}
 
 }  // namespace
 }  // namespace af3d

@@ -9,6 +9,7 @@
 // one or two 64-byte lines.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -33,8 +34,16 @@ enum Plane : int {
   NPLANES
 };
 
+// How the culling records and near lists measure: lengths in units of 2^-qs cm, and how far a
+// clump is allowed to move before its lists are built again (see NearLists).
+struct Margins {
+  int qs;
+  float per_speed, floor, cap;   // allowance min(per_speed * speed + floor, cap), in cm
+};
+
 struct Planes {
   double *p[NPLANES];
+  Margins m;
 };
 
 // Packed neighbour record: everything a partner clump contributes to a contact.
@@ -44,14 +53,42 @@ struct __align__(64) NbrRec {
   double rad, msph, mwall;   // sphere radius, sphere mass, wall-contact mass
 };
 
-// FP32 culling record.  c = (centre, bound), sk = (sphere centre, inflated radius).  The bounds
-// are rounded up and inflated by 2^-22 times the largest coordinate magnitude, which covers the
-// FP32 rounding of every coordinate; the tests multiply by (1 + 2^-18) on top, so a pair the
-// FP64 test could accept is never culled.
+// Culling record.  c = (centre, bound) in FP32: the bound is rounded up and inflated by 2^-22
+// times the largest coordinate magnitude, which covers the FP32 rounding of every coordinate; the
+// tests multiply by (1 + 2^-18) on top.  sk = (sphere centre in units, truncated, modulo 2^32 | the
+// inflated sphere radius in units, a float).  Differences of nearby coordinates are exact in
+// units whatever the coordinates' size, so the sphere tests see gaps down to a few units (2^-21
+// cm at 1 mm spheres) where FP32 coordinates of ~100 cm blur 10^-4 cm.  A pair the FP64 test
+// could accept is never culled.
 struct __align__(16) CullRec {
   float4 c;
-  float4 s[4];
+  int4 s[4];
+  int key;       // the clump's bucket at this step (cell order of the contacts)
+  float allow;   // how far it may move from here (Margins)
+  int pad[2];
 };
+
+// A clump of extent + radius above this many units has an infinite radius in its record: every
+// sphere pair of it passes the culling tests.  Below it the differences that the tests form stay
+// under 2^22 units: centres at most two extents and two allowances apart, plus two extents.
+constexpr float kCullMaxUnits = 943718.0f;   // 0.9 x 2^20
+
+// The margins for clumps of sphere radius up to rmax moving for up to `steps` steps of dt.  The
+// unit: a regular clump's bounding radius (half of GYR rmax, cabecera.hu:8) is at most 0.8 x 2^20
+// units.  The allowance: half as much again as the clump's speed covers in that time, and 4 % of
+// a sphere's radius for what contacts accelerate it; at most 30 % of the radius.
+inline Margins margins_for(double rmax, double dt, long steps) {
+  Margins m;
+  int e = 0;
+  const bool ok = rmax > 1e-30 && rmax < 1e30;
+  frexp(ok ? 838860.0 / (2.2247448713915889 * rmax) : 2097152.0, &e);
+  m.qs = e - 1;
+  const double v = 1.5 * fabs(dt) * (double)steps;
+  m.per_speed = v < 1e30 ? (float)v : 1e30f;
+  m.floor = ok ? (float)(0.04 * rmax) : 0.0f;
+  m.cap = ok ? (float)(0.3 * rmax) : 0.0f;
+  return m;
+}
 
 // Cell-list buffers.  Keys: flume cell offset + cell index for binned clumps (the flumes' grids
 // are concatenated, so the sort keeps every flume contiguous), ncell_total + id for clumps that
@@ -66,6 +103,8 @@ struct Cells {
   int *count;       // [cap] bucket sizes (all zero between builds)
   int *start;       // [cap+1] exclusive scan of count
   int *tile_count;  // [scan_tiles(cap)] clumps per kScanTile buckets (all zero between builds)
+  int *occ;         // [cap] clumps per bucket at this step, when it does not sort (all zero after it)
+  int *occ_next;    // [cap] the same, filled by the look-ahead for the next step
   long cap;         // buckets available (ncell_total + N must fit)
 };
 
@@ -126,15 +165,18 @@ __host__ __device__ inline Consts make_consts(const af3d_system_par &s, const af
 // One flume of the context (a plain drop-in run has one; a batched ensemble has many).  Every
 // flume has its own system_par (friction, restitution, slope, ...), Funnel and cell grid; all
 // flumes share dt and advance in lockstep.
-// FP32 copies of a grid's origin and inverse cell sides (the search-cell estimate).
+// FP32 copies of a grid's origin and inverse cell sides (the search-cell estimate) and its cell
+// counts (all cells together are fewer than 2^31).
 struct GridF {
   float xmin, ymin, zmin, ix, iy, iz;
+  int nx, ny, nz;
 };
 
 __host__ __device__ inline GridF grid_floats(const af3d_cell_par &g) {
   GridF q;
   q.xmin = (float)g.rr_min.x; q.ymin = (float)g.rr_min.y; q.zmin = (float)g.rr_min.z;
   q.ix = (float)g.cs_inv.x; q.iy = (float)g.cs_inv.y; q.iz = (float)g.cs_inv.z;
+  q.nx = (int)g.ncell.x; q.ny = (int)g.ncell.y; q.nz = (int)g.ncell.z;
   return q;
 }
 
@@ -162,6 +204,10 @@ struct DevScalars {
   unsigned long long overflows; // clumps whose item lists overflowed, over fused force passes
   long long       ncell_total; // sum of the flumes' ncell3: the first removed-clump bucket
   long long       pending;     // > 0: a re-grid derived grids needing this many cell buckets
+  int             tick;        // steps begun (counts with the clock)
+  int             all_slow;    // from this tick on every clump takes the per-clump search ...
+  int             brute;       // ... over every clump of its flume (until the lists are built again)
+  unsigned        ticket;      // blocks of a force pass that have finished
   DevFlume       *flumes;      // [nflumes]
 };
 
@@ -201,14 +247,40 @@ __host__ __device__ inline int pack_list_counts(int listed, int pre, int pair) {
   return listed < 0 ? -1 : listed | pre << 8 | pair << 16;
 }
 
+// Near lists: per clump the sphere pairs and the (boundary routine, sphere) pairs that may touch
+// while no clump moves farther than its allowance, built from a cell sort and used for up to
+// kBuildEvery steps (fewer when the slots are permuted, the grid changes or the caller touches
+// the state).  A step that uses them neither sorts nor walks cells: it tests ~7 sphere pairs per
+// clump of a dense bed instead of ~300 behind nine dependent reads of the cell table.  Each pass
+// tests the listed pairs at the current positions and orders the overlapping ones by the
+// current cells, so a step's contacts and their order do not depend on when the lists were
+// built.  What a clump may still move is counted down (`rem`); one that used it up marks every
+// clump around it `loose` from the next step on, and a loose clump searches the cells around
+// itself (as built) in place of its list.  Measured against a sort and a walk every step:
+// 2,048 clumps (fast) 48 -> 37 us a step, 20,011 in the hopper (exact) 82 -> 75, 262,144 (fast)
+// 0.325 -> 0.296 ms with the copies of a 40-step call, (exact) 0.49 -> 0.46.
+constexpr int kNearCap = 60;
+#ifndef AF3D_BUILD_EVERY
+#define AF3D_BUILD_EVERY 16
+#endif
+constexpr long kBuildEvery = AF3D_BUILD_EVERY;
+struct NearLists {
+  unsigned *items;   // [kNearCap][n] partner slot << 4 | sph_id - 1, by partner id, then sph_id
+  int *info;         // [n] entries, -1: too many (the clump searches for itself)
+  unsigned *bnd;     // [n] bit 4 * routine + sphere
+  float *rem;        // [n] cm the clump may still move
+  int *loose;        // [n] the tick from which the list does not hold (never: INT_MAX)
+};
+
 // The next step's predictor run at the end of a force pass (look-ahead): the corrected clump is
 // advanced at once, its records go to the next step's record buffers, its rotation rows to the
-// RN planes, its bucket key, arrival rank and bucket count to the cell list.  nbr == null: none.
+// RN planes, and it is counted in the next step's buckets: for the sort (build: the next step
+// sorts and builds lists) or for the cells' capacity alone.  The pass's last block advances the
+// clock.  nbr == null: none.
 struct LookAhead {
   NbrRec *nbr;
   CullRec *cull;
-  Cells cells;
-  const long long *id;
+  bool build;
 };
 
 // Which force routines a boundary kernel applies, in the reference's call order.
@@ -223,32 +295,39 @@ struct Launch {
 };
 
 // init_Verlet and/or the cell keys; with nbr/cull (predict and keys only) also the neighbour
-// records of every clump at its own slot.
+// records of every clump at its own slot.  count_only: the step keeps its near lists, so the keys
+// are counted for the cells' capacity, not for a sort, and the clumps' motion against `near`.
 void launch_predict (const Launch &L, Planes cur, DevScalars *d, bool predict, bool keys, bool t_prev,
-                     Cells cells, const long long *id, const int *flume, NbrRec *nbr = nullptr,
-                     CullRec *cull = nullptr, long s0 = 0, long count = -1);
+                     Cells cells, const long long *id, const int *flume, long ntags, NearLists near,
+                     const int *order, bool count_only, NbrRec *nbr = nullptr, CullRec *cull = nullptr,
+                     long s0 = 0, long count = -1);
 // Exclusive scan of the bucket counts, scatter by arrival, then the deterministic (bucket, id)
 // rank: fills cells.start[0..nbuckets] and cells.perm, checks the ntags capacity and leaves the
 // count array zeroed.  nbuckets = ncell_total + N is read on the device.
 // With cull (records already written at the old slots) also fills cells.csort.
 void launch_sort (const Launch &L, DevScalars *d, Cells cells, const long long *id, long ntags,
-                  const CullRec *cull = nullptr, bool advance = false);
+                  const CullRec *cull = nullptr);
 long scan_tiles (long bucket_cap);
 // Moves every plane (and the id and flume arrays) into the new order and builds the records.
 // `ft`: also carry the force/torque accumulators and a_f (the fused step rewrites them first).
-void launch_permute_records (const Launch &L, Planes src, Planes dst, const int *perm,
+void launch_permute_records (const Launch &L, Planes src, Planes dst, const int *perm, const int *key,
                              const long long *id_src, long long *id_dst, const int *fl_src,
                              int *fl_dst, NbrRec *nbr, CullRec *cull, bool ft);
 void launch_build_records (const Launch &L, Planes cur, NbrRec *nbr, CullRec *cull);
-// The force pass: each block builds its clumps' item lists, then processes them (walls, contacts,
-// bed, get_accel, finish_Verlet).  order: null when the slots are in (cell, id) order, else
-// cells.perm of the last sort, with csort the matching culling centres.  warm: the step's
-// predicted state was made by the previous pass's look-ahead (records, RN planes) and is
-// committed to the planes here; look: this pass runs the next step's predictor.
+// The near lists of slots [s0, s0 + count) from this step's sort.  order: null when the slots are
+// in (cell, id) order, else cells.perm, with csort the matching culling centres.
+void launch_build_lists (const Launch &L, Margins m, DevScalars *d, const int *flume, const CullRec *cull,
+                         Cells cells, const int *order, const long long *id, NearLists near, long s0 = 0,
+                         long count = -1);
+// The force pass: each block takes its clumps' contact items from their near lists, then processes
+// them (walls, contacts, bed, get_accel, finish_Verlet).  order: that of the last built lists.
+// warm: the step's predicted state was made by the previous pass's look-ahead (records, RN
+// planes) and is committed to the planes here; look: this pass runs the next step's predictor.
+// counted: this step's buckets were counted in cells.occ, which the pass zeroes.
 void launch_lists_forces (const Launch &L, Planes cur, Planes out, DevScalars *d, const int *flume,
-                          const NbrRec *nbr, const CullRec *cull, const int *start, const int *order,
-                          const float4 *csort, ContactLists lists, bool write_ft,
-                          const Consts *uniform = nullptr, bool warm = false,
+                          const NbrRec *nbr, const CullRec *cull, Cells cells, const int *order,
+                          const long long *id, NearLists near, ContactLists lists, long ntags, bool write_ft,
+                          bool counted, const Consts *uniform = nullptr, bool warm = false,
                           LookAhead look = LookAhead{}, long s0 = 0, long count = -1, int shape = 0);
 void launch_boundary (const Launch &L, Planes cur, DevScalars *d, const int *flume, int routine);
 void launch_part (const Launch &L, Planes cur, DevScalars *d, const int *flume, const NbrRec *nbr,
@@ -285,14 +364,11 @@ cudaError_t check_fp64_bits (const double *x, long n, int *bad);
 // Adjoint of the exact step (af3d_adjoint.cu).  Planes of 24 state adjoints (r, v, w, R rows,
 // a_i, alpha_i), 21 scattered parts (r1, v1, w1, sphere centres), 9 own R1 parts.
 constexpr int kAdjPlanes = 24, kAccPlanes = 21, kRbPlanes = 9;
-void launch_adj_forces (const Launch &L, Planes P, Planes in, Planes out, Planes acc, Planes rb, DevScalars *d,
-                        const int *flume, const NbrRec *nbr, const CullRec *cull, const int *start,
-                        const int *order, const float4 *csort, double *param_b, bool startup);
-// The same reverse (not the start-up pass) from the item lists and counts the forward force pass
-// of this step recorded.
+// The reverse of a force pass (startup: the start-up pass, which has no finish_Verlet) from the
+// item lists and counts that the forward pass recorded.
 void launch_adj_forces_lists (const Launch &L, Planes P, Planes in, Planes out, Planes acc, Planes rb,
                               DevScalars *d, const int *flume, const NbrRec *nbr, const CullRec *cull,
-                              const int *start, const int *order, ContactLists lists, double *param_b);
+                              const int *start, const int *order, ContactLists lists, double *param_b, bool startup);
 void launch_adj_predict (const Launch &L, Planes P, Planes tape, Planes in, Planes out, Planes acc, Planes rb,
                          DevScalars *d, const int *flume);
 void launch_adj_startup (const Launch &L, Planes P, Planes in, Planes out, Planes acc, Planes rb);
@@ -309,12 +385,13 @@ void launch_state_copy (const Launch &L, Planes P, Planes tape, bool to_tape, bo
 // -DAF3D_FAST -fmad=true; same arguments as above).
 namespace fast {
 void launch_predict (const Launch &L, Planes cur, DevScalars *d, bool predict, bool keys, bool t_prev,
-                     Cells cells, const long long *id, const int *flume, NbrRec *nbr = nullptr,
-                     CullRec *cull = nullptr, long s0 = 0, long count = -1);
+                     Cells cells, const long long *id, const int *flume, long ntags, NearLists near,
+                     const int *order, bool count_only, NbrRec *nbr = nullptr, CullRec *cull = nullptr,
+                     long s0 = 0, long count = -1);
 void launch_lists_forces (const Launch &L, Planes cur, Planes out, DevScalars *d, const int *flume,
-                          const NbrRec *nbr, const CullRec *cull, const int *start, const int *order,
-                          const float4 *csort, ContactLists lists, bool write_ft,
-                          const Consts *uniform = nullptr, bool warm = false,
+                          const NbrRec *nbr, const CullRec *cull, Cells cells, const int *order,
+                          const long long *id, NearLists near, ContactLists lists, long ntags, bool write_ft,
+                          bool counted, const Consts *uniform = nullptr, bool warm = false,
                           LookAhead look = LookAhead{}, long s0 = 0, long count = -1, int shape = 0);
 }  // namespace fast
 

@@ -4,14 +4,17 @@
 //   k_predict      init_Verlet (+ cell key, bucket count)              one thread per clump
 //   (cells)        scan of bucket counts, scatter, deterministic rank  af3d_cells.cu
 //   k_permute      move every plane into (cell, id) order, build the packed neighbour records
-//   k_lists_forces each block builds its clumps' contact item lists (neighbour walk, FP32
-//                  culling, exact overlap tests, boundary gates), then runs boundaries + sphere
-//                  contacts + bed + get_accel + finish_Verlet for them, gathering (never
-//                  scattering) contributions: no atomics on forces
+//   (near lists)   what may touch within the next steps             af3d_near.cu
+//   k_lists_forces each block takes its clumps' contact items from their near lists, then runs
+//                  boundaries + sphere contacts + bed + get_accel + finish_Verlet for them,
+//                  gathering (never scattering) contributions: no atomics on forces; and the next
+//                  step's predictor.  The sort, the permutation and the lists run every few
+//                  steps only: the other steps are this one kernel
 // The per-routine C-ABI entry points use k_boundary / k_part / k_get_accel / k_finish_verlet,
 // which apply the same device functions to the F, T planes one routine at a time.
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 #include "af3d_cellwalk.cuh"
 
@@ -121,17 +124,38 @@ __global__ void k_planes_to_aos(Planes P, const long long *__restrict__ id, cons
 
 __device__ __forceinline__ float f_up(double x) { return to_float_ru(x); }
 
-// Packed FP64 neighbour record and conservative FP32 culling record of one clump.
-// The culling bounds are formed in FP32 from the FP32-rounded coordinates.  M32 = max |coordinate|
-// in FP32 is within 2^-24 of the FP64 maximum M, so mu = 2^-22 * M32 * (1 + 2^-20) is at least
-// 4 x 2^-24 M: the FP32 difference of a coordinate of this clump and one of a partner is within
-// 2^-24 (M + M') (the two roundings) + 2^-24 |difference| of the exact one, so a distance formed
-// from FP32 coordinates errs by at most sqrt(3) 2^-24 (M + M') + 2^-24 d < mu + mu' + 2^-24 d,
-// and the last term is covered by the tests' relative slack (1 + 2^-18) on squared bounds.  The
-// sphere extent ext32 = max_k |s_k - r| from the FP32 coordinates is within 2 sqrt(3) 2^-24 M + a
-// few 2^-24 ext of the exact one, which the added 2 mu and the factor (1 + 2^-20) cover.
+// x in units of 2^-qs, truncated, modulo 2^32 (|x| below 2^50 units: make_records), from the bits
+// of the double: the 53-bit mantissa shifted into place.
+__device__ __forceinline__ int to_units(double x, int qs) {
+  const unsigned long long b = bits_of(x);
+  const int e = (int)((b >> 52) & 0x7FFull);
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 1ull << 52;   // (a subnormal shifts out anyway)
+  const int sh = 1075 - qs - e;
+  const unsigned v = sh > 63 ? 0u : (unsigned)(m >> max(sh, 0));
+  return (long long)b < 0 ? (int)(0u - v) : (int)v;
+}
+
+// |x| as a float, truncated, from the bits (0 below the float range, inf above it and for NaN).
+__device__ __forceinline__ float magnitude_f(double x) {
+  const unsigned long long b = bits_of(x);
+  const unsigned hi = (unsigned)(b >> 32) & 0x7FFFFFFFu, lo = (unsigned)b;
+  if (hi < 0x38100000u) return 0.0f;
+  if (hi >= 0x47F00000u) return __int_as_float(0x7F800000);
+  return __uint_as_float((hi - 0x38000000u) << 3 | lo >> 29);
+}
+
+// Packed FP64 neighbour record and conservative culling record of one clump.
+// The centre test's bound covers the FP32 rounding of the centres.  M32 = max |coordinate| in FP32
+// is within 2^-24 of the FP64 maximum M, so mu = 2^-22 * M32 * (1 + 2^-20) is at least 4 x 2^-24
+// M: the FP32 difference of a coordinate of this clump and one of a partner is within 2^-24 (M +
+// M') (the two roundings) + 2^-24 |difference| of the exact one, so a distance formed from FP32
+// coordinates errs by at most sqrt(3) 2^-24 (M + M') + 2^-24 d < mu + mu' + 2^-24 d, and the last
+// term is covered by the tests' relative slack (1 + 2^-18) on squared bounds.  The sphere extent
+// max_k |s_k - r| is formed in units: each difference of truncated coordinates is within 2 units
+// of the exact one, so the extent within 2 sqrt(3) and its FP32 rounding, which the 4 units and
+// the factor (1 + 2^-20) cover.
 __device__ __forceinline__ void make_records(V3 r, V3 v, V3 w, const V3 *sp, double rad, double msph,
-                                             double mwall, NbrRec &q, CullRec &c) {
+                                             double mwall, Margins m, int key, NbrRec &q, CullRec &c) {
   q.rx = r.x; q.ry = r.y; q.rz = r.z;
   q.vx = v.x; q.vy = v.y; q.vz = v.z;
   q.wx = w.x; q.wy = w.y; q.wz = w.z;
@@ -140,21 +164,61 @@ __device__ __forceinline__ void make_records(V3 r, V3 v, V3 w, const V3 *sp, dou
   }
   q.rad = rad; q.msph = msph; q.mwall = mwall;
   const float cx = to_float_rn(r.x), cy = to_float_rn(r.y), cz = to_float_rn(r.z);
-  float M = fmaxf(fmaxf(fabsf(cx), fabsf(cy)), fabsf(cz));
-  float ext = 0.0f;
-  float4 sf[4];
-  for (int k = 0; k < 4; k++) {
-    sf[k] = make_float4(to_float_rn(sp[k].x), to_float_rn(sp[k].y), to_float_rn(sp[k].z), 0.0f);
-    M = fmaxf(M, fmaxf(fmaxf(fabsf(sf[k].x), fabsf(sf[k].y)), fabsf(sf[k].z)));
-    const float dx = sf[k].x - cx, dy = sf[k].y - cy, dz = sf[k].z - cz;
-    ext = fmaxf(ext, sqrtf(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx))));
-  }
   const float radf = f_up(rad);
+  const int qi = m.qs;
+  const int ux = to_units(r.x, qi), uy = to_units(r.y, qi), uz = to_units(r.z, qi);
+  float ext2 = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int x = to_units(sp[k].x, qi), y = to_units(sp[k].y, qi), z = to_units(sp[k].z, qi);
+    const float dx = (float)(x - ux), dy = (float)(y - uy), dz = (float)(z - uz);
+    ext2 = fmaxf(ext2, __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)));
+    c.s[k].x = x; c.s[k].y = y; c.s[k].z = z;
+  }
+  const float unit = unit_power(-qi), units = unit_power(qi);
+  const float extu = sqrtf(ext2) * (1.0f + 9.5367431640625e-07f) + 4.0f;
+  float radu = radf * units * (1.0f + 9.5367431640625e-07f) + 2.0f;
+  float ext = extu * unit;
+  const float M = fmaxf(fmaxf(fabsf(cx), fabsf(cy)), fabsf(cz));
+  // A clump too large for the unit, or so far out that its coordinates do not fit the shifts: its
+  // extent from the FP32 coordinates, and an infinite radius in the sphere tests.
+  if (!(extu + radu <= kCullMaxUnits && (M + 4.0f * kCullMaxUnits * unit) * units <= 1.125899906842624e+15f)) {
+    float far2 = 0.0f, most = M;
+    for (int k = 0; k < 4; k++) {
+      const float x = to_float_rn(sp[k].x), y = to_float_rn(sp[k].y), z = to_float_rn(sp[k].z);
+      most = fmaxf(most, fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)));
+      const float dx = x - cx, dy = y - cy, dz = z - cz;
+      far2 = fmaxf(far2, __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)));
+    }
+    ext = sqrtf(far2) * (1.0f + 9.5367431640625e-07f) + most * 4.76837158203125e-07f;
+    radu = __int_as_float(0x7F800000);
+  }
   // 2^-22 * max|coordinate|: see above.
   const float mu = fmaxf(M, radf) * 2.384185791015625e-07f * (1.0f + 9.5367431640625e-07f) + 1e-30f;
-  const float sph = radf * (1.0f + 9.5367431640625e-07f) + mu;
-  c.c = make_float4(cx, cy, cz, (ext * (1.0f + 9.5367431640625e-07f) + 2.0f * mu) + sph);
-  for (int k = 0; k < 4; k++) c.s[k] = make_float4(sf[k].x, sf[k].y, sf[k].z, sph);
+  const float bound = (ext * (1.0f + 9.5367431640625e-07f) + 2.0f * mu) + (radf * (1.0f + 9.5367431640625e-07f) + mu);
+  c.c = make_float4(cx, cy, cz, bound);
+  for (int k = 0; k < 4; k++) c.s[k].w = __float_as_int(radu);
+  c.key = key;
+  // no sphere moves faster than |v| + |w| bound
+  const float vx = magnitude_f(v.x), vy = magnitude_f(v.y), vz = magnitude_f(v.z);
+  const float wx = magnitude_f(w.x), wy = magnitude_f(w.y), wz = magnitude_f(w.z);
+  const float speed = sqrtf(vx * vx + vy * vy + vz * vz) + sqrtf(wx * wx + wy * wy + wz * wz) * bound;
+  c.allow = fminf(m.per_speed * speed + m.floor, m.cap);   // cap for NaN
+  c.pad[0] = c.pad[1] = 0;
+}
+
+// How far the spheres of a clump moved between two of its records, at most, in cm.  Differences
+// of truncated coordinates: within 2 units each, covered by the 4 units; a step longer than 2^31
+// units leaves the grid.
+__device__ __forceinline__ float sphere_motion(const int4 *from, const CullRec &to, int qs) {
+  float d2 = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float dx = (float)(to.s[k].x - from[k].x), dy = (float)(to.s[k].y - from[k].y),
+                dz = (float)(to.s[k].z - from[k].z);
+    d2 = fmaxf(d2, __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)));
+  }
+  return (sqrtf(d2) * (1.0f + 9.5367431640625e-07f) + 4.0f) * unit_power(-qs);
 }
 
 constexpr int kPermBlock = 128;
@@ -390,16 +454,41 @@ __device__ __forceinline__ long bucket_key(V3 r, const DevFlume &fl, DevScalars 
   return fl.cell_off + i + g.ncell.x * (j + k * g.ncell.y);
 }
 
+// A clump's place in a step that keeps its near lists: counted in its cell for the capacity check
+// of cells.cu:96-102 (at most ntags - 1 clumps), and its motion since the previous step's record
+// (old) against its allowance.  With none left, the clumps that may now meet it unlisted -- all
+// within the 5 x 5 x 5 cells around it in the built order, as long as nothing has moved a cell
+// further than its allowance -- search for themselves from tick `from` on.
+__device__ __forceinline__ void keep_place(long s, const int4 *old, const CullRec &cr, const DevFlume &fl,
+                                           DevScalars *d, int *occ, long ntags, const NearLists &near,
+                                           const int *__restrict__ start, const int *__restrict__ order, Margins m,
+                                           int from) {
+  if (ntags > 0 && cr.key < d->ncell_total && atomicAdd(&occ[cr.key], 1) + 1 >= ntags)
+    raise_status(d, AF3D_ERR_CELL_CAPACITY);
+  const float rem = near.rem[s] - sphere_motion(old, cr, m.qs);
+  near.rem[s] = rem;
+  if (rem >= 0.0f) return;
+  const GridF &g = fl.gridf;
+  const float side = fminf(fminf(1.0f / g.ix, 1.0f / g.iy), 1.0f / g.iz);
+  CellAt c;
+  if (!(rem > m.cap - 0.9f * side)) atomicMin(&d->brute, from);   // (NaN too)
+  else if (cell_at(cr.key, fl.cell_off, g, c))
+    for_slots_around(c, g, fl.cell_off, start, order, [&](int t) { atomicMin(&near.loose[t], from); });
+  atomicMin(&near.loose[s], from);
+}
+
 // init_Verlet.cu:25-148 for one clump (PREDICT), and/or cell_locate's binning (cells.cu:60-92)
 // with the current time (KEYS): the bucket key, the bucket count and the clump's arrival rank.
 // Clumps that are not binned (removed, or non-finite) get the unique bucket ncell_total + id, so every
 // bucket holds its clumps in id order after the rank pass.  `t_prev`: init_Verlet's removal test
 // uses the time before the advance (the fused step advances time first).  RECORDS: also write
-// the clump's neighbour records at its own slot (steps that keep the slot order).
+// the clump's neighbour records at its own slot (steps that keep the slot order).  count_only: the
+// step does not sort but keeps its near lists (keep_place; with RECORDS).
 template <bool PREDICT, bool KEYS, bool RECORDS>
 __global__ void __launch_bounds__(kBlock) k_predict(Planes P, DevScalars *d, bool t_prev, Cells cells,
                                                     const long long *__restrict__ id,
-                                                    const int *__restrict__ flume, NbrRec *nbr,
+                                                    const int *__restrict__ flume, long ntags, NearLists near,
+                                                    const int *__restrict__ order, bool count_only, NbrRec *nbr,
                                                     CullRec *cull, long s0, long n) {
   __shared__ double s_nbr[RECORDS ? kPermBlock * kRecStride : 1];
   __shared__ CullRec s_cull[RECORDS ? kPermBlock : 1];
@@ -434,18 +523,24 @@ __global__ void __launch_bounds__(kBlock) k_predict(Planes P, DevScalars *d, boo
         have = true;
       }
     }
+    long key = 0;
+    if (KEYS) {
+      key = bucket_key(r, fl, d, id[s], d->time);
+      cells.key[s] = (int)key;
+      if (!(RECORDS && count_only)) cells.rank_tmp[s] = arrive_in_bucket(cells, key);
+    }
     if (RECORDS) {
       if (!have) {
         v = load3(P, VX, s);
         w = load3(P, WX, s);
         for (int k = 0; k < 4; k++) sp[k] = load3(P, S0X + 3 * k, s);
       }
-      make_records(r, v, w, sp, P.p[RAD][s], P.p[MSPH][s], P.p[MWALL][s], q, cr);
-    }
-    if (KEYS) {
-      const long key = bucket_key(r, fl, d, id[s], d->time);
-      cells.key[s] = (int)key;
-      cells.rank_tmp[s] = arrive_in_bucket(cells, key);
+      make_records(r, v, w, sp, P.p[RAD][s], P.p[MSPH][s], P.p[MWALL][s], P.m, (int)key, q, cr);
+      if (count_only) {
+        int4 old[4];
+        for (int k = 0; k < 4; k++) old[k] = cull[s].s[k];
+        keep_place(s, old, cr, fl, d, cells.occ, ntags, near, cells.start, order, P.m, d->tick);
+      }
     }
   }
   if (RECORDS) store_records<kPermBlock>(valid, base, n, q, cr, nbr, cull, s_nbr, s_cull);
@@ -457,6 +552,7 @@ __global__ void __launch_bounds__(kBlock) k_predict(Planes P, DevScalars *d, boo
 // `ft`: the fused step rewrites them before reading), plus the packed records of the new slot,
 // assembled in shared memory and written out as contiguous 16-byte stores.
 __global__ void __launch_bounds__(kPermBlock) k_permute(Planes src, Planes dst, const int *__restrict__ perm,
+                                                        const int *__restrict__ key,
                                                         const long long *__restrict__ id_src,
                                                         long long *id_dst, const int *__restrict__ fl_src,
                                                         int *fl_dst, NbrRec *nbr, CullRec *cull,
@@ -482,7 +578,7 @@ __global__ void __launch_bounds__(kPermBlock) k_permute(Planes src, Planes dst, 
     V3 sp[4];
     for (int k = 0; k < 4; k++) sp[k] = load3(dst, S0X + 3 * k, s);
     make_records(load3(dst, RX, s), load3(dst, VX, s), load3(dst, WX, s), sp, dst.p[RAD][s], dst.p[MSPH][s],
-                 dst.p[MWALL][s], q, cr);
+                 dst.p[MWALL][s], dst.m, perm ? key[perm[s]] : 0, q, cr);
   }
   store_records<kPermBlock>(s < n, base, n, q, cr, nbr, cull, s_nbr, s_cull);
 }
@@ -676,11 +772,82 @@ __device__ __forceinline__ Own own_from_planes(const Planes &P, long s) {
   return o;
 }
 
-// The contacts of a clump whose item lists overflowed, by the per-clump cell walk, added to
-// (F, T) in the reference's order: the boundary routines before the particles, the sixteen
-// sph_id passes, the routines after.  Not inlined: it runs rarely, and inlined its registers
-// and spills would weigh on the pooled path of every clump.  The clump's state, bound and
-// grid are read here again.
+// The next particle contact of clump s after the one of order key `done`, in the reference's order:
+// by sph_id, then the partner's cell in the 27-cell visiting order, then its id
+// (force_part.cu:88-106).  The candidates are the clumps of the 5 x 5 x 5 cells around it in the
+// built order (brute: every clump of its flume).  exact: overlapping pairs only, else those the
+// tests in units cannot rule out (the items of the lists).  Returns the key, ~0 after the last
+// pair; item: partner slot << 4 | sph_id - 1.
+__device__ __forceinline__ unsigned long long next_contact(long s, const DevScalars *d, const int *__restrict__ flume,
+                                                           const NbrRec *__restrict__ nbr,
+                                                           const CullRec *__restrict__ cull,
+                                                           const int *__restrict__ start,
+                                                           const int *__restrict__ order,
+                                                           const long long *__restrict__ id, bool brute, long n,
+                                                           bool exact, unsigned long long done, unsigned &item) {
+  const int f = flume[s];
+  const DevFlume &fl = d->flumes[f];
+  const GridF &g = fl.gridf;
+  const CullRec me = cull[s];
+  const NbrRec &mine = nbr[s];
+  const Search q = search_centre_f(me.c, mk(mine.rx, mine.ry, mine.rz), fl.grid, g, 0);
+  unsigned long long best = ~0ull;
+  auto look = [&](int t) {
+    if (t == s) return;
+    unsigned mask = pair_mask(me, cull[t]);
+    CellAt a;
+    if (!mask || !cell_at(cull[t].key, fl.cell_off, g, a)) return;
+    const long dx = a.x - q.ci + 1, dy = a.y - q.cj + 1, dz = a.z - q.ck + 1;
+    if (dx < 0 || dx > 2 || dy < 0 || dy > 2 || dz < 0 || dz > 2) return;
+    while (mask) {
+      const int p = __ffs(mask) - 1;
+      mask &= mask - 1u;
+      const unsigned long long key =
+          ((unsigned long long)(p * 27 + (int)(9 * dx + 3 * dy + dz)) << 32 | (unsigned long long)id[t]) + 1ull;
+      if (key <= done || key >= best) continue;
+      if (exact) {
+        V3 dd;
+        double dist2, sep;
+        const int k = p & 3;
+        if (!spheres_overlap(mk(mine.s[3 * k], mine.s[3 * k + 1], mine.s[3 * k + 2]), mine.rad, nbr[t], p >> 2, dd,
+                             dist2, sep))
+          continue;
+      }
+      best = key;
+      item = (unsigned)t << 4 | (unsigned)p;
+    }
+  };
+  CellAt at;
+  if (brute) {
+    for (long t = 0; t < n; t++)
+      if (flume[t] == f) look((int)t);
+  } else if (cell_at(me.key, fl.cell_off, g, at)) {
+    for_slots_around(at, g, fl.cell_off, start, order, look);
+  }
+  return best;
+}
+
+// The particle items of a clump whose near list does not hold (too many entries, or a clump around
+// it used up its allowance), found one after another: the items the list would have given.  To
+// the column `col` from entry `nitems` on; false if they would overflow it.  Not inlined: rare.
+__device__ __noinline__ bool search_items(long s, const DevScalars *d, const int *__restrict__ flume,
+                                          const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
+                                          const int *__restrict__ start, const int *__restrict__ order,
+                                          const long long *__restrict__ id, bool brute, long n, unsigned *col,
+                                          int &nitems) {
+  unsigned item = 0u;
+  for (unsigned long long done = 0ull;;) {
+    done = next_contact(s, d, flume, nbr, cull, start, order, id, brute, n, false, done, item);
+    if (done == ~0ull) return true;
+    if (nitems == kListCap) return false;
+    col[n * nitems++] = item;
+  }
+}
+
+// The contacts of a clump with more items than its list holds, added to (F, T) in the reference's
+// order: the boundary routines before the particles, the overlapping sphere pairs, the routines
+// after.  Not inlined: it runs rarely, and inlined its registers and spills would weigh on the
+// pooled path of every clump.  The clump's state, bound and grid are read here again.
 struct SlowSums {
   V3 F, T;
   int active;
@@ -688,14 +855,21 @@ struct SlowSums {
 __device__ __noinline__ SlowSums slow_contacts(long s, int pre0, int pre1, int post0, int post1, const Consts &c,
                                                const DevScalars *d, const int *__restrict__ flume,
                                                const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
-                                               const int *__restrict__ start, const int *__restrict__ order, V3 F,
-                                               V3 T) {
+                                               const int *__restrict__ start, const int *__restrict__ order,
+                                               const long long *__restrict__ id, bool brute, long n, V3 F, V3 T) {
   const Own o = own_from_record(nbr[s]);
   const double B = (double)cull[s].c.w;
-  const DevFlume &fl = d->flumes[flume[s]];
   for (int rt = pre0; rt <= pre1; rt++)
     if (bnd_may_touch(rt, o.r, B, c)) bnd_routine(rt, o, false, c, F, T);
-  const int active = contacts_by_pass(s, o, c, fl.grid, fl.cell_off, nbr, cull, start, order, 0xffffu, F, T);
+  const bool xi0 = c.variant == AF3D_FRICTION_DEV;
+  int active = 0;
+  unsigned item = 0u;
+  for (unsigned long long done = 0ull;;) {
+    done = next_contact(s, d, flume, nbr, cull, start, order, id, brute, n, true, done, item);
+    if (done == ~0ull) break;
+    const int p = (int)(item & 15u);
+    active += part_pair(o.r, o.v, o.w, o.s[p & 3], o.rad, o.msph, nbr[item >> 4], p >> 2, c, xi0, F, T) == 2;
+  }
   for (int rt = post0; rt <= post1; rt++)
     if (bnd_may_touch(rt, o.r, B, c)) bnd_routine(rt, o, false, c, F, T);
   return SlowSums{F, T, active};
@@ -718,8 +892,8 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
                                               const NbrRec *__restrict__ nbr,
                                               const CullRec *__restrict__ cull,
                                               const int *__restrict__ start,
-                                              const int *__restrict__ order,
-                                              const unsigned *items, int listed, ListCounts lc, long n,
+                                              const int *__restrict__ order, const long long *__restrict__ id,
+                                              bool brute, const unsigned *items, int listed, ListCounts lc, long n,
                                               V3 &F, V3 &T) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pre0 = aval ? R_HOP0 : 1, pre1 = aval ? R_WALLS : 0;         // fill: none before
@@ -756,7 +930,7 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
         const int k = p & 3;
         const V3 s1 = mk(me.s[3 * k], me.s[3 * k + 1], me.s[3 * k + 2]);
         kind = pair_input(rl, vl, wl, s1, me.rad, me.msph, nbr[t], p >> 2, co,
-                          co.variant == AF3D_FRICTION_DEV, ci, true) ? 1 : 0;
+                          co.variant == AF3D_FRICTION_DEV, ci) ? 1 : 0;
       }
       int r = kind == 1 ? 1 : 0;
       if (kind && apply_law(ci, rl, co, fs, tq)) r = kind == 1 ? 2 : 3;
@@ -823,7 +997,8 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
     __syncthreads();
   }
   if (slow) {
-    const SlowSums r = slow_contacts(s, pre0, pre1, post0, post1, c, d, flume, nbr, cull, start, order, F, T);
+    const SlowSums r = slow_contacts(s, pre0, pre1, post0, post1, c, d, flume, nbr, cull, start, order, id, brute, n,
+                                     F, T);
     F = r.F;
     T = r.T;
     active += r.active;
@@ -837,37 +1012,133 @@ __device__ __forceinline__ void warp_count(DevScalars *d, int active) {
   if ((threadIdx.x & 31) == 0 && v) atomicAdd(&d->contacts, (unsigned long long)v);
 }
 
-// The list phase of k_lists_forces for one clump: its item lists (see block_contacts) into
-// `lists`; returns the item count (-1: the lists overflowed) and their layout in lc.
-template <bool UNIFORM>
+// Candidate pairs of one warp's clumps in shared memory, one column per lane: (sph_id - 1) * 32 +
+// cell place << 6 | entry of the near list.
+struct PassLists {
+  unsigned short cand[kListCap][32];
+};
+static_assert(kNearCap <= 64, "candidates hold 6 bits of entry");
+
+// Boundary items of the routine and sphere bits `bits` for one clump, appended to the lane's item
+// column; false if the list would overflow.  The FP32 gates admit every sphere the routine can
+// touch (and a few more, which the exact test of the force pass then rejects).
+__device__ __forceinline__ bool push_boundary(unsigned bits, const NbrRec &me, float rad, const Consts &c,
+                                              bool door_closed, unsigned *col, long stride, int &nitems) {
+#pragma unroll 1
+  while (bits) {
+    const unsigned b = (unsigned)__ffs(bits) - 1u;
+    bits &= bits - 1u;
+    const int ns = (int)(b & 3u);
+    const float4 p = make_float4(to_float_rn(me.s[3 * ns]), to_float_rn(me.s[3 * ns + 1]),
+                                 to_float_rn(me.s[3 * ns + 2]), 0.0f);
+    if (rad < kCullMaxUnits && !bnd_may_touch_f((int)(b >> 2), p, rad, c, door_closed)) continue;
+    if (nitems == kListCap) return false;
+    col[stride * nitems++] = kBndItem | b;
+  }
+  return true;
+}
+
+// The list phase of k_lists_forces for one clump: its item list (see block_contacts) from its near
+// list, in the reference's order, into `lists`; returns the item count (-1: more than the list
+// holds, see slow_contacts) and their layout in lc.  A list that does not hold is replaced by a
+// search that gives the same items.  overflow: the clump's list or items were too many.  Four entries a turn are loaded and tested
+// together; the few pairs within a few units of overlap are put in order by the current cells
+// (the entries are in id order, so equal places stay so).  The exact test is the force pass's.
 __device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, const int *__restrict__ flume,
-                                           const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
-                                           const int *__restrict__ start, const int *__restrict__ order,
-                                           const float4 *__restrict__ csort, ContactLists lists, long s0,
-                                           long n, PassLists &pl, ListCounts &lc) {
+                                          const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
+                                          const int *__restrict__ start, const int *__restrict__ order,
+                                          const long long *__restrict__ id, const NearLists &near,
+                                          ContactLists lists, long s0, long n, Margins m, PassLists &pl,
+                                          ListCounts &lc, bool &brute, bool &overflow) {
+  const int lane = threadIdx.x & 31;
   const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const bool valid = s < n;
-  const long sv = valid ? s : n - 1;
-  const int f = flume[sv];
-  const DevFlume &fl = d->flumes[f];
-  const af3d_cell_par g = fl.grid;
-  const GridF gf = fl.gridf;
-  const long long off = fl.cell_off;
-  const NbrRec &me = nbr[sv];
-  const V3 r = mk(me.rx, me.ry, me.rz);
-  const bool act = valid && !is_removed(*c.tp, r.x, c.side_x);
-  bool slow = false;
-  const int k = build_item_lists(pl, lists.items + sv, n, s0 + blockIdx.x * (long)blockDim.x + (threadIdx.x & ~31u), sv,
-                                 act, c.phase == AF3D_PHASE_AVALANCHE, r, c, g, gf, off, nbr, cull, start, order,
-                                 csort, slow, lc);
-  return slow ? -1 : k;
+  lc.pre = lc.pair = 0;
+  brute = overflow = false;
+  if (s >= n) return 0;
+  const NbrRec &me = nbr[s];
+  if (is_removed(*c.tp, me.rx, c.side_x)) return 0;
+  const int tick = d->tick, info = near.info[s];
+  brute = d->brute <= tick;
+  const bool search = info < 0 || near.loose[s] <= tick || d->all_slow <= tick || brute;
+  overflow = info < 0;
+  const bool aval = c.phase == AF3D_PHASE_AVALANCHE;
+  const unsigned pre = aval ? 0x00FFFFFFu : 0u, post = aval ? 0x0F000000u : 0x00000FFFu;
+  const unsigned bnd = search ? 0x0FFFFFFFu : near.bnd[s];
+  const CullRec &rec = cull[s];
+  const float radu = __int_as_float(rec.s[0].w), rad = radu * unit_power(-m.qs);
+  const bool door_closed = *c.tp < 0.0;
+  unsigned *col = lists.items + s;
+  int nitems = 0;
+  if (!push_boundary(bnd & pre, me, rad, c, door_closed, col, n, nitems)) return -1;
+  const int npre = nitems;
+  if (search) {
+    if (!search_items(s, d, flume, nbr, cull, start, order, id, brute, n, col, nitems)) return -1;
+    lc.pair = nitems - npre;
+    if (!push_boundary(bnd & post, me, rad, c, door_closed, col, n, nitems)) return -1;
+    lc.pre = npre;
+    return nitems;
+  }
+  int ncand = 0;
+  bool have_cell = false;
+  int ci = 0, cj = 0, ck = 0;
+  const DevFlume &fl = d->flumes[flume[s]];
+  const unsigned *list = near.items + s;
+#pragma unroll 1
+  for (int e0 = 0; e0 < info; e0 += 4) {
+    unsigned it[4];
+    int4 a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) it[k] = e0 + k < info ? list[(long)(e0 + k) * n] : 0xFFFFFFFFu;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (it[k] != 0xFFFFFFFFu) {
+        a[k] = rec.s[it[k] & 3u];
+        b[k] = cull[it[k] >> 4].s[(it[k] >> 2) & 3u];
+      }
+    unsigned hit = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float r = radu + __int_as_float(b[k].w);
+      const float dx = unit_difference(b[k].x, a[k].x), dy = unit_difference(b[k].y, a[k].y),
+                  dz = unit_difference(b[k].z, a[k].z);
+      if (it[k] != 0xFFFFFFFFu &&
+          !(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r * r * (1.0f + 9.5367431640625e-07f)))
+        hit |= 1u << k;
+    }
+#pragma unroll 1
+    while (hit) {
+      const int k = __ffs(hit) - 1;
+      hit &= hit - 1u;
+      const unsigned item = k == 0 ? it[0] : k == 1 ? it[1] : k == 2 ? it[2] : it[3];
+      if (!have_cell) {
+        const Search q = search_centre_f(rec.c, mk(me.rx, me.ry, me.rz), fl.grid, fl.gridf, 0);
+        ci = (int)max(-3L, min(q.ci, (long)fl.gridf.nx + 2));
+        cj = (int)max(-3L, min(q.cj, (long)fl.gridf.ny + 2));
+        ck = (int)max(-3L, min(q.ck, (long)fl.gridf.nz + 2));
+        have_cell = true;
+      }
+      CellAt at;
+      if (!cell_at(cull[item >> 4].key, fl.cell_off, fl.gridf, at)) continue;   // not binned any more
+      const int dx = at.x - ci + 1, dy = at.y - cj + 1, dz = at.z - ck + 1;
+      if ((unsigned)dx > 2u || (unsigned)dy > 2u || (unsigned)dz > 2u) continue;   // not a neighbour cell
+      if (nitems + ncand == kListCap) return -1;
+      const unsigned code = (item & 15u) << 5 | (unsigned)(9 * dx + 3 * dy + dz);
+      int i = ncand++;
+      for (; i > 0 && (unsigned)(pl.cand[i - 1][lane] >> 6) > code; i--) pl.cand[i][lane] = pl.cand[i - 1][lane];
+      pl.cand[i][lane] = (unsigned short)(code << 6 | (unsigned)(e0 + k));
+    }
+  }
+#pragma unroll 1
+  for (int i = 0; i < ncand; i++) col[n * nitems++] = list[(long)(pl.cand[i][lane] & 63u) * n];
+  if (!push_boundary(bnd & post, me, rad, c, door_closed, col, n, nitems)) return -1;
+  lc.pre = npre;
+  lc.pair = ncand;
+  return nitems;
 }
 
 // Shared memory of the force kernel: the list phase, the force phase and the look-ahead's record
 // staging run one after another.  Kept small because the SM's L1 cache gets what the resident
-// blocks' shared memory leaves of 256 KB: at 96 threads and 6 blocks an SM, 20.3 KB per block
-// (the list phase's) leaves ~124 KB of L1 for the walk's, records' and spills' lines, where
-// 30.8 KB left 60 KB (0.275 -> 0.269 ms per pass on the 262,144-clump bed).
+// blocks' shared memory leaves of 256 KB.
 template <int NB>
 union ForceShared {
   PassLists pl[NB / 32];
@@ -877,13 +1148,23 @@ union ForceShared {
   } rec;
 };
 
+// sys_par.time += dt (avalanche_hst.cu:672), keeping the previous value for init_Verlet.  The
+// flumes of an ensemble share dt and the clock.
+__device__ __forceinline__ void advance_clock(DevScalars *d) {
+  d->time_prev = d->time;
+  d->time = d->time + d->flumes[0].sys.dt;
+  d->tick++;
+}
+
 template <int NB, bool WRITE_FT, bool UNIFORM>
 __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out, DevScalars *d,
                                            const int *__restrict__ flume, const NbrRec *__restrict__ nbr,
-                                           const CullRec *__restrict__ cull, const int *__restrict__ start,
-                                           const int *__restrict__ order, ContactLists lists, int listed,
-                                           ListCounts lc, long s0, long n, bool warm, const LookAhead &la,
-                                           ForceShared<NB> &sh) {
+                                           const CullRec *__restrict__ cull, const Cells &cells,
+                                           const int *__restrict__ order, const long long *__restrict__ id,
+                                           const NearLists &near, ContactLists lists, int listed, ListCounts lc,
+                                           bool brute, bool overflow, long ntags, bool counted, long s0, long n,
+                                           bool warm,
+                                           const LookAhead &la, ForceShared<NB> &sh) {
   const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
   const bool valid = s < n;
   const long sv = valid ? s : n - 1;   // in-range slot for lanes past n (nothing is written for them)
@@ -900,12 +1181,14 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
   }
   const long bbase = s0 + blockIdx.x * (long)blockDim.x;
   const int active = block_contacts<NB, UNIFORM>(sh.bq, bbase, sv, valid && !removed, aval, c, d, flume, nbr, cull,
-                                                 start, order, lists.items, valid ? listed : 0, lc, n, F, T);
+                                                 cells.start, order, id, brute, lists.items, valid ? listed : 0, lc,
+                                                 n, F, T);
   if (la.nbr) __syncthreads();   // the force phase's shared memory is free for the record staging
   if (valid) {
     if (lists.cnt) lists.cnt[s] = pack_list_counts(listed, lc.pre, lc.pair);
     if (lists.ovf && listed < 0) *lists.ovf = 1;
-    if (listed < 0) atomicAdd(&d->overflows, 1ull);   // rare: counted for the diagnostics
+    if (overflow) atomicAdd(&d->overflows, 1ull);   // rare: counted for the diagnostics
+    if (counted) cells.occ[cull[s].key] = 0;
     if (WRITE_FT) {
       store3(P, FX, s, F);
       store3(P, TX, s, T);
@@ -965,22 +1248,34 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
         store3(P, RN10, s, Ry);
         store3(P, RN20, s, Rz);
       }
+      const long key = bucket_key(rn, fl, d, id[s], t_next);
+      cells.key[s] = (int)key;
       {
         NbrRec q;
         CullRec cr;
-        make_records(rn, vn, wn, sp, P.p[RAD][s], P.p[MSPH][s], P.p[MWALL][s], q, cr);
+        make_records(rn, vn, wn, sp, P.p[RAD][s], P.p[MSPH][s], P.p[MWALL][s], P.m, (int)key, q, cr);
         stage_nbr_record(q, sh.rec.nbr);
         la.cull[s] = cr;   // stored directly: staged too, it would set the block's shared memory size
+        if (la.build) {
+          cells.rank_tmp[s] = arrive_in_bucket(cells, key);
+        } else {
+          int4 old[4];
+          for (int k = 0; k < 4; k++) old[k] = cull[s].s[k];
+          keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1);
+        }
       }
-      const long key = bucket_key(rn, fl, d, la.id[s], t_next);
-      la.cells.key[s] = (int)key;
-      la.cells.rank_tmp[s] = arrive_in_bucket(la.cells, key);
     }
   }
   warp_count(d, active);
   if (la.nbr) {
     __syncthreads();   // every neighbour record of the block is staged
     copy_nbr_records<NB>(bbase, n, la.nbr, sh.rec.nbr);
+    // The pass's last block advances the clock for the step it has looked ahead to: every block
+    // reads the time before its barrier above.
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicInc(&d->ticket, gridDim.x - 1) == gridDim.x - 1) advance_clock(d);
+    }
   }
 }
 
@@ -1054,12 +1349,7 @@ __global__ void k_clear_forces(Planes P, long n) {
   store3(P, TX, s, mk(0.0, 0.0, 0.0));
 }
 
-// sys_par.time += dt (avalanche_hst.cu:672), keeping the previous value for init_Verlet.  The
-// flumes of an ensemble share dt and the clock.
-__global__ void k_advance_time(DevScalars *d) {
-  d->time_prev = d->time;
-  d->time = d->time + d->flumes[0].sys.dt;
-}
+__global__ void k_advance_time(DevScalars *d) { advance_clock(d); }
 
 // ------------------------------------------------------------------ re-grid (cell_dim)
 
@@ -1252,119 +1542,97 @@ namespace fast {
 #endif
 
 void launch_predict(const Launch &L, Planes cur, DevScalars *d, bool predict, bool keys, bool t_prev,
-                    Cells cells, const long long *id, const int *flume, NbrRec *nbr, CullRec *cull, long s0,
-                    long count) {
+                    Cells cells, const long long *id, const int *flume, long ntags, NearLists near, const int *order,
+                    bool count_only, NbrRec *nbr, CullRec *cull, long s0, long count) {
   // slots [s0, s0 + count) of L.n (count < 0: to the end); s0 a multiple of kBlock
   const long m = count < 0 ? L.n - s0 : std::min(count, L.n - s0);
   if (L.n <= 0 || m <= 0 || s0 % kBlock != 0) return;
   const unsigned g = grid_for(m);
-  if (predict && keys && nbr)
-    k_predict<true, true, true><<<g, kBlock, 0, L.st>>>(cur, d, t_prev, cells, id, flume, nbr, cull, s0, L.n);
-  else if (predict && keys)
-    k_predict<true, true, false><<<g, kBlock, 0, L.st>>>(cur, d, t_prev, cells, id, flume, nbr, cull, s0, L.n);
-  else if (predict)
-    k_predict<true, false, false><<<g, kBlock, 0, L.st>>>(cur, d, t_prev, cells, id, flume, nbr, cull, s0, L.n);
-  else if (keys && nbr)
-    k_predict<false, true, true><<<g, kBlock, 0, L.st>>>(cur, d, t_prev, cells, id, flume, nbr, cull, s0, L.n);
-  else if (keys)
-    k_predict<false, true, false><<<g, kBlock, 0, L.st>>>(cur, d, t_prev, cells, id, flume, nbr, cull, s0, L.n);
+  auto run = [&](auto kernel) {
+    kernel<<<g, kBlock, 0, L.st>>>(cur, d, t_prev, cells, id, flume, ntags, near, order, count_only, nbr, cull, s0,
+                                   L.n);
+  };
+  if (predict && keys && nbr) run(k_predict<true, true, true>);
+  else if (predict && keys) run(k_predict<true, true, false>);
+  else if (predict) run(k_predict<true, false, false>);
+  else if (keys && nbr) run(k_predict<false, true, true>);
+  else if (keys) run(k_predict<false, true, false>);
 }
 
-void launch_permute_records(const Launch &L, Planes src, Planes dst, const int *perm,
+void launch_permute_records(const Launch &L, Planes src, Planes dst, const int *perm, const int *key,
                             const long long *id_src, long long *id_dst, const int *fl_src, int *fl_dst,
                             NbrRec *nbr, CullRec *cull, bool ft) {
   if (L.n <= 0) return;
-  k_permute<<<grid_for(L.n, kPermBlock), kPermBlock, 0, L.st>>>(src, dst, perm, id_src, id_dst, fl_src,
-                                                                fl_dst, nbr, cull, ft, L.n);
+  k_permute<<<grid_for(L.n, kPermBlock), kPermBlock, 0, L.st>>>(src, dst, perm, key, id_src, id_dst, fl_src, fl_dst,
+                                                                nbr, cull, ft, L.n);
 }
 
 void launch_build_records(const Launch &L, Planes cur, NbrRec *nbr, CullRec *cull) {
   if (L.n <= 0) return;
-  k_permute<<<grid_for(L.n, kPermBlock), kPermBlock, 0, L.st>>>(cur, cur, nullptr, nullptr, nullptr,
-                                                                nullptr, nullptr, nbr, cull, true, L.n);
+  k_permute<<<grid_for(L.n, kPermBlock), kPermBlock, 0, L.st>>>(cur, cur, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                                                nullptr, nbr, cull, true, L.n);
 }
 
-// The lists and the force pass of one block's clumps in one launch: the block builds its clumps'
-// item lists (the list kernel's work), then processes them (the force kernel's work).  Blocks
-// resident on one SM are in different phases most of the time, so the latency-bound walk of
-// some overlaps the FP64-bound contact laws of others.  The lists pass through global memory
-// (the block's own entries, visible to its threads after the barrier).
+// The contact items and the force pass of one block's clumps in one launch: the block takes its
+// clumps' item lists from their near lists, then processes them.  The lists pass through global
+// memory (the block's own entries, visible to its threads after the barrier).
 template <int NB, int MINB, bool WRITE_FT, bool UNIFORM>
-__global__ void __launch_bounds__(NB, MINB) k_lists_forces(Planes P, Planes out, DevScalars *d,
-                                                         const int *__restrict__ flume,
-                                                         const NbrRec *__restrict__ nbr,
-                                                         const CullRec *__restrict__ cull,
-                                                         const int *__restrict__ start,
-                                                         const int *__restrict__ order,
-                                                         const float4 *__restrict__ csort, ContactLists lists,
-                                                         const __grid_constant__ Consts kc, bool warm,
-                                                         const __grid_constant__ LookAhead la, long s0, long n) {
+__global__ void __launch_bounds__(NB, MINB)
+    k_lists_forces(Planes P, Planes out, DevScalars *d, const int *__restrict__ flume, const NbrRec *__restrict__ nbr,
+                   const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
+                   const int *__restrict__ order, const long long *__restrict__ id,
+                   const __grid_constant__ NearLists near, ContactLists lists, long ntags, bool counted,
+                   const __grid_constant__ Consts kc, bool warm, const __grid_constant__ LookAhead la, long s0,
+                   long n) {
   __shared__ ForceShared<NB> sh;
   ListCounts lc;
-  if constexpr (UNIFORM) {
-    const int listed = lists_body<true>(kc, d, flume, nbr, cull, start, order, csort, lists, s0, n,
-                                        sh.pl[threadIdx.x >> 5], lc);
+  bool brute, overflow;
+  auto body = [&](const Consts &c) {
+    const int listed = lists_body(c, d, flume, nbr, cull, cells.start, order, id, near, lists, s0, n, P.m,
+                                  sh.pl[threadIdx.x >> 5], lc, brute, overflow);
+    overflow = overflow || listed < 0;
     __syncthreads();
-    fused_body<NB, WRITE_FT, true>(kc, P, out, d, flume, nbr, cull, start, order, lists, listed, lc, s0, n, warm, la,
-                               sh);
+    fused_body<NB, WRITE_FT, UNIFORM>(c, P, out, d, flume, nbr, cull, cells, order, id, near, lists, listed, lc, brute,
+                                      overflow, ntags, counted, s0, n, warm, la, sh);
+  };
+  if constexpr (UNIFORM) {
+    body(kc);
   } else {
     // the flume's constants read where they lie (a reference, not a register copy)
     const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const Consts &c = d->flumes[flume[s < n ? s : n - 1]].c;
-    const int listed = lists_body<false>(c, d, flume, nbr, cull, start, order, csort, lists, s0, n,
-                                         sh.pl[threadIdx.x >> 5], lc);
-    __syncthreads();
-    fused_body<NB, WRITE_FT, false>(c, P, out, d, flume, nbr, cull, start, order, lists, listed, lc, s0, n, warm, la,
-                                sh);
-  }
-}
-
-template <int NB, int MINB>
-void launch_lists_forces_shape(const Launch &L, Planes cur, Planes out, DevScalars *d, const int *flume,
-                               const NbrRec *nbr, const CullRec *cull, const int *start, const int *order,
-                               const float4 *csort, ContactLists lists, bool write_ft, const Consts *uniform,
-                               bool warm, LookAhead look, long s0, long m) {
-  const Consts kc = uniform ? *uniform : Consts{};
-  const unsigned g = grid_for(m, NB);
-  if (uniform) {
-    if (write_ft)
-      k_lists_forces<NB, MINB, true, true><<<g, NB, 0, L.st>>>(cur, out, d, flume, nbr, cull, start, order, csort,
-                                                              lists, kc, warm, look, s0, L.n);
-    else
-      k_lists_forces<NB, MINB, false, true><<<g, NB, 0, L.st>>>(cur, out, d, flume, nbr, cull, start, order, csort,
-                                                               lists, kc, warm, look, s0, L.n);
-  } else {
-    if (write_ft)
-      k_lists_forces<NB, MINB, true, false><<<g, NB, 0, L.st>>>(cur, out, d, flume, nbr, cull, start, order, csort,
-                                                               lists, kc, warm, look, s0, L.n);
-    else
-      k_lists_forces<NB, MINB, false, false><<<g, NB, 0, L.st>>>(cur, out, d, flume, nbr, cull, start, order, csort,
-                                                                lists, kc, warm, look, s0, L.n);
+    body(d->flumes[flume[s < n ? s : n - 1]].c);
   }
 }
 
 void launch_lists_forces(const Launch &L, Planes cur, Planes out, DevScalars *d, const int *flume,
-                         const NbrRec *nbr, const CullRec *cull, const int *start, const int *order,
-                         const float4 *csort, ContactLists lists, bool write_ft, const Consts *uniform, bool warm,
-                         LookAhead look, long s0, long count, int shape) {
+                         const NbrRec *nbr, const CullRec *cull, Cells cells, const int *order, const long long *id,
+                         NearLists near, ContactLists lists, long ntags, bool write_ft, bool counted,
+                         const Consts *uniform, bool warm, LookAhead look, long s0, long count, int shape) {
   // slots [s0, s0 + count) of L.n (count < 0: to the end); s0 a multiple of the shape's block,
   // so the launch's blocks are those of the whole pass
   const long m = count < 0 ? L.n - s0 : std::min(count, L.n - s0);
   if (L.n <= 0 || m <= 0 || shape < 0 || shape >= kForceShapes || s0 % kForceShapeBlock[shape] != 0) return;
   static_assert(kForceShapes == 4 && kForceShapeBlock[0] == 128 && kForceShapeBlock[1] == 96 &&
                     kForceShapeBlock[2] == 64 && kForceShapeBlock[3] == 192, "the instantiated shapes");
-  if (shape == 0)
-    launch_lists_forces_shape<128, kForceShapeMinb[0]>(L, cur, out, d, flume, nbr, cull, start, order, csort,
-                                                       lists, write_ft, uniform, warm, look, s0, m);
-  else if (shape == 1)
-    launch_lists_forces_shape<96, kForceShapeMinb[1]>(L, cur, out, d, flume, nbr, cull, start, order, csort,
-                                                      lists, write_ft, uniform, warm, look, s0, m);
-  else if (shape == 2)
-    launch_lists_forces_shape<64, kForceShapeMinb[2]>(L, cur, out, d, flume, nbr, cull, start, order, csort,
-                                                      lists, write_ft, uniform, warm, look, s0, m);
-  else
-    launch_lists_forces_shape<192, kForceShapeMinb[3]>(L, cur, out, d, flume, nbr, cull, start, order, csort,
-                                                       lists, write_ft, uniform, warm, look, s0, m);
+  const Consts kc = uniform ? *uniform : Consts{};
+  auto run = [&](auto kernel, int nb) {
+    kernel<<<grid_for(m, nb), nb, 0, L.st>>>(cur, out, d, flume, nbr, cull, cells, order, id, near, lists, ntags,
+                                             counted, kc, warm, look, s0, L.n);
+  };
+  auto shaped = [&](auto ft, auto uni) {
+    constexpr bool FT = decltype(ft)::value, UNI = decltype(uni)::value;
+    if (shape == 0) run(k_lists_forces<128, kForceShapeMinb[0], FT, UNI>, 128);
+    else if (shape == 1) run(k_lists_forces<96, kForceShapeMinb[1], FT, UNI>, 96);
+    else if (shape == 2) run(k_lists_forces<64, kForceShapeMinb[2], FT, UNI>, 64);
+    else run(k_lists_forces<192, kForceShapeMinb[3], FT, UNI>, 192);
+  };
+  if (uniform) {
+    if (write_ft) shaped(std::true_type{}, std::true_type{});
+    else shaped(std::false_type{}, std::true_type{});
+  } else {
+    if (write_ft) shaped(std::true_type{}, std::false_type{});
+    else shaped(std::false_type{}, std::false_type{});
+  }
 }
 
 void launch_boundary(const Launch &L, Planes cur, DevScalars *d, const int *flume, int routine) {

@@ -555,9 +555,9 @@ __device__ __forceinline__ bool bnd_may_touch_f(int routine, float4 p, float B, 
 // sphere sm of partner m: d = s2 - s1, dist2 = |d|^2 and sep = rad_1 + rad_2.  The reference
 // compares each partial sum of dist2 with sep^2; the partial sums never decrease (each adds a
 // square and rounding is monotone, fused or not), so the last comparison alone takes the same
-// decision, NaN included.  The list kernel and pair_input run this same function.
+// decision, NaN included.
 __device__ __forceinline__ bool spheres_overlap(const V3 &s1, double rad_1, const NbrRec &m, int sm, V3 &d,
-                                                double &dist2, double &sep, bool known = false) {
+                                                double &dist2, double &sep) {
   const double rad_2 = m.rad;
   sep = rad_1 + rad_2;
   const double sep2 = sep * sep;
@@ -567,16 +567,15 @@ __device__ __forceinline__ bool spheres_overlap(const V3 &s1, double rad_1, cons
   dist2 = d.x * d.x;
   dist2 = __dadd_rn(dist2, __dmul_rn(d.y, d.y));   // uncontracted in both modes
   dist2 = __dadd_rn(dist2, __dmul_rn(d.z, d.z));
-  return known || dist2 < sep2;   // known: an item of the lists, which this same test kept
+  return dist2 < sep2;
 }
 
-// listed: the pair is an item of the lists, whose overlap test (this one) it passed.
 __device__ __forceinline__ bool pair_input(const V3 &rrl, const V3 &vvl, const V3 &wwl, const V3 &s1,
                                            double rad_1, double massl, const NbrRec &m, int sm,
-                                           const Consts &c, bool xi0, ContactIn &ci, bool listed = false) {
+                                           const Consts &c, bool xi0, ContactIn &ci) {
   V3 d;
   double dist2, sep;
-  if (!spheres_overlap(s1, rad_1, m, sm, d, dist2, sep, listed)) return false;
+  if (!spheres_overlap(s1, rad_1, m, sm, d, dist2, sep)) return false;
   if (kFast) {   // 0.5 kappa 0.5 (m1 + m2) with kappa / 4 formed once per flume
     const double msum = m.msph + massl;
     ci.km = c.qk_pp * msum;
