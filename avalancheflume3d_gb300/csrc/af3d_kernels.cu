@@ -135,15 +135,6 @@ __device__ __forceinline__ int to_units(double x, int qs) {
   return (long long)b < 0 ? (int)(0u - v) : (int)v;
 }
 
-// |x| as a float, truncated, from the bits (0 below the float range, inf above it and for NaN).
-__device__ __forceinline__ float magnitude_f(double x) {
-  const unsigned long long b = bits_of(x);
-  const unsigned hi = (unsigned)(b >> 32) & 0x7FFFFFFFu, lo = (unsigned)b;
-  if (hi < 0x38100000u) return 0.0f;
-  if (hi >= 0x47F00000u) return __int_as_float(0x7F800000);
-  return __uint_as_float((hi - 0x38000000u) << 3 | lo >> 29);
-}
-
 // Packed FP64 neighbour record and conservative culling record of one clump.
 // The centre test's bound covers the FP32 rounding of the centres.  M32 = max |coordinate| in FP32
 // is within 2^-24 of the FP64 maximum M, so mu = 2^-22 * M32 * (1 + 2^-20) is at least 4 x 2^-24
@@ -284,6 +275,22 @@ __device__ __forceinline__ long bin_axis(double x, double xmin, double inv, long
   return i;
 }
 
+// The same from the FP32 rounding of x and the FP32 grid copies where that is certain (the
+// estimate of search_axis_f, which lies on the same side of every integer as the FP64 product).
+__device__ __forceinline__ long bin_axis_f(double x, float xminf, float invf, double xmin, double inv, long n) {
+  const float xf = to_float_rn(x);
+  const float q = (xf - xminf) * invf;
+  const float E = 4.76837158203125e-07f * ((fabsf(xf) + fabsf(xminf)) * invf + 3.0f * q);   // 2^-21 (...)
+  if (q > E && q < 4.0e6f) {
+    const float tq = truncf(q), fr = q - tq;
+    if (fr > E && fr < 1.0f - E) {
+      const long i = (long)(int)tq;
+      return i == n ? i - 1 : i;
+    }
+  }
+  return bin_axis(x, xmin, inv, n);
+}
+
 constexpr double kSmallAngle2 = 9.765625e-04;   // (2^-5)^2
 
 // sin t and cos t of a rotation angle t >= 0 with t2 = t^2 (rounded).  Below 2^-5 rad (a step of
@@ -349,7 +356,7 @@ __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, 
     } else {
       mag = sqrt_rn(mag2);
     }
-    if (mag > 0.0) {
+    if (positive_bits(mag)) {
       // Rodrigues rotation about dO/|dO| by |dO| (init_Verlet.cu:63-83)
       V3 u;
       double c, sn;
@@ -438,9 +445,10 @@ __device__ __forceinline__ long bucket_key(V3 r, const DevFlume &fl, DevScalars 
     raise_status(d, AF3D_ERR_NAN);
     return d->ncell_total + id;
   }
-  long i = bin_axis(r.x, g.rr_min.x, g.cs_inv.x, g.ncell.x);
-  long j = bin_axis(r.y, g.rr_min.y, g.cs_inv.y, g.ncell.y);
-  long k = bin_axis(r.z, g.rr_min.z, g.cs_inv.z, g.ncell.z);
+  const GridF &gf = fl.gridf;
+  long i = bin_axis_f(r.x, gf.xmin, gf.ix, g.rr_min.x, g.cs_inv.x, g.ncell.x);
+  long j = bin_axis_f(r.y, gf.ymin, gf.iy, g.rr_min.y, g.cs_inv.y, g.ncell.y);
+  long k = bin_axis_f(r.z, gf.zmin, gf.iz, g.rr_min.z, g.cs_inv.z, g.ncell.z);
   if (i < 0 || j < 0 || k < 0) {
     raise_status(d, AF3D_ERR_NEGATIVE_CELL);
     i = i < 0 ? 0 : i; j = j < 0 ? 0 : j; k = k < 0 ? 0 : k;

@@ -85,6 +85,42 @@ __device__ __forceinline__ bool in_open_range_bits(double x, double lo, double h
   return b - l - 1ull < (unsigned long long)__double_as_longlong(hi) - l - 1ull;
 }
 
+// x > 0.0 (false for NaN).
+__device__ __forceinline__ bool positive_bits(double x) {
+  return bits_of(x) - 1ull < 0x7FF0000000000000ull;
+}
+
+// x is NaN.
+__device__ __forceinline__ bool nan_bits(double x) {
+  return (bits_of(x) & 0x7FFFFFFFFFFFFFFFull) > 0x7FF0000000000000ull;
+}
+
+// a < b for b >= +0 or NaN and a not -0 (false when either is a positive NaN, as arithmetic makes).
+__device__ __forceinline__ bool less_bits(double a, double b) {
+  return (long long)bits_of(a) < (long long)bits_of(b) && bits_of(b) <= 0x7FF0000000000000ull;
+}
+
+// x > y for any two values (false for NaN).
+__device__ __forceinline__ bool greater_bits(double x, double y) {
+  auto key = [](double v) {   // order-preserving, both zeros alike
+    const long long b = (long long)bits_of(v);
+    return b < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)b) : b;
+  };
+  return key(x) > key(y) && !nan_bits(x) && !nan_bits(y);
+}
+
+// x as a float, truncated, from the bits (0 below the float range, inf above it and for NaN).
+__device__ __forceinline__ float magnitude_f(double x) {
+  const unsigned long long b = bits_of(x);
+  const unsigned hi = (unsigned)(b >> 32) & 0x7FFFFFFFu, lo = (unsigned)b;
+  if (hi < 0x38100000u) return 0.0f;
+  if (hi >= 0x47F00000u) return __int_as_float(0x7F800000);
+  return __uint_as_float((hi - 0x38000000u) << 3 | lo >> 29);
+}
+__device__ __forceinline__ float truncated_f(double x) {
+  return __uint_as_float(__float_as_uint(magnitude_f(x)) | ((unsigned)(bits_of(x) >> 32) & 0x80000000u));
+}
+
 // (float)x, round to nearest even: the top 23 mantissa bits, rounded on the 29 below.
 __device__ __forceinline__ float to_float_rn(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
@@ -128,7 +164,20 @@ __device__ __forceinline__ Consts load_consts(const DevScalars *d, int f) {
 
 // time > 0 && x > side.x (init_Verlet.cu:29, cells.cu:65, force_part.cu:47, ...)
 __device__ __forceinline__ bool is_removed(double time, double x, double side_x) {
-  return time > 0.0 && x > side_x;
+  return positive_bits(time) && greater_bits(x, side_x);
+}
+
+// Whether the tangential displacement xi = dt |v_t| of a contact is certainly cut to zero by the
+// gate cns_1 normal < |xi| of the law (normal > 0), decided in FP32 with a margin: |v_t| formed from
+// operands truncated to floats is within 2^-19 |dv| of the exact one.  The gate's threshold is
+// ~10^-12 of the normal force (force_part.cu:221), so it cuts nearly every moving contact's xi.
+__device__ __forceinline__ bool surely_gated(V3 dv, V3 n, double normal, double cns_1, double dt) {
+  const float x = truncated_f(dv.x), y = truncated_f(dv.y), z = truncated_f(dv.z);
+  const float nx = truncated_f(n.x), ny = truncated_f(n.y), nz = truncated_f(n.z);
+  const float vn = x * nx + y * ny + z * nz;
+  const float tx = x - vn * nx, ty = y - vn * ny, tz = z - vn * nz;
+  const float vt = sqrtf(tx * tx + ty * ty + tz * tz), v = sqrtf(x * x + y * y + z * z);
+  return magnitude_f(dt) * (vt - 4e-6f * v) > 1.001f * magnitude_f(cns_1) * magnitude_f(normal) + 1e-36f;
 }
 
 // Spring-dashpot normal force + Cundall-Strack tangential force with the Coulomb cap; the common
@@ -139,21 +188,26 @@ __device__ __forceinline__ bool contact_law_fast(V3 dvvc, V3 n, double comp, dou
                                                  double mass_t, double mu, double cns_1, double dt,
                                                  double inv_dt, bool xi0, bool gate, V3 &f) {
   const double vn = dvvc.x * n.x + dvvc.y * n.y + dvvc.z * n.z;
+  const double normal = km * comp + gm * (-vn);
+  const bool push = positive_bits(normal);
+  if (gate ? !push && !nan_bits(normal) : !push) return false;
+  f = mk(-normal * n.x, -normal * n.y, -normal * n.z);
+  const bool gated = surely_gated(dvvc, n, normal, cns_1, dt);
+  if (gated && !xi0) return true;   // no displacement, no Coulomb branch: the normal force alone
   const V3 vt = mk(dvvc.x - vn * n.x, dvvc.y - vn * n.y, dvvc.z - vn * n.z);
   const double vt2 = vt.x * vt.x + vt.y * vt.y + vt.z * vt.z;
   double inv_vt;                             // +inf for vt = 0: the tangential part is then skipped,
   const double vt_mag = sqrt_and_inverse(vt2, inv_vt);   // as in the exact law
-  // dvvc . vt / |vt| = |vt| up to the rounding of vt's orthogonality to n, which the exact law
-  // also rounds: the fast law takes |vt| itself
-  const double vt_sig = vt_mag;
-  const double normal = km * comp + gm * (-vn);
-  if (gate ? (normal <= 0.0) : !(normal > 0.0)) return false;
-  f = mk(-normal * n.x, -normal * n.y, -normal * n.z);
-  double xi = dt * vt_sig;
-  if (cns_1 * normal < fabs(xi)) xi = 0.0;
-  const double fsdt = 1.0e12 * mass_t * xi + 2.0e6 * mass_t * (xi * inv_dt);
-  if (vt_mag > 0.0) {
-    if (fabs(fsdt) > mu * normal || (xi0 && xi == 0.0)) {
+  double xi = 0.0, fsdt = 0.0;
+  if (!gated) {
+    // dvvc . vt / |vt| = |vt| up to the rounding of vt's orthogonality to n, which the exact law
+    // also rounds: the fast law takes |vt| itself
+    xi = dt * vt_mag;
+    if (less_bits(cns_1 * normal, fabs(xi))) xi = 0.0;
+    fsdt = 1.0e12 * mass_t * xi + 2.0e6 * mass_t * (xi * inv_dt);
+  }
+  if (positive_bits(vt_mag)) {
+    if (less_bits(mu * normal, fabs(fsdt)) || (xi0 && !nonzero_bits(xi))) {
       // af = 0.8 mu N / |vt|, t0 = m / af, af / (1 + (dt / t0)^2) = af m^2 / (m^2 + (dt af)^2)
       const double af = 0.8 * mu * normal * inv_vt;
       const double dta = dt * af;
@@ -175,33 +229,43 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
                                             double mass_t, double mu, double cns_1, double dt,
                                             bool xi0, bool gate, V3 &f) {
   double vn = dvvc.x * n.x + dvvc.y * n.y + dvvc.z * n.z;
+  double normal = km * comp + gm * (-vn);
+  const bool push = positive_bits(normal);
+  if (gate ? !push && !nan_bits(normal) : !push) return false;
+  f.x = -normal * n.x;
+  f.y = -normal * n.y;
+  f.z = -normal * n.z;
+  const bool gated = surely_gated(dvvc, n, normal, cns_1, dt);
+  if (gated && !xi0) {
+    // xi = 0 and no Coulomb branch: the law adds (0 vt_i) / |vt| to each component, which changes
+    // only a zero's sign, where n_i = 0 and so vt_i = dvvc_i: -0 + 0 = +0
+    if (!nonzero_bits(f.x) && positive_bits(dvvc.x)) f.x = 0.0;
+    if (!nonzero_bits(f.y) && positive_bits(dvvc.y)) f.y = 0.0;
+    if (!nonzero_bits(f.z) && positive_bits(dvvc.z)) f.z = 0.0;
+    return true;
+  }
   V3 vt;
   vt.x = dvvc.x - vn * n.x;
   vt.y = dvvc.y - vn * n.y;
   vt.z = dvvc.z - vn * n.z;
-  double vt_mag = sqrt_rn(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
+  const double vt_mag = sqrt_rn(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
   const Divisor vt_div = divisor_of(vt_mag);
-  V3 tv;
-  tv.x = div_by(vt.x, vt_div);
-  tv.y = div_by(vt.y, vt_div);
-  tv.z = div_by(vt.z, vt_div);
-  double vt_sig = dvvc.x * tv.x + dvvc.y * tv.y + dvvc.z * tv.z;
-  double normal = km * comp + gm * (-vn);
-  if (gate ? (normal <= 0.0) : !(normal > 0.0)) return false;
-  f.x = -normal * n.x;
-  f.y = -normal * n.y;
-  f.z = -normal * n.z;
-  double xi = dt * vt_sig;
-  if (cns_1 * normal < fabs(xi)) xi = 0.0;
-  double xi_dot = nonzero_bits(xi) ? div_rn(xi, dt) : xi;   // dt > 0
-  double fsdt = 1.0e12 * mass_t * xi + 2.0e6 * mass_t * xi_dot;
-  if (vt_mag > 0.0) {
+  double xi = 0.0, fsdt = 0.0;
+  if (!gated) {
+    const V3 tv = mk(div_by(vt.x, vt_div), div_by(vt.y, vt_div), div_by(vt.z, vt_div));
+    const double vt_sig = dvvc.x * tv.x + dvvc.y * tv.y + dvvc.z * tv.z;
+    xi = dt * vt_sig;
+    if (less_bits(cns_1 * normal, fabs(xi))) xi = 0.0;
+    const double xi_dot = nonzero_bits(xi) ? div_rn(xi, dt) : xi;   // dt > 0
+    fsdt = 1.0e12 * mass_t * xi + 2.0e6 * mass_t * xi_dot;
+  }
+  if (positive_bits(vt_mag)) {
     // Coulomb branch:  af = 0.8 mu N / |vt|; t0 = m / af; af /= 1 + (dt/t0)^2; f += af vt.
     // Otherwise:       f_i += fsdt vt_i / |vt| where vt_i != 0.
     // The two branches' first three divisions run as one sequence with per-lane operands, so
     // a warp whose lanes take different branches executes three divisions, not seven; every
     // lane still evaluates exactly its own branch's operations.
-    const bool coulomb = fabs(fsdt) > mu * normal || (xi0 && xi == 0.0);
+    const bool coulomb = less_bits(mu * normal, fabs(fsdt)) || (xi0 && !nonzero_bits(xi));
     const double q1 = div_by(coulomb ? 0.8 * mu * normal : fsdt * vt.x, vt_div);   // af  | f_x term
     const double q2 = div_rn(coulomb ? mass_t : fsdt * vt.y, coulomb ? q1 : vt_mag);   // t0 | f_y
     const double q3 = div_rn(coulomb ? dt : fsdt * vt.z, coulomb ? q2 : vt_mag);   // dt/t0 | f_z
@@ -567,7 +631,7 @@ __device__ __forceinline__ bool spheres_overlap(const V3 &s1, double rad_1, cons
   dist2 = d.x * d.x;
   dist2 = __dadd_rn(dist2, __dmul_rn(d.y, d.y));   // uncontracted in both modes
   dist2 = __dadd_rn(dist2, __dmul_rn(d.z, d.z));
-  return dist2 < sep2;
+  return less_bits(dist2, sep2);
 }
 
 __device__ __forceinline__ bool pair_input(const V3 &rrl, const V3 &vvl, const V3 &wwl, const V3 &s1,
@@ -662,8 +726,9 @@ __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 
     a.z = div_by(f.z, by) - adrag * v.z - kGRAV;
   }
   V3 wb, tb, ab;
-  if (kFast && I.x == I.y && I.y == I.z && I.x > 0.0 && isfinite(I.x) && isfinite(w.x) && isfinite(w.y) &&
-      isfinite(w.z)) {
+  const bool isotropic =
+      bits_of(I.x) == bits_of(I.y) && bits_of(I.y) == bits_of(I.z) && positive_bits(I.x) && finite_bits(I.x);
+  if (kFast && isotropic && finite_bits(w.x) && finite_bits(w.y) && finite_bits(w.z)) {
     // Fast mode, isotropic inertia: the Euler term C w_b x w_b is zero (C = 0), so the body-frame
     // spin is not formed; alpha = R (R^T T) / I.
     tb.x = t.x * Rx.x + t.y * Ry.x + t.z * Rz.x;
@@ -675,14 +740,43 @@ __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 
     al.z = ab.x * Rz.x + ab.y * Rz.y + ab.z * Rz.z;
     return;
   }
-  wb.x = w.x * Rx.x + w.y * Ry.x + w.z * Rz.x;
-  wb.y = w.x * Rx.y + w.y * Ry.y + w.z * Rz.y;
-  wb.z = w.x * Rx.z + w.y * Ry.z + w.z * Rz.z;
   tb.x = t.x * Rx.x + t.y * Ry.x + t.z * Rz.x;
   tb.y = t.x * Rx.y + t.y * Ry.y + t.z * Rz.y;
   tb.z = t.x * Rx.z + t.y * Ry.z + t.z * Rz.z;
-  if (I.x == I.y && I.y == I.z && isfinite(wb.x) && isfinite(wb.y) && isfinite(wb.z) && I.x > 0.0 &&
-      isfinite(I.x)) {
+  if (!kFast && isotropic) {
+    // Only the signs of the body-frame spin are needed, and only where a quotient is zero
+    // (a clump without contacts): taken in FP32 where they are certain.
+    const Divisor by = divisor_of(I.x);
+    ab = mk(div_by(tb.x, by), div_by(tb.y, by), div_by(tb.z, by));
+    const float wx = truncated_f(w.x), wy = truncated_f(w.y), wz = truncated_f(w.z);
+    const float r[9] = {truncated_f(Rx.x), truncated_f(Ry.x), truncated_f(Rz.x), truncated_f(Rx.y), truncated_f(Ry.y),
+                        truncated_f(Rz.y), truncated_f(Rx.z), truncated_f(Ry.z), truncated_f(Rz.z)};
+    bool sure = fabsf(wx) < 1e18f && fabsf(wy) < 1e18f && fabsf(wz) < 1e18f;   // and so wb is finite
+    float sb[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const float x = wx * r[3 * k], y = wy * r[3 * k + 1], z = wz * r[3 * k + 2];
+      sb[k] = x + y + z;
+      sure = sure && fabsf(r[3 * k]) < 4.0f && fabsf(r[3 * k + 1]) < 4.0f && fabsf(r[3 * k + 2]) < 4.0f &&
+             fabsf(sb[k]) > 1e-5f * (fabsf(x) + fabsf(y) + fabsf(z)) + 1e-30f;
+    }
+    if (sure) {
+      // (a zero plus a signed zero is -0 when both are)
+      auto plus_zero = [](double q, float a, float b) {
+        const unsigned long long z = (unsigned long long)((__float_as_uint(a) ^ __float_as_uint(b)) & 0x80000000u) << 32;
+        return nonzero_bits(q) ? q : of_bits(bits_of(q) & z);
+      };
+      ab = mk(plus_zero(ab.x, sb[1], sb[2]), plus_zero(ab.y, sb[2], sb[0]), plus_zero(ab.z, sb[0], sb[1]));
+      al.x = ab.x * Rx.x + ab.y * Rx.y + ab.z * Rx.z;
+      al.y = ab.x * Ry.x + ab.y * Ry.y + ab.z * Ry.z;
+      al.z = ab.x * Rz.x + ab.y * Rz.y + ab.z * Rz.z;
+      return;
+    }
+  }
+  wb.x = w.x * Rx.x + w.y * Ry.x + w.z * Rz.x;
+  wb.y = w.x * Rx.y + w.y * Ry.y + w.z * Rz.y;
+  wb.z = w.x * Rx.z + w.y * Ry.z + w.z * Rz.z;
+  if (isotropic && finite_bits(wb.x) && finite_bits(wb.y) && finite_bits(wb.z)) {
     if (kFast) {
       ab.x = tb.x * iI + signed_zero_product(wb.y, wb.z);
       ab.y = tb.y * iI + signed_zero_product(wb.z, wb.x);
