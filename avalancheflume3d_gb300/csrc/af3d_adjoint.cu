@@ -42,44 +42,53 @@ __device__ __forceinline__ bool contact_law_fwd_rev(const ContactIn &ci, double 
   // forward, as contact_law
   const V3 dv = ci.dvvc, n = ci.n;
   const double vn = dv.x * n.x + dv.y * n.y + dv.z * n.z;
-  V3 vt;
-  vt.x = dv.x - vn * n.x;
-  vt.y = dv.y - vn * n.y;
-  vt.z = dv.z - vn * n.z;
-  const double vt_mag = sqrt(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
-  V3 tv;
-  tv.x = vt.x / vt_mag;
-  tv.y = vt.y / vt_mag;
-  tv.z = vt.z / vt_mag;
-  const double vt_sig = dv.x * tv.x + dv.y * tv.y + dv.z * tv.z;
   const double normal = ci.km * ci.comp + ci.gm * (-vn);
-  if (ci.gate ? (normal <= 0.0) : !(normal > 0.0)) return false;
+  const bool push = positive_bits(normal);
+  if (ci.gate ? !push && !nan_bits(normal) : !push) return false;
   V3 f;
   f.x = -normal * n.x;
   f.y = -normal * n.y;
   f.z = -normal * n.z;
-  double xi = dt * vt_sig;
-  const bool zeroed = ci.cns * normal < fabs(xi);
-  if (zeroed) xi = 0.0;
-  const double xi_dot = xi / dt;
+  // a displacement that is surely cut and no Coulomb branch: the normal force alone
+  const bool gated = surely_gated(dv, n, normal, ci.cns, dt);
+  const bool plain = gated && !ci.xi0;
   const double m = ci.mass_t;
-  const double fsdt = 1.0e12 * m * xi + 2.0e6 * m * xi_dot;
-  const bool tang = vt_mag > 0.0;
-  const bool coul = tang && (fabs(fsdt) > ci.mu * normal || (ci.xi0 && xi == 0.0));
-  double q1 = 0.0, q3 = 0.0;
-  if (tang) {
-    q1 = (coul ? 0.8 * ci.mu * normal : fsdt * vt.x) / vt_mag;
-    const double q2 = (coul ? m : fsdt * vt.y) / (coul ? q1 : vt_mag);
-    q3 = (coul ? dt : fsdt * vt.z) / (coul ? q2 : vt_mag);
-    if (coul) {
-      const double af = q1 / (1.0 + q3 * q3);
-      f.x += af * vt.x;
-      f.y += af * vt.y;
-      f.z += af * vt.z;
-    } else {
-      if (vt.x != 0.0) f.x += q1;
-      if (vt.y != 0.0) f.y += q2;
-      if (vt.z != 0.0) f.z += q3;
+  V3 vt = mk(0.0, 0.0, 0.0), tv = vt;
+  double vt_mag = 0.0, fsdt = 0.0, ivt = 0.0, q1 = 0.0, q3 = 0.0;
+  bool zeroed = true, tang = false, coul = false;
+  if (!plain) {
+    vt.x = dv.x - vn * n.x;
+    vt.y = dv.y - vn * n.y;
+    vt.z = dv.z - vn * n.z;
+    vt_mag = sqrt_rn(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
+    const Divisor by = divisor_of(vt_mag);
+    tv = mk(div_by(vt.x, by), div_by(vt.y, by), div_by(vt.z, by));
+    double xi = 0.0;
+    if (!gated) {
+      const double vt_sig = dv.x * tv.x + dv.y * tv.y + dv.z * tv.z;
+      xi = dt * vt_sig;
+      zeroed = less_bits(ci.cns * normal, fabs(xi));
+      if (zeroed) xi = 0.0;
+      const double xi_dot = nonzero_bits(xi) ? div_rn(xi, dt) : xi;
+      fsdt = 1.0e12 * m * xi + 2.0e6 * m * xi_dot;
+    }
+    tang = positive_bits(vt_mag);
+    coul = tang && (less_bits(ci.mu * normal, fabs(fsdt)) || (ci.xi0 && !nonzero_bits(xi)));
+    if (tang) {
+      q1 = div_by(coul ? 0.8 * ci.mu * normal : fsdt * vt.x, by);
+      const double q2 = div_rn(coul ? m : fsdt * vt.y, coul ? q1 : vt_mag);
+      q3 = div_rn(coul ? dt : fsdt * vt.z, coul ? q2 : vt_mag);
+      if (coul) {
+        const double af = div_rn(q1, 1.0 + q3 * q3);
+        f.x += af * vt.x;
+        f.y += af * vt.y;
+        f.z += af * vt.z;
+      } else {
+        if (nonzero_bits(vt.x)) f.x += q1;
+        if (nonzero_bits(vt.y)) f.y += q2;
+        if (nonzero_bits(vt.z)) f.z += q3;
+      }
+      ivt = reciprocal(vt_mag);
     }
   }
   // reverse: F += f, T += e x f
@@ -90,11 +99,10 @@ __device__ __forceinline__ bool contact_law_fwd_rev(const ContactIn &ci, double 
   V3 dv_b = mk(0.0, 0.0, 0.0), vt_b = mk(0.0, 0.0, 0.0);
   double vtmag_b = 0.0, mu_b = 0.0;
   if (tang) {
-    const double ivt = 1.0 / vt_mag;
     if (coul) {
       // af = 0.8 mu N / |vt| (q1);  r = dt / (m / af) (q3);  f += af / (1 + r^2) vt
       const double af = q1, r = q3;
-      const double iden = 1.0 / (1.0 + r * r);
+      const double iden = reciprocal(1.0 + r * r);
       const double af2 = af * iden;
       const double af2_b = dot(fb, vt);
       vt_b = madd(af2, fb, vt_b);
@@ -106,9 +114,9 @@ __device__ __forceinline__ bool contact_law_fwd_rev(const ContactIn &ci, double 
       // f_i += fsdt vt_i / |vt| for every component with vt_i != 0
       const double g = fsdt * ivt;
       double g_b = 0.0;
-      if (vt.x != 0.0) { vt_b.x += g * fb.x; g_b += fb.x * vt.x; }
-      if (vt.y != 0.0) { vt_b.y += g * fb.y; g_b += fb.y * vt.y; }
-      if (vt.z != 0.0) { vt_b.z += g * fb.z; g_b += fb.z * vt.z; }
+      if (nonzero_bits(vt.x)) { vt_b.x += g * fb.x; g_b += fb.x * vt.x; }
+      if (nonzero_bits(vt.y)) { vt_b.y += g * fb.y; g_b += fb.y * vt.y; }
+      if (nonzero_bits(vt.z)) { vt_b.z += g * fb.z; g_b += fb.z * vt.z; }
       const double fsdt_b = g_b * ivt;
       vtmag_b -= g_b * g * ivt;
       if (!zeroed) {
@@ -189,7 +197,8 @@ __device__ __forceinline__ void pair_rev(V3 rl, V3 vl, V3 wl, V3 s1, double rad1
   const V3 sp = mk(m.s[3 * sm], m.s[3 * sm + 1], m.s[3 * sm + 2]);
   const V3 rm = mk(m.rx, m.ry, m.rz), wm = mk(m.wx, m.wy, m.wz);
   const V3 d = sp - s1;
-  const double dist = sqrt(d.x * d.x + d.y * d.y + d.z * d.z);
+  double idist;
+  sqrt_and_inverse(d.x * d.x + d.y * d.y + d.z * d.z, idist);
   const V3 n = ci.n;
   const V3 e_m = rrc - rm;
   const double meff = 0.5 * (m.msph + massl);
@@ -211,7 +220,7 @@ __device__ __forceinline__ void pair_rev(V3 rl, V3 vl, V3 wl, V3 s1, double rad1
   // rrc = s1 + rad1 n;  comp = sep - dist;  n = d / dist;  d = sp - s1
   V3 n_b = madd(rad1, rrc_b, lb.n);
   const double dist_b = -lb.comp;
-  const V3 d_b = madd(dist_b, n, (1.0 / dist) * madd(-dot(n, n_b), n, n_b));
+  const V3 d_b = madd(dist_b, n, idist * madd(-dot(n, n_b), n, n_b));
   ob.s += rrc_b;
   ob.s -= d_b;
   ps_b = d_b;
@@ -483,18 +492,20 @@ __device__ __forceinline__ void adj_head(long s, bool act, bool valid, int start
     ob.w = w2_b;
     // get_accel: a_f = F/m - adrag0 |v1| v1 - g z;  alpha_f = R1 (R1^T T) / I (isotropic I)
     const double m = P.p[MASS][s], I = P.p[IXX][s], adrag0 = P.p[ADRAG][s];
-    Fb = (1.0 / m) * af_b;
-    const double vmag = sqrt(dot(o.v, o.v));
-    if (vmag > 0.0) ob.v -= adrag0 * vmag * af_b + (adrag0 * dot(o.v, af_b) / vmag) * o.v;
+    Fb = reciprocal(m) * af_b;
+    const double vmag = sqrt_rn(dot(o.v, o.v));
+    if (positive_bits(vmag))
+      ob.v -= adrag0 * vmag * af_b + (adrag0 * dot(o.v, af_b) * reciprocal(vmag)) * o.v;
     const V3 Rx = ld3(P, R00, s), Ry = ld3(P, R10, s), Rz = ld3(P, R20, s);
     const V3 T = ld3(P, TX, s);
     const V3 tb = mk(T.x * Rx.x + T.y * Ry.x + T.z * Rz.x, T.x * Rx.y + T.y * Ry.y + T.z * Rz.y,
                      T.x * Rx.z + T.y * Ry.z + T.z * Rz.z);
-    const V3 ab = (1.0 / I) * tb;
+    const double iI = reciprocal(I);
+    const V3 ab = iI * tb;
     const V3 ab_b = mk(alf_b.x * Rx.x + alf_b.y * Ry.x + alf_b.z * Rz.x,
                        alf_b.x * Rx.y + alf_b.y * Ry.y + alf_b.z * Rz.y,
                        alf_b.x * Rx.z + alf_b.y * Ry.z + alf_b.z * Rz.z);
-    const V3 tb_b = (1.0 / I) * ab_b;
+    const V3 tb_b = iI * ab_b;
     Tb = mk(dot(Rx, tb_b), dot(Ry, tb_b), dot(Rz, tb_b));
     // R1 adjoint: alpha_i = sum_j R_ij ab_j and tb_j = sum_i R_ij T_i
     V3 RbX = ld3(in, ARM, s), RbY = ld3(in, ARM + 3, s), RbZ = ld3(in, ARM + 6, s);

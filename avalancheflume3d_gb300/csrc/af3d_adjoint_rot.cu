@@ -32,18 +32,18 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_predict(Planes P, Planes tape
   V3 r1_b = ld3(in, AR, s) + ld3(acc, CR, s);
   const V3 v1_b = ld3(acc, CV, s), w1_b = ld3(acc, CW, s);
   V3 Rb3[3] = {ld3(rb, 0, s), ld3(rb, 3, s), ld3(rb, 6, s)};
-  fold_spheres(acc, s, P.p[RAD][s] / kROOT2, r1_b, Rb3);
+  fold_spheres(acc, s, P.p[RAD][s] * (1.0 / kROOT2), r1_b, Rb3);
   double R1b[3][3];
   for (int i = 0; i < 3; i++) {
     R1b[i][0] = Rb3[i].x; R1b[i][1] = Rb3[i].y; R1b[i][2] = Rb3[i].z;
   }
   // forward re-evaluation of the rotation update
   const V3 dO = mk(dt * (w.x + hdt * al.x), dt * (w.y + hdt * al.y), dt * (w.z + hdt * al.z));
-  const double mag = sqrt(dO.x * dO.x + dO.y * dO.y + dO.z * dO.z);
+  const double mag = sqrt_rn(dO.x * dO.x + dO.y * dO.y + dO.z * dO.z);
   double dR[3][3];
   V3 u = mk(0.0, 0.0, 0.0);
   double c = 1.0, sn = 0.0, omc = 0.0;
-  const double imag = mag > 0.0 ? 1.0 / mag : 0.0;
+  const double imag = mag > 0.0 ? reciprocal(mag) : 0.0;
   if (mag > 0.0) {
     u = mk(dO.x * imag, dO.y * imag, dO.z * imag);
     if (mag < 0.03125) {
@@ -73,12 +73,12 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_predict(Planes P, Planes tape
   double T[3][3], nrm[3];
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++) T[i][j] = dR[i][0] * R[0][j] + dR[i][1] * R[1][j] + dR[i][2] * R[2][j];
-  for (int j = 0; j < 3; j++) nrm[j] = sqrt(T[0][j] * T[0][j] + T[1][j] * T[1][j] + T[2][j] * T[2][j]);
+  for (int j = 0; j < 3; j++) nrm[j] = sqrt_rn(T[0][j] * T[0][j] + T[1][j] * T[1][j] + T[2][j] * T[2][j]);
   // column normalisation R1_ij = T_ij / n_j (the derivative needs no bit-exact quotient: one
   // reciprocal per column)
   double Tb[3][3];
   for (int j = 0; j < 3; j++) {
-    const double in = 1.0 / nrm[j];
+    const double in = reciprocal(nrm[j]);
     double q[3], sj = 0.0;
     for (int i = 0; i < 3; i++) {
       q[i] = T[i][j] * in;
@@ -133,7 +133,7 @@ __global__ void k_adj_startup(Planes P, Planes in, Planes out, Planes acc, Plane
   if (s >= n) return;
   V3 r_b = ld3(in, AR, s) + ld3(acc, CR, s);
   V3 Rb3[3] = {ld3(rb, 0, s), ld3(rb, 3, s), ld3(rb, 6, s)};
-  fold_spheres(acc, s, P.p[RAD][s] / kROOT2, r_b, Rb3);
+  fold_spheres(acc, s, P.p[RAD][s] * (1.0 / kROOT2), r_b, Rb3);
   st3(out, AR, s, r_b);
   st3(out, AV, s, ld3(in, AV, s) + ld3(acc, CV, s));
   st3(out, AW, s, ld3(in, AW, s) + ld3(acc, CW, s));
