@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "af3d_cellwalk.cuh"
+#include "af3d_fixed.cuh"
 
 namespace af3d {
 
@@ -311,17 +312,19 @@ __device__ __forceinline__ void sincos_step(double t, double t2, double &sn, dou
   c = __fma_rn(-t2, __fma_rn(-t2, q, 0.5), 1.0);
 }
 
-// init_Verlet.cu:25-148 for one clump that is not removed: r, v, w and the rotation rows move
-// one step with a_i, alpha_i; sp receives the new sphere centres.
-__device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, V3 &Rx, V3 &Ry, V3 &Rz, V3 *sp,
-                                              double rad, double dt, double hdt) {
-  r.x += dt * (v.x + hdt * a.x);
-  r.y += dt * (v.y + hdt * a.y);
-  r.z += dt * (v.z + hdt * a.z);
-  v.x += dt * a.x;
-  v.y += dt * a.y;
-  v.z += dt * a.z;
-  V3 dO = mk(dt * (w.x + hdt * al.x), dt * (w.y + hdt * al.y), dt * (w.z + hdt * al.z));
+struct Rows {
+  V3 x, y, z;
+};
+
+// init_Verlet.cu:63-114: the rotation rows turned by the angle vector dO, columns renormalised.
+// In the fast mode the path of turns of 2^-10 rad and more and of unnormalised input (the others
+// run in fixed point, predict_state), not inlined there.
+#ifdef AF3D_FAST
+__device__ __noinline__
+#else
+__device__ __forceinline__
+#endif
+Rows turn_rows(V3 dO, V3 Rx, V3 Ry, V3 Rz) {
   const double mag2 = dO.x * dO.x + dO.y * dO.y + dO.z * dO.z;
   double mag, imag = 0.0;
   V3 dRx, dRy, dRz;
@@ -406,12 +409,11 @@ __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, 
     by = divisor_of(sqrt_rn(Tx.z * Tx.z + Ty.z * Ty.z + Tz.z * Tz.z));
     Rx.z = div_by(Tx.z, by); Ry.z = div_by(Ty.z, by); Rz.z = div_by(Tz.z, by);
   }
-  w.x += dt * al.x;
-  w.y += dt * al.y;
-  w.z += dt * al.z;
-  // sphere centres r + (radius/sqrt2) R (+-1,+-1,+-1) (init_Verlet.cu:130-142)
-  constexpr Divisor root2 = constant_divisor(kROOT2, 0x3FF6A09E667F3BCCull);
-  const double pos = kFast ? rad * (1.0 / kROOT2) : div_by(rad, root2);
+  return Rows{Rx, Ry, Rz};
+}
+
+// init_Verlet.cu:130-142: the sphere centres r + (radius/sqrt2) R (+-1,+-1,+-1).
+__device__ __forceinline__ void place_spheres(V3 r, V3 Rx, V3 Ry, V3 Rz, double pos, V3 *sp) {
   if (kFast) {
     // the four patterns (a + c, b - c, c - a, -(b + c)) with a = x + y, b = x - y, from the
     // two partial sums r0 + pos c and r0 - pos c: eight operations per row
@@ -434,6 +436,50 @@ __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, 
              r.z + pos * (-Rz.x - Rz.y + Rz.z));
   sp[3] = mk(r.x + pos * (-Rx.x + Rx.y - Rx.z), r.y + pos * (-Ry.x + Ry.y - Ry.z),
              r.z + pos * (-Rz.x + Rz.y - Rz.z));
+}
+
+// init_Verlet.cu:25-148 for one clump that is not removed: r, v, w and the rotation rows move
+// one step with a_i, alpha_i; sp receives the new sphere centres.  Fast mode: the rotation and the
+// spheres in fixed point (af3d_fixed.cuh), 18 FP64 instructions instead of 123: a step of
+// 262,144 clumps 198 -> 190 us, of 582,320 in 64 flumes 414 -> 398 us (2,048 clumps, where one warp
+// has an SM's sub-partition to itself and latency counts: 35.4 -> 37.3 us).
+__device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, V3 &Rx, V3 &Ry, V3 &Rz, V3 *sp,
+                                              double rad, double dt, double hdt, int qs) {
+  r.x += dt * (v.x + hdt * a.x);
+  r.y += dt * (v.y + hdt * a.y);
+  r.z += dt * (v.z + hdt * a.z);
+  v.x += dt * a.x;
+  v.y += dt * a.y;
+  v.z += dt * a.z;
+  const V3 dO = mk(dt * (w.x + hdt * al.x), dt * (w.y + hdt * al.y), dt * (w.z + hdt * al.z));
+  w.x += dt * al.x;
+  w.y += dt * al.y;
+  w.z += dt * al.z;
+  constexpr Divisor root2 = constant_divisor(kROOT2, 0x3FF6A09E667F3BCCull);
+  const double pos = kFast ? rad * (1.0 / kROOT2) : div_by(rad, root2);
+  if (kFast) {
+    const double angle[3] = {dO.x, dO.y, dO.z};
+    const double R[9] = {Rx.x, Rx.y, Rx.z, Ry.x, Ry.y, Ry.z, Rz.x, Rz.y, Rz.z};
+    long long turned[9];
+    if (rotate_fixed(angle, R, turned)) {
+      Rx = mk(double_of(turned[0], 62), double_of(turned[1], 62), double_of(turned[2], 62));
+      Ry = mk(double_of(turned[3], 62), double_of(turned[4], 62), double_of(turned[5], 62));
+      Rz = mk(double_of(turned[6], 62), double_of(turned[7], 62), double_of(turned[8], 62));
+      const double at[3] = {r.x, r.y, r.z};
+      double c[12];
+      if (spheres_fixed(turned, at, pos, qs + 38, c)) {
+        for (int k = 0; k < 4; k++) sp[k] = mk(c[3 * k], c[3 * k + 1], c[3 * k + 2]);
+        return;
+      }
+    } else {
+      const Rows t = turn_rows(dO, Rx, Ry, Rz);
+      Rx = t.x; Ry = t.y; Rz = t.z;
+    }
+  } else {
+    const Rows t = turn_rows(dO, Rx, Ry, Rz);
+    Rx = t.x; Ry = t.y; Rz = t.z;
+  }
+  place_spheres(r, Rx, Ry, Rz, pos, sp);
 }
 
 // cell_locate's bucket of a clump at r (cells.cu:60-92) at time t: the flume's cell offset + cell
@@ -520,7 +566,7 @@ __global__ void __launch_bounds__(kBlock) k_predict(Planes P, DevScalars *d, boo
         w = load3(P, WX, s);
         V3 Rx = load3(P, R00, s), Ry = load3(P, R10, s), Rz = load3(P, R20, s);
         predict_state(r, v, w, load3(P, AIX, s), load3(P, ALIX, s), Rx, Ry, Rz, sp, P.p[RAD][s], fl.sys.dt,
-                      fl.sys.hdt);
+                      fl.sys.hdt, P.m.qs);
         store3(P, RX, s, r);
         store3(P, VX, s, v);
         store3(P, WX, s, w);
@@ -707,22 +753,14 @@ struct BlockQueue {
   int base[NB + 1];   // exclusive prefix of the clumps' item counts
   int pbase[NB + 1];  // ... of their particle item counts (kind-sorted pass)
   int qbase[NB + 1];  // ... of their boundary item counts (kind-sorted pass)
-  int npre[NB];       // boundary items before the particle items, per clump
   int wsum[3][NB / 32];
   double res[6][kBatch];  // [component][item in the batch]
+  unsigned item[kBatch];        // the batch's items in the order they are processed
+  unsigned char owner[kBatch];  // ... their owners' threads
+  unsigned char place[kBatch];  // ... and places in the owners' lists
   unsigned char flag[kBatch];
 };
-
-// The thread whose range [base[t], base[t+1]) holds position j.
-template <int NB>
-__device__ __forceinline__ int block_owner_of(const int *base, int j) {
-  int lo = 0, hi = NB - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (base[mid] <= j) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
+static_assert(kBatch <= 256, "owners and places are bytes");
 
 // Block-wide exclusive prefixes of three per-thread counts (all threads call this).
 template <int NB>
@@ -837,17 +875,18 @@ __device__ __forceinline__ unsigned long long next_contact(long s, const DevScal
 
 // The particle items of a clump whose near list does not hold (too many entries, or a clump around
 // it used up its allowance), found one after another: the items the list would have given.  To
-// the column `col` from entry `nitems` on; false if they would overflow it.  Not inlined: rare.
-__device__ __noinline__ bool search_items(long s, const DevScalars *d, const int *__restrict__ flume,
+// the column `col` from entry `nitems` on; returns the entries then, -1 if they would overflow it.
+// Not inlined: rare.
+__device__ __noinline__ int search_items(long s, const DevScalars *d, const int *__restrict__ flume,
                                           const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
                                           const int *__restrict__ start, const int *__restrict__ order,
                                           const long long *__restrict__ id, bool brute, long n, unsigned *col,
-                                          int &nitems) {
+                                          int nitems) {
   unsigned item = 0u;
   for (unsigned long long done = 0ull;;) {
     done = next_contact(s, d, flume, nbr, cull, start, order, id, brute, n, false, done, item);
-    if (done == ~0ull) return true;
-    if (nitems == kListCap) return false;
+    if (done == ~0ull) return nitems;
+    if (nitems == kListCap) return -1;
     col[n * nitems++] = item;
   }
 }
@@ -883,12 +922,23 @@ __device__ __noinline__ SlowSums slow_contacts(long s, int pre0, int pre1, int p
   return SlowSums{F, T, active};
 }
 
-// A boundary item's contact, prepared for the law.  Not inlined: the seven routines' input code
-// inlined into the pooled item loop raised its register pressure enough to spill on every
-// clump's path (636 bytes of spill stores against 212), while boundary items are a minority of
-// the items.
-__device__ __noinline__ bool bnd_input_call(int rt, const Sph &q, const Consts &co, ContactIn &ci) {
-  return bnd_input(rt, q, co, ci);
+// A boundary item of owner record `me`: its force and torque terms into res (components `stride`
+// apart); 3 with a force, else 0.  Not inlined: the seven routines' inputs raise the register
+// pressure of whatever they are inlined into, and a round of items is of one kind.
+__device__ __noinline__ int bnd_contact(unsigned it, const NbrRec *me, const Consts &co, double *res, int stride) {
+  const int rt = (int)((it >> 2) & 7u), ns = (int)(it & 3u);
+  Sph q;
+  q.r = mk(me->rx, me->ry, me->rz);
+  q.v = mk(me->vx, me->vy, me->vz);
+  q.w = mk(me->wx, me->wy, me->wz);
+  q.s = mk(me->s[3 * ns], me->s[3 * ns + 1], me->s[3 * ns + 2]);
+  q.rad = me->rad;
+  q.mwall = me->mwall;
+  V3 fs, tq;
+  if (!bnd_sphere(rt, q, co, fs, tq)) return 0;
+  res[0] = fs.x; res[stride] = fs.y; res[2 * stride] = fs.z;
+  res[3 * stride] = tq.x; res[4 * stride] = tq.y; res[5 * stride] = tq.z;
+  return 3;
 }
 
 // UNIFORM: every clump of the launch belongs to one flume, whose constants `c` are (a
@@ -909,56 +959,35 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
   const bool slow = act && listed < 0;
   const int nitems = act && listed > 0 ? listed : 0;
   const int npair = nitems > 0 ? lc.pair : 0;
-  bq.npre[tid] = nitems > 0 ? lc.pre : 0;
   block_prefix3<NB>(bq, nitems, npair, nitems - npair);
   const int base = bq.base[tid], total = bq.base[NB];
   const int ptotal = bq.pbase[NB];
-  // One item: its contact into the batch's result slot jb.
-  auto process = [&](int lo, int idx, int jb) {
-    const unsigned it = items[(long)idx * n + bbase + lo];   // written in this launch
-    const NbrRec &me = nbr[bbase + lo];   // owners hold clumps, so bbase + lo < n
-    // Prepare the item's contact (type-specific, short), then run the contact law.
-    auto contact = [&](const Consts &co, V3 &fs, V3 &tq) -> int {
-      ContactIn ci;
-      V3 rl = mk(me.rx, me.ry, me.rz);
-      int kind;   // 0 nothing, 1 sphere pair, 2 wall
-      if (it >= kBndItem) {
-        const int rt = (int)((it >> 2) & 7u), ns = (int)(it & 3u);
-        Sph q;
-        q.r = rl;
-        q.v = mk(me.vx, me.vy, me.vz);
-        q.w = mk(me.wx, me.wy, me.wz);
-        q.s = mk(me.s[3 * ns], me.s[3 * ns + 1], me.s[3 * ns + 2]);
-        q.rad = me.rad;
-        q.mwall = me.mwall;
-        kind = bnd_input_call(rt, q, co, ci) ? 2 : 0;
-      } else {
-        const int t = (int)(it >> 4), p = (int)(it & 15u);
-        const V3 vl = mk(me.vx, me.vy, me.vz), wl = mk(me.wx, me.wy, me.wz);
-        const int k = p & 3;
-        const V3 s1 = mk(me.s[3 * k], me.s[3 * k + 1], me.s[3 * k + 2]);
-        kind = pair_input(rl, vl, wl, s1, me.rad, me.msph, nbr[t], p >> 2, co,
-                          co.variant == AF3D_FRICTION_DEV, ci) ? 1 : 0;
-      }
-      int r = kind == 1 ? 1 : 0;
-      if (kind && apply_law(ci, rl, co, fs, tq)) r = kind == 1 ? 2 : 3;
-      return r;
-    };
-    V3 fs, tq;
-    int r;
+  // One item: its contact into its owner's place of the batch.
+  auto constants_of = [&](long os) -> const Consts & {
     if constexpr (UNIFORM) {
-      r = contact(c, fs, tq);
-    } else {
-      // the owner's flume may differ from this thread's at a flume boundary of an ensemble
-      const int of = flume[bbase + lo];
-      const Consts &co = of == flume[s] ? c : d->flumes[of].c;
-      r = contact(co, fs, tq);
+      return c;
+    } else {   // the owner's flume may differ from this thread's at a flume boundary of an ensemble
+      const int of = flume[os];
+      return of == flume[s] ? c : d->flumes[of].c;
     }
-    bq.flag[jb] = (unsigned char)r;
-    if (r >= 2) {
+  };
+  auto pair = [&](unsigned it, long os, int jb) {
+    const NbrRec &me = nbr[os];
+    const Consts &co = constants_of(os);
+    const int t = (int)(it >> 4), p = (int)(it & 15u), k = p & 3;
+    const V3 rl = mk(me.rx, me.ry, me.rz);
+    ContactIn ci;
+    V3 fs, tq;
+    int r = 0;
+    if (pair_input(rl, mk(me.vx, me.vy, me.vz), mk(me.wx, me.wy, me.wz),
+                   mk(me.s[3 * k], me.s[3 * k + 1], me.s[3 * k + 2]), me.rad, me.msph, nbr[t], p >> 2, co,
+                   co.variant == AF3D_FRICTION_DEV, ci) &&
+        apply_law(ci, rl, co, fs, tq)) {
+      r = 2;
       bq.res[0][jb] = fs.x; bq.res[1][jb] = fs.y; bq.res[2][jb] = fs.z;
       bq.res[3][jb] = tq.x; bq.res[4][jb] = tq.y; bq.res[5][jb] = tq.z;
     }
+    bq.flag[jb] = (unsigned char)r;
   };
   int active = 0;
   // Owners add their items' terms in list order.
@@ -975,29 +1004,38 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
     }
   };
   // A block whose items fit one batch takes them in kind order: every particle item of the
-  // block, then every boundary item, 32 a round per warp, so that each round runs one input
-  // routine; results go to the items' places in the owners' lists.  Otherwise batches of kBatch
-  // items in the owners' order.
+  // block, then every boundary item, 32 a round, so that a round is of one kind and no lane is
+  // idle but in each kind's last round; results go to the items' places in the owners' lists.
+  // Otherwise batches of kBatch items in the owners' order, particle items then boundary items of
+  // each.  The owners first lay their items out in shared memory in that order.
+  constexpr int kWarps = NB / 32;
   const bool kind_order = total <= kBatch;
+  const int pb = bq.pbase[tid], qb = ptotal + bq.qbase[tid];
   for (int b0 = 0; b0 < total; b0 += kBatch) {
     const int bn = total - b0 < kBatch ? total - b0 : kBatch;
-    for (int r0 = warp * 32; r0 < bn; r0 += NB) {
-      const int i = r0 + lane;
-      if (i < bn) {
-        int lo, idx;
-        if (kind_order && i < ptotal) {
-          lo = block_owner_of<NB>(bq.pbase, i);
-          idx = bq.npre[lo] + (i - bq.pbase[lo]);
-        } else if (kind_order) {
-          const int ib = i - ptotal;
-          lo = block_owner_of<NB>(bq.qbase, ib);
-          const int b = ib - bq.qbase[lo], np = bq.npre[lo];
-          idx = b < np ? b : b + (bq.pbase[lo + 1] - bq.pbase[lo]);
-        } else {
-          lo = block_owner_of<NB>(bq.base, b0 + i);   // the thread whose list holds item b0 + i
-          idx = b0 + i - bq.base[lo];
-        }
-        process(lo, idx, kind_order ? bq.base[lo] + idx : i);
+    const int e0 = base > b0 ? 0 : b0 - base, e1 = nitems < b0 + bn - base ? nitems : b0 + bn - base;
+    for (int e = e0; e < e1; e++) {
+      const unsigned it = items[(long)e * n + s];
+      const int at = base + e - b0;
+      const int j = !kind_order ? at : it < kBndItem ? pb + (e - lc.pre) : qb + (e < lc.pre ? e : e - npair);
+      bq.item[j] = it;
+      bq.owner[j] = (unsigned char)tid;
+      bq.place[j] = (unsigned char)at;
+    }
+    __syncthreads();
+    const int np = kind_order ? ptotal : bn, q0 = kind_order ? ptotal : 0;
+    for (int i = tid; i < np; i += NB) {
+      const unsigned it = bq.item[i];
+      if (it < kBndItem) pair(it, bbase + bq.owner[i], bq.place[i]);
+    }
+    // the boundary rounds go to the warps after those that took the last particle rounds
+    const int w0 = (warp + kWarps - (np + 31) / 32 % kWarps) % kWarps;
+    for (int i = q0 + 32 * w0 + lane; i < bn; i += NB) {
+      const unsigned it = bq.item[i];
+      const int at = bq.place[i];
+      if (it >= kBndItem) {
+        const long os = bbase + bq.owner[i];
+        bq.flag[at] = (unsigned char)bnd_contact(it, nbr + os, constants_of(os), &bq.res[0][at], kBatch);
       }
     }
     __syncthreads();
@@ -1080,7 +1118,8 @@ __device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, 
   if (!push_boundary(bnd & pre, me, rad, c, door_closed, col, n, nitems)) return -1;
   const int npre = nitems;
   if (search) {
-    if (!search_items(s, d, flume, nbr, cull, start, order, id, brute, n, col, nitems)) return -1;
+    nitems = search_items(s, d, flume, nbr, cull, start, order, id, brute, n, col, nitems);
+    if (nitems < 0) return -1;
     lc.pair = nitems - npre;
     if (!push_boundary(bnd & post, me, rad, c, door_closed, col, n, nitems)) return -1;
     lc.pre = npre;
@@ -1251,7 +1290,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
         store3(P, RN10, s, Ry);
         store3(P, RN20, s, Rz);
       } else {
-        predict_state(rn, vn, wn, a, al, Rx, Ry, Rz, sp, P.p[RAD][s], fl.sys.dt, fl.sys.hdt);
+        predict_state(rn, vn, wn, a, al, Rx, Ry, Rz, sp, P.p[RAD][s], fl.sys.dt, fl.sys.hdt, P.m.qs);
         store3(P, RN00, s, Rx);
         store3(P, RN10, s, Ry);
         store3(P, RN20, s, Rz);
