@@ -41,7 +41,7 @@ UNITS = [
 ]
 HOST_UNITS = [("af3d_hostio.cpp", "af3d_hostio", ["-O2", "-ffp-contract=off"])]
 
-HEADERS = ["af3d_internal.h", "af3d_physics.cuh", "af3d_cellwalk.cuh", "af3d_adjoint.cuh", "af3d_intfp64.cuh", "af3d_fixed.cuh"]
+HEADERS = ["af3d_internal.h", "af3d_physics.cuh", "af3d_cellwalk.cuh", "af3d_adjoint.cuh", "af3d_intfp64.cuh", "af3d_fixed.cuh", "af3d_wide.cuh"]
 
 
 def _run(cmd: list[str]) -> str:

@@ -45,19 +45,18 @@ AF3D_HD double double_of(long long v, int q) {
   return of_bits(r | ((unsigned long long)v & 0x8000000000000000ull));
 }
 
-// The rotation rows R (row-major) turned by the angle vector w (|w| < 2^-10) and its columns
-// renormalised, in units of 2^-62, into out; false when the angle is larger or a column's squared
-// norm is further than 2^-29 from one (a state read from text), which the FP64 formulas take.
-// dR - 1 = -(1/2 - t/24) (t 1 - w w^T) + (1 - t/6 + t^2/120) [w]x, t = |w|^2 (Rodrigues' matrix by
-// its Maclaurin series; the first omitted terms are below 2^-62).  An exact rotation keeps the
-// columns' norms, so what is renormalised is the rounding left by the step before: R_ij - R_ij
-// (|R_j|^2 - 1) / 2.
-AF3D_HD bool rotate_fixed(const double *w, const double *R, long long *out) {
+// dR - 1 of a turn by the angle vector w, |w| < 2^-10, in Q72, each entry as 2^32 hi + lo with both
+// halves signed: -(1/2 - t/24) (t 1 - w w^T) + (1 - t/6 + t^2/120) [w]x, t = |w|^2 (Rodrigues'
+// matrix by its Maclaurin series; the first omitted terms are below 2^-62).
+struct Turn {
+  int hi[9], lo[9];
+};
+
+// False for a larger angle, which the FP64 formulas take.
+AF3D_HD bool turn_fixed(const double *w, Turn &turn) {
   bool small = true;
 #pragma unroll
   for (int i = 0; i < 3; i++) small = small && ((bits_of(w[i]) >> 52) & 0x7FFull) < 1013ull;   // |w_i| < 2^-10
-#pragma unroll
-  for (int i = 0; i < 9; i++) small = small && ((bits_of(R[i]) >> 52) & 0x7FFull) < 1024ull;   // |R_ij| < 2
   if (!small) return false;
   long long x[3];
 #pragma unroll
@@ -79,62 +78,95 @@ AF3D_HD bool rotate_fixed(const double *w, const double *R, long long *out) {
   for (int i = 0; i < 3; i++) s[i] = x[i] - ((x[i] >> 32) * (long long)t6 >> 20);
   const long long D[9] = {-(yy + zz), xy - s[2], xz + s[1], xy + s[2], -(xx + zz), yz - s[0],
                           xz - s[1], yz + s[0], -(xx + yy)};
-  // 64-bit values as 2^32 hi + lo with both halves signed
-  int dh[9], dl[9];
 #pragma unroll
   for (int i = 0; i < 9; i++) {
-    dh[i] = (int)((D[i] + 0x80000000ll) >> 32);
-    dl[i] = (int)D[i];
-  }
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    long long f[3];
-    int rh[3], rl[3];
-    long long norm = -(1ll << 60);   // |R_j|^2 - 1 in Q60
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      f[i] = fixed_of(R[3 * i + j], 62);
-      rh[i] = (int)((f[i] + 0x80000000ll) >> 32);
-      rl[i] = (int)f[i];
-      norm += mulhi_ll(f[i], f[i]);
-    }
-    if (norm >= 0x7FFFFFFFll || norm <= -0x7FFFFFFFll) return false;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      long long acc = 0;   // sum over k of D_ik R_kj in Q70
-      int low = 0;
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        acc += (long long)dh[3 * i + k] * rh[k];
-        low += mulhi_s(dh[3 * i + k], rl[k]) + mulhi_s(dl[3 * i + k], rh[k]);
-      }
-      out[3 * i + j] = f[i] + ((acc + low + 128) >> 8) - ((long long)rh[i] * (long long)(int)norm >> 29);
-    }
+    turn.hi[i] = (int)((D[i] + 0x80000000ll) >> 32);
+    turn.lo[i] = (int)D[i];
   }
   return true;
 }
 
-// The four sphere centres r + pos R (1,1,1), (1,-1,-1), (-1,-1,1), (-1,1,-1) (init_Verlet.cu:
-// 130-142) for R in units of 2^-62, rounded once; pos < 2^(60 - q).  The offsets are formed in
-// units of 2^-q and added to each coordinate in units 2^-8 of its last place or finer.  False when
-// r or pos does not fit.
-AF3D_HD bool spheres_fixed(const long long *R, const double *r, double pos, int q, double *s) {
+// Column j of the turned rotation, renormalised, in units of 2^-62, from the column R.  An exact
+// rotation keeps its norm, so what is renormalised is the rounding left by the step before: R_i -
+// R_i (|R|^2 - 1) / 2.  False when the squared norm is further than 2^-29 from one (a state read
+// from text), which the FP64 formulas take.
+AF3D_HD bool column_fixed(const Turn &turn, const double *R, long long *out) {
+  bool small = true;
+#pragma unroll
+  for (int i = 0; i < 3; i++) small = small && ((bits_of(R[i]) >> 52) & 0x7FFull) < 1024ull;   // |R_i| < 2
+  if (!small) return false;
+  long long f[3];
+  int rh[3], rl[3];
+  long long norm = -(1ll << 60);   // |R|^2 - 1 in Q60
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    f[i] = fixed_of(R[i], 62);
+    rh[i] = (int)((f[i] + 0x80000000ll) >> 32);
+    rl[i] = (int)f[i];
+    norm += mulhi_ll(f[i], f[i]);
+  }
+  if (norm >= 0x7FFFFFFFll || norm <= -0x7FFFFFFFll) return false;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    long long acc = 0;   // sum over k of D_ik R_k in Q70
+    int low = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      acc += (long long)turn.hi[3 * i + k] * rh[k];
+      low += mulhi_s(turn.hi[3 * i + k], rl[k]) + mulhi_s(turn.lo[3 * i + k], rh[k]);
+    }
+    out[i] = f[i] + ((acc + low + 128) >> 8) - ((long long)rh[i] * (long long)(int)norm >> 29);
+  }
+  return true;
+}
+
+// The rotation rows R (row-major) turned by w and renormalised, in units of 2^-62.
+AF3D_HD bool rotate_fixed(const double *w, const double *R, long long *out) {
+  Turn turn;
+  if (!turn_fixed(w, turn)) return false;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const double col[3] = {R[j], R[3 + j], R[6 + j]};
+    long long c[3];
+    if (!column_fixed(turn, col, c)) return false;
+#pragma unroll
+    for (int i = 0; i < 3; i++) out[3 * i + j] = c[i];
+  }
+  return true;
+}
+
+// Whether spheres_fixed takes a clump: pos < 2^(60 - q), and coordinates whose units fit.
+AF3D_HD bool spheres_fit(const double *r, double pos, int q) {
   bool fits = ((bits_of(pos) >> 52) & 0x7FFull) < (unsigned long long)(1023 + 60 - q);
 #pragma unroll
   for (int i = 0; i < 3; i++) fits = fits && ((bits_of(r[i]) >> 52) & 0x7FFull) < (unsigned long long)(1082 - q + 60);
-  if (!fits) return false;
+  return fits;
+}
+
+// One coordinate of the four sphere centres r + pos R (1,1,1), (1,-1,-1), (-1,-1,1), (-1,1,-1)
+// (init_Verlet.cu:130-142) from the row R in units of 2^-62, rounded once.  The offsets are formed
+// in units of 2^-q and added to r in units 2^-8 of its last place or finer.
+AF3D_HD void spheres_row_fixed(const long long *R, double r, double pos, int q, double *s) {
   const long long p = fixed_of(pos, q) << 2;   // mulhi(p, Q62) is in Q(q)
+  const int e = (int)((bits_of(r) >> 52) & 0x7FFull);
+  const int qi = q < 1082 - e ? q : 1082 - e, sh = q - qi;   // |r| and the sums below 2^62 units
+  const long long a = mulhi_ll(p, R[0] + R[1]), b = mulhi_ll(p, R[0] - R[1]), c = mulhi_ll(p, R[2]);
+  const long long o = fixed_of(r, qi);
+  s[0] = double_of(o + ((c + a) >> sh), qi);
+  s[1] = double_of(o + ((b - c) >> sh), qi);
+  s[2] = double_of(o + ((c - a) >> sh), qi);
+  s[3] = double_of(o - ((b + c) >> sh), qi);
+}
+
+// The four sphere centres (s[3 k + i]); false when r or pos does not fit.
+AF3D_HD bool spheres_fixed(const long long *R, const double *r, double pos, int q, double *s) {
+  if (!spheres_fit(r, pos, q)) return false;
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    const int e = (int)((bits_of(r[i]) >> 52) & 0x7FFull);
-    const int qi = q < 1082 - e ? q : 1082 - e, sh = q - qi;   // |r_i| and the sums below 2^62 units
-    const long long x = R[3 * i], y = R[3 * i + 1];
-    const long long a = mulhi_ll(p, x + y), b = mulhi_ll(p, x - y), c = mulhi_ll(p, R[3 * i + 2]);
-    const long long o = fixed_of(r[i], qi);
-    s[i] = double_of(o + ((c + a) >> sh), qi);
-    s[3 + i] = double_of(o + ((b - c) >> sh), qi);
-    s[6 + i] = double_of(o + ((c - a) >> sh), qi);
-    s[9 + i] = double_of(o - ((b + c) >> sh), qi);
+    double c[4];
+    spheres_row_fixed(R + 3 * i, r[i], pos, q, c);
+#pragma unroll
+    for (int k = 0; k < 4; k++) s[3 * k + i] = c[k];
   }
   return true;
 }

@@ -228,6 +228,13 @@ constexpr long kForceAlign = 384;
 static_assert(kForceAlign % 128 == 0 && kForceAlign % 96 == 0 && kForceAlign % 64 == 0 && kForceAlign % 192 == 0,
               "a multiple of every shape's block");
 
+// Up to this many clumps a force pass runs in blocks of 32 clumps on 128 threads whatever the shape
+// (af3d_wide.cuh).
+#ifndef AF3D_WIDE_CLUMPS
+#define AF3D_WIDE_CLUMPS 24576
+#endif
+constexpr long kWideClumps = AF3D_WIDE_CLUMPS;
+
 // Per-clump item lists of one force pass, from the list phase to the force phase of the force
 // kernel: entry e of slot s at items[e * n + s] (an item is a boundary (routine, sphere) or a
 // particle (partner slot, sph_id) contact).  With cnt, the pass also records each clump's list

@@ -412,30 +412,33 @@ Rows turn_rows(V3 dO, V3 Rx, V3 Ry, V3 Rz) {
   return Rows{Rx, Ry, Rz};
 }
 
-// init_Verlet.cu:130-142: the sphere centres r + (radius/sqrt2) R (+-1,+-1,+-1).
-__device__ __forceinline__ void place_spheres(V3 r, V3 Rx, V3 Ry, V3 Rz, double pos, V3 *sp) {
+// init_Verlet.cu:130-142: one coordinate of the sphere centres r + (radius/sqrt2) R (+-1,+-1,+-1)
+// from the rotation row R.
+__device__ __forceinline__ void place_row(double r0, V3 R, double pos, double *s) {
   if (kFast) {
     // the four patterns (a + c, b - c, c - a, -(b + c)) with a = x + y, b = x - y, from the
     // two partial sums r0 + pos c and r0 - pos c: eight operations per row
-    auto row = [&](double r0, const V3 &R, double &s0, double &s1, double &s2, double &s3) {
-      const double a = R.x + R.y, b = R.x - R.y;
-      const double up = r0 + pos * R.z, dn = r0 - pos * R.z;
-      s0 = up + pos * a;
-      s2 = up - pos * a;
-      s1 = dn + pos * b;
-      s3 = dn - pos * b;
-    };
-    row(r.x, Rx, sp[0].x, sp[1].x, sp[2].x, sp[3].x);
-    row(r.y, Ry, sp[0].y, sp[1].y, sp[2].y, sp[3].y);
-    row(r.z, Rz, sp[0].z, sp[1].z, sp[2].z, sp[3].z);
+    const double a = R.x + R.y, b = R.x - R.y;
+    const double up = r0 + pos * R.z, dn = r0 - pos * R.z;
+    s[0] = up + pos * a;
+    s[2] = up - pos * a;
+    s[1] = dn + pos * b;
+    s[3] = dn - pos * b;
     return;
   }
-  sp[0] = mk(r.x + pos * (Rx.x + Rx.y + Rx.z), r.y + pos * (Ry.x + Ry.y + Ry.z), r.z + pos * (Rz.x + Rz.y + Rz.z));
-  sp[1] = mk(r.x + pos * (Rx.x - Rx.y - Rx.z), r.y + pos * (Ry.x - Ry.y - Ry.z), r.z + pos * (Rz.x - Rz.y - Rz.z));
-  sp[2] = mk(r.x + pos * (-Rx.x - Rx.y + Rx.z), r.y + pos * (-Ry.x - Ry.y + Ry.z),
-             r.z + pos * (-Rz.x - Rz.y + Rz.z));
-  sp[3] = mk(r.x + pos * (-Rx.x + Rx.y - Rx.z), r.y + pos * (-Ry.x + Ry.y - Ry.z),
-             r.z + pos * (-Rz.x + Rz.y - Rz.z));
+  s[0] = r0 + pos * (R.x + R.y + R.z);
+  s[1] = r0 + pos * (R.x - R.y - R.z);
+  s[2] = r0 + pos * (-R.x - R.y + R.z);
+  s[3] = r0 + pos * (-R.x + R.y - R.z);
+}
+
+__device__ __forceinline__ void place_spheres(V3 r, V3 Rx, V3 Ry, V3 Rz, double pos, V3 *sp) {
+  double x[4], y[4], z[4];
+  place_row(r.x, Rx, pos, x);
+  place_row(r.y, Ry, pos, y);
+  place_row(r.z, Rz, pos, z);
+#pragma unroll
+  for (int k = 0; k < 4; k++) sp[k] = mk(x[k], y[k], z[k]);
 }
 
 // init_Verlet.cu:25-148 for one clump that is not removed: r, v, w and the rotation rows move
@@ -922,6 +925,16 @@ __device__ __noinline__ SlowSums slow_contacts(long s, int pre0, int pre1, int p
   return SlowSums{F, T, active};
 }
 
+// A removed clump's contacts: hop, funnel and fcorners only (walls, part and flume skip it).  B: its
+// sphere offsets + radius, rounded up.  Not inlined: rare.
+__device__ __noinline__ SlowSums removed_contacts(const NbrRec *me, double B, const Consts &c) {
+  const Own o = own_from_record(*me);
+  SlowSums r = {mk(0.0, 0.0, 0.0), mk(0.0, 0.0, 0.0), 0};
+  for (int rt = R_HOP0; rt <= R_FCORNERS; rt++)
+    if (bnd_may_touch(rt, o.r, B, c)) bnd_routine(rt, o, true, c, r.F, r.T);
+  return r;
+}
+
 // A boundary item of owner record `me`: its force and torque terms into res (components `stride`
 // apart); 3 with a force, else 0.  Not inlined: the seven routines' inputs raise the register
 // pressure of whatever they are inlined into, and a round of items is of one kind.
@@ -1065,11 +1078,11 @@ struct PassLists {
 };
 static_assert(kNearCap <= 64, "candidates hold 6 bits of entry");
 
-// Boundary items of the routine and sphere bits `bits` for one clump, appended to the lane's item
-// column; false if the list would overflow.  The FP32 gates admit every sphere the routine can
-// touch (and a few more, which the exact test of the force pass then rejects).
-__device__ __forceinline__ bool push_boundary(unsigned bits, const NbrRec &me, float rad, const Consts &c,
-                                              bool door_closed, unsigned *col, long stride, int &nitems) {
+// Of the routine and sphere bits `bits` of one clump, those whose FP32 gates admit the sphere:
+// every sphere the routine can touch (and a few more, which its exact test rejects).
+__device__ __forceinline__ unsigned touching(unsigned bits, const NbrRec &me, float rad, const Consts &c) {
+  const bool door_closed = *c.tp < 0.0;
+  unsigned out = 0u;
 #pragma unroll 1
   while (bits) {
     const unsigned b = (unsigned)__ffs(bits) - 1u;
@@ -1077,65 +1090,30 @@ __device__ __forceinline__ bool push_boundary(unsigned bits, const NbrRec &me, f
     const int ns = (int)(b & 3u);
     const float4 p = make_float4(to_float_rn(me.s[3 * ns]), to_float_rn(me.s[3 * ns + 1]),
                                  to_float_rn(me.s[3 * ns + 2]), 0.0f);
-    if (rad < kCullMaxUnits && !bnd_may_touch_f((int)(b >> 2), p, rad, c, door_closed)) continue;
-    if (nitems == kListCap) return false;
-    col[stride * nitems++] = kBndItem | b;
+    if (!(rad < kCullMaxUnits) || bnd_may_touch_f((int)(b >> 2), p, rad, c, door_closed)) out |= 1u << b;
   }
-  return true;
+  return out;
 }
 
-// The list phase of k_lists_forces for one clump: its item list (see block_contacts) from its near
-// list, in the reference's order, into `lists`; returns the item count (-1: more than the list
-// holds, see slow_contacts) and their layout in lc.  A list that does not hold is replaced by a
-// search that gives the same items.  overflow: the clump's list or items were too many.  Four entries a turn are loaded and tested
-// together; the few pairs within a few units of overlap are put in order by the current cells
-// (the entries are in id order, so equal places stay so).  The exact test is the force pass's.
-__device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, const int *__restrict__ flume,
-                                          const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
-                                          const int *__restrict__ start, const int *__restrict__ order,
-                                          const long long *__restrict__ id, const NearLists &near,
-                                          ContactLists lists, long s0, long n, Margins m, PassLists &pl,
-                                          ListCounts &lc, bool &brute, bool &overflow) {
+// The near-list pairs of clump s within a few units of overlap into its column of pl, in the
+// reference's order; returns their count, -1 for more than an item list holds.  Four entries a turn
+// are loaded and tested together; the few hits are put in order by the current cells (the
+// entries are in id order, so equal places stay so).  The exact test is the force pass's.
+__device__ __forceinline__ int near_pairs(long s, int entries, const DevFlume &fl, const NbrRec &me,
+                                          const CullRec *__restrict__ cull, const unsigned *list, long n,
+                                          PassLists &pl) {
   const int lane = threadIdx.x & 31;
-  const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
-  lc.pre = lc.pair = 0;
-  brute = overflow = false;
-  if (s >= n) return 0;
-  const NbrRec &me = nbr[s];
-  if (is_removed(*c.tp, me.rx, c.side_x)) return 0;
-  const int tick = d->tick, info = near.info[s];
-  brute = d->brute <= tick;
-  const bool search = info < 0 || near.loose[s] <= tick || d->all_slow <= tick || brute;
-  overflow = info < 0;
-  const bool aval = c.phase == AF3D_PHASE_AVALANCHE;
-  const unsigned pre = aval ? 0x00FFFFFFu : 0u, post = aval ? 0x0F000000u : 0x00000FFFu;
-  const unsigned bnd = search ? 0x0FFFFFFFu : near.bnd[s];
   const CullRec &rec = cull[s];
-  const float radu = __int_as_float(rec.s[0].w), rad = radu * unit_power(-m.qs);
-  const bool door_closed = *c.tp < 0.0;
-  unsigned *col = lists.items + s;
-  int nitems = 0;
-  if (!push_boundary(bnd & pre, me, rad, c, door_closed, col, n, nitems)) return -1;
-  const int npre = nitems;
-  if (search) {
-    nitems = search_items(s, d, flume, nbr, cull, start, order, id, brute, n, col, nitems);
-    if (nitems < 0) return -1;
-    lc.pair = nitems - npre;
-    if (!push_boundary(bnd & post, me, rad, c, door_closed, col, n, nitems)) return -1;
-    lc.pre = npre;
-    return nitems;
-  }
+  const float radu = __int_as_float(rec.s[0].w);
   int ncand = 0;
   bool have_cell = false;
   int ci = 0, cj = 0, ck = 0;
-  const DevFlume &fl = d->flumes[flume[s]];
-  const unsigned *list = near.items + s;
 #pragma unroll 1
-  for (int e0 = 0; e0 < info; e0 += 4) {
+  for (int e0 = 0; e0 < entries; e0 += 4) {
     unsigned it[4];
     int4 a[4], b[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) it[k] = e0 + k < info ? list[(long)(e0 + k) * n] : 0xFFFFFFFFu;
+    for (int k = 0; k < 4; k++) it[k] = e0 + k < entries ? list[(long)(e0 + k) * n] : 0xFFFFFFFFu;
 #pragma unroll
     for (int k = 0; k < 4; k++)
       if (it[k] != 0xFFFFFFFFu) {
@@ -1168,18 +1146,69 @@ __device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, 
       if (!cell_at(cull[item >> 4].key, fl.cell_off, fl.gridf, at)) continue;   // not binned any more
       const int dx = at.x - ci + 1, dy = at.y - cj + 1, dz = at.z - ck + 1;
       if ((unsigned)dx > 2u || (unsigned)dy > 2u || (unsigned)dz > 2u) continue;   // not a neighbour cell
-      if (nitems + ncand == kListCap) return -1;
+      if (ncand == kListCap) return -1;
       const unsigned code = (item & 15u) << 5 | (unsigned)(9 * dx + 3 * dy + dz);
       int i = ncand++;
       for (; i > 0 && (unsigned)(pl.cand[i - 1][lane] >> 6) > code; i--) pl.cand[i][lane] = pl.cand[i - 1][lane];
       pl.cand[i][lane] = (unsigned short)(code << 6 | (unsigned)(e0 + k));
     }
   }
+  return ncand;
+}
+
+// Boundary routines before and after the particles, as bits of NearLists::bnd.
+__device__ __forceinline__ unsigned bits_before(bool aval) { return aval ? 0x00FFFFFFu : 0u; }
+__device__ __forceinline__ unsigned bits_after(bool aval) { return aval ? 0x0F000000u : 0x00000FFFu; }
+
+// Whether clump s must search for its pairs because its near list does not hold.
+__device__ __forceinline__ bool must_search(long s, const DevScalars *d, const NearLists &near, int info, bool &brute) {
+  const int tick = d->tick;
+  brute = d->brute <= tick;
+  return info < 0 || near.loose[s] <= tick || d->all_slow <= tick || brute;
+}
+
+// The list phase of k_lists_forces for one clump: its item list (see block_contacts) from its near
+// list, in the reference's order, into `lists`; returns the item count (-1: more than the list
+// holds, see slow_contacts) and their layout in lc.  A list that does not hold is replaced by a
+// search that gives the same items.  overflow: the clump's list or items were too many.
+__device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, const int *__restrict__ flume,
+                                          const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
+                                          const int *__restrict__ start, const int *__restrict__ order,
+                                          const long long *__restrict__ id, const NearLists &near,
+                                          ContactLists lists, long s0, long n, Margins m, PassLists &pl,
+                                          ListCounts &lc, bool &brute, bool &overflow) {
+  const int lane = threadIdx.x & 31;
+  const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
+  lc.pre = lc.pair = 0;
+  brute = overflow = false;
+  if (s >= n) return 0;
+  const NbrRec &me = nbr[s];
+  if (is_removed(*c.tp, me.rx, c.side_x)) return 0;
+  const int info = near.info[s];
+  const bool search = must_search(s, d, near, info, brute);
+  overflow = info < 0;
+  const bool aval = c.phase == AF3D_PHASE_AVALANCHE;
+  const float rad = __int_as_float(cull[s].s[0].w) * unit_power(-m.qs);
+  unsigned *col = lists.items + s;
+  const unsigned bnd = touching(search ? 0x0FFFFFFFu : near.bnd[s], me, rad, c);
+  unsigned before = bnd & bits_before(aval), after = bnd & bits_after(aval);
+  const int npre = __popc(before);
+  int nitems = 0;
+  for (; before; before &= before - 1u) col[n * nitems++] = kBndItem | ((unsigned)__ffs(before) - 1u);
+  if (search) {
+    nitems = search_items(s, d, flume, nbr, cull, start, order, id, brute, n, col, nitems);
+    if (nitems < 0) return -1;
+  } else {
+    const unsigned *list = near.items + s;
+    const int np = near_pairs(s, info, d->flumes[flume[s]], me, cull, list, n, pl);
+    if (np < 0 || nitems + np > kListCap) return -1;
 #pragma unroll 1
-  for (int i = 0; i < ncand; i++) col[n * nitems++] = list[(long)(pl.cand[i][lane] & 63u) * n];
-  if (!push_boundary(bnd & post, me, rad, c, door_closed, col, n, nitems)) return -1;
+    for (int i = 0; i < np; i++) col[n * nitems++] = list[(long)(pl.cand[i][lane] & 63u) * n];
+  }
+  lc.pair = nitems - npre;
+  if (nitems + __popc(after) > kListCap) return -1;
+  for (; after; after &= after - 1u) col[n * nitems++] = kBndItem | ((unsigned)__ffs(after) - 1u);
   lc.pre = npre;
-  lc.pair = ncand;
   return nitems;
 }
 
@@ -1219,12 +1248,10 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
   const bool removed = is_removed(*c.tp, nbr[sv].rx, c.side_x);
   V3 F = mk(0.0, 0.0, 0.0), T = mk(0.0, 0.0, 0.0);
   const bool aval = c.phase == AF3D_PHASE_AVALANCHE;
-  // Removed clumps get hop, funnel and fcorners only (walls, part and flume skip them).
   if (valid && removed && aval) {
-    const Own o = own_from_record(nbr[sv]);
-    const double B = (double)cull[sv].c.w;   // sphere offsets + radius, rounded up
-    for (int rt = R_HOP0; rt <= R_FCORNERS; rt++)
-      if (bnd_may_touch(rt, o.r, B, c)) bnd_routine(rt, o, true, c, F, T);
+    const SlowSums r = removed_contacts(nbr + sv, (double)cull[sv].c.w, c);
+    F = r.F;
+    T = r.T;
   }
   const long bbase = s0 + blockIdx.x * (long)blockDim.x;
   const int active = block_contacts<NB, UNIFORM>(sh.bq, bbase, sv, valid && !removed, aval, c, d, flume, nbr, cull,
@@ -1651,6 +1678,8 @@ __global__ void __launch_bounds__(NB, MINB)
   }
 }
 
+#include "af3d_wide.cuh"
+
 void launch_lists_forces(const Launch &L, Planes cur, Planes out, DevScalars *d, const int *flume,
                          const NbrRec *nbr, const CullRec *cull, Cells cells, const int *order, const long long *id,
                          NearLists near, ContactLists lists, long ntags, bool write_ft, bool counted,
@@ -1662,6 +1691,15 @@ void launch_lists_forces(const Launch &L, Planes cur, Planes out, DevScalars *d,
   static_assert(kForceShapes == 4 && kForceShapeBlock[0] == 128 && kForceShapeBlock[1] == 96 &&
                     kForceShapeBlock[2] == 64 && kForceShapeBlock[3] == 192, "the instantiated shapes");
   const Consts kc = uniform ? *uniform : Consts{};
+  if (L.n <= kWideClumps) {
+    auto wide = [&](auto kernel) {
+      kernel<<<grid_for(m, kWide), kWideThreads, 0, L.st>>>(cur, out, d, flume, nbr, cull, cells, order, id, near, lists,
+                                                           ntags, write_ft, counted, kc, warm, look, s0, L.n);
+    };
+    if (uniform) wide(k_forces_wide<true>);
+    else wide(k_forces_wide<false>);
+    return;
+  }
   auto run = [&](auto kernel, int nb) {
     kernel<<<grid_for(m, nb), nb, 0, L.st>>>(cur, out, d, flume, nbr, cull, cells, order, id, near, lists, ntags,
                                              counted, kc, warm, look, s0, L.n);

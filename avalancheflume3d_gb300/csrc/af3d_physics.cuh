@@ -704,6 +704,12 @@ __device__ __forceinline__ double signed_zero_product(double a, double b) {
   return __longlong_as_double((long long)((sa ^ sb) & 0x8000000000000000ull));
 }
 
+// The sum of a quotient and a zero with the sign of a b: -0 when both are, else the quotient.
+__device__ __forceinline__ double plus_signed_zero(double q, float a, float b) {
+  const unsigned long long z = (unsigned long long)((__float_as_uint(a) ^ __float_as_uint(b)) & 0x80000000u) << 32;
+  return nonzero_bits(q) ? q : of_bits(bits_of(q) & z);
+}
+
 // get_accel.cu:21-75 for one clump; R rows Rx, Ry, Rz.  `adrag0` = DRAG*rad*rad/m (the same
 // expression, precomputed per clump).  For isotropic inertia (Ix == Iy == Iz, the reference's
 // clumps, calculate_particle_parameters.cu:33) the Euler coupling terms C*wb*wb are (+0*wb)*wb,
@@ -761,12 +767,8 @@ __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 
              fabsf(sb[k]) > 1e-5f * (fabsf(x) + fabsf(y) + fabsf(z)) + 1e-30f;
     }
     if (sure) {
-      // (a zero plus a signed zero is -0 when both are)
-      auto plus_zero = [](double q, float a, float b) {
-        const unsigned long long z = (unsigned long long)((__float_as_uint(a) ^ __float_as_uint(b)) & 0x80000000u) << 32;
-        return nonzero_bits(q) ? q : of_bits(bits_of(q) & z);
-      };
-      ab = mk(plus_zero(ab.x, sb[1], sb[2]), plus_zero(ab.y, sb[2], sb[0]), plus_zero(ab.z, sb[0], sb[1]));
+      ab = mk(plus_signed_zero(ab.x, sb[1], sb[2]), plus_signed_zero(ab.y, sb[2], sb[0]),
+              plus_signed_zero(ab.z, sb[0], sb[1]));
       al.x = ab.x * Rx.x + ab.y * Rx.y + ab.z * Rx.z;
       al.y = ab.x * Ry.x + ab.y * Ry.y + ab.z * Ry.z;
       al.z = ab.x * Rz.x + ab.y * Rz.y + ab.z * Rz.z;
