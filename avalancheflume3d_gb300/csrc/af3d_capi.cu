@@ -138,6 +138,7 @@ struct af3d_ctx {
   // in nbr/cull (records), the RN planes (rotation rows) and the cell keys; the planes still hold
   // the last step's corrected state.
   bool look = false;
+  bool taping = false;    // every step's state is read from the planes (the adjoint's tape)
   ContactLists lists{};   // the item lists of the current force pass
   NearLists near{};       // what may touch within the next steps
   long since_build = kBuildEvery;   // steps the near lists have served (kBuildEvery: build them anew)
@@ -372,7 +373,7 @@ void forces_for(af3d_ctx *c, bool write_ft, Planes out, bool warm = false, bool 
     uni = &kc;
   }
   LookAhead la{};
-  if (look) la = LookAhead{c->nbr_next, c->cull_next, next_builds};
+  if (look) la = LookAhead{c->nbr_next, c->cull_next, next_builds, look && !c->taping};
   auto run = c->fp_mode == AF3D_FP_FAST ? fast::launch_lists_forces : launch_lists_forces;
   run(c->L(), c->cur, out, c->d, c->fl_cur, c->nbr, c->cull, c->cells, c->built_order, c->id_cur, c->near, c->lists,
       c->ntags, write_ft, counted, uni, warm, la, s0, count, c->force_shape);
@@ -1761,6 +1762,11 @@ extern "C" af3d_status af3d_adjoint(af3d_ctx *c, long steps, long ckpt_every, do
     ~ModeBack() { c->fp_mode = m; }
   } mode_back{c, mode};
   drop_graphs(c);
+  c->taping = true;
+  struct TapingDone {
+    af3d_ctx *c;
+    ~TapingDone() { c->taping = false; }
+  } taping_done{c};
   AdjBuffers buf;
   Planes state0{}, fin{}, adjA{}, adjB{}, acc{}, rb{}, rnext{};
   cudaError_t e = buf.planes(kAdjPlanes + 12, n, state0);   // with the sphere centres

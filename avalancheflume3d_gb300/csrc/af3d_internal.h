@@ -229,9 +229,11 @@ static_assert(kForceAlign % 128 == 0 && kForceAlign % 96 == 0 && kForceAlign % 6
               "a multiple of every shape's block");
 
 // Up to this many clumps a force pass runs in blocks of 32 clumps on 128 threads whatever the shape
-// (af3d_wide.cuh).
+// (af3d_wide.cuh).  The line lies where its blocks fill the 152 SMs once (four an SM, 19,456 clumps);
+// us a step of a dense bed, wide against the shapes: 16,384 clumps fast 31 and 44, exact 42 and 58;
+// 20,000 45 and 46, 62 and 65; 24,576 50 and 48, 72 and 66.
 #ifndef AF3D_WIDE_CLUMPS
-#define AF3D_WIDE_CLUMPS 24576
+#define AF3D_WIDE_CLUMPS 20480
 #endif
 constexpr long kWideClumps = AF3D_WIDE_CLUMPS;
 
@@ -283,11 +285,14 @@ struct NearLists {
 // advanced at once, its records go to the next step's record buffers, its rotation rows to the
 // RN planes, and it is counted in the next step's buckets: for the sort (build: the next step
 // sorts and builds lists) or for the cells' capacity alone.  The pass's last block advances the
-// clock.  nbr == null: none.
+// clock.  The records carry r, v, w and the sphere centres from step to step and the RN planes the
+// rotation: a pass with `keep` stores 240 B per clump less (262,144 clumps: a step 171 -> 167 us, 582,320 in 64 flumes 358 -> 346).
+// nbr == null: none.
 struct LookAhead {
   NbrRec *nbr;
   CullRec *cull;
   bool build;
+  bool keep;   // the planes need not receive this step's state: the next step overwrites it
 };
 
 // Which force routines a boundary kernel applies, in the reference's call order.

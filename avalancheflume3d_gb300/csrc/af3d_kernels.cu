@@ -1274,7 +1274,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
     const V3 v = mk(me.vx, me.vy, me.vz), w = mk(me.wx, me.wy, me.wz);
     const int R0 = warm ? RN00 : R00;
     V3 Rx = load3(P, R0, s), Ry = load3(P, R0 + 3, s), Rz = load3(P, R0 + 6, s);
-    if (warm) {   // commit the predicted state to the planes
+    if (warm && !la.keep) {   // commit the predicted state to the planes
       store3(P, RX, s, r);
       for (int k = 0; k < 4; k++) store3(P, S0X + 3 * k, s, mk(me.s[3 * k], me.s[3 * k + 1], me.s[3 * k + 2]));
       store3(P, R00, s, Rx);
@@ -1301,8 +1301,10 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
       store3(P, AFX, s, a);
       store3(P, ALFX, s, al);
     }
-    store3(out, VX, s, v2);
-    store3(out, WX, s, w2);
+    if (!la.keep) {
+      store3(out, VX, s, v2);
+      store3(out, WX, s, w2);
+    }
     if (la.nbr) {
       // The next step's init_Verlet (removal test at this step's time, a_i = this a_f), cell key
       // (at the next step's time) and records, exactly as k_predict<1,1,1> would make them
@@ -1323,7 +1325,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
         store3(P, RN20, s, Rz);
       }
       const long key = bucket_key(rn, fl, d, id[s], t_next);
-      cells.key[s] = (int)key;
+      if (la.build) cells.key[s] = (int)key;
       {
         NbrRec q;
         CullRec cr;

@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
         P.p[FX + i][s] = Fi;
         P.p[TX + i][s] = Ti;
       }
-      if (warm) {   // commit the predicted state to the planes
+      if (warm && !la.keep) {   // commit the predicted state to the planes
         P.p[RX + i][s] = mr[i];
 #pragma unroll
         for (int k = 0; k < 4; k++) P.p[S0X + 3 * k + i][s] = me.s[3 * k + i];
@@ -288,8 +288,10 @@ __global__ void __launch_bounds__(kWideThreads, 4)
       }
       P.p[AFX + i][s] = ai;
       P.p[ALFX + i][s] = ali;
-      out.p[VX + i][s] = v2;
-      out.p[WX + i][s] = w2;
+      if (!la.keep) {
+        out.p[VX + i][s] = v2;
+        out.p[WX + i][s] = w2;
+      }
     }
     if (!la.nbr) return;
 
@@ -321,7 +323,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
     long key = 0;
     if (w == 3 && valid) {
       key = bucket_key(r1, fl, d, id[s], t_next);
-      cells.key[s] = (int)key;
+      if (la.build) cells.key[s] = (int)key;
       if (removed) P.p[RAD][s] = 0.0;
     }
     constexpr Divisor root2 = constant_divisor(kROOT2, 0x3FF6A09E667F3BCCull);
