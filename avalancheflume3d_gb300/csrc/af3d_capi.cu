@@ -352,8 +352,10 @@ void sort_for(af3d_ctx *c, bool with_centres) {
 }
 
 // The near lists from the sort just made (order: null when the slots were permuted into it).
-void build_lists(af3d_ctx *c, const int *order, long s0 = 0, long count = -1) {
-  launch_build_lists(c->L(), c->cur.m, c->d, c->fl_cur, c->cull, c->cells, order, c->id_cur, c->near, s0, count);
+void build_lists(af3d_ctx *c, cudaStream_t st, const int *order, long s0 = 0, long count = -1) {
+  Launch L = c->L();
+  L.st = st;
+  launch_build_lists(L, c->cur.m, c->d, c->fl_cur, c->cull, c->cells, order, c->id_cur, c->near, s0, count);
   c->launches++;
   c->built_order = order;
   c->since_build = 0;
@@ -423,10 +425,10 @@ void step_predict(af3d_ctx *c, const StepPlan &p) {
 void step_lists(af3d_ctx *c, const StepPlan &p) {
   if (p.resort) {
     enqueue_cell_build(c, true, true, false);   // F, T and a_f are rewritten before being read
-    build_lists(c, nullptr);
+    build_lists(c, c->st, nullptr);
   } else if (p.build) {
     sort_for(c, true);
-    build_lists(c, c->cells.perm);
+    build_lists(c, c->st, c->cells.perm);
   }
 }
 
@@ -862,13 +864,14 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
     if (!e) AF3D_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   // Part boundaries on whole blocks.  The first part to leave the device (force pass, then copy
   // out) and the last part to arrive (copy in, then conversion and predictor) are the ones
-  // whose work nothing overlaps, so they get half a part's share of the clumps and the others
-  // share the rest: `out_at` splits the export, `in_at` (the mirror image) the import.
+  // whose work nothing overlaps, so they get less than a part's share of the clumps (the first to
+  // leave enough that its copy lasts while the second part computes) and the others share the
+  // rest: `out_at` splits the export, `in_at` the import.
   auto round_up = [](long x) { return (x + kForceAlign - 1) / kForceAlign * kForceAlign; };
   const long edge = (n + 2 * kHostParts - 1) / (2 * kHostParts);
   long out_at[kHostParts + 1], in_at[kHostParts + 1];
   out_at[0] = 0;
-  out_at[1] = std::min(n, round_up(edge));
+  out_at[1] = std::min(n, round_up(n * 2 / (3 * kHostParts)));
   for (int j = 2; j <= kHostParts; j++)
     out_at[j] = std::min(n, out_at[1] + round_up((n - out_at[1]) * (j - 1) / (kHostParts - 1)));
   out_at[kHostParts] = n;
@@ -880,6 +883,15 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   // Each part's copy to the device (copy stream) releases its conversion to planes and its
   // predictor (the step's stream) while the next part copies.  The copy stream waits for the
   // context's stream first: the staging buffers may still be in use.
+  struct OneStep {   // the lists serve this step alone: no clump needs an allowance
+    af3d_ctx *c;
+    explicit OneStep(af3d_ctx *c) : c(c) {
+      Margins m = c->cur.m;
+      m.per_speed = m.floor = m.cap = 0.0f;
+      c->cur.m = c->alt.m = m;
+    }
+    ~OneStep() { set_margins(c); }
+  } one_step(c);
   AF3D_CUDA(cudaEventRecord(c->part_done[0], c->st));
   AF3D_CUDA(cudaStreamWaitEvent(c->xfer, c->part_done[0], 0));
   drop_graphs(c);   // the slot order changes (the next af3d_step permutes when it is due)
@@ -909,10 +921,19 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   c->sorted = false;
   c->look = false;
   c->since_sort = c->resort_every;
-  // The rest of the step (a kept-order step of af3d_step): the sort, then the near lists and the
-  // force pass in kHostParts launches of whole blocks; after each, the part's clumps go to the AoS staging
-  // buffer and, on the copy stream, to the host while the next part computes.
+  // The rest of the step (a kept-order step of af3d_step): the sort and the near lists,
+  // then the force pass in kHostParts launches of whole blocks; after each, the part's clumps go
+  // to the AoS staging buffer and, on the copy stream, to the host while the next part computes.
+  // The lists of all parts but the first are built on the copy stream, idle until the first
+  // part leaves, beside the first part's.
   sort_for(c, true);
+  if (out_at[1] < n) {
+    AF3D_CUDA(cudaEventRecord(c->part_in[0], c->st));
+    AF3D_CUDA(cudaStreamWaitEvent(c->xfer, c->part_in[0], 0));
+    build_lists(c, c->xfer, c->cells.perm, out_at[1], n - out_at[1]);
+    AF3D_CUDA(cudaEventRecord(c->part_in[1], c->xfer));
+  }
+  build_lists(c, c->st, c->cells.perm, 0, out_at[1]);
   Planes after = c->cur;   // the plane set as the step leaves it (accelerations swapped)
   swap_accel_planes(after);
   const int in_parts = parts;
@@ -920,7 +941,7 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   for (int j = 0; j < kHostParts; j++) {
     const long s0 = out_at[j], cnt = out_at[j + 1] - s0;
     if (cnt <= 0) continue;
-    build_lists(c, c->cells.perm, s0, cnt);
+    if (j == 1) AF3D_CUDA(cudaStreamWaitEvent(c->st, c->part_in[1], 0));
     forces_for(c, false, c->cur, false, false, false, false, s0, cnt);
     launch_planes_to_aos(c->L(), after, c->id_cur, c->fl_cur, c->d_aos, acc_out ? c->d_acc : nullptr,
                          anga_out ? c->d_anga : nullptr, c->d, s0, cnt);
@@ -1259,7 +1280,7 @@ af3d_status af3d_forces(af3d_ctx *c) {
   enqueue_cell_build(c, false, false);
   c->cells_valid = true;
   // Corrected velocities go to the dead plane set and are dropped: this pass stops at get_accel.
-  build_lists(c, nullptr);
+  build_lists(c, c->st, nullptr);
   forces_for(c, true, c->alt);
   drop_lists(c);
   c->records_valid = true;
@@ -1474,7 +1495,7 @@ af3d_status af3d_step_profile(af3d_ctx *c, long k, double *ms) {
     AF3D_CUDA(cudaEventRecord(ev[3], c->st));
     if (p.resort) enqueue_permutation(c, false);
     AF3D_CUDA(cudaEventRecord(ev[4], c->st));
-    if (p.build) build_lists(c, p.resort ? nullptr : c->cells.perm);
+    if (p.build) build_lists(c, c->st, p.resort ? nullptr : c->cells.perm);
     step_forces(c, p, false);
     AF3D_CUDA(cudaEventRecord(ev[5], c->st));
     c->since_sort = resort ? 0 : c->since_sort + 1;
@@ -1726,7 +1747,7 @@ af3d_status set_device_time(af3d_ctx *c, double t) {
 void enqueue_startup_pass(af3d_ctx *c) {
   predict_for(c, false, true, false, true);
   sort_for(c, true);
-  build_lists(c, c->cells.perm);
+  build_lists(c, c->st, c->cells.perm);
   forces_for(c, true, c->alt);   // corrected velocities go to the dead set
   drop_lists(c);
 }
