@@ -5,7 +5,7 @@
 // clumps of one cell -- and of neighbouring cells along x -- sit in consecutive slots and all
 // per-clump kernels read and write coalesced.  Two plane sets (cur / alt) are ping-ponged by the
 // permutation.  Neighbour-visible data is additionally packed per slot into an FP64 record
-// (NbrRec, 192 B) and an FP32 culling record (CullRec, 80 B) so that a neighbour gather touches
+// (NbrRec, 192 B) and a culling record (CullRec, 96 B) so that a neighbour gather touches
 // one or two 64-byte lines.
 #pragma once
 
@@ -39,6 +39,7 @@ enum Plane : int {
 struct Margins {
   int qs;
   float per_speed, floor, cap;   // allowance min(per_speed * speed + floor, cap), in cm
+  float most;                    // bounding radius that the near lists' cell ranges reach for, in cm
 };
 
 struct Planes {
@@ -76,13 +77,19 @@ constexpr float kCullMaxUnits = 943718.0f;   // 0.9 x 2^20
 // The margins for clumps of sphere radius up to rmax moving for up to `steps` steps of dt.  The
 // unit: a regular clump's bounding radius (half of GYR rmax, cabecera.hu:8) is at most 0.8 x 2^20
 // units.  The allowance: half as much again as the clump's speed covers in that time, and 4 % of
-// a sphere's radius for what contacts accelerate it; at most 30 % of the radius.
+// a sphere's radius for what contacts accelerate it; at most 30 % of the radius.  The bounding
+// radius to reach for is that of a regular clump of rmax and 5 % (a state with a larger one has
+// every clump search its cells): reaching for all that a record can hold, 0.9 x 2^20 units, took
+// 17 rows of 4 cells a clump for 10 of 3 (262,144 clumps fast 10.44 ms, now 10.24; 100,003 from
+// host memory 726 us, now 714).
 inline Margins margins_for(double rmax, double dt, long steps) {
   Margins m;
   int e = 0;
   const bool ok = rmax > 1e-30 && rmax < 1e30;
   frexp(ok ? 838860.0 / (2.2247448713915889 * rmax) : 2097152.0, &e);
   m.qs = e - 1;
+  const double holds = ldexp((double)kCullMaxUnits, -m.qs);
+  m.most = (float)(ok ? fmin(1.05 * 2.2247448713915889 * rmax, holds) : holds);
   const double v = 1.5 * fabs(dt) * (double)steps;
   m.per_speed = v < 1e30 ? (float)v : 1e30f;
   m.floor = ok ? (float)(0.04 * rmax) : 0.0f;

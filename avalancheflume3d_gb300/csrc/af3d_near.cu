@@ -49,8 +49,9 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
   const CullRec &rec = cull[sv];
   const float4 mc = rec.c;
   const float allow = rec.allow, grown = allow * (1.0f + 1e-5f);
-  const float unit = unit_power(-m.qs);
-  const bool coarse = !(__int_as_float(rec.s[0].w) < kCullMaxUnits);   // too large for the lists
+  const float sum = fabsf(mc.x) + fabsf(mc.y) + fabsf(mc.z);
+  const bool coarse = !(__int_as_float(rec.s[0].w) < kCullMaxUnits) ||
+                      !(mc.w <= m.most + 1e-6f * (sum + 10.0f));   // too large for the lists
   if (w == 0 && valid) {
     near.loose[s] = INT_MAX;
     near.rem[s] = allow * (1.0f - 1e-5f);
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
     if (coarse) atomicMin(&d->all_slow, d->tick);   // every clump searches for itself
   }
   // the cells within reach of any partner's bound and allowance, FP32 with slack
-  const float most = kCullMaxUnits * unit + 1e-6f * (fabsf(mc.x) + fabsf(mc.y) + fabsf(mc.z) + 10.0f) + m.cap;
+  const float most = m.most + 1e-6f * (sum + 20.0f) + m.cap;
   const float reach = (mc.w + grown + most) * (1.0f + 1e-5f);
   auto range = [&](float x, float xmin, float inv, int cells, int &lo, int &hi) {
     const float q = (x - xmin) * inv, r = reach * inv;

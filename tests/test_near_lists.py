@@ -78,3 +78,24 @@ def test_kept_lists_equal_new_ones(af3d, mode, speed, n, nflumes, phase):
             assert x.tobytes() == y.tobytes()
         if speed < 100.0:
             assert kept.list_overflows() > 0
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("scale", [1.0, 1.04, 1.06, 1.5])
+def test_clumps_up_to_and_past_the_reach(af3d, mode, scale):
+    """The largest clump of the flume's rmax, 5 % more (the largest the lists reach for) and more
+    than that (every clump searches its cells): kept lists equal new ones, bit for bit."""
+    from tests.states import flume_system, wall_state
+    n = 301
+    sys, fun = flume_system(n)
+    pp = wall_state(n, 43, sys, vel=200.0, omega=50.0)
+    pp["radius"][::7] = scale * float(np.ravel(sys["rmax"])[0])
+    af3d.sphere_centres(pp)
+    with start(af3d, sys, fun, pp, mode, 1, 200.0, 1) as kept, start(af3d, sys, fun, pp, mode, 1, 200.0, 1) as new:
+        for _ in range(STEPS):
+            new.step(1)
+            new.import_particles(*new.export_particles())
+        kept.step(STEPS)
+        assert kept.contact_count() > 0
+        for x, y in zip(kept.export_particles(), new.export_particles()):
+            assert x.tobytes() == y.tobytes()
