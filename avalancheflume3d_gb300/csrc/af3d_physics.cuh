@@ -62,7 +62,7 @@ __device__ __forceinline__ V3 mk(double x, double y, double z) {
 }
 
 // ---- FP64 tests and conversions on the integer pipe ----------------------------------------
-// The FP64 pipe of this GPU retires one warp instruction per ~19 SM cycles, and conversions and
+// The FP64 pipe of this GPU retires one warp instruction per 16 (DFMA) to 19 SM cycles, and conversions and
 // comparisons of doubles occupy it like arithmetic does.  These helpers take the same decisions
 // and give the same bits as the hardware instructions they replace, from the operands' bit
 // patterns, on the integer pipe; values outside their fast range (zero, subnormal or huge

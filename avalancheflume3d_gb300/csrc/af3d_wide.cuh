@@ -382,11 +382,9 @@ __global__ void __launch_bounds__(kWideThreads, 4)
       if (turns && w < 3) {
         double e[3] = {i == 0 ? 1.0 : 0.0, i == 1 ? 1.0 : 0.0, i == 2 ? 1.0 : 0.0};
         if (positive_bits(mag)) {
-          const double u[3] = {sh.aux[0][lane], sh.aux[1][lane], sh.aux[2][lane]};
           const double omc = 1.0 - cs, ui = sh.aux[i][lane], u1 = sh.aux[i1][lane], u2 = sh.aux[i2][lane];
           // (i, i): omc u_i u_i + c;  (i, i1): omc u_i u_i1 - sn u_i2;  (i, i2): omc u_i u_i2 + sn u_i1
           const double d0 = omc * ui * ui + cs, d1 = omc * ui * u1 - sn * u2, d2 = omc * ui * u2 + sn * u1;
-          (void)u;
           e[0] = i == 0 ? d0 : i1 == 0 ? d1 : d2;
           e[1] = i == 1 ? d0 : i1 == 1 ? d1 : d2;
           e[2] = i == 2 ? d0 : i1 == 2 ? d1 : d2;
