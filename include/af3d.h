@@ -192,15 +192,17 @@ af3d_status af3d_swap_accel (af3d_ctx *ctx);          /* avalanche_hst.cu:845-85
    reference's order, get_accel into a_f (avalanche_hst.cu:678-707; fill :445-464). */
 af3d_status af3d_forces (af3d_ctx *ctx);
 
-/* k steps of the current phase, fused and replayed from CUDA graphs, with the reference's
+/* k steps of the current phase, fused (whole permutation periods replayed from a CUDA graph, the
+   rest launched one by one), with the reference's
    re-grid every 2000 steps (avalanche_hst.cu:713-748).  Returns the first error status raised
    by the device checks during those steps. */
 af3d_status af3d_step (af3d_ctx *ctx, long k);
 
 /* Same steps as af3d_step, enqueued without graphs and with CUDA events between the kernels on
    the context stream; adds the milliseconds of each phase to ms[AF3D_NPROF]:
-   0 time advance, 1 init_Verlet + cell keys, 2 cell sort, 3 permutation + neighbour records,
-   4 force kernel (contact lists, walls, contacts, bed, get_accel, finish_Verlet), 5 re-grid. */
+   0 time advance, 1 init_Verlet + cell keys, 2 cell sort and near lists (one step in 16),
+   3 permutation + neighbour records, 4 force kernel (contacts, walls, bed, get_accel,
+   finish_Verlet, the next step's init_Verlet), 5 re-grid. */
 enum { AF3D_NPROF = 6 };
 af3d_status af3d_step_profile (af3d_ctx *ctx, long k, double *ms);
 /* Kernels executed on the device by this context so far (graph replays included). */
@@ -270,7 +272,7 @@ af3d_status af3d_autotune (af3d_ctx *ctx, long steps_per_trial, long *resort_eve
 /* The fused force kernel's block (no counterpart in the reference): 64, 96, 128 or 192 threads,
    one clump per thread, the block's clumps pooling their contact items; each runs at the
    resident blocks per SM that measured fastest for it (10, 6, 5 and 3).  Results do not depend
-   on it.  A new context starts with the block of 64, 96 and 128 whose last wave is fullest for
+   on it, and up to 20,480 clumps the steps run in a shape of their own.  A new context starts with the block of 64, 96 and 128 whose last wave is fullest for
    its clump count on the current device; af3d_set_force_block overrides it. */
 af3d_status af3d_set_force_block (af3d_ctx *ctx, int block);
 af3d_status af3d_get_force_block (af3d_ctx *ctx, int *block);
