@@ -160,7 +160,7 @@ struct af3d_ctx {
   StepGraph graphs[4];
   int graph_next = 0;
   // af3d_step_host: the stream of its device-to-host copies and the events that release them
-  cudaStream_t xfer = nullptr;
+  cudaStream_t xfer = nullptr, side = nullptr;   // side: the near lists of the later parts
   cudaEvent_t part_done[kHostParts] = {}, part_in[kHostParts] = {};
   long launches = 0;          // kernels executed (graph replays included)
 
@@ -720,6 +720,10 @@ af3d_status af3d_destroy(af3d_ctx *c) {
                   (void *)c->d_acc, (void *)c->d_anga, (void *)c->d_tmp, (void *)c->d_count})
     if (p) cudaFree(p);
   if (c->own_stream && c->st) cudaStreamDestroy(c->st);
+  if (c->side) {
+    cudaStreamSynchronize(c->side);
+    cudaStreamDestroy(c->side);
+  }
   if (c->xfer) {
     cudaStreamSynchronize(c->xfer);
     cudaStreamDestroy(c->xfer);
@@ -858,6 +862,7 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   if (!c->d_acc) AF3D_CUDA(cudaMalloc(&c->d_acc, sizeof(double) * 3 * m));
   if (!c->d_anga) AF3D_CUDA(cudaMalloc(&c->d_anga, sizeof(double) * 3 * m));
   if (!c->xfer) AF3D_CUDA(cudaStreamCreateWithFlags(&c->xfer, cudaStreamNonBlocking));
+  if (!c->side) AF3D_CUDA(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
   for (cudaEvent_t &e : c->part_done)
     if (!e) AF3D_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (cudaEvent_t &e : c->part_in)
@@ -924,16 +929,17 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   // The rest of the step (a kept-order step of af3d_step): the sort and the near lists,
   // then the force pass in kHostParts launches of whole blocks; after each, the part's clumps go
   // to the AoS staging buffer and, on the copy stream, to the host while the next part computes.
-  // The lists of all parts but the first are built on the copy stream, idle until the first
-  // part leaves, beside the first part's.
+  // The lists of all parts but the first are built on a stream of their own beside the parts
+  // before them.
   sort_for(c, true);
-  if (out_at[1] < n) {
-    AF3D_CUDA(cudaEventRecord(c->part_in[0], c->st));
-    AF3D_CUDA(cudaStreamWaitEvent(c->xfer, c->part_in[0], 0));
-    build_lists(c, c->xfer, c->cells.perm, out_at[1], n - out_at[1]);
-    AF3D_CUDA(cudaEventRecord(c->part_in[1], c->xfer));
-  }
+  AF3D_CUDA(cudaEventRecord(c->part_in[0], c->st));
+  AF3D_CUDA(cudaStreamWaitEvent(c->side, c->part_in[0], 0));
   build_lists(c, c->st, c->cells.perm, 0, out_at[1]);
+  for (int j = 1; j < kHostParts; j++) {
+    if (out_at[j] >= n) break;
+    build_lists(c, c->side, c->cells.perm, out_at[j], out_at[j + 1] - out_at[j]);
+    AF3D_CUDA(cudaEventRecord(c->part_in[j], c->side));
+  }
   Planes after = c->cur;   // the plane set as the step leaves it (accelerations swapped)
   swap_accel_planes(after);
   const int in_parts = parts;
@@ -941,7 +947,7 @@ af3d_status af3d_step_host(af3d_ctx *c, const af3d_particle *in, const af3d_vec3
   for (int j = 0; j < kHostParts; j++) {
     const long s0 = out_at[j], cnt = out_at[j + 1] - s0;
     if (cnt <= 0) continue;
-    if (j == 1) AF3D_CUDA(cudaStreamWaitEvent(c->st, c->part_in[1], 0));
+    if (j > 0) AF3D_CUDA(cudaStreamWaitEvent(c->st, c->part_in[j], 0));
     forces_for(c, false, c->cur, false, false, false, false, s0, cnt);
     launch_planes_to_aos(c->L(), after, c->id_cur, c->fl_cur, c->d_aos, acc_out ? c->d_acc : nullptr,
                          anga_out ? c->d_anga : nullptr, c->d, s0, cnt);
