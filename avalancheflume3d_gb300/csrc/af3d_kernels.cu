@@ -324,8 +324,8 @@ struct Rows {
 };
 
 // init_Verlet.cu:63-114: the rotation rows turned by the angle vector dO, columns renormalised.
-// In the fast mode the path of turns of 2^-10 rad and more and of unnormalised input (the others
-// run in fixed point, predict_state), not inlined there.
+// In the fast mode the path of the device friction law, of turns of 2^-10 rad and more and of
+// unnormalised input (the others run in fixed point, predict_state), not inlined there.
 #ifdef AF3D_FAST
 __device__ __noinline__
 #else
@@ -452,9 +452,10 @@ __device__ __forceinline__ void place_spheres(V3 r, V3 Rx, V3 Ry, V3 Rz, double 
 // one step with a_i, alpha_i; sp receives the new sphere centres.  Fast mode: the rotation and the
 // spheres in fixed point (af3d_fixed.cuh), 18 FP64 instructions instead of 123: a step of
 // 262,144 clumps 198 -> 190 us, of 582,320 in 64 flumes 414 -> 398 us (2,048 clumps, where one warp
-// has an SM's sub-partition to itself and latency counts: 35.4 -> 37.3 us).
+// has an SM's sub-partition to itself and latency counts: 35.4 -> 37.3 us).  dev: the device friction
+// law, whose runs show every last bit (af3d_physics.cuh): in FP64.
 __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, V3 &Rx, V3 &Ry, V3 &Rz, V3 *sp,
-                                              double rad, double dt, double hdt, int qs) {
+                                              double rad, double dt, double hdt, int qs, bool dev) {
   r.x += dt * (v.x + hdt * a.x);
   r.y += dt * (v.y + hdt * a.y);
   r.z += dt * (v.z + hdt * a.z);
@@ -467,7 +468,7 @@ __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, 
   w.z += dt * al.z;
   constexpr Divisor root2 = constant_divisor(kROOT2, 0x3FF6A09E667F3BCCull);
   const double pos = kFast ? rad * (1.0 / kROOT2) : div_by(rad, root2);
-  if (kFast) {
+  if (kFast && !dev) {
     const double angle[3] = {dO.x, dO.y, dO.z};
     const double R[9] = {Rx.x, Rx.y, Rx.z, Ry.x, Ry.y, Ry.z, Rz.x, Rz.y, Rz.z};
     long long turned[9];
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(kBlock) k_predict(Planes P, DevScalars *d, boo
         w = load3(P, WX, s);
         V3 Rx = load3(P, R00, s), Ry = load3(P, R10, s), Rz = load3(P, R20, s);
         predict_state(r, v, w, load3(P, AIX, s), load3(P, ALIX, s), Rx, Ry, Rz, sp, P.p[RAD][s], fl.sys.dt,
-                      fl.sys.hdt, P.m.qs);
+                      fl.sys.hdt, P.m.qs, d->variant == AF3D_FRICTION_DEV);
         store3(P, RX, s, r);
         store3(P, VX, s, v);
         store3(P, WX, s, w);
@@ -1305,7 +1306,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
     V3 v2, w2, a, al;
     if (!removed) {
       get_accel_one(F, T, v, w, Rx, Ry, Rz, P.p[MASS][s], P.p[ADRAG][s], load3(P, IXX, s), a, al, P.p[IMASS][s],
-                    P.p[IINER][s]);
+                    P.p[IINER][s], c.variant == AF3D_FRICTION_DEV);
       store3(P, AFX, s, a);
       store3(P, ALFX, s, al);
       const V3 ai = load3(P, AIX, s), ali = load3(P, ALIX, s);
@@ -1340,7 +1341,8 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
         store3(P, RN10, s, Ry);
         store3(P, RN20, s, Rz);
       } else {
-        predict_state(rn, vn, wn, a, al, Rx, Ry, Rz, sp, P.p[RAD][s], fl.sys.dt, fl.sys.hdt, P.m.qs);
+        predict_state(rn, vn, wn, a, al, Rx, Ry, Rz, sp, P.p[RAD][s], fl.sys.dt, fl.sys.hdt, P.m.qs,
+                      c.variant == AF3D_FRICTION_DEV);
         store3(P, RN00, s, Rx);
         store3(P, RN10, s, Ry);
         store3(P, RN20, s, Rz);
@@ -1413,7 +1415,8 @@ __global__ void k_get_accel(Planes P, DevScalars *d, const int *__restrict__ flu
   if (is_removed(d->time, P.p[RX][s], d->flumes[flume[s]].sys.side.x)) return;
   V3 a, al;
   get_accel_one(load3(P, FX, s), load3(P, TX, s), load3(P, VX, s), load3(P, WX, s), load3(P, R00, s),
-                load3(P, R10, s), load3(P, R20, s), P.p[MASS][s], P.p[ADRAG][s], load3(P, IXX, s), a, al, P.p[IMASS][s], P.p[IINER][s]);
+                load3(P, R10, s), load3(P, R20, s), P.p[MASS][s], P.p[ADRAG][s], load3(P, IXX, s), a, al,
+                P.p[IMASS][s], P.p[IINER][s], d->variant == AF3D_FRICTION_DEV);
   store3(P, AFX, s, a);
   store3(P, ALFX, s, al);
 }

@@ -9,8 +9,18 @@
 // Fast mode (built with -DAF3D_FAST -fmad=true): the same FP64 physics with multiply-adds
 // contracted, normals and tangents from a reciprocal square root instead of three divisions,
 // and quotients by a shared divisor taken as products with one reciprocal.  Each of these
-// changes a result by a few units in the last place, so forces agree with the reference to
-// ~1e-14 relative rather than bit for bit.
+// changes a result by a few units in the last place, so one pass's forces agree with the
+// reference to ~1e-14 relative rather than bit for bit.
+//
+// Under the device friction law every pushing pair slides in the Coulomb branch, whose direction
+// v_t / |v_t| divides a last-bit difference of two runs by the slip: over tens of steps such
+// differences reached 3e-8 of max(rms alpha, |alpha|) in single clumps (168,000 clumps, 29 steps).
+// A change of rounding anywhere in a step therefore shows in a run under that law, so its
+// arithmetic is kept to the bit: |v_t|, the normals and the drag's |v| from CUDA's rsqrt, the Coulomb
+// quotient by a division, the rotation and the sphere centres in FP64 (predict_state).  Under
+// the host law, whose gate cuts the tangential part of nearly every pair, the same differences
+// stayed below 9e-9 (80 runs), and |v_t|, the normals and the Coulomb quotient come from integer-pipe roots and
+// reciprocals (af3d_intfp64.cuh), the rotation and the centres from fixed point (af3d_fixed.cuh).
 //
 // Geometry stays exact in both modes.  The distances that decide whether a contact exists, and
 // whose difference from the radius is the contact's compression, are evaluated with
@@ -184,10 +194,12 @@ __device__ __forceinline__ bool surely_gated(V3 dv, V3 n, double normal, double 
 // tail of every contact type (force_part.cu:189-241, force_walls.cu:123-177, ...).
 //   xi0:  Coulomb branch also when xi was zeroed (walls; DEV particle variant)
 //   gate: false -> proceed when normal > 0; true -> proceed unless normal <= 0 (fcorners)
+//   dev:  the device friction law (see the header comment)
 __device__ __forceinline__ bool contact_law_fast(V3 dvvc, V3 n, double comp, double km, double gm,
                                                  double mass_t, double mu, double cns_1, double dt,
-                                                 double inv_dt, bool xi0, bool gate, V3 &f) {
-  const double vn = dvvc.x * n.x + dvvc.y * n.y + dvvc.z * n.z;
+                                                 double inv_dt, bool xi0, bool gate, bool dev, V3 &f) {
+  // the multiply-adds named, so that every kernel rounds alike
+  const double vn = __fma_rn(dvvc.z, n.z, __fma_rn(dvvc.x, n.x, dvvc.y * n.y));
   const double normal = km * comp + gm * (-vn);
   const bool push = positive_bits(normal);
   if (gate ? !push && !nan_bits(normal) : !push) return false;
@@ -196,8 +208,13 @@ __device__ __forceinline__ bool contact_law_fast(V3 dvvc, V3 n, double comp, dou
   if (gated && !xi0) return true;   // no displacement, no Coulomb branch: the normal force alone
   const V3 vt = mk(dvvc.x - vn * n.x, dvvc.y - vn * n.y, dvvc.z - vn * n.z);
   const double vt2 = vt.x * vt.x + vt.y * vt.y + vt.z * vt.z;
-  double inv_vt;                             // +inf for vt = 0: the tangential part is then skipped,
-  const double vt_mag = sqrt_and_inverse(vt2, inv_vt);   // as in the exact law
+  double inv_vt, vt_mag;   // +inf and 0 (dev: NaN) for vt = 0: the tangential part is then skipped, as in the exact law
+  if (dev) {
+    inv_vt = rsqrt(vt2);
+    vt_mag = vt2 * inv_vt;
+  } else {
+    vt_mag = sqrt_and_inverse(vt2, inv_vt);
+  }
   double xi = 0.0, fsdt = 0.0;
   if (!gated) {
     // dvvc . vt / |vt| = |vt| up to the rounding of vt's orthogonality to n, which the exact law
@@ -211,7 +228,8 @@ __device__ __forceinline__ bool contact_law_fast(V3 dvvc, V3 n, double comp, dou
       // af = 0.8 mu N / |vt|, t0 = m / af, af / (1 + (dt / t0)^2) = af m^2 / (m^2 + (dt af)^2)
       const double af = 0.8 * mu * normal * inv_vt;
       const double dta = dt * af;
-      const double a = af * (mass_t * mass_t) * reciprocal(mass_t * mass_t + dta * dta);
+      const double num = af * (mass_t * mass_t), den = mass_t * mass_t + dta * dta;
+      const double a = dev ? div_rn(num, den) : num * reciprocal(den);
       f.x += a * vt.x;
       f.y += a * vt.y;
       f.z += a * vt.z;
@@ -359,7 +377,7 @@ __device__ __forceinline__ void wall_input(const Sph &o, V3 rrc, V3 n, double co
 // The contact law on a prepared contact: force fs and its torque term about the clump centre r.
 __device__ __forceinline__ bool apply_law(const ContactIn &ci, V3 r, const Consts &c, V3 &fs, V3 &tq) {
   const bool on = kFast ? contact_law_fast(ci.dvvc, ci.n, ci.comp, ci.km, ci.gm, ci.mass_t, ci.mu, ci.cns, c.dt,
-                                           c.inv_dt, ci.xi0, ci.gate, fs)
+                                           c.inv_dt, ci.xi0, ci.gate, c.variant == AF3D_FRICTION_DEV, fs)
                         : contact_law(ci.dvvc, ci.n, ci.comp, ci.km, ci.gm, ci.mass_t, ci.mu, ci.cns, c.dt,
                                       ci.xi0, ci.gate, fs);
   if (!on) return false;
@@ -651,8 +669,14 @@ __device__ __forceinline__ bool pair_input(const V3 &rrl, const V3 &vvl, const V
   }
   double dist;
   if (kFast) {
+    // dist correctly rounded: the compression sep - dist is the exact mode's
     double inv;
-    dist = sqrt_and_inverse(dist2, inv);   // correctly rounded: the compression sep - dist is the exact mode's
+    if (c.variant == AF3D_FRICTION_DEV) {
+      inv = rsqrt(dist2);
+      dist = sqrt_rn(dist2);
+    } else {
+      dist = sqrt_and_inverse(dist2, inv);
+    }
     ci.n = mk(d.x * inv, d.y * inv, d.z * inv);
   } else {
     dist = sqrt_rn(dist2);
@@ -710,6 +734,12 @@ __device__ __forceinline__ double plus_signed_zero(double q, float a, float b) {
   return nonzero_bits(q) ? q : of_bits(bits_of(q) & z);
 }
 
+// |v| of the drag from v2 = |v|^2 (dev: the device friction law, see the header comment).
+__device__ __forceinline__ double speed_of(double v2, bool dev) {
+  if (kFast && dev) return v2 == 0.0 ? 0.0 : v2 * rsqrt(v2);   // NaN stays NaN
+  return sqrt_rn(v2);
+}
+
 // get_accel.cu:21-75 for one clump; R rows Rx, Ry, Rz.  `adrag0` = DRAG*rad*rad/m (the same
 // expression, precomputed per clump).  For isotropic inertia (Ix == Iy == Iz, the reference's
 // clumps, calculate_particle_parameters.cu:33) the Euler coupling terms C*wb*wb are (+0*wb)*wb,
@@ -717,9 +747,10 @@ __device__ __forceinline__ double plus_signed_zero(double q, float a, float b) {
 // multiplications, which gives the same bits for finite angular velocities.
 // (fast mode: im = 1/m and iI = 1/I.x, formed once at import, replace the divisions)
 __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 Ry, V3 Rz, double m,
-                                              double adrag0, V3 I, V3 &a, V3 &al, double im, double iI) {
+                                              double adrag0, V3 I, V3 &a, V3 &al, double im, double iI,
+                                              bool dev) {
   const double v2 = v.x * v.x + v.y * v.y + v.z * v.z;
-  double vmag = sqrt_rn(v2);
+  double vmag = speed_of(v2, dev);
   double adrag = adrag0 * vmag;
   if (kFast) {
     a.x = f.x * im - adrag * v.x;

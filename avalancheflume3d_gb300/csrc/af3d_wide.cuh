@@ -41,9 +41,9 @@ struct Accel {
 };
 // get_accel of a whole clump (inertia that is not isotropic, spins whose signs FP32 leaves open).
 __device__ __noinline__ Accel get_accel_whole(V3 f, V3 t, V3 v, V3 w, Rows R, double m, double adrag0, V3 I, double im,
-                                              double iI) {
+                                              double iI, bool dev) {
   Accel r;
-  get_accel_one(f, t, v, w, R.x, R.y, R.z, m, adrag0, I, r.a, r.al, im, iI);
+  get_accel_one(f, t, v, w, R.x, R.y, R.z, m, adrag0, I, r.a, r.al, im, iI, dev);
   return r;
 }
 
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
   auto body = [&](const Consts &c) {
     const NbrRec &me = nbr[sv];
     const bool removed = is_removed(*c.tp, me.rx, c.side_x), act = valid && !removed;
-    const bool aval = c.phase == AF3D_PHASE_AVALANCHE;
+    const bool aval = c.phase == AF3D_PHASE_AVALANCHE, dev = c.variant == AF3D_FRICTION_DEV;
     const int info = near.info[sv];
     bool brute = false;
     const bool search = act && must_search(sv, d, near, info, brute);
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
                     plus_signed_zero(ab.z, sb[0], sb[1]));
           }
           const double v2s = v.x * v.x + v.y * v.y + v.z * v.z;
-          const double adrag = adrag0 * sqrt_rn(v2s);
+          const double adrag = adrag0 * speed_of(v2s, dev);
           const double vi = comp(v, i);
           if (kFast) ai = Fi * im - adrag * vi;
           else ai = div_by(Fi, divisor_of(mass)) - adrag * vi;
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
         } else {
           const Rows R = {load3(P, R0, s), load3(P, R0 + 3, s), load3(P, R0 + 6, s)};
           const Accel r = get_accel_whole(mk(sh.aux[0][lane], sh.aux[1][lane], sh.aux[2][lane]), T, v, om, R, mass,
-                                          adrag0, I, im, iI);
+                                          adrag0, I, im, iI, dev);
           ai = comp(r.a, i);
           ali = comp(r.al, i);
         }
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
     const bool turns = valid && !removed;
     if constexpr (kFast) {
       bool ok = false;
-      if (turns && w < 3) {
+      if (turns && w < 3 && !dev) {
         const double angle[3] = {dO.x, dO.y, dO.z};
         Turn turn;
         long long t[3];
