@@ -1,5 +1,5 @@
 """Writes fast_device.npz: runs of the fast FP64 mode under the device friction law, as commit d99b290
-computed them on a GB300 (python -m tests.golden.make_fast_device on that commit's tree).
+computed them on a GB300 (python -m tests.runs.make_fast_device on that commit's tree).
 
 Under that law every pushing pair slides in the Coulomb branch, and its direction v_t / |v_t| shows a
 last-bit difference divided by the slip, so the runs are kept bit for bit.  One count per shape of the

@@ -1,11 +1,11 @@
 """The fast FP64 mode under the device friction law computes the same bits as it did when
-tests/golden/fast_device.npz was written: under that law a last-bit difference anywhere in a step grows
+tests/runs/fast_device.npz was written: under that law a last-bit difference anywhere in a step grows
 by the ratio of speed to slip at every sliding pair, so a run shows whatever a kernel rounds
 otherwise (af3d_physics.cuh)."""
 import numpy as np
 import pytest
 
-from tests.golden.make_fast_device import PATH, RUNS, run
+from tests.runs.make_fast_device import PATH, RUNS, run
 
 pytestmark = pytest.mark.gpu
 
