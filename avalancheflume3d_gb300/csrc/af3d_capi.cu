@@ -347,7 +347,7 @@ void predict_for(af3d_ctx *c, bool predict, bool keys, bool t_prev, bool records
 }
 
 void sort_for(af3d_ctx *c, bool with_centres) {
-  launch_sort(c->L(), c->d, c->cells, c->id_cur, c->ntags, with_centres ? c->cull : nullptr);
+  launch_sort(c->L(), c->cur.m, c->d, c->cells, c->id_cur, c->ntags, with_centres ? c->cull : nullptr);
   c->launches += kKernelsPerSort;
 }
 

@@ -121,7 +121,7 @@ __global__ void k_scatter(const int *__restrict__ key, const int *__restrict__ r
 __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ start,
                        const int *__restrict__ tmp_slot, const long long *__restrict__ id, int *perm,
                        const CullRec *__restrict__ cull, float4 *csort, int *count, int *tile_count,
-                       DevScalars *d, long ntags, long n) {
+                       Margins m, DevScalars *d, long ntags, long n) {
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (s >= n) return;
   const long ncell3 = d->ncell_total;
@@ -137,6 +137,8 @@ __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ star
     float4 c = cull[s].c;
     c.w += cull[s].allow * (1.0f + 1e-5f);
     csort[b + r] = c;
+    // before any force pass of the step, whose first parts may run beside the later lists' builds
+    if (beyond_reach(cull[s], m)) atomicMin(&d->all_slow, d->tick);
   }
   // cells.cu:96-102: a cell may hold at most ntags - 1 clumps
   if (ntags > 0 && k < ncell3 && r == 0 && (e - b) >= ntags)
@@ -147,7 +149,8 @@ __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ star
 
 long scan_tiles(long bucket_cap) { return (bucket_cap + kTile - 1) / kTile; }
 
-void launch_sort(const Launch &L, DevScalars *d, Cells c, const long long *id, long ntags, const CullRec *cull) {
+void launch_sort(const Launch &L, Margins m, DevScalars *d, Cells c, const long long *id, long ntags,
+                 const CullRec *cull) {
   // Launch sizes follow the capacity; the kernels read the bucket count in use from the device,
   // so a captured graph stays valid across device-side re-grids.
   const long ntiles = scan_tiles(c.cap);
@@ -155,7 +158,7 @@ void launch_sort(const Launch &L, DevScalars *d, Cells c, const long long *id, l
   if (L.n <= 0) return;
   const unsigned g = (unsigned)((L.n + 127) / 128);
   k_scatter<<<g, 128, 0, L.st>>>(c.key, c.rank_tmp, c.start, c.tmp_slot, L.n);
-  k_rank<<<g, 128, 0, L.st>>>(c.key, c.start, c.tmp_slot, id, c.perm, cull, c.csort, c.count, c.tile_count, d,
+  k_rank<<<g, 128, 0, L.st>>>(c.key, c.start, c.tmp_slot, id, c.perm, cull, c.csort, c.count, c.tile_count, m, d,
                               ntags, L.n);
 }
 

@@ -97,6 +97,15 @@ inline Margins margins_for(double rmax, double dt, long steps) {
   return m;
 }
 
+#ifdef __CUDACC__
+// Whether a clump's bounding sphere is larger than the near lists reach for (an infinite sphere radius
+// marks one that the unit cannot hold).
+__device__ __forceinline__ bool beyond_reach(const CullRec &r, const Margins &m) {
+  const float sum = fabsf(r.c.x) + fabsf(r.c.y) + fabsf(r.c.z);
+  return !(__int_as_float(r.s[0].w) < kCullMaxUnits) || !(r.c.w <= m.most + 1e-6f * (sum + 10.0f));
+}
+#endif
+
 // Cell-list buffers.  Keys: flume cell offset + cell index for binned clumps (the flumes' grids
 // are concatenated, so the sort keeps every flume contiguous), ncell_total + id for clumps that
 // are not binned (removed), so every bucket holds its clumps in id order after the rank pass and
@@ -323,8 +332,9 @@ void launch_predict (const Launch &L, Planes cur, DevScalars *d, bool predict, b
 // Exclusive scan of the bucket counts, scatter by arrival, then the deterministic (bucket, id)
 // rank: fills cells.start[0..nbuckets] and cells.perm, checks the ntags capacity and leaves the
 // count array zeroed.  nbuckets = ncell_total + N is read on the device.
-// With cull (records already written at the old slots) also fills cells.csort.
-void launch_sort (const Launch &L, DevScalars *d, Cells cells, const long long *id, long ntags,
+// With cull (records already written at the old slots) also fills cells.csort and lowers d->all_slow for
+// a clump beyond the near lists' reach.
+void launch_sort (const Launch &L, Margins m, DevScalars *d, Cells cells, const long long *id, long ntags,
                   const CullRec *cull = nullptr);
 long scan_tiles (long bucket_cap);
 // Moves every plane (and the id and flume arrays) into the new order and builds the records.

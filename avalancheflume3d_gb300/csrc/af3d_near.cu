@@ -50,8 +50,7 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
   const float4 mc = rec.c;
   const float allow = rec.allow, grown = allow * (1.0f + 1e-5f);
   const float sum = fabsf(mc.x) + fabsf(mc.y) + fabsf(mc.z);
-  const bool coarse = !(__int_as_float(rec.s[0].w) < kCullMaxUnits) ||
-                      !(mc.w <= m.most + 1e-6f * (sum + 10.0f));   // too large for the lists
+  const bool coarse = beyond_reach(rec, m);
   if (w == 0 && valid) {
     near.loose[s] = INT_MAX;
     near.rem[s] = allow * (1.0f - 1e-5f);
@@ -64,7 +63,8 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
     for (int rt = R_HOP0; rt <= last; rt++)
       if (bnd_may_touch_f(rt, mc, mc.w + grown, c, door_closed)) bnd |= 15u << (4 * rt);
     near.bnd[s] = bnd;
-    if (coarse) atomicMin(&d->all_slow, d->tick);   // every clump searches for itself
+    // every clump searches for itself (with `order` the sort has said so)
+    if (coarse && !order) atomicMin(&d->all_slow, d->tick);
   }
   // the cells within reach of any partner's bound and allowance, FP32 with slack
   const float most = m.most + 1e-6f * (sum + 20.0f) + m.cap;
