@@ -347,7 +347,8 @@ void predict_for(af3d_ctx *c, bool predict, bool keys, bool t_prev, bool records
 }
 
 void sort_for(af3d_ctx *c, bool with_centres) {
-  launch_sort(c->L(), c->cur.m, c->d, c->cells, c->id_cur, c->ntags, with_centres ? c->cull : nullptr);
+  launch_sort(c->L(), c->cur.m, c->d, c->cells, c->id_cur, c->fl_cur, c->near, c->ntags,
+              with_centres ? c->cull : nullptr);
   c->launches += kKernelsPerSort;
 }
 
@@ -648,6 +649,8 @@ af3d_status af3d_create_ensemble(int nflumes, const af3d_system_par *sys, const 
   ok = ok && cudaMalloc((void **)&c->near.bnd, sizeof(unsigned) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->near.rem, sizeof(float) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->near.loose, sizeof(int) * n) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&c->near.chain, sizeof(unsigned long long) * 2 * n) == cudaSuccess;
+  ok = ok && cudaMalloc((void **)&c->near.chain_next, sizeof(int) * 2 * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->cells.key, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->cells.rank_tmp, sizeof(int) * n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&c->cells.tmp_slot, sizeof(int) * n) == cudaSuccess;
@@ -687,7 +690,8 @@ af3d_status af3d_create_ensemble(int nflumes, const af3d_system_par *sys, const 
   ds.variant = c->variant;
   ds.nflumes = nflumes;
   ds.flumes = c->flumes;
-  ds.all_slow = ds.brute = INT_MAX;
+  ds.runaway = INT_MAX;
+  cudaMemsetAsync(c->near.chain, 0, sizeof(unsigned long long) * 2 * n, c->st);
   cudaMemsetAsync(c->plane_mem[0], 0, sizeof(double) * n * NPLANES, c->st);
   cudaMemsetAsync(c->plane_mem[1], 0, sizeof(double) * n * NPLANES, c->st);
   cudaMemcpyAsync(c->flume_of_id, fid.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->st);
@@ -716,7 +720,8 @@ af3d_status af3d_destroy(af3d_ctx *c) {
                   (void *)c->cull, (void *)c->lists.items, (void *)c->nbr_next, (void *)c->cull_next, (void *)c->cells.key, (void *)c->cells.rank_tmp, (void *)c->cells.tmp_slot,
                   (void *)c->cells.perm, (void *)c->cells.csort, (void *)c->cells.count, (void *)c->cells.start,
                   (void *)c->cells.tile_count, (void *)c->cells.occ, (void *)c->cells.occ_next, (void *)c->near.items,
-                  (void *)c->near.info, (void *)c->near.bnd, (void *)c->near.rem, (void *)c->near.loose, (void *)c->d, (void *)c->flumes, (void *)c->d_aos,
+                  (void *)c->near.info, (void *)c->near.bnd, (void *)c->near.rem, (void *)c->near.loose,
+                  (void *)c->near.chain, (void *)c->near.chain_next, (void *)c->d, (void *)c->flumes, (void *)c->d_aos,
                   (void *)c->d_acc, (void *)c->d_anga, (void *)c->d_tmp, (void *)c->d_count})
     if (p) cudaFree(p);
   if (c->own_stream && c->st) cudaStreamDestroy(c->st);

@@ -12,7 +12,7 @@
 // Integer work only; HBM-bound.
 #include <climits>
 
-#include "af3d_internal.h"
+#include "af3d_cellwalk.cuh"
 
 namespace af3d {
 
@@ -73,10 +73,10 @@ __device__ __forceinline__ long n_buckets(const DevScalars *d, long n) { return 
 
 // Each tile adds the clump counts of the tiles before it (counted at arrival; integer sums are
 // exact in any order), then scans its own buckets.
-// Lists are built from the sort, so the marks that clumps left since the last ones are void.
+// Lists are built from the sort, so the runaways and marks since the last ones are void (k_scatter).
 __global__ void k_scan_final(const int *__restrict__ count, const int *__restrict__ tile_count,
                              int *start, DevScalars *d, long n) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) d->all_slow = d->brute = INT_MAX;
+  if (blockIdx.x == 0 && threadIdx.x == 0) d->runaway = INT_MAX;
   const long nb = n_buckets(d, n);
   if (blockIdx.x == 0 && threadIdx.x == 0) start[nb] = (int)n;   // every clump has one bucket
   if (blockIdx.x * (long)kTile >= nb) return;   // a tile past the buckets in use
@@ -110,9 +110,10 @@ __global__ void k_scan_final(const int *__restrict__ count, const int *__restric
 }
 
 __global__ void k_scatter(const int *__restrict__ key, const int *__restrict__ rank_tmp,
-                          const int *__restrict__ start, int *tmp_slot, long n) {
+                          const int *__restrict__ start, int *tmp_slot, int *loose, long n) {
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (s >= n) return;
+  loose[s] = INT_MAX;
   tmp_slot[start[key[s]] + rank_tmp[s]] = (int)s;
 }
 
@@ -121,7 +122,7 @@ __global__ void k_scatter(const int *__restrict__ key, const int *__restrict__ r
 __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ start,
                        const int *__restrict__ tmp_slot, const long long *__restrict__ id, int *perm,
                        const CullRec *__restrict__ cull, float4 *csort, int *count, int *tile_count,
-                       Margins m, DevScalars *d, long ntags, long n) {
+                       Margins m, DevScalars *d, const int *__restrict__ flume, int *loose, long ntags, long n) {
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (s >= n) return;
   const long ncell3 = d->ncell_total;
@@ -138,7 +139,10 @@ __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ star
     c.w += cull[s].allow * (1.0f + 1e-5f);
     csort[b + r] = c;
     // before any force pass of the step, whose first parts may run beside the later lists' builds
-    if (beyond_reach(cull[s], m)) atomicMin(&d->all_slow, d->tick);
+    const DevFlume &fl = d->flumes[flume[s]];
+    CellAt at;
+    if (beyond_reach(cull[s], m) && cell_at(k, fl.cell_off, fl.gridf, at))
+      mark_around(at, fl.gridf, fl.cell_off, start, tmp_slot, loose, d->tick);
   }
   // cells.cu:96-102: a cell may hold at most ntags - 1 clumps
   if (ntags > 0 && k < ncell3 && r == 0 && (e - b) >= ntags)
@@ -149,17 +153,17 @@ __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ star
 
 long scan_tiles(long bucket_cap) { return (bucket_cap + kTile - 1) / kTile; }
 
-void launch_sort(const Launch &L, Margins m, DevScalars *d, Cells c, const long long *id, long ntags,
-                 const CullRec *cull) {
+void launch_sort(const Launch &L, Margins m, DevScalars *d, Cells c, const long long *id, const int *flume,
+                 NearLists near, long ntags, const CullRec *cull) {
   // Launch sizes follow the capacity; the kernels read the bucket count in use from the device,
   // so a captured graph stays valid across device-side re-grids.
   const long ntiles = scan_tiles(c.cap);
   k_scan_final<<<(unsigned)ntiles, kScanThreads, 0, L.st>>>(c.count, c.tile_count, c.start, d, L.n);
   if (L.n <= 0) return;
   const unsigned g = (unsigned)((L.n + 127) / 128);
-  k_scatter<<<g, 128, 0, L.st>>>(c.key, c.rank_tmp, c.start, c.tmp_slot, L.n);
+  k_scatter<<<g, 128, 0, L.st>>>(c.key, c.rank_tmp, c.start, c.tmp_slot, near.loose, L.n);
   k_rank<<<g, 128, 0, L.st>>>(c.key, c.start, c.tmp_slot, id, c.perm, cull, c.csort, c.count, c.tile_count, m, d,
-                              ntags, L.n);
+                              flume, near.loose, ntags, L.n);
 }
 
 }  // namespace af3d

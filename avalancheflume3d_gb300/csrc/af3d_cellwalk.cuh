@@ -229,6 +229,36 @@ __device__ __forceinline__ void for_slots_around(const CellAt &c, const GridF &g
     }
 }
 
+// Clump s, in cell `c` of key `key`, may meet clumps that their near lists do not hold: those around it as
+// built search for themselves from tick `from` on (a plain look first: most were marked before).
+__device__ __forceinline__ void mark_around(const CellAt &c, const GridF &g, long long off,
+                                            const int *__restrict__ start, const int *__restrict__ order, int *loose,
+                                            int from) {
+  for_slots_around(c, g, off, start, order, [&](int t) {
+    if (loose[t] > from) atomicMin(&loose[t], from);
+  });
+}
+
+// Clump s joins the chain of its cell's key for tick `from`; once for a clump and tick.
+__device__ __forceinline__ void join_chain(const NearLists &near, long s, int key, int from, long n) {
+  const long half = (from & 1) * n;
+  const unsigned long long old =
+      atomicExch(&near.chain[half + key % n], (unsigned long long)(unsigned)from << 32 | (unsigned)s);
+  near.chain_next[half + s] = (unsigned)(old >> 32) == (unsigned)from ? (int)(unsigned)old : -1;
+}
+
+// Visits the runaways in cell `key` at tick `tick`.
+template <typename F>
+__device__ __forceinline__ void for_chain(const NearLists &near, const CullRec *__restrict__ cull, int key, int tick,
+                                          long n, F &&f) {
+  const long half = (tick & 1) * n;
+  const unsigned long long head = near.chain[half + key % n];
+  int t = (unsigned)(head >> 32) == (unsigned)tick ? (int)(unsigned)head : -1;
+#pragma unroll 1
+  for (; t >= 0; t = near.chain_next[half + t])
+    if (cull[t].key == key) f(t);
+}
+
 // A clump's list layout: `pre` boundary items, then `pair` particle items, then the rest.
 struct ListCounts {
   int pre, pair;

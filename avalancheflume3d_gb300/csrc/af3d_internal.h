@@ -221,8 +221,7 @@ struct DevScalars {
   long long       ncell_total; // sum of the flumes' ncell3: the first removed-clump bucket
   long long       pending;     // > 0: a re-grid derived grids needing this many cell buckets
   int             tick;        // steps begun (counts with the clock)
-  int             all_slow;    // from this tick on every clump takes the per-clump search ...
-  int             brute;       // ... over every clump of its flume (until the lists are built again)
+  int             runaway;     // from this tick on a search looks at the runaways' chains too (NearLists)
   unsigned        ticket;      // blocks of a force pass that have finished
   DevFlume       *flumes;      // [nflumes]
 };
@@ -281,7 +280,11 @@ __host__ __device__ inline int pack_list_counts(int listed, int pre, int pair) {
 // current cells, so a step's contacts and their order do not depend on when the lists were
 // built.  What a clump may still move is counted down (`rem`); one that used it up marks every
 // clump around it `loose` from the next step on, and a loose clump searches the cells around
-// itself (as built) in place of its list.  Measured against a sort and a walk every step:
+// itself (as built) in place of its list.  A clump that moved about a cell (a runaway) is no longer near
+// the cell it was built in: it joins the chain of the cell it is in, which the searches of the clumps
+// around that cell follow, so that however fast it is it costs them alone.  A clump too large for the
+// lists (beyond_reach) has used up its allowance from the start.  Clumps in no cell (removed, not
+// finite) meet nobody and mark nobody.  Measured against a sort and a walk every step:
 // 2,048 clumps (fast) 48 -> 37 us a step, 20,011 in the hopper (exact) 82 -> 75, 262,144 (fast)
 // 0.325 -> 0.296 ms with the copies of a 40-step call, (exact) 0.49 -> 0.46.
 constexpr int kNearCap = 60;
@@ -295,6 +298,11 @@ struct NearLists {
   unsigned *bnd;     // [n] bit 4 * routine + sphere
   float *rem;        // [n] cm the clump may still move
   int *loose;        // [n] the tick from which the list does not hold (never: INT_MAX)
+  // The runaways' chains, of odd and even ticks (a pass follows one while it makes the next): a cell's
+  // chain starts at entry key mod n with tick << 32 | slot (an older tick: empty) and goes on
+  // at chain_next (-1: the end); it holds the clumps of all cells with that remainder.
+  unsigned long long *chain;   // [2][n]
+  int *chain_next;             // [2][n]
 };
 
 // The next step's predictor run at the end of a force pass (look-ahead): the corrected clump is
@@ -332,10 +340,10 @@ void launch_predict (const Launch &L, Planes cur, DevScalars *d, bool predict, b
 // Exclusive scan of the bucket counts, scatter by arrival, then the deterministic (bucket, id)
 // rank: fills cells.start[0..nbuckets] and cells.perm, checks the ntags capacity and leaves the
 // count array zeroed.  nbuckets = ncell_total + N is read on the device.
-// With cull (records already written at the old slots) also fills cells.csort and lowers d->all_slow for
-// a clump beyond the near lists' reach.
-void launch_sort (const Launch &L, Margins m, DevScalars *d, Cells cells, const long long *id, long ntags,
-                  const CullRec *cull = nullptr);
+// With cull (records already written at the old slots) also fills cells.csort and marks the clumps
+// around one beyond the near lists' reach.
+void launch_sort (const Launch &L, Margins m, DevScalars *d, Cells cells, const long long *id, const int *flume,
+                  NearLists near, long ntags, const CullRec *cull = nullptr);
 long scan_tiles (long bucket_cap);
 // Moves every plane (and the id and flume arrays) into the new order and builds the records.
 // `ft`: also carry the force/torque accumulators and a_f (the fused step rewrites them first).

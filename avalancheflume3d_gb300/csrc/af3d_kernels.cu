@@ -522,24 +522,26 @@ __device__ __forceinline__ long bucket_key(V3 r, const DevFlume &fl, DevScalars 
 // A clump's place in a step that keeps its near lists: counted in its cell for the capacity check
 // of cells.cu:96-102 (at most ntags - 1 clumps), and its motion since the previous step's record
 // (old) against its allowance.  With none left, the clumps that may now meet it unlisted -- all
-// within the 5 x 5 x 5 cells around it in the built order, as long as nothing has moved a cell
-// further than its allowance -- search for themselves from tick `from` on.
+// within the 5 x 5 x 5 cells around it in the built order, as long as neither moved a cell further
+// than its allowance -- search for themselves from tick `from` on; beyond that it is a runaway.
 __device__ __forceinline__ void keep_place(long s, const int4 *old, const CullRec &cr, const DevFlume &fl,
                                            DevScalars *d, int *occ, long ntags, const NearLists &near,
                                            const int *__restrict__ start, const int *__restrict__ order, Margins m,
-                                           int from) {
+                                           int from, long n) {
   if (ntags > 0 && cr.key < d->ncell_total && atomicAdd(&occ[cr.key], 1) + 1 >= ntags)
     raise_status(d, AF3D_ERR_CELL_CAPACITY);
   const float rem = near.rem[s] - sphere_motion(old, cr, m.qs);
   near.rem[s] = rem;
-  if (rem >= 0.0f) return;
   const GridF &g = fl.gridf;
-  const float side = fminf(fminf(1.0f / g.ix, 1.0f / g.iy), 1.0f / g.iz);
   CellAt c;
-  if (!(rem > m.cap - 0.9f * side)) atomicMin(&d->brute, from);   // (NaN too)
-  else if (cell_at(cr.key, fl.cell_off, g, c))
-    for_slots_around(c, g, fl.cell_off, start, order, [&](int t) { atomicMin(&near.loose[t], from); });
+  if (rem >= 0.0f || !cell_at(cr.key, fl.cell_off, g, c)) return;
+  mark_around(c, g, fl.cell_off, start, order, near.loose, from);
   atomicMin(&near.loose[s], from);
+  const float side = fminf(fminf(1.0f / g.ix, 1.0f / g.iy), 1.0f / g.iz);
+  if (!(rem > m.cap - 0.9f * side)) {
+    join_chain(near, s, cr.key, from, n);
+    atomicMin(&d->runaway, from);
+  }
 }
 
 // init_Verlet.cu:25-148 for one clump (PREDICT), and/or cell_locate's binning (cells.cu:60-92)
@@ -604,7 +606,7 @@ __global__ void __launch_bounds__(kBlock) k_predict(Planes P, DevScalars *d, boo
       if (count_only) {
         int4 old[4];
         for (int k = 0; k < 4; k++) old[k] = cull[s].s[k];
-        keep_place(s, old, cr, fl, d, cells.occ, ntags, near, cells.start, order, P.m, d->tick);
+        keep_place(s, old, cr, fl, d, cells.occ, ntags, near, cells.start, order, P.m, d->tick, n);
       }
     }
   }
@@ -846,7 +848,7 @@ __device__ __forceinline__ Own own_from_planes(const Planes &P, long s) {
 // The next particle contact of clump s after the one of order key `done`, in the reference's order:
 // by sph_id, then the partner's cell in the 27-cell visiting order, then its id
 // (force_part.cu:88-106).  The candidates are the clumps of the 5 x 5 x 5 cells around it in the
-// built order (brute: every clump of its flume).  exact: overlapping pairs only, else those the
+// built order and, with `away`, the runaways in the 27 cells around it.  exact: overlapping pairs only, else those the
 // tests in units cannot rule out (the items of the lists).  Returns the key, ~0 after the last
 // pair; item: partner slot << 4 | sph_id - 1.
 __device__ __forceinline__ unsigned long long next_contact(long s, const DevScalars *d, const int *__restrict__ flume,
@@ -854,8 +856,9 @@ __device__ __forceinline__ unsigned long long next_contact(long s, const DevScal
                                                            const CullRec *__restrict__ cull,
                                                            const int *__restrict__ start,
                                                            const int *__restrict__ order,
-                                                           const long long *__restrict__ id, bool brute, long n,
-                                                           bool exact, unsigned long long done, unsigned &item) {
+                                                           const long long *__restrict__ id,
+                                                           const NearLists &near, bool away, long n, bool exact,
+                                                           unsigned long long done, unsigned &item) {
   const int f = flume[s];
   const DevFlume &fl = d->flumes[f];
   const GridF &g = fl.gridf;
@@ -889,11 +892,15 @@ __device__ __forceinline__ unsigned long long next_contact(long s, const DevScal
     }
   };
   CellAt at;
-  if (brute) {
-    for (long t = 0; t < n; t++)
-      if (flume[t] == f) look((int)t);
-  } else if (cell_at(me.key, fl.cell_off, g, at)) {
-    for_slots_around(at, g, fl.cell_off, start, order, look);
+  if (cell_at(me.key, fl.cell_off, g, at)) for_slots_around(at, g, fl.cell_off, start, order, look);
+  if (away) {
+    const int tick = d->tick;
+#pragma unroll 1
+    for (int k = 0; k < 27; k++) {
+      const long x = q.ci + k / 9 - 1, y = q.cj + k / 3 % 3 - 1, z = q.ck + k % 3 - 1;
+      if (x < 0 || y < 0 || z < 0 || x >= g.nx || y >= g.ny || z >= g.nz) continue;
+      for_chain(near, cull, (int)(fl.cell_off + x + (long)g.nx * (y + (long)g.ny * z)), tick, n, look);
+    }
   }
   return best;
 }
@@ -905,11 +912,11 @@ __device__ __forceinline__ unsigned long long next_contact(long s, const DevScal
 __device__ __noinline__ int search_items(long s, const DevScalars *d, const int *__restrict__ flume,
                                           const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
                                           const int *__restrict__ start, const int *__restrict__ order,
-                                          const long long *__restrict__ id, bool brute, long n, unsigned *col,
-                                          int nitems) {
+                                          const long long *__restrict__ id, const NearLists &near, bool away, long n,
+                                          unsigned *col, int nitems) {
   unsigned item = 0u;
   for (unsigned long long done = 0ull;;) {
-    done = next_contact(s, d, flume, nbr, cull, start, order, id, brute, n, false, done, item);
+    done = next_contact(s, d, flume, nbr, cull, start, order, id, near, away, n, false, done, item);
     if (done == ~0ull) return nitems;
     if (nitems == kListCap) return -1;
     col[n * nitems++] = item;
@@ -928,7 +935,8 @@ __device__ __noinline__ SlowSums slow_contacts(long s, int pre0, int pre1, int p
                                                const DevScalars *d, const int *__restrict__ flume,
                                                const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
                                                const int *__restrict__ start, const int *__restrict__ order,
-                                               const long long *__restrict__ id, bool brute, long n, V3 F, V3 T) {
+                                               const long long *__restrict__ id, const NearLists &near, bool away,
+                                               long n, V3 F, V3 T) {
   const Own o = own_from_record(nbr[s]);
   const double B = (double)cull[s].c.w;
   for (int rt = pre0; rt <= pre1; rt++)
@@ -937,7 +945,7 @@ __device__ __noinline__ SlowSums slow_contacts(long s, int pre0, int pre1, int p
   int active = 0;
   unsigned item = 0u;
   for (unsigned long long done = 0ull;;) {
-    done = next_contact(s, d, flume, nbr, cull, start, order, id, brute, n, true, done, item);
+    done = next_contact(s, d, flume, nbr, cull, start, order, id, near, away, n, true, done, item);
     if (done == ~0ull) break;
     const int p = (int)(item & 15u);
     active += part_pair(o.r, o.v, o.w, o.s[p & 3], o.rad, o.msph, nbr[item >> 4], p >> 2, c, xi0, F, T) == 2;
@@ -986,7 +994,8 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
                                               const CullRec *__restrict__ cull,
                                               const int *__restrict__ start,
                                               const int *__restrict__ order, const long long *__restrict__ id,
-                                              bool brute, const unsigned *items, int listed, ListCounts lc, long n,
+                                              const NearLists &near, bool away, const unsigned *items, int listed,
+                                              ListCounts lc, long n,
                                               V3 &F, V3 &T) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pre0 = aval ? R_HOP0 : 1, pre1 = aval ? R_WALLS : 0;         // fill: none before
@@ -1078,8 +1087,8 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
     __syncthreads();
   }
   if (slow) {
-    const SlowSums r = slow_contacts(s, pre0, pre1, post0, post1, c, d, flume, nbr, cull, start, order, id, brute, n,
-                                     F, T);
+    const SlowSums r = slow_contacts(s, pre0, pre1, post0, post1, c, d, flume, nbr, cull, start, order, id, near, away,
+                                     n, F, T);
     F = r.F;
     T = r.T;
     active += r.active;
@@ -1182,11 +1191,12 @@ __device__ __forceinline__ int near_pairs(long s, int entries, const DevFlume &f
 __device__ __forceinline__ unsigned bits_before(bool aval) { return aval ? 0x00FFFFFFu : 0u; }
 __device__ __forceinline__ unsigned bits_after(bool aval) { return aval ? 0x0F000000u : 0x00000FFFu; }
 
-// Whether clump s must search for its pairs because its near list does not hold.
-__device__ __forceinline__ bool must_search(long s, const DevScalars *d, const NearLists &near, int info, bool &brute) {
+// Whether clump s must search for its pairs because its near list does not hold; away: there are
+// runaways to look for.
+__device__ __forceinline__ bool must_search(long s, const DevScalars *d, const NearLists &near, int info, bool &away) {
   const int tick = d->tick;
-  brute = d->brute <= tick;
-  return info < 0 || near.loose[s] <= tick || d->all_slow <= tick || brute;
+  away = d->runaway <= tick;
+  return info < 0 || near.loose[s] <= tick;
 }
 
 // The list phase of k_lists_forces for one clump: its item list (see block_contacts) from its near
@@ -1198,16 +1208,16 @@ __device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, 
                                           const int *__restrict__ start, const int *__restrict__ order,
                                           const long long *__restrict__ id, const NearLists &near,
                                           ContactLists lists, long s0, long n, Margins m, PassLists &pl,
-                                          ListCounts &lc, bool &brute, bool &overflow) {
+                                          ListCounts &lc, bool &away, bool &overflow) {
   const int lane = threadIdx.x & 31;
   const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
   lc.pre = lc.pair = 0;
-  brute = overflow = false;
+  away = overflow = false;
   if (s >= n) return 0;
   const NbrRec &me = nbr[s];
   if (is_removed(*c.tp, me.rx, c.side_x)) return 0;
   const int info = near.info[s];
-  const bool search = must_search(s, d, near, info, brute);
+  const bool search = must_search(s, d, near, info, away);
   overflow = info < 0;
   const bool aval = c.phase == AF3D_PHASE_AVALANCHE;
   const float rad = __int_as_float(cull[s].s[0].w) * unit_power(-m.qs);
@@ -1218,7 +1228,7 @@ __device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, 
   int nitems = 0;
   for (; before; before &= before - 1u) col[n * nitems++] = kBndItem | ((unsigned)__ffs(before) - 1u);
   if (search) {
-    nitems = search_items(s, d, flume, nbr, cull, start, order, id, brute, n, col, nitems);
+    nitems = search_items(s, d, flume, nbr, cull, start, order, id, near, away, n, col, nitems);
     if (nitems < 0) return -1;
   } else {
     const unsigned *list = near.items + s;
@@ -1260,7 +1270,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
                                            const CullRec *__restrict__ cull, const Cells &cells,
                                            const int *__restrict__ order, const long long *__restrict__ id,
                                            const NearLists &near, ContactLists lists, int listed, ListCounts lc,
-                                           bool brute, bool overflow, long ntags, bool counted, long s0, long n,
+                                           bool away, bool overflow, long ntags, bool counted, long s0, long n,
                                            bool warm,
                                            const LookAhead &la, ForceShared<NB> &sh) {
   const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -1277,7 +1287,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
   }
   const long bbase = s0 + blockIdx.x * (long)blockDim.x;
   const int active = block_contacts<NB, UNIFORM>(sh.bq, bbase, sv, valid && !removed, aval, c, d, flume, nbr, cull,
-                                                 cells.start, order, id, brute, lists.items, valid ? listed : 0, lc,
+                                                 cells.start, order, id, near, away, lists.items, valid ? listed : 0, lc,
                                                  n, F, T);
   if (la.nbr) __syncthreads();   // the force phase's shared memory is free for the record staging
   if (valid) {
@@ -1360,7 +1370,8 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
         } else {
           int4 old[4];
           for (int k = 0; k < 4; k++) old[k] = cull[s].s[k];
-          keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1);
+          keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1,
+                     n);
         }
       }
     }
@@ -1686,13 +1697,13 @@ __global__ void __launch_bounds__(NB, MINB)
                    long n) {
   __shared__ ForceShared<NB> sh;
   ListCounts lc;
-  bool brute, overflow;
+  bool away, overflow;
   auto body = [&](const Consts &c) {
     const int listed = lists_body(c, d, flume, nbr, cull, cells.start, order, id, near, lists, s0, n, P.m,
-                                  sh.pl[threadIdx.x >> 5], lc, brute, overflow);
+                                  sh.pl[threadIdx.x >> 5], lc, away, overflow);
     overflow = overflow || listed < 0;
     __syncthreads();
-    fused_body<NB, WRITE_FT, UNIFORM>(c, P, out, d, flume, nbr, cull, cells, order, id, near, lists, listed, lc, brute,
+    fused_body<NB, WRITE_FT, UNIFORM>(c, P, out, d, flume, nbr, cull, cells, order, id, near, lists, listed, lc, away,
                                       overflow, ntags, counted, s0, n, warm, la, sh);
   };
   if constexpr (UNIFORM) {

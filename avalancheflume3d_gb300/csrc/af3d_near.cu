@@ -3,8 +3,6 @@
 //
 // Integer and FP32 work on the culling records; built from the sorted cell list once every
 // kBuildEvery steps.
-#include <climits>
-
 #include "af3d_cellwalk.cuh"
 
 namespace af3d {
@@ -52,8 +50,7 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
   const float sum = fabsf(mc.x) + fabsf(mc.y) + fabsf(mc.z);
   const bool coarse = beyond_reach(rec, m);
   if (w == 0 && valid) {
-    near.loose[s] = INT_MAX;
-    near.rem[s] = allow * (1.0f - 1e-5f);
+    near.rem[s] = coarse ? -1e-30f : allow * (1.0f - 1e-5f);   // (none left, yet not a runaway)
     // boundaries: the routines' gates are 1-Lipschitz in the sphere centre, so the allowance adds
     // to the bound; a door that is closed now may open, one that is open stays open
     const Consts &c = fl.c;
@@ -63,8 +60,9 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
     for (int rt = R_HOP0; rt <= last; rt++)
       if (bnd_may_touch_f(rt, mc, mc.w + grown, c, door_closed)) bnd |= 15u << (4 * rt);
     near.bnd[s] = bnd;
-    // every clump searches for itself (with `order` the sort has said so)
-    if (coarse && !order) atomicMin(&d->all_slow, d->tick);
+    CellAt at;   // (with `order` the sort has marked them)
+    if (coarse && !order && cell_at(rec.key, fl.cell_off, g, at))
+      mark_around(at, g, fl.cell_off, start, order, near.loose, d->tick);
   }
   // the cells within reach of any partner's bound and allowance, FP32 with slack
   const float most = m.most + 1e-6f * (sum + 20.0f) + m.cap;

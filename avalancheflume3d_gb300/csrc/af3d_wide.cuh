@@ -66,14 +66,14 @@ __global__ void __launch_bounds__(kWideThreads, 4)
     const bool removed = is_removed(*c.tp, me.rx, c.side_x), act = valid && !removed;
     const bool aval = c.phase == AF3D_PHASE_AVALANCHE, dev = c.variant == AF3D_FRICTION_DEV;
     const int info = near.info[sv];
-    bool brute = false;
-    const bool search = act && must_search(sv, d, near, info, brute);
+    bool away = false;
+    const bool search = act && must_search(sv, d, near, info, away);
     const unsigned *list = near.items + sv;
     unsigned *col = lists.items + sv;
     // the clumps' items: near pairs (warp 0), boundary spheres (warp 1)
     if (w == 0) {
       int np = 0;
-      if (search) np = search_items(sv, d, flume, nbr, cull, cells.start, order, id, brute, n, col, 0);
+      if (search) np = search_items(sv, d, flume, nbr, cull, cells.start, order, id, near, away, n, col, 0);
       else if (act) np = near_pairs(sv, info, fl, me, cull, list, n, sh.pl);
       sh.npair[lane] = np;
     } else if (w == 1) {
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
       const int post0 = aval ? R_FLUME : R_HOP0, post1 = aval ? R_FLUME : R_HOP2;
       const V3 zero = mk(0.0, 0.0, 0.0);
       const SlowSums r = slow_contacts(sv, pre0, pre1, post0, post1, c, d, flume, nbr, cull, cells.start, order, id,
-                                       brute, n, zero, zero);
+                                       near, away, n, zero, zero);
       if (w < 3) {
         Fi = comp(r.F, w);
         Ti = comp(r.T, w);
@@ -442,7 +442,8 @@ __global__ void __launch_bounds__(kWideThreads, 4)
         } else {
           int4 old[4];
           for (int k = 0; k < 4; k++) old[k] = cull[s].s[k];
-          keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1);
+          keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1,
+                     n);
         }
       }
     } else {
