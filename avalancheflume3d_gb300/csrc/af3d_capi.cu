@@ -690,7 +690,7 @@ af3d_status af3d_create_ensemble(int nflumes, const af3d_system_par *sys, const 
   ds.variant = c->variant;
   ds.nflumes = nflumes;
   ds.flumes = c->flumes;
-  ds.runaway = INT_MAX;
+  ds.away = INT_MAX;
   cudaMemsetAsync(c->near.chain, 0, sizeof(unsigned long long) * 2 * n, c->st);
   cudaMemsetAsync(c->plane_mem[0], 0, sizeof(double) * n * NPLANES, c->st);
   cudaMemsetAsync(c->plane_mem[1], 0, sizeof(double) * n * NPLANES, c->st);

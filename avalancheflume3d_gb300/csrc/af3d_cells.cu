@@ -73,10 +73,10 @@ __device__ __forceinline__ long n_buckets(const DevScalars *d, long n) { return 
 
 // Each tile adds the clump counts of the tiles before it (counted at arrival; integer sums are
 // exact in any order), then scans its own buckets.
-// Lists are built from the sort, so the runaways and marks since the last ones are void (k_scatter).
+// Lists are built from the sort, so the chains and marks since the last ones are void (k_scatter).
 __global__ void k_scan_final(const int *__restrict__ count, const int *__restrict__ tile_count,
                              int *start, DevScalars *d, long n) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) d->runaway = INT_MAX;
+  if (blockIdx.x == 0 && threadIdx.x == 0) d->away = INT_MAX;
   const long nb = n_buckets(d, n);
   if (blockIdx.x == 0 && threadIdx.x == 0) start[nb] = (int)n;   // every clump has one bucket
   if (blockIdx.x * (long)kTile >= nb) return;   // a tile past the buckets in use
@@ -122,7 +122,8 @@ __global__ void k_scatter(const int *__restrict__ key, const int *__restrict__ r
 __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ start,
                        const int *__restrict__ tmp_slot, const long long *__restrict__ id, int *perm,
                        const CullRec *__restrict__ cull, float4 *csort, int *count, int *tile_count,
-                       Margins m, DevScalars *d, const int *__restrict__ flume, int *loose, long ntags, long n) {
+                       const __grid_constant__ Margins m, DevScalars *d, const int *__restrict__ flume,
+                       const __grid_constant__ NearLists near, long ntags, long n) {
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (s >= n) return;
   const long ncell3 = d->ncell_total;
@@ -142,7 +143,7 @@ __global__ void k_rank(const int *__restrict__ key, const int *__restrict__ star
     const DevFlume &fl = d->flumes[flume[s]];
     CellAt at;
     if (beyond_reach(cull[s], m) && cell_at(k, fl.cell_off, fl.gridf, at))
-      mark_around(at, fl.gridf, fl.cell_off, start, tmp_slot, loose, d->tick);
+      go_away(s, cull[s].c, k, at, m, fl, d, start, tmp_slot, near, d->tick, n);
   }
   // cells.cu:96-102: a cell may hold at most ntags - 1 clumps
   if (ntags > 0 && k < ncell3 && r == 0 && (e - b) >= ntags)
@@ -163,7 +164,7 @@ void launch_sort(const Launch &L, Margins m, DevScalars *d, Cells c, const long 
   const unsigned g = (unsigned)((L.n + 127) / 128);
   k_scatter<<<g, 128, 0, L.st>>>(c.key, c.rank_tmp, c.start, c.tmp_slot, near.loose, L.n);
   k_rank<<<g, 128, 0, L.st>>>(c.key, c.start, c.tmp_slot, id, c.perm, cull, c.csort, c.count, c.tile_count, m, d,
-                              flume, near.loose, ntags, L.n);
+                              flume, near, ntags, L.n);
 }
 
 }  // namespace af3d

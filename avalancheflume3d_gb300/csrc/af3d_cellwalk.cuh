@@ -213,41 +213,87 @@ __device__ __forceinline__ bool cell_at(int key, long long off, const GridF &g, 
   return true;
 }
 
-// Visits the slots that the last built cell order holds in the 5 x 5 x 5 cells around `c`.
+// The cells that a bounding sphere of `reach` around `c` meets, in FP32 with slack.
+struct CellRange {
+  int x0, x1, y0, y1, z0, z1;
+};
+__device__ __forceinline__ CellRange cells_within(float4 c, float reach, const GridF &g) {
+  auto range = [&](float x, float xmin, float inv, int cells, int &lo, int &hi) {
+    const float q = (x - xmin) * inv, r = reach * inv;
+    const float e = 2e-6f * ((fabsf(x) + fabsf(xmin)) * inv + fabsf(q) + r + 1.0f);
+    lo = (int)fminf(fmaxf(floorf(q - r - e), 0.0f), (float)(cells - 1));
+    hi = (int)fminf(fmaxf(floorf(q + r + e), 0.0f), (float)(cells - 1));
+  };
+  CellRange b;
+  range(c.x, g.xmin, g.ix, g.nx, b.x0, b.x1);
+  range(c.y, g.ymin, g.iy, g.ny, b.y0, b.y1);
+  range(c.z, g.zmin, g.iz, g.nz, b.z0, b.z1);
+  return b;
+}
+
+// The largest bounding radius and allowance of a clump of the near lists, about the centre c.
+__device__ __forceinline__ float partner_reach(float4 c, const Margins &m) {
+  return m.most + 1e-6f * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z) + 20.0f) + m.cap;
+}
+
+// Visits the slots of the clumps that may touch a clump with the bounding sphere c (radius c.w) in cell
+// `at` and are not away: in the last built cell order, where none of them is further than its allowance
+// from its place.  Whatever c.w is, that is the cells next to `at` (contacts are between neighbour
+// cells) and as many more as an allowance spans.
 template <typename F>
-__device__ __forceinline__ void for_slots_around(const CellAt &c, const GridF &g, long long off,
-                                                 const int *__restrict__ start, const int *__restrict__ order, F &&f) {
-  const int x0 = max(c.x - 2, 0), x1 = min(c.x + 2, g.nx - 1);
+__device__ __forceinline__ void for_slots_around(float4 c, const CellAt &at, const Margins &m, const GridF &g,
+                                                 long long off, const int *__restrict__ start,
+                                                 const int *__restrict__ order, F &&f) {
+  CellRange b = cells_within(c, (c.w + partner_reach(c, m)) * (1.0f + 1e-5f), g);
+  auto clip = [&](int &lo, int &hi, int k, float inv) {
+    const int more = 2 + (int)fminf(m.cap * inv, 1e6f);
+    lo = max(lo, k - more);
+    hi = min(hi, k + more);
+  };
+  clip(b.x0, b.x1, at.x, g.ix);
+  clip(b.y0, b.y1, at.y, g.iy);
+  clip(b.z0, b.z1, at.z, g.iz);
+  if (b.x0 > b.x1 || b.y0 > b.y1 || b.z0 > b.z1) return;
+  const int ny = b.y1 - b.y0 + 1, rows = ny * (b.z1 - b.z0 + 1);
 #pragma unroll 1
-  for (int z = max(c.z - 2, 0); z <= min(c.z + 2, g.nz - 1); z++)
-#pragma unroll 1
-    for (int y = max(c.y - 2, 0); y <= min(c.y + 2, g.ny - 1); y++) {
-      const int *row = start + off + (long long)g.nx * (y + (long long)g.ny * z);
-      const int t1 = __ldg(row + x1 + 1);
-#pragma unroll 1
-      for (int t = __ldg(row + x0); t < t1; t++) f(order ? __ldg(&order[t]) : t);
+  for (int r0 = 0; r0 < rows; r0 += 4) {   // four rows' ends side by side
+    int k[4], end[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      k[q] = end[q] = 0;
+      if (r0 + q < rows) {
+        const int z = (r0 + q) / ny, y = r0 + q - z * ny;
+        const int *row = start + off + (long long)g.nx * (b.y0 + y + (long long)g.ny * (b.z0 + z));
+        k[q] = __ldg(row + b.x0);
+        end[q] = __ldg(row + b.x1 + 1);
+      }
     }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll 1
+      for (; k[q] < end[q]; k[q]++) f(order ? __ldg(&order[k[q]]) : k[q]);
+  }
 }
 
-// Clump s, in cell `c` of key `key`, may meet clumps that their near lists do not hold: those around it as
-// built search for themselves from tick `from` on (a plain look first: most were marked before).
-__device__ __forceinline__ void mark_around(const CellAt &c, const GridF &g, long long off,
-                                            const int *__restrict__ start, const int *__restrict__ order, int *loose,
-                                            int from) {
-  for_slots_around(c, g, off, start, order, [&](int t) {
-    if (loose[t] > from) atomicMin(&loose[t], from);
-  });
-}
-
-// Clump s joins the chain of its cell's key for tick `from`; once for a clump and tick.
-__device__ __forceinline__ void join_chain(const NearLists &near, long s, int key, int from, long n) {
-  const long half = (from & 1) * n;
+// Clump s with the bounding sphere c, in cell `at` of bucket `key`, is away at tick `tick`: it joins the
+// chain of its cell, and the clumps around it, whose near lists may not hold it, are loose (a plain
+// look first: most were marked before).  Once for a clump and tick.  Not inlined: rare.
+static __device__ __noinline__ void go_away(long s, float4 c, int key, CellAt at, const Margins &m, const DevFlume &fl,
+                                            DevScalars *d, const int *__restrict__ start,
+                                            const int *__restrict__ order, const NearLists &near, int tick, long n) {
+  const long half = (tick & 1) * n;
   const unsigned long long old =
-      atomicExch(&near.chain[half + key % n], (unsigned long long)(unsigned)from << 32 | (unsigned)s);
-  near.chain_next[half + s] = (unsigned)(old >> 32) == (unsigned)from ? (int)(unsigned)old : -1;
+      atomicExch(&near.chain[half + key % n], (unsigned long long)(unsigned)tick << 32 | (unsigned)s);
+  near.chain_next[half + s] = (unsigned)(old >> 32) == (unsigned)tick ? (int)(unsigned)old : -1;
+  if (d->away > tick) atomicMin(&d->away, tick);
+  auto mark = [&](int t) {
+    if (near.loose[t] > tick) atomicMin(&near.loose[t], tick);
+  };
+  for_slots_around(c, at, m, fl.gridf, fl.cell_off, start, order, mark);
+  mark((int)s);
 }
 
-// Visits the runaways in cell `key` at tick `tick`.
+// Visits the clumps away in cell `key` at tick `tick`.
 template <typename F>
 __device__ __forceinline__ void for_chain(const NearLists &near, const CullRec *__restrict__ cull, int key, int tick,
                                           long n, F &&f) {

@@ -66,7 +66,8 @@ struct __align__(16) CullRec {
   int4 s[4];
   int key;       // the clump's bucket at this step (cell order of the contacts)
   float allow;   // how far it may move from here (Margins)
-  int pad[2];
+  int away;      // it is in a chain (NearLists)
+  int pad;
 };
 
 // A clump of extent + radius above this many units has an infinite radius in its record: every
@@ -221,7 +222,7 @@ struct DevScalars {
   long long       ncell_total; // sum of the flumes' ncell3: the first removed-clump bucket
   long long       pending;     // > 0: a re-grid derived grids needing this many cell buckets
   int             tick;        // steps begun (counts with the clock)
-  int             runaway;     // from this tick on a search looks at the runaways' chains too (NearLists)
+  int             away;        // from this tick on there are clumps in the chains of NearLists
   unsigned        ticket;      // blocks of a force pass that have finished
   DevFlume       *flumes;      // [nflumes]
 };
@@ -278,13 +279,12 @@ __host__ __device__ inline int pack_list_counts(int listed, int pre, int pair) {
 // clump of a dense bed instead of ~300 behind nine dependent reads of the cell table.  Each pass
 // tests the listed pairs at the current positions and orders the overlapping ones by the
 // current cells, so a step's contacts and their order do not depend on when the lists were
-// built.  What a clump may still move is counted down (`rem`); one that used it up marks every
-// clump around it `loose` from the next step on, and a loose clump searches the cells around
-// itself (as built) in place of its list.  A clump that moved about a cell (a runaway) is no longer near
-// the cell it was built in: it joins the chain of the cell it is in, which the searches of the clumps
-// around that cell follow, so that however fast it is it costs them alone.  A clump too large for the
-// lists (beyond_reach) has used up its allowance from the start.  Clumps in no cell (removed, not
-// finite) meet nobody and mark nobody.  Measured against a sort and a walk every step:
+// built.  What a clump may still move is counted down (`rem`).  One that used it up is away from the
+// cell it was built in: it joins the chain of the cell it is in, and marks the clumps around it, found
+// in the built order, `loose` from the next step on.  A loose clump searches the cells around itself as
+// built and the chains in place of its list.  So however fast a clump is, it costs the clumps around it
+// alone.  A clump too large for the lists (beyond_reach) is away from the start; clumps in no cell
+// (removed, not finite) meet nobody and mark nobody.  Measured against a sort and a walk every step:
 // 2,048 clumps (fast) 48 -> 37 us a step, 20,011 in the hopper (exact) 82 -> 75, 262,144 (fast)
 // 0.325 -> 0.296 ms with the copies of a 40-step call, (exact) 0.49 -> 0.46.
 constexpr int kNearCap = 60;
@@ -298,9 +298,9 @@ struct NearLists {
   unsigned *bnd;     // [n] bit 4 * routine + sphere
   float *rem;        // [n] cm the clump may still move
   int *loose;        // [n] the tick from which the list does not hold (never: INT_MAX)
-  // The runaways' chains, of odd and even ticks (a pass follows one while it makes the next): a cell's
-  // chain starts at entry key mod n with tick << 32 | slot (an older tick: empty) and goes on
-  // at chain_next (-1: the end); it holds the clumps of all cells with that remainder.
+  // The chains of the clumps away, of odd and even ticks (a pass follows one while it makes the next):
+  // a cell's starts at entry key mod n with tick << 32 | slot (an older tick: empty) and goes on at
+  // chain_next (-1: the end); it holds the clumps of all cells with that remainder.
   unsigned long long *chain;   // [2][n]
   int *chain_next;             // [2][n]
 };

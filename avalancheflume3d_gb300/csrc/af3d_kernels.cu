@@ -203,7 +203,7 @@ __device__ __forceinline__ void make_records(V3 r, V3 v, V3 w, const V3 *sp, dou
   const float wx = magnitude_f(w.x), wy = magnitude_f(w.y), wz = magnitude_f(w.z);
   const float speed = sqrtf(vx * vx + vy * vy + vz * vz) + sqrtf(wx * wx + wy * wy + wz * wz) * bound;
   c.allow = fminf(m.per_speed * speed + m.floor, m.cap);   // cap for NaN
-  c.pad[0] = c.pad[1] = 0;
+  c.away = c.pad = 0;
 }
 
 // How far the spheres of a clump moved between two of its records, at most, in cm.  Differences
@@ -521,27 +521,19 @@ __device__ __forceinline__ long bucket_key(V3 r, const DevFlume &fl, DevScalars 
 
 // A clump's place in a step that keeps its near lists: counted in its cell for the capacity check
 // of cells.cu:96-102 (at most ntags - 1 clumps), and its motion since the previous step's record
-// (old) against its allowance.  With none left, the clumps that may now meet it unlisted -- all
-// within the 5 x 5 x 5 cells around it in the built order, as long as neither moved a cell further
-// than its allowance -- search for themselves from tick `from` on; beyond that it is a runaway.
-__device__ __forceinline__ void keep_place(long s, const int4 *old, const CullRec &cr, const DevFlume &fl,
-                                           DevScalars *d, int *occ, long ntags, const NearLists &near,
-                                           const int *__restrict__ start, const int *__restrict__ order, Margins m,
-                                           int from, long n) {
+// (old) against its allowance: with none left it is away at tick `tick`.
+__device__ __forceinline__ void keep_place(long s, const int4 *old, CullRec &cr, const DevFlume &fl, DevScalars *d,
+                                           int *occ, long ntags, const NearLists &near,
+                                           const int *__restrict__ start, const int *__restrict__ order,
+                                           const Margins &m, int tick, long n) {
   if (ntags > 0 && cr.key < d->ncell_total && atomicAdd(&occ[cr.key], 1) + 1 >= ntags)
     raise_status(d, AF3D_ERR_CELL_CAPACITY);
   const float rem = near.rem[s] - sphere_motion(old, cr, m.qs);
   near.rem[s] = rem;
-  const GridF &g = fl.gridf;
-  CellAt c;
-  if (rem >= 0.0f || !cell_at(cr.key, fl.cell_off, g, c)) return;
-  mark_around(c, g, fl.cell_off, start, order, near.loose, from);
-  atomicMin(&near.loose[s], from);
-  const float side = fminf(fminf(1.0f / g.ix, 1.0f / g.iy), 1.0f / g.iz);
-  if (!(rem > m.cap - 0.9f * side)) {
-    join_chain(near, s, cr.key, from, n);
-    atomicMin(&d->runaway, from);
-  }
+  CellAt at;
+  if (rem >= 0.0f || !cell_at(cr.key, fl.cell_off, fl.gridf, at)) return;
+  cr.away = 1;
+  go_away(s, cr.c, cr.key, at, m, fl, d, start, order, near, tick, n);
 }
 
 // init_Verlet.cu:25-148 for one clump (PREDICT), and/or cell_locate's binning (cells.cu:60-92)
@@ -552,9 +544,10 @@ __device__ __forceinline__ void keep_place(long s, const int4 *old, const CullRe
 // the clump's neighbour records at its own slot (steps that keep the slot order).  count_only: the
 // step does not sort but keeps its near lists (keep_place; with RECORDS).
 template <bool PREDICT, bool KEYS, bool RECORDS>
-__global__ void __launch_bounds__(kBlock) k_predict(Planes P, DevScalars *d, bool t_prev, Cells cells,
+__global__ void __launch_bounds__(kBlock) k_predict(const __grid_constant__ Planes P, DevScalars *d, bool t_prev, Cells cells,
                                                     const long long *__restrict__ id,
-                                                    const int *__restrict__ flume, long ntags, NearLists near,
+                                                    const int *__restrict__ flume, long ntags,
+                                                    const __grid_constant__ NearLists near,
                                                     const int *__restrict__ order, bool count_only, NbrRec *nbr,
                                                     CullRec *cull, long s0, long n) {
   __shared__ double s_nbr[RECORDS ? kPermBlock * kRecStride : 1];
@@ -845,82 +838,107 @@ __device__ __forceinline__ Own own_from_planes(const Planes &P, long s) {
   return o;
 }
 
-// The next particle contact of clump s after the one of order key `done`, in the reference's order:
-// by sph_id, then the partner's cell in the 27-cell visiting order, then its id
-// (force_part.cu:88-106).  The candidates are the clumps of the 5 x 5 x 5 cells around it in the
-// built order and, with `away`, the runaways in the 27 cells around it.  exact: overlapping pairs only, else those the
-// tests in units cannot rule out (the items of the lists).  Returns the key, ~0 after the last
-// pair; item: partner slot << 4 | sph_id - 1.
+// Visits the sphere pairs of clump s that the tests in units cannot rule out: the clumps around it in
+// the built order and those away in the 27 cells around it (an oversize clump may be both).
+// f(key, item): the pair's place in the reference's order -- by sph_id, then the partner's cell in the
+// 27-cell visiting order, then its id (force_part.cu:88-106) -- and partner slot << 4 | sph_id - 1.
+template <typename F>
+__device__ __forceinline__ void for_pairs(long s, const DevScalars *d, const int *__restrict__ flume,
+                                          const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
+                                          const int *__restrict__ start, const int *__restrict__ order,
+                                          const long long *__restrict__ id, const NearLists &near, const Margins &m,
+                                          long n, F &&f) {
+  const DevFlume &fl = d->flumes[flume[s]];
+  const GridF &g = fl.gridf;
+  const CullRec me = cull[s];
+  CellAt at;
+  if (!cell_at(me.key, fl.cell_off, g, at)) return;
+  const Search q = search_centre_f(me.c, mk(nbr[s].rx, nbr[s].ry, nbr[s].rz), fl.grid, g, 0);
+  auto look = [&](int t) {
+    unsigned mask = pair_mask(me, cull[t]);
+    CellAt a;
+    if (!mask || !cell_at(cull[t].key, fl.cell_off, g, a)) return;
+    const long dx = a.x - q.ci + 1, dy = a.y - q.cj + 1, dz = a.z - q.ck + 1;
+    if (dx < 0 || dx > 2 || dy < 0 || dy > 2 || dz < 0 || dz > 2) return;
+    const unsigned long long place = (unsigned long long)(9 * dx + 3 * dy + dz) << 32 | (unsigned long long)id[t];
+    while (mask) {
+      const int p = __ffs(mask) - 1;
+      mask &= mask - 1u;
+      f(((unsigned long long)(p * 27) << 32) + place + 1ull, (unsigned)t << 4 | (unsigned)p);
+    }
+  };
+  for_slots_around(me.c, at, m, g, fl.cell_off, start, order, [&](int t) {
+    if (t != s && !cull[t].away) look(t);
+  });
+  const int tick = d->tick;
+  if (d->away > tick) return;
+#pragma unroll 1
+  for (int k = 0; k < 27; k++) {
+    const long x = q.ci + k / 9 - 1, y = q.cj + k / 3 % 3 - 1, z = q.ck + k % 3 - 1;
+    if (x < 0 || y < 0 || z < 0 || x >= g.nx || y >= g.ny || z >= g.nz) continue;
+    for_chain(near, cull, (int)(fl.cell_off + x + (long)g.nx * (y + (long)g.ny * z)), tick, n, [&](int t) {
+      if (t != s) look(t);
+    });
+  }
+}
+
+// The particle items of a clump whose near list does not hold (too many entries, or a clump around it is
+// away): the items the list would have given, put in order as they are found.  To the column `col` from
+// entry `nitems` on; returns the entries then, -1 if they would overflow it.  Not inlined: rare.
+__device__ __noinline__ int search_items(long s, const DevScalars *d, const int *__restrict__ flume,
+                                          const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
+                                          const int *__restrict__ start, const int *__restrict__ order,
+                                          const long long *__restrict__ id, const NearLists &near, const Margins &m,
+                                          long n, unsigned *col, int nitems) {
+  unsigned long long keys[kListCap];
+  unsigned items[kListCap];
+  const int room = kListCap - nitems;
+  int found = 0;
+  bool over = false;
+  for_pairs(s, d, flume, nbr, cull, start, order, id, near, m, n, [&](unsigned long long key, unsigned item) {
+    int i = found;
+    while (i > 0 && keys[i - 1] > key) i--;
+    if (i > 0 && keys[i - 1] == key) return;
+    if (found == room) {
+      over = true;
+      return;
+    }
+    for (int j = found++; j > i; j--) {
+      keys[j] = keys[j - 1];
+      items[j] = items[j - 1];
+    }
+    keys[i] = key;
+    items[i] = item;
+  });
+  if (over) return -1;
+  for (int i = 0; i < found; i++) col[n * nitems++] = items[i];
+  return nitems;
+}
+
+// The next overlapping sphere pair of clump s after the one of key `done` (for_pairs): its key, ~0 after
+// the last one.
 __device__ __forceinline__ unsigned long long next_contact(long s, const DevScalars *d, const int *__restrict__ flume,
                                                            const NbrRec *__restrict__ nbr,
                                                            const CullRec *__restrict__ cull,
                                                            const int *__restrict__ start,
                                                            const int *__restrict__ order,
                                                            const long long *__restrict__ id,
-                                                           const NearLists &near, bool away, long n, bool exact,
+                                                           const NearLists &near, const Margins &m, long n,
                                                            unsigned long long done, unsigned &item) {
-  const int f = flume[s];
-  const DevFlume &fl = d->flumes[f];
-  const GridF &g = fl.gridf;
-  const CullRec me = cull[s];
   const NbrRec &mine = nbr[s];
-  const Search q = search_centre_f(me.c, mk(mine.rx, mine.ry, mine.rz), fl.grid, g, 0);
   unsigned long long best = ~0ull;
-  auto look = [&](int t) {
-    if (t == s) return;
-    unsigned mask = pair_mask(me, cull[t]);
-    CellAt a;
-    if (!mask || !cell_at(cull[t].key, fl.cell_off, g, a)) return;
-    const long dx = a.x - q.ci + 1, dy = a.y - q.cj + 1, dz = a.z - q.ck + 1;
-    if (dx < 0 || dx > 2 || dy < 0 || dy > 2 || dz < 0 || dz > 2) return;
-    while (mask) {
-      const int p = __ffs(mask) - 1;
-      mask &= mask - 1u;
-      const unsigned long long key =
-          ((unsigned long long)(p * 27 + (int)(9 * dx + 3 * dy + dz)) << 32 | (unsigned long long)id[t]) + 1ull;
-      if (key <= done || key >= best) continue;
-      if (exact) {
-        V3 dd;
-        double dist2, sep;
-        const int k = p & 3;
-        if (!spheres_overlap(mk(mine.s[3 * k], mine.s[3 * k + 1], mine.s[3 * k + 2]), mine.rad, nbr[t], p >> 2, dd,
-                             dist2, sep))
-          continue;
-      }
-      best = key;
-      item = (unsigned)t << 4 | (unsigned)p;
-    }
-  };
-  CellAt at;
-  if (cell_at(me.key, fl.cell_off, g, at)) for_slots_around(at, g, fl.cell_off, start, order, look);
-  if (away) {
-    const int tick = d->tick;
-#pragma unroll 1
-    for (int k = 0; k < 27; k++) {
-      const long x = q.ci + k / 9 - 1, y = q.cj + k / 3 % 3 - 1, z = q.ck + k % 3 - 1;
-      if (x < 0 || y < 0 || z < 0 || x >= g.nx || y >= g.ny || z >= g.nz) continue;
-      for_chain(near, cull, (int)(fl.cell_off + x + (long)g.nx * (y + (long)g.ny * z)), tick, n, look);
-    }
-  }
+  for_pairs(s, d, flume, nbr, cull, start, order, id, near, m, n, [&](unsigned long long key, unsigned it) {
+    if (key <= done || key >= best) return;
+    V3 dd;
+    double dist2, sep;
+    const int k = it & 3;
+    if (!spheres_overlap(mk(mine.s[3 * k], mine.s[3 * k + 1], mine.s[3 * k + 2]), mine.rad, nbr[it >> 4],
+                         (it >> 2) & 3, dd, dist2, sep))
+      return;
+    best = key;
+    item = it;
+  });
   return best;
-}
-
-// The particle items of a clump whose near list does not hold (too many entries, or a clump around
-// it used up its allowance), found one after another: the items the list would have given.  To
-// the column `col` from entry `nitems` on; returns the entries then, -1 if they would overflow it.
-// Not inlined: rare.
-__device__ __noinline__ int search_items(long s, const DevScalars *d, const int *__restrict__ flume,
-                                          const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
-                                          const int *__restrict__ start, const int *__restrict__ order,
-                                          const long long *__restrict__ id, const NearLists &near, bool away, long n,
-                                          unsigned *col, int nitems) {
-  unsigned item = 0u;
-  for (unsigned long long done = 0ull;;) {
-    done = next_contact(s, d, flume, nbr, cull, start, order, id, near, away, n, false, done, item);
-    if (done == ~0ull) return nitems;
-    if (nitems == kListCap) return -1;
-    col[n * nitems++] = item;
-  }
 }
 
 // The contacts of a clump with more items than its list holds, added to (F, T) in the reference's
@@ -935,8 +953,8 @@ __device__ __noinline__ SlowSums slow_contacts(long s, int pre0, int pre1, int p
                                                const DevScalars *d, const int *__restrict__ flume,
                                                const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull,
                                                const int *__restrict__ start, const int *__restrict__ order,
-                                               const long long *__restrict__ id, const NearLists &near, bool away,
-                                               long n, V3 F, V3 T) {
+                                               const long long *__restrict__ id, const NearLists &near,
+                                               const Margins &m, long n, V3 F, V3 T) {
   const Own o = own_from_record(nbr[s]);
   const double B = (double)cull[s].c.w;
   for (int rt = pre0; rt <= pre1; rt++)
@@ -945,7 +963,7 @@ __device__ __noinline__ SlowSums slow_contacts(long s, int pre0, int pre1, int p
   int active = 0;
   unsigned item = 0u;
   for (unsigned long long done = 0ull;;) {
-    done = next_contact(s, d, flume, nbr, cull, start, order, id, near, away, n, true, done, item);
+    done = next_contact(s, d, flume, nbr, cull, start, order, id, near, m, n, done, item);
     if (done == ~0ull) break;
     const int p = (int)(item & 15u);
     active += part_pair(o.r, o.v, o.w, o.s[p & 3], o.rad, o.msph, nbr[item >> 4], p >> 2, c, xi0, F, T) == 2;
@@ -994,8 +1012,8 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
                                               const CullRec *__restrict__ cull,
                                               const int *__restrict__ start,
                                               const int *__restrict__ order, const long long *__restrict__ id,
-                                              const NearLists &near, bool away, const unsigned *items, int listed,
-                                              ListCounts lc, long n,
+                                              const NearLists &near, const Margins &m, const unsigned *items,
+                                              int listed, ListCounts lc, long n,
                                               V3 &F, V3 &T) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pre0 = aval ? R_HOP0 : 1, pre1 = aval ? R_WALLS : 0;         // fill: none before
@@ -1087,8 +1105,8 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
     __syncthreads();
   }
   if (slow) {
-    const SlowSums r = slow_contacts(s, pre0, pre1, post0, post1, c, d, flume, nbr, cull, start, order, id, near, away,
-                                     n, F, T);
+    const SlowSums r = slow_contacts(s, pre0, pre1, post0, post1, c, d, flume, nbr, cull, start, order, id, near, m, n,
+                                     F, T);
     F = r.F;
     T = r.T;
     active += r.active;
@@ -1191,12 +1209,9 @@ __device__ __forceinline__ int near_pairs(long s, int entries, const DevFlume &f
 __device__ __forceinline__ unsigned bits_before(bool aval) { return aval ? 0x00FFFFFFu : 0u; }
 __device__ __forceinline__ unsigned bits_after(bool aval) { return aval ? 0x0F000000u : 0x00000FFFu; }
 
-// Whether clump s must search for its pairs because its near list does not hold; away: there are
-// runaways to look for.
-__device__ __forceinline__ bool must_search(long s, const DevScalars *d, const NearLists &near, int info, bool &away) {
-  const int tick = d->tick;
-  away = d->runaway <= tick;
-  return info < 0 || near.loose[s] <= tick;
+// Whether clump s must search for its pairs because its near list does not hold.
+__device__ __forceinline__ bool must_search(long s, const DevScalars *d, const NearLists &near, int info) {
+  return info < 0 || near.loose[s] <= d->tick;
 }
 
 // The list phase of k_lists_forces for one clump: its item list (see block_contacts) from its near
@@ -1208,16 +1223,16 @@ __device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, 
                                           const int *__restrict__ start, const int *__restrict__ order,
                                           const long long *__restrict__ id, const NearLists &near,
                                           ContactLists lists, long s0, long n, Margins m, PassLists &pl,
-                                          ListCounts &lc, bool &away, bool &overflow) {
+                                          ListCounts &lc, bool &overflow) {
   const int lane = threadIdx.x & 31;
   const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
   lc.pre = lc.pair = 0;
-  away = overflow = false;
+  overflow = false;
   if (s >= n) return 0;
   const NbrRec &me = nbr[s];
   if (is_removed(*c.tp, me.rx, c.side_x)) return 0;
   const int info = near.info[s];
-  const bool search = must_search(s, d, near, info, away);
+  const bool search = must_search(s, d, near, info);
   overflow = info < 0;
   const bool aval = c.phase == AF3D_PHASE_AVALANCHE;
   const float rad = __int_as_float(cull[s].s[0].w) * unit_power(-m.qs);
@@ -1228,7 +1243,7 @@ __device__ __forceinline__ int lists_body(const Consts &c, const DevScalars *d, 
   int nitems = 0;
   for (; before; before &= before - 1u) col[n * nitems++] = kBndItem | ((unsigned)__ffs(before) - 1u);
   if (search) {
-    nitems = search_items(s, d, flume, nbr, cull, start, order, id, near, away, n, col, nitems);
+    nitems = search_items(s, d, flume, nbr, cull, start, order, id, near, m, n, col, nitems);
     if (nitems < 0) return -1;
   } else {
     const unsigned *list = near.items + s;
@@ -1270,7 +1285,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
                                            const CullRec *__restrict__ cull, const Cells &cells,
                                            const int *__restrict__ order, const long long *__restrict__ id,
                                            const NearLists &near, ContactLists lists, int listed, ListCounts lc,
-                                           bool away, bool overflow, long ntags, bool counted, long s0, long n,
+                                           bool overflow, long ntags, bool counted, long s0, long n,
                                            bool warm,
                                            const LookAhead &la, ForceShared<NB> &sh) {
   const long s = s0 + blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -1287,7 +1302,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
   }
   const long bbase = s0 + blockIdx.x * (long)blockDim.x;
   const int active = block_contacts<NB, UNIFORM>(sh.bq, bbase, sv, valid && !removed, aval, c, d, flume, nbr, cull,
-                                                 cells.start, order, id, near, away, lists.items, valid ? listed : 0, lc,
+                                                 cells.start, order, id, near, P.m, lists.items, valid ? listed : 0, lc,
                                                  n, F, T);
   if (la.nbr) __syncthreads();   // the force phase's shared memory is free for the record staging
   if (valid) {
@@ -1364,7 +1379,6 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
         CullRec cr;
         make_records(rn, vn, wn, sp, P.p[RAD][s], P.p[MSPH][s], P.p[MWALL][s], P.m, (int)key, q, cr);
         stage_nbr_record(q, sh.rec.nbr);
-        la.cull[s] = cr;   // stored directly: staged too, it would set the block's shared memory size
         if (la.build) {
           cells.rank_tmp[s] = arrive_in_bucket(cells, key);
         } else {
@@ -1373,6 +1387,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
           keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1,
                      n);
         }
+        la.cull[s] = cr;   // stored directly: staged too, it would set the block's shared memory size
       }
     }
   }
@@ -1689,7 +1704,7 @@ void launch_build_records(const Launch &L, Planes cur, NbrRec *nbr, CullRec *cul
 // memory (the block's own entries, visible to its threads after the barrier).
 template <int NB, int MINB, bool WRITE_FT, bool UNIFORM>
 __global__ void __launch_bounds__(NB, MINB)
-    k_lists_forces(Planes P, Planes out, DevScalars *d, const int *__restrict__ flume, const NbrRec *__restrict__ nbr,
+    k_lists_forces(const __grid_constant__ Planes P, const __grid_constant__ Planes out, DevScalars *d, const int *__restrict__ flume, const NbrRec *__restrict__ nbr,
                    const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
                    const int *__restrict__ order, const long long *__restrict__ id,
                    const __grid_constant__ NearLists near, ContactLists lists, long ntags, bool counted,
@@ -1697,13 +1712,13 @@ __global__ void __launch_bounds__(NB, MINB)
                    long n) {
   __shared__ ForceShared<NB> sh;
   ListCounts lc;
-  bool away, overflow;
+  bool overflow;
   auto body = [&](const Consts &c) {
     const int listed = lists_body(c, d, flume, nbr, cull, cells.start, order, id, near, lists, s0, n, P.m,
-                                  sh.pl[threadIdx.x >> 5], lc, away, overflow);
+                                  sh.pl[threadIdx.x >> 5], lc, overflow);
     overflow = overflow || listed < 0;
     __syncthreads();
-    fused_body<NB, WRITE_FT, UNIFORM>(c, P, out, d, flume, nbr, cull, cells, order, id, near, lists, listed, lc, away,
+    fused_body<NB, WRITE_FT, UNIFORM>(c, P, out, d, flume, nbr, cull, cells, order, id, near, lists, listed, lc,
                                       overflow, ntags, counted, s0, n, warm, la, sh);
   };
   if constexpr (UNIFORM) {

@@ -30,12 +30,13 @@ struct NearShared {
 // the partners with smaller ids.  Bound by the latency of its chain of loads and tests, so it is
 // split over four warps: a whole clump per thread took 47 us at 8,192 clumps, 49 at 32,768 and
 // about 200 for 100,003 in four parts; so it is 31, 38 and 75 (in one launch).
-__global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalars *d, const int *__restrict__ flume,
+__global__ void __launch_bounds__(kNearBlock) k_build_lists(const __grid_constant__ Margins m, DevScalars *d, const int *__restrict__ flume,
                                                             const CullRec *__restrict__ cull,
                                                             const int *__restrict__ start,
                                                             const int *__restrict__ order,
                                                             const float4 *__restrict__ csort,
-                                                            const long long *__restrict__ id, NearLists near, long s0, long s1,
+                                                            const long long *__restrict__ id,
+                                                            const __grid_constant__ NearLists near, long s0, long s1,
                                                             long n) {
   __shared__ NearShared sh;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -47,10 +48,9 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
   const CullRec &rec = cull[sv];
   const float4 mc = rec.c;
   const float allow = rec.allow, grown = allow * (1.0f + 1e-5f);
-  const float sum = fabsf(mc.x) + fabsf(mc.y) + fabsf(mc.z);
   const bool coarse = beyond_reach(rec, m);
   if (w == 0 && valid) {
-    near.rem[s] = coarse ? -1e-30f : allow * (1.0f - 1e-5f);   // (none left, yet not a runaway)
+    near.rem[s] = coarse ? -1.0f : allow * (1.0f - 1e-5f);
     // boundaries: the routines' gates are 1-Lipschitz in the sphere centre, so the allowance adds
     // to the bound; a door that is closed now may open, one that is open stays open
     const Consts &c = fl.c;
@@ -62,22 +62,11 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
     near.bnd[s] = bnd;
     CellAt at;   // (with `order` the sort has marked them)
     if (coarse && !order && cell_at(rec.key, fl.cell_off, g, at))
-      mark_around(at, g, fl.cell_off, start, order, near.loose, d->tick);
+      go_away(s, mc, rec.key, at, m, fl, d, start, order, near, d->tick, n);
   }
   // the cells within reach of any partner's bound and allowance, FP32 with slack
-  const float most = m.most + 1e-6f * (sum + 20.0f) + m.cap;
-  const float reach = (mc.w + grown + most) * (1.0f + 1e-5f);
-  auto range = [&](float x, float xmin, float inv, int cells, int &lo, int &hi) {
-    const float q = (x - xmin) * inv, r = reach * inv;
-    const float e = 2e-6f * ((fabsf(x) + fabsf(xmin)) * inv + fabsf(q) + r + 1.0f);
-    lo = (int)fminf(fmaxf(floorf(q - r - e), 0.0f), (float)(cells - 1));
-    hi = (int)fminf(fmaxf(floorf(q + r + e), 0.0f), (float)(cells - 1));
-  };
-  int x0, x1, y0, y1, z0, z1;
-  range(mc.x, g.xmin, g.ix, g.nx, x0, x1);
-  range(mc.y, g.ymin, g.iy, g.ny, y0, y1);
-  range(mc.z, g.zmin, g.iz, g.nz, z0, z1);
-  const int ny = y1 - y0 + 1, rows = valid && !coarse ? ny * (z1 - z0 + 1) : 0;
+  const CellRange b = cells_within(mc, (mc.w + grown + partner_reach(mc, m)) * (1.0f + 1e-5f), g);
+  const int ny = b.y1 - b.y0 + 1, rows = valid && !coarse ? ny * (b.z1 - b.z0 + 1) : 0;
   const float mine = mc.w + grown;
   auto centre = [&](int k) {
     if (order) return __ldg(&csort[k]);
@@ -95,9 +84,9 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(Margins m, DevScalar
       k[q] = end[q] = 0;
       if (r < rows) {
         const int z = r / ny, y = r - z * ny;
-        const int *row = start + fl.cell_off + (long long)g.nx * (y0 + y + (long long)g.ny * (z0 + z));
-        k[q] = __ldg(row + x0);
-        end[q] = __ldg(row + x1 + 1);
+        const int *row = start + fl.cell_off + (long long)g.nx * (b.y0 + y + (long long)g.ny * (b.z0 + z));
+        k[q] = __ldg(row + b.x0);
+        end[q] = __ldg(row + b.x1 + 1);
       }
     }
 #pragma unroll 1

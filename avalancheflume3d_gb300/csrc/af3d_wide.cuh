@@ -66,14 +66,13 @@ __global__ void __launch_bounds__(kWideThreads, 4)
     const bool removed = is_removed(*c.tp, me.rx, c.side_x), act = valid && !removed;
     const bool aval = c.phase == AF3D_PHASE_AVALANCHE, dev = c.variant == AF3D_FRICTION_DEV;
     const int info = near.info[sv];
-    bool away = false;
-    const bool search = act && must_search(sv, d, near, info, away);
+    const bool search = act && must_search(sv, d, near, info);
     const unsigned *list = near.items + sv;
     unsigned *col = lists.items + sv;
     // the clumps' items: near pairs (warp 0), boundary spheres (warp 1)
     if (w == 0) {
       int np = 0;
-      if (search) np = search_items(sv, d, flume, nbr, cull, cells.start, order, id, near, away, n, col, 0);
+      if (search) np = search_items(sv, d, flume, nbr, cull, cells.start, order, id, near, P.m, n, col, 0);
       else if (act) np = near_pairs(sv, info, fl, me, cull, list, n, sh.pl);
       sh.npair[lane] = np;
     } else if (w == 1) {
@@ -194,7 +193,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
       const int post0 = aval ? R_FLUME : R_HOP0, post1 = aval ? R_FLUME : R_HOP2;
       const V3 zero = mk(0.0, 0.0, 0.0);
       const SlowSums r = slow_contacts(sv, pre0, pre1, post0, post1, c, d, flume, nbr, cull, cells.start, order, id,
-                                       near, away, n, zero, zero);
+                                       near, P.m, n, zero, zero);
       if (w < 3) {
         Fi = comp(r.F, w);
         Ti = comp(r.T, w);
@@ -436,7 +435,6 @@ __global__ void __launch_bounds__(kWideThreads, 4)
         V3 sp[4];
         for (int k = 0; k < 4; k++) sp[k] = mk(o[9 + 3 * k], o[10 + 3 * k], o[11 + 3 * k]);
         make_records(r1, mk(o[3], o[4], o[5]), mk(o[6], o[7], o[8]), sp, o[21], o[22], o[23], P.m, (int)key, q, cr);
-        la.cull[s] = cr;
         if (la.build) {
           cells.rank_tmp[s] = arrive_in_bucket(cells, key);
         } else {
@@ -445,6 +443,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
           keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1,
                      n);
         }
+        la.cull[s] = cr;
       }
     } else {
       const long cnt = n - bbase < kWide ? n - bbase : kWide;
