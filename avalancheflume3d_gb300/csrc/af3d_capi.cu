@@ -71,7 +71,9 @@ struct PtrState {
 struct StepGraph {
   PtrState start{}, end{};      // before and after the captured steps
   bool look_last = false;       // the last captured force pass looks ahead
+  long build_every = 0;
   long since_build = 0;         // steps the near lists have served at its end
+  const int *built_order = nullptr;
   long kernels = 0;
   cudaGraphExec_t exec = nullptr;
 };
@@ -141,7 +143,8 @@ struct af3d_ctx {
   bool taping = false;    // every step's state is read from the planes (the adjoint's tape)
   ContactLists lists{};   // the item lists of the current force pass
   NearLists near{};       // what may touch within the next steps
-  long since_build = kBuildEvery;   // steps the near lists have served (kBuildEvery: build them anew)
+  long build_every = kBuildEvery;   // steps the near lists serve (list_interval)
+  long since_build = kBuildEvery;   // steps they have served (build_every or more: build them anew)
   const int *built_order = nullptr;   // the slots' place in the sort they were built from (null: in that order)
   Cells cells{};
   DevScalars *d = nullptr;
@@ -207,11 +210,20 @@ bool same_state(const PtrState &a, const PtrState &b) {
 void set_margins(af3d_ctx *c) {
   double rmax = 0.0;
   for (const auto &s : c->sys) rmax = std::max(rmax, s.rmax);
-  c->cur.m = c->alt.m = margins_for(rmax, c->sys[0].dt, kBuildEvery);
+  c->cur.m = c->alt.m = margins_for(rmax, c->sys[0].dt, c->build_every);
 }
 
 // The state, the grid or the slots changed other than by a step: the next step builds its lists.
 void drop_lists(af3d_ctx *c) { c->since_build = kBuildEvery; }
+
+// The interval of the next lists from the counts of the last; between steps that look ahead.
+void choose_interval(af3d_ctx *c, const int *outrun) {
+  const long every = list_interval(outrun, c->n, c->build_every);
+  if (every == c->build_every) return;
+  c->build_every = every;   // (graphs are kept by their interval)
+  set_margins(c);
+  drop_lists(c);
+}
 
 void drop_graphs(af3d_ctx *c) {
   for (auto &g : c->graphs) {
@@ -413,9 +425,9 @@ StepPlan plan_step(const af3d_ctx *c, bool resort, bool look) {
   StepPlan p;
   p.resort = resort;
   p.warm = !resort && c->look;
-  p.build = resort || c->since_build >= kBuildEvery;
+  p.build = resort || c->since_build >= c->build_every;
   p.look = look;
-  p.next_builds = (p.build ? 1 : c->since_build + 1) >= kBuildEvery;
+  p.next_builds = (p.build ? 1 : c->since_build + 1) >= c->build_every;
   return p;
 }
 
@@ -483,7 +495,9 @@ af3d_status run_steps(af3d_ctx *c, long m, bool launch = true) {
     const PtrState now = ptr_state(c);
     StepGraph *g = nullptr;
     for (auto &cand : c->graphs)
-      if (cand.exec && cand.look_last == look_last && same_state(cand.start, now)) g = &cand;
+      if (cand.exec && cand.look_last == look_last && cand.build_every == c->build_every &&
+          same_state(cand.start, now))
+        g = &cand;
     if (!g) {
       g = &c->graphs[c->graph_next];
       c->graph_next = (c->graph_next + 1) % 4;
@@ -491,6 +505,7 @@ af3d_status run_steps(af3d_ctx *c, long m, bool launch = true) {
       *g = StepGraph{};
       g->start = now;
       g->look_last = look_last;
+      g->build_every = c->build_every;
       const long launches0 = c->launches;
       cudaGraph_t graph;
       AF3D_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
@@ -498,6 +513,7 @@ af3d_status run_steps(af3d_ctx *c, long m, bool launch = true) {
       AF3D_CUDA(cudaStreamEndCapture(c->st, &graph));
       g->end = ptr_state(c);
       g->since_build = c->since_build;
+      g->built_order = c->built_order;
       g->kernels = c->launches - launches0;
       c->launches = launches0;
       set_ptr_state(c, now);
@@ -516,7 +532,7 @@ af3d_status run_steps(af3d_ctx *c, long m, bool launch = true) {
     c->sorted = false;   // the last captured step keeps the slot order
     c->since_sort = len - 1;
     c->since_build = g->since_build;
-    c->built_order = len > kBuildEvery ? c->cells.perm : nullptr;
+    c->built_order = g->built_order;
     m -= len;
   }
   for (; launch && m > 0; m--) {
@@ -528,13 +544,16 @@ af3d_status run_steps(af3d_ctx *c, long m, bool launch = true) {
   return AF3D_OK;
 }
 
-af3d_status read_status(af3d_ctx *c, int *flags) {
-  int st = 0, zero = 0;
-  AF3D_CUDA(cudaMemcpyAsync(&st, &c->d->status, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+// The status bits, cleared; outrun (may be null): also the counts of the last lists.
+af3d_status read_status(af3d_ctx *c, int *flags, int *outrun = nullptr) {
+  int st[kIntervals] = {}, zero = 0;
+  static_assert(offsetof(DevScalars, outrun) == offsetof(DevScalars, status) + sizeof(int), "read together");
+  AF3D_CUDA(cudaMemcpyAsync(st, &c->d->status, outrun ? sizeof(st) : sizeof(int), cudaMemcpyDeviceToHost, c->st));
   AF3D_CUDA(cudaMemcpyAsync(&c->d->status, &zero, sizeof(int), cudaMemcpyHostToDevice, c->st));
   AF3D_CUDA(cudaStreamSynchronize(c->st));
   AF3D_CUDA(cudaGetLastError());
-  *flags = st;
+  *flags = st[0];
+  if (outrun) std::copy(st + 1, st + kIntervals, outrun);
   return AF3D_OK;
 }
 
@@ -1295,9 +1314,10 @@ af3d_status af3d_forces(af3d_ctx *c) {
   forces_for(c, true, c->alt);
   drop_lists(c);
   c->records_valid = true;
-  int flags = 0;
-  af3d_status s = read_status(c, &flags);
+  int flags = 0, outrun[kIntervals - 1];
+  af3d_status s = read_status(c, &flags, outrun);
   if (s) return s;
+  choose_interval(c, outrun);
   return first_error(flags);
 }
 
@@ -1318,13 +1338,17 @@ af3d_status af3d_step(af3d_ctx *c, long k) {
     c->cells_valid = true;
     c->records_valid = false;
     if (do_regrid) {
+      int outrun[kIntervals - 1] = {};   // (the re-grid waits for the steps as it is)
+      AF3D_CUDA(cudaMemcpyAsync(outrun, &c->d->outrun, sizeof(outrun), cudaMemcpyDeviceToHost, c->st));
       s = regrid(c);
       if (s) return s;
+      if (k > 0) choose_interval(c, outrun);
     }
   }
-  int flags = 0;
-  af3d_status s = read_status(c, &flags);
+  int flags = 0, outrun[kIntervals - 1];
+  af3d_status s = read_status(c, &flags, outrun);
   if (s) return s;
+  choose_interval(c, outrun);
   return first_error(flags);
 }
 

@@ -76,7 +76,10 @@ __device__ __forceinline__ long n_buckets(const DevScalars *d, long n) { return 
 // Lists are built from the sort, so the chains and marks since the last ones are void (k_scatter).
 __global__ void k_scan_final(const int *__restrict__ count, const int *__restrict__ tile_count,
                              int *start, DevScalars *d, long n) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) d->away = INT_MAX;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    d->away = INT_MAX;
+    for (int b = 0; b < kIntervals - 1; b++) d->outrun[b] = 0;
+  }
   const long nb = n_buckets(d, n);
   if (blockIdx.x == 0 && threadIdx.x == 0) start[nb] = (int)n;   // every clump has one bucket
   if (blockIdx.x * (long)kTile >= nb) return;   // a tile past the buckets in use

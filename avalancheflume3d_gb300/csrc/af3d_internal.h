@@ -34,11 +34,27 @@ enum Plane : int {
   NPLANES
 };
 
+// The steps between list builds: 16, or 8, 4 or 2 where the flow would outrun the lists' largest allowance
+// (kBuildEvery >> b for b < kIntervals).  A build costs about what a step does (262,144 clumps: sort 26 us, lists
+// 190; 2,048: 10 and 30), a search several times what a list's tests do, and a clump that has used up its
+// allowance makes about ten around it search and with them most of their warps.  So each interval is kept while at most
+// n / 2048, n / 512 and n / 16 clumps outrun it, by the counts of the last lists, and a longer one comes back at
+// a quarter of that.  Results do not depend on it.
+constexpr int kIntervals = 4;
+constexpr long kBuildEvery = 16;
+inline long list_interval(const int *outrun, long n, long now) {
+  const long share[kIntervals - 1] = {2048, 512, 16};
+  for (int b = 0; b < kIntervals - 1; b++)
+    if (outrun[b] <= n / share[b] / (kBuildEvery >> b > now ? 4 : 1)) return kBuildEvery >> b;
+  return kBuildEvery >> (kIntervals - 1);
+}
+
 // How the culling records and near lists measure: lengths in units of 2^-qs cm, and how far a
 // clump is allowed to move before its lists are built again (see NearLists).
 struct Margins {
   int qs;
   float per_speed, floor, cap;   // allowance min(per_speed * speed + floor, cap), in cm
+  float steps;                   // the steps it is for
   float most;                    // bounding radius that the near lists' cell ranges reach for, in cm
 };
 
@@ -67,7 +83,7 @@ struct __align__(16) CullRec {
   int key;       // the clump's bucket at this step (cell order of the contacts)
   float allow;   // how far it may move from here (Margins)
   int away;      // it is in a chain (NearLists)
-  int pad;
+  float pace;    // per_speed * speed (Margins)
 };
 
 // A clump of extent + radius above this many units has an infinite radius in its record: every
@@ -93,6 +109,7 @@ inline Margins margins_for(double rmax, double dt, long steps) {
   m.most = (float)(ok ? fmin(1.05 * 2.2247448713915889 * rmax, holds) : holds);
   const double v = 1.5 * fabs(dt) * (double)steps;
   m.per_speed = v < 1e30 ? (float)v : 1e30f;
+  m.steps = (float)steps;
   m.floor = ok ? (float)(0.04 * rmax) : 0.0f;
   m.cap = ok ? (float)(0.3 * rmax) : 0.0f;
   return m;
@@ -215,8 +232,9 @@ struct DevScalars {
   double          time_prev;  // time before the last advance (init_Verlet's removal test)
   int             phase;      // AF3D_PHASE_*
   int             variant;    // AF3D_FRICTION_*
-  int             status;     // bitmask of 1 << AF3D_ERR_*
   int             nflumes;
+  int             status;     // bitmask of 1 << AF3D_ERR_*
+  int             outrun[kIntervals - 1];   // clumps that lists kept for kBuildEvery >> b steps would not serve
   unsigned long long contacts; // active sphere-sphere contacts summed over fused force passes
   unsigned long long overflows; // clumps whose item lists overflowed, over fused force passes
   long long       ncell_total; // sum of the flumes' ncell3: the first removed-clump bucket
@@ -274,7 +292,7 @@ __host__ __device__ inline int pack_list_counts(int listed, int pre, int pair) {
 
 // Near lists: per clump the sphere pairs and the (boundary routine, sphere) pairs that may touch
 // while no clump moves farther than its allowance, built from a cell sort and used for up to
-// kBuildEvery steps (fewer when the slots are permuted, the grid changes or the caller touches
+// list_interval steps (fewer when the slots are permuted, the grid changes or the caller touches
 // the state).  A step that uses them neither sorts nor walks cells: it tests ~7 sphere pairs per
 // clump of a dense bed instead of ~300 behind nine dependent reads of the cell table.  Each pass
 // tests the listed pairs at the current positions and orders the overlapping ones by the
@@ -288,10 +306,6 @@ __host__ __device__ inline int pack_list_counts(int listed, int pre, int pair) {
 // 2,048 clumps (fast) 48 -> 37 us a step, 20,011 in the hopper (exact) 82 -> 75, 262,144 (fast)
 // 0.325 -> 0.296 ms with the copies of a 40-step call, (exact) 0.49 -> 0.46.
 constexpr int kNearCap = 60;
-#ifndef AF3D_BUILD_EVERY
-#define AF3D_BUILD_EVERY 16
-#endif
-constexpr long kBuildEvery = AF3D_BUILD_EVERY;
 struct NearLists {
   unsigned *items;   // [kNearCap][n] partner slot << 4 | sph_id - 1, by partner id, then sph_id
   int *info;         // [n] entries, -1: too many (the clump searches for itself)

@@ -202,8 +202,9 @@ __device__ __forceinline__ void make_records(V3 r, V3 v, V3 w, const V3 *sp, dou
   const float vx = magnitude_f(v.x), vy = magnitude_f(v.y), vz = magnitude_f(v.z);
   const float wx = magnitude_f(w.x), wy = magnitude_f(w.y), wz = magnitude_f(w.z);
   const float speed = sqrtf(vx * vx + vy * vy + vz * vz) + sqrtf(wx * wx + wy * wy + wz * wz) * bound;
-  c.allow = fminf(m.per_speed * speed + m.floor, m.cap);   // cap for NaN
-  c.away = c.pad = 0;
+  c.pace = m.per_speed * speed;
+  c.allow = fminf(c.pace + m.floor, m.cap);   // cap for NaN
+  c.away = 0;
 }
 
 // How far the spheres of a clump moved between two of its records, at most, in cm.  Differences
@@ -521,8 +522,8 @@ __device__ __forceinline__ long bucket_key(V3 r, const DevFlume &fl, DevScalars 
 
 // A clump's place in a step that keeps its near lists: counted in its cell for the capacity check
 // of cells.cu:96-102 (at most ntags - 1 clumps), and its motion since the previous step's record
-// (old) against its allowance: with none left it is away at tick `tick`.
-__device__ __forceinline__ void keep_place(long s, const int4 *old, CullRec &cr, const DevFlume &fl, DevScalars *d,
+// (old) against its allowance: with none left it is away at tick `tick` (true, for its record).
+__device__ __forceinline__ bool keep_place(long s, const int4 *old, const CullRec &cr, const DevFlume &fl, DevScalars *d,
                                            int *occ, long ntags, const NearLists &near,
                                            const int *__restrict__ start, const int *__restrict__ order,
                                            const Margins &m, int tick, long n) {
@@ -531,9 +532,9 @@ __device__ __forceinline__ void keep_place(long s, const int4 *old, CullRec &cr,
   const float rem = near.rem[s] - sphere_motion(old, cr, m.qs);
   near.rem[s] = rem;
   CellAt at;
-  if (rem >= 0.0f || !cell_at(cr.key, fl.cell_off, fl.gridf, at)) return;
-  cr.away = 1;
+  if (rem >= 0.0f || !cell_at(cr.key, fl.cell_off, fl.gridf, at)) return false;
   go_away(s, cr.c, cr.key, at, m, fl, d, start, order, near, tick, n);
+  return true;
 }
 
 // init_Verlet.cu:25-148 for one clump (PREDICT), and/or cell_locate's binning (cells.cu:60-92)
@@ -599,7 +600,7 @@ __global__ void __launch_bounds__(kBlock) k_predict(const __grid_constant__ Plan
       if (count_only) {
         int4 old[4];
         for (int k = 0; k < 4; k++) old[k] = cull[s].s[k];
-        keep_place(s, old, cr, fl, d, cells.occ, ntags, near, cells.start, order, P.m, d->tick, n);
+        cr.away = keep_place(s, old, cr, fl, d, cells.occ, ntags, near, cells.start, order, P.m, d->tick, n);
       }
     }
   }
@@ -1379,15 +1380,15 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
         CullRec cr;
         make_records(rn, vn, wn, sp, P.p[RAD][s], P.p[MSPH][s], P.p[MWALL][s], P.m, (int)key, q, cr);
         stage_nbr_record(q, sh.rec.nbr);
+        la.cull[s] = cr;   // stored directly: staged too, it would set the block's shared memory size
         if (la.build) {
           cells.rank_tmp[s] = arrive_in_bucket(cells, key);
         } else {
           int4 old[4];
           for (int k = 0; k < 4; k++) old[k] = cull[s].s[k];
-          keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1,
-                     n);
+          if (keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1, n))
+            la.cull[s].away = 1;
         }
-        la.cull[s] = cr;   // stored directly: staged too, it would set the block's shared memory size
       }
     }
   }

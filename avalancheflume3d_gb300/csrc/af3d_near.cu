@@ -2,7 +2,7 @@
 // while no clump moves farther than its allowance (NearLists in af3d_internal.h).
 //
 // Integer and FP32 work on the culling records; built from the sorted cell list once every
-// kBuildEvery steps.
+// 2 to 16 steps (list_interval).
 #include "af3d_cellwalk.cuh"
 
 namespace af3d {
@@ -63,6 +63,16 @@ __global__ void __launch_bounds__(kNearBlock) k_build_lists(const __grid_constan
     CellAt at;   // (with `order` the sort has marked them)
     if (coarse && !order && cell_at(rec.key, fl.cell_off, g, at))
       go_away(s, mc, rec.key, at, m, fl, d, start, order, near, d->tick, n);
+  }
+  // the clumps that lists kept for each interval would not serve: their speed (the allowance is for half as
+  // much again) takes them past the largest allowance, with 5 % to spare
+  if (w == 0 && m.cap > 0.0f) {
+    const float pace = valid && (unsigned)rec.key < (unsigned)d->ncell_total ? 0.7f * rec.pace / m.steps : 0.0f;
+    for (int b = 0; b < kIntervals - 1; b++) {
+      const unsigned past = __ballot_sync(0xffffffffu, pace * (float)(kBuildEvery >> b) > m.cap);
+      if (!past) break;
+      if (lane == 0) atomicAdd(&d->outrun[b], __popc(past));
+    }
   }
   // the cells within reach of any partner's bound and allowance, FP32 with slack
   const CellRange b = cells_within(mc, (mc.w + grown + partner_reach(mc, m)) * (1.0f + 1e-5f), g);

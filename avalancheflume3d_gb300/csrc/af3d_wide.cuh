@@ -435,15 +435,15 @@ __global__ void __launch_bounds__(kWideThreads, 4)
         V3 sp[4];
         for (int k = 0; k < 4; k++) sp[k] = mk(o[9 + 3 * k], o[10 + 3 * k], o[11 + 3 * k]);
         make_records(r1, mk(o[3], o[4], o[5]), mk(o[6], o[7], o[8]), sp, o[21], o[22], o[23], P.m, (int)key, q, cr);
+        la.cull[s] = cr;
         if (la.build) {
           cells.rank_tmp[s] = arrive_in_bucket(cells, key);
         } else {
           int4 old[4];
           for (int k = 0; k < 4; k++) old[k] = cull[s].s[k];
-          keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1,
-                     n);
+          if (keep_place(s, old, cr, fl, d, cells.occ_next, ntags, near, cells.start, order, P.m, d->tick + 1, n))
+            la.cull[s].away = 1;
         }
-        la.cull[s] = cr;
       }
     } else {
       const long cnt = n - bbase < kWide ? n - bbase : kWide;
