@@ -59,6 +59,14 @@ inline double sqrt_instr(double x) { return std::sqrt(x); }
 #define AF3D_HD inline
 #endif
 
+// The FP32 estimate y of a number in (1/2, 1], in Q23: y + 1 in (1.5, 2] holds it in its last 23 bits.
+// An estimate past 1 (of the reciprocal or root of a mantissa at or just above 1) is one unit below
+// it, as 1 is, so that it fits 31 bits in Q31 and the Newton step takes it from there.
+AF3D_HD unsigned estimate_q23(float y) {
+  const unsigned e = bits_of_float(y + 1.0f) - 0x3F800001u;
+  return e < 0x7FFFFFu ? e : 0x7FFFFFu;
+}
+
 // A divisor's 53-bit mantissa and the reciprocal of (mantissa / 2^52) in Q31, within two units.
 struct Divisor {
   double b;
@@ -72,10 +80,8 @@ AF3D_HD Divisor divisor_of(double b) {
   Divisor d;
   d.b = b;
   d.m = ((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
-  // FP32 estimate y of 1/b for b in [1, 2), then y + 1 in [1.5, 2] holds it in its last 23 bits
   const unsigned top = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
-  const float y = rcp_estimate(float_of_bits(0x3F800000u | top));
-  const unsigned r0 = (bits_of_float(y + 1.0f) - 0x3F800001u) << 8;   // Q31, below 2^31
+  const unsigned r0 = estimate_q23(rcp_estimate(float_of_bits(0x3F800000u | top))) << 8;   // Q31, below 2^31
   // one Newton step: r0 + r0 (1 - b r0), the residual in Q50
   const unsigned bh = (unsigned)(d.m >> 21);   // Q31
   const long long e = (1LL << 62) - (long long)((unsigned long long)bh * r0);
@@ -111,8 +117,7 @@ AF3D_HD double div_by(double a, const Divisor &d) {
 
 // 1/sqrt(v) for v = M / 2^52 in [1, 4), in Q31 within two units.
 AF3D_HD unsigned rsqrt_q31(unsigned long long M, unsigned hi_float) {
-  const float y = rsqrt_estimate(float_of_bits(hi_float));
-  const unsigned r23 = bits_of_float(y + 1.0f) - 0x3F800001u;   // Q23, below 2^23
+  const unsigned r23 = estimate_q23(rsqrt_estimate(float_of_bits(hi_float)));
   const unsigned vh = (unsigned)(M >> 22);                       // Q30
   const unsigned t = (unsigned)(((unsigned long long)r23 * r23) >> 15);   // y^2 in Q31
   const long long e = (1LL << 61) - (long long)((unsigned long long)vh * t);   // 1 - v y^2 in Q61
