@@ -49,9 +49,8 @@ __device__ __forceinline__ bool contact_law_fwd_rev(const ContactIn &ci, double 
   f.x = -normal * n.x;
   f.y = -normal * n.y;
   f.z = -normal * n.z;
-  // a displacement that is surely cut and no Coulomb branch: the normal force alone
   const bool gated = surely_gated(dv, n, normal, ci.cns, dt);
-  const bool plain = gated && !ci.xi0;
+  const bool plain = normal_only(gated, ci.xi0, ci.mu);
   const double m = ci.mass_t;
   V3 vt = mk(0.0, 0.0, 0.0), tv = vt;
   double vt_mag = 0.0, fsdt = 0.0, ivt = 0.0, q1 = 0.0, q3 = 0.0;

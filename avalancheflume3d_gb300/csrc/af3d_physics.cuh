@@ -190,6 +190,12 @@ __device__ __forceinline__ bool surely_gated(V3 dv, V3 n, double normal, double 
   return magnitude_f(dt) * (vt - 4e-6f * v) > 1.001f * magnitude_f(cns_1) * magnitude_f(normal) + 1e-36f;
 }
 
+// Whether the law leaves the normal force alone: no displacement (gated), no Coulomb branch for want of
+// one, nor for |0| > mu normal, which a negative friction takes.
+__device__ __forceinline__ bool normal_only(bool gated, bool xi0, double mu) {
+  return gated && !xi0 && bits_of(mu) <= 0x8000000000000000ull;
+}
+
 // Spring-dashpot normal force + Cundall-Strack tangential force with the Coulomb cap; the common
 // tail of every contact type (force_part.cu:189-241, force_walls.cu:123-177, ...).
 //   xi0:  Coulomb branch also when xi was zeroed (walls; DEV particle variant)
@@ -205,7 +211,7 @@ __device__ __forceinline__ bool contact_law_fast(V3 dvvc, V3 n, double comp, dou
   if (gate ? !push && !nan_bits(normal) : !push) return false;
   f = mk(-normal * n.x, -normal * n.y, -normal * n.z);
   const bool gated = surely_gated(dvvc, n, normal, cns_1, dt);
-  if (gated && !xi0) return true;   // no displacement, no Coulomb branch: the normal force alone
+  if (normal_only(gated, xi0, mu)) return true;
   const V3 vt = mk(dvvc.x - vn * n.x, dvvc.y - vn * n.y, dvvc.z - vn * n.z);
   const double vt2 = vt.x * vt.x + vt.y * vt.y + vt.z * vt.z;
   double inv_vt, vt_mag;   // +inf and 0 (dev: NaN) for vt = 0: the tangential part is then skipped, as in the exact law
@@ -254,8 +260,8 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
   f.y = -normal * n.y;
   f.z = -normal * n.z;
   const bool gated = surely_gated(dvvc, n, normal, cns_1, dt);
-  if (gated && !xi0) {
-    // xi = 0 and no Coulomb branch: the law adds (0 vt_i) / |vt| to each component, which changes
+  if (normal_only(gated, xi0, mu)) {
+    // the law adds (0 vt_i) / |vt| to each component, which changes
     // only a zero's sign, where n_i = 0 and so vt_i = dvvc_i: -0 + 0 = +0
     if (!nonzero_bits(f.x) && positive_bits(dvvc.x)) f.x = 0.0;
     if (!nonzero_bits(f.y) && positive_bits(dvvc.y)) f.y = 0.0;
@@ -274,7 +280,7 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
     const double vt_sig = dvvc.x * tv.x + dvvc.y * tv.y + dvvc.z * tv.z;
     xi = dt * vt_sig;
     if (less_bits(cns_1 * normal, fabs(xi))) xi = 0.0;
-    const double xi_dot = nonzero_bits(xi) ? div_rn(xi, dt) : xi;   // dt > 0
+    const double xi_dot = nonzero_bits(xi) ? div_rn(xi, dt) : xi;
     fsdt = 1.0e12 * mass_t * xi + 2.0e6 * mass_t * xi_dot;
   }
   if (positive_bits(vt_mag)) {
