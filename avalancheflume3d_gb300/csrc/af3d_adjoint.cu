@@ -68,7 +68,7 @@ __device__ __forceinline__ bool contact_law_fwd_rev(const ContactIn &ci, double 
       xi = dt * vt_sig;
       zeroed = less_bits(ci.cns * normal, fabs(xi));
       if (zeroed) xi = 0.0;
-      const double xi_dot = nonzero_bits(xi) ? div_rn(xi, dt) : xi;
+      const double xi_dot = nonzero_bits(xi) || !nonzero_bits(dt) ? div_rn(xi, dt) : xi;
       fsdt = 1.0e12 * m * xi + 2.0e6 * m * xi_dot;
     }
     tang = positive_bits(vt_mag);

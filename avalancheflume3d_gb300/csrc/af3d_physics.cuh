@@ -280,7 +280,7 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
     const double vt_sig = dvvc.x * tv.x + dvvc.y * tv.y + dvvc.z * tv.z;
     xi = dt * vt_sig;
     if (less_bits(cns_1 * normal, fabs(xi))) xi = 0.0;
-    const double xi_dot = nonzero_bits(xi) ? div_rn(xi, dt) : xi;
+    const double xi_dot = nonzero_bits(xi) || !nonzero_bits(dt) ? div_rn(xi, dt) : xi;
     fsdt = 1.0e12 * mass_t * xi + 2.0e6 * mass_t * xi_dot;
   }
   if (positive_bits(vt_mag)) {

@@ -1,5 +1,6 @@
 """The contact law where its shortcuts must not be taken: a negative friction puts a contact whose
-displacement the gate cuts into the Coulomb branch (|0| > mu N, force_part.cu:224-232).  One force pass of moving, overlapping clumps against the oracle,
+displacement the gate cuts into the Coulomb branch (|0| > mu N, force_part.cu:224-232), and a time step of
+zero makes the displacement's rate 0 / 0.  One force pass of moving, overlapping clumps against the oracle,
 bit for bit."""
 import numpy as np
 import pytest
@@ -22,7 +23,7 @@ def af3d():
 
 @pytest.mark.parametrize("friction", [FRICTION_HST, FRICTION_DEV])
 @pytest.mark.parametrize("n", [400, 21000])   # either shape of the force pass
-@pytest.mark.parametrize("mu,dt", [(-0.3, 2e-6), (0.0, 2e-6)])
+@pytest.mark.parametrize("mu,dt", [(-0.3, 2e-6), (0.0, 2e-6), (0.5, 0.0)])
 def test_force_pass_equals_the_oracle(af3d, oracle, friction, n, mu, dt):
     sys, fun = flume_system(n, time=0.001)
     sys["mu_pp"] = mu
@@ -34,8 +35,13 @@ def test_force_pass_equals_the_oracle(af3d, oracle, friction, n, mu, dt):
     with af3d.Engine(sys, fun, ntags=0, friction=friction) as e:
         e.set_grid(run.cp)
         e.import_particles(pp)
-        e.forces()
+        try:
+            e.forces()
+        except Exception:
+            assert dt == 0.0   # NaN accelerations are raised
         F, T = e.get_forces()
         assert e.contact_count() > n // 8
         for got, want in ((F, run.bufs["F"]), (T, run.bufs["T"])):
-            assert got.tobytes() == want.tobytes()
+            nan = np.isnan(want)
+            assert np.array_equal(np.isnan(got), nan)
+            assert np.where(nan, 0.0, got).tobytes() == np.where(nan, 0.0, want).tobytes()
