@@ -300,6 +300,8 @@ __device__ __forceinline__ long bin_axis_f(double x, float xminf, float invf, do
   return bin_axis(x, xmin, inv, n);
 }
 
+constexpr bool kCall = !kFast;   // k_lists_forces calls its quotients (af3d_physics.cuh)
+
 constexpr double kSmallAngle2 = 9.765625e-04;   // (2^-5)^2
 
 // sin t and cos t of a rotation angle t >= 0 with t2 = t^2 (rounded).  Below 2^-5 rad (a step of
@@ -327,6 +329,7 @@ struct Rows {
 // init_Verlet.cu:63-114: the rotation rows turned by the angle vector dO, columns renormalised.
 // In the fast mode the path of the device friction law, of turns of 2^-10 rad and more and of
 // unnormalised input (the others run in fixed point, predict_state), not inlined there.
+template <bool CALL = false>
 #ifdef AF3D_FAST
 __device__ __noinline__
 #else
@@ -365,7 +368,7 @@ Rows turn_rows(V3 dO, V3 Rx, V3 Ry, V3 Rz) {
       imag = rsqrt(mag2);
       mag = mag2 * imag;
     } else {
-      mag = sqrt_rn(mag2);
+      mag = root<CALL>(mag2);
     }
     if (positive_bits(mag)) {
       // Rodrigues rotation about dO/|dO| by |dO| (init_Verlet.cu:63-83)
@@ -375,8 +378,7 @@ Rows turn_rows(V3 dO, V3 Rx, V3 Ry, V3 Rz) {
         u = mk(dO.x * imag, dO.y * imag, dO.z * imag);
         sincos(mag, &sn, &c);
       } else {
-        const Divisor by = divisor_of(mag);
-        u = mk(div_by(dO.x, by), div_by(dO.y, by), div_by(dO.z, by));
+        u = div3<CALL>(dO, mag);
         sincos_step(mag, mag2, sn, c);   // init_Verlet.cu's cos and sin
       }
       const double omc = 1.0 - c;
@@ -410,12 +412,12 @@ Rows turn_rows(V3 dO, V3 Rx, V3 Ry, V3 Rz) {
     in = inv_norm(Tx.z * Tx.z + Ty.z * Ty.z + Tz.z * Tz.z);
     Rx.z = Tx.z * in; Ry.z = Ty.z * in; Rz.z = Tz.z * in;
   } else {
-    Divisor by = divisor_of(sqrt_rn(Tx.x * Tx.x + Ty.x * Ty.x + Tz.x * Tz.x));
-    Rx.x = div_by(Tx.x, by); Ry.x = div_by(Ty.x, by); Rz.x = div_by(Tz.x, by);
-    by = divisor_of(sqrt_rn(Tx.y * Tx.y + Ty.y * Ty.y + Tz.y * Tz.y));
-    Rx.y = div_by(Tx.y, by); Ry.y = div_by(Ty.y, by); Rz.y = div_by(Tz.y, by);
-    by = divisor_of(sqrt_rn(Tx.z * Tx.z + Ty.z * Ty.z + Tz.z * Tz.z));
-    Rx.z = div_by(Tx.z, by); Ry.z = div_by(Ty.z, by); Rz.z = div_by(Tz.z, by);
+    V3 q = div3<CALL>(mk(Tx.x, Ty.x, Tz.x), root<CALL>(Tx.x * Tx.x + Ty.x * Ty.x + Tz.x * Tz.x));
+    Rx.x = q.x; Ry.x = q.y; Rz.x = q.z;
+    q = div3<CALL>(mk(Tx.y, Ty.y, Tz.y), root<CALL>(Tx.y * Tx.y + Ty.y * Ty.y + Tz.y * Tz.y));
+    Rx.y = q.x; Ry.y = q.y; Rz.y = q.z;
+    q = div3<CALL>(mk(Tx.z, Ty.z, Tz.z), root<CALL>(Tx.z * Tx.z + Ty.z * Ty.z + Tz.z * Tz.z));
+    Rx.z = q.x; Ry.z = q.y; Rz.z = q.z;
   }
   return Rows{Rx, Ry, Rz};
 }
@@ -455,6 +457,7 @@ __device__ __forceinline__ void place_spheres(V3 r, V3 Rx, V3 Ry, V3 Rz, double 
 // 262,144 clumps 198 -> 190 us, of 582,320 in 64 flumes 414 -> 398 us (2,048 clumps, where one warp
 // has an SM's sub-partition to itself and latency counts: 35.4 -> 37.3 us).  dev: the device friction
 // law, whose runs show every last bit (af3d_physics.cuh): in FP64.
+template <bool CALL = false>
 __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, V3 &Rx, V3 &Ry, V3 &Rz, V3 *sp,
                                               double rad, double dt, double hdt, int qs, bool dev) {
   r.x += dt * (v.x + hdt * a.x);
@@ -484,11 +487,11 @@ __device__ __forceinline__ void predict_state(V3 &r, V3 &v, V3 &w, V3 a, V3 al, 
         return;
       }
     } else {
-      const Rows t = turn_rows(dO, Rx, Ry, Rz);
+      const Rows t = turn_rows<CALL>(dO, Rx, Ry, Rz);
       Rx = t.x; Ry = t.y; Rz = t.z;
     }
   } else {
-    const Rows t = turn_rows(dO, Rx, Ry, Rz);
+    const Rows t = turn_rows<CALL>(dO, Rx, Ry, Rz);
     Rx = t.x; Ry = t.y; Rz = t.z;
   }
   place_spheres(r, Rx, Ry, Rz, pos, sp);
@@ -987,6 +990,7 @@ __device__ __noinline__ SlowSums removed_contacts(const NbrRec *me, double B, co
 // A boundary item of owner record `me`: its force and torque terms into res (components `stride`
 // apart); 3 with a force, else 0.  Not inlined: the seven routines' inputs raise the register
 // pressure of whatever they are inlined into, and a round of items is of one kind.
+template <bool CALL = false>
 __device__ __noinline__ int bnd_contact(unsigned it, const NbrRec *me, const Consts &co, double *res, int stride) {
   const int rt = (int)((it >> 2) & 7u), ns = (int)(it & 3u);
   Sph q;
@@ -997,7 +1001,7 @@ __device__ __noinline__ int bnd_contact(unsigned it, const NbrRec *me, const Con
   q.rad = me->rad;
   q.mwall = me->mwall;
   V3 fs, tq;
-  if (!bnd_sphere(rt, q, co, fs, tq)) return 0;
+  if (!bnd_sphere<CALL>(rt, q, co, fs, tq)) return 0;
   res[0] = fs.x; res[stride] = fs.y; res[2 * stride] = fs.z;
   res[3 * stride] = tq.x; res[4 * stride] = tq.y; res[5 * stride] = tq.z;
   return 3;
@@ -1042,10 +1046,10 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
     ContactIn ci;
     V3 fs, tq;
     int r = 0;
-    if (pair_input(rl, mk(me.vx, me.vy, me.vz), mk(me.wx, me.wy, me.wz),
+    if (pair_input<kCall>(rl, mk(me.vx, me.vy, me.vz), mk(me.wx, me.wy, me.wz),
                    mk(me.s[3 * k], me.s[3 * k + 1], me.s[3 * k + 2]), me.rad, me.msph, nbr[t], p >> 2, co,
                    co.variant == AF3D_FRICTION_DEV, ci) &&
-        apply_law(ci, rl, co, fs, tq)) {
+        apply_law<kCall>(ci, rl, co, fs, tq)) {
       r = 2;
       bq.res[0][jb] = fs.x; bq.res[1][jb] = fs.y; bq.res[2][jb] = fs.z;
       bq.res[3][jb] = tq.x; bq.res[4][jb] = tq.y; bq.res[5][jb] = tq.z;
@@ -1098,7 +1102,7 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
       const int at = bq.place[i];
       if (it >= kBndItem) {
         const long os = bbase + bq.owner[i];
-        bq.flag[at] = (unsigned char)bnd_contact(it, nbr + os, constants_of(os), &bq.res[0][at], kBatch);
+        bq.flag[at] = (unsigned char)bnd_contact<kCall>(it, nbr + os, constants_of(os), &bq.res[0][at], kBatch);
       }
     }
     __syncthreads();
@@ -1331,7 +1335,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
     }
     V3 v2, w2, a, al;
     if (!removed) {
-      get_accel_one(F, T, v, w, Rx, Ry, Rz, P.p[MASS][s], P.p[ADRAG][s], load3(P, IXX, s), a, al, P.p[IMASS][s],
+      get_accel_one<kCall>(F, T, v, w, Rx, Ry, Rz, P.p[MASS][s], P.p[ADRAG][s], load3(P, IXX, s), a, al, P.p[IMASS][s],
                     P.p[IINER][s], c.variant == AF3D_FRICTION_DEV);
       store3(P, AFX, s, a);
       store3(P, ALFX, s, al);
@@ -1367,7 +1371,7 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
         store3(P, RN10, s, Ry);
         store3(P, RN20, s, Rz);
       } else {
-        predict_state(rn, vn, wn, a, al, Rx, Ry, Rz, sp, P.p[RAD][s], fl.sys.dt, fl.sys.hdt, P.m.qs,
+        predict_state<kCall>(rn, vn, wn, a, al, Rx, Ry, Rz, sp, P.p[RAD][s], fl.sys.dt, fl.sys.hdt, P.m.qs,
                       c.variant == AF3D_FRICTION_DEV);
         store3(P, RN00, s, Rx);
         store3(P, RN10, s, Ry);

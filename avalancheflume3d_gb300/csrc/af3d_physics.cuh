@@ -71,6 +71,36 @@ __device__ __forceinline__ V3 mk(double x, double y, double z) {
   return r;
 }
 
+// ---- Quotients and roots, inlined or called ----------------------------------------------------
+// CALL: the exact mode's force kernel of large counts calls them.  Its some thirty integer-pipe quotients
+// and roots inlined made it 818 KB of code (663 KB so), and blocks that drift out of phase in a long launch
+// then wait for instructions: 64 flumes of 32,768 clumps, device friction law, 4207 us a step inlined,
+// 3532 called (3789 with the hardware's); 262,144 clumps 8.28 and 8.18 ms a 20-step call.  Elsewhere a
+// call costs up to 1.5 % (9,973 clumps 3.35 -> 3.41 ms a 100-step call), and the fast mode forms fewer.
+static __device__ __noinline__ V3 div3_called(V3 a, double b) {
+  const Divisor by = divisor_of(b);
+  return mk(div_by(a.x, by), div_by(a.y, by), div_by(a.z, by));
+}
+static __device__ __noinline__ double quot_called(double a, double b) { return div_rn(a, b); }
+static __device__ __noinline__ double root_called(double x) { return sqrt_rn(x); }
+
+template <bool CALL>
+__device__ __forceinline__ V3 div3(V3 a, double b) {
+  if constexpr (CALL) return div3_called(a, b);
+  const Divisor by = divisor_of(b);
+  return mk(div_by(a.x, by), div_by(a.y, by), div_by(a.z, by));
+}
+template <bool CALL>
+__device__ __forceinline__ double quot(double a, double b) {
+  if constexpr (CALL) return quot_called(a, b);
+  return div_rn(a, b);
+}
+template <bool CALL>
+__device__ __forceinline__ double root(double x) {
+  if constexpr (CALL) return root_called(x);
+  return sqrt_rn(x);
+}
+
 // ---- FP64 tests and conversions on the integer pipe ----------------------------------------
 // The FP64 pipe of this GPU retires one warp instruction per 16 (DFMA) to 19 SM cycles, and conversions and
 // comparisons of doubles occupy it like arithmetic does.  These helpers take the same decisions
@@ -249,6 +279,7 @@ __device__ __forceinline__ bool contact_law_fast(V3 dvvc, V3 n, double comp, dou
   return true;
 }
 
+template <bool CALL = false>
 __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double km, double gm,
                                             double mass_t, double mu, double cns_1, double dt,
                                             bool xi0, bool gate, V3 &f) {
@@ -272,15 +303,20 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
   vt.x = dvvc.x - vn * n.x;
   vt.y = dvvc.y - vn * n.y;
   vt.z = dvvc.z - vn * n.z;
-  const double vt_mag = sqrt_rn(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
-  const Divisor vt_div = divisor_of(vt_mag);
+  const double vt_mag = root<CALL>(vt.x * vt.x + vt.y * vt.y + vt.z * vt.z);
+  Divisor vt_div;
+  if constexpr (!CALL) vt_div = divisor_of(vt_mag);
+  auto over_vt = [&](double x) {   // x / |vt|
+    if constexpr (CALL) return quot_called(x, vt_mag);
+    else return div_by(x, vt_div);
+  };
   double xi = 0.0, fsdt = 0.0;
   if (!gated) {
-    const V3 tv = mk(div_by(vt.x, vt_div), div_by(vt.y, vt_div), div_by(vt.z, vt_div));
+    const V3 tv = CALL ? div3<CALL>(vt, vt_mag) : mk(over_vt(vt.x), over_vt(vt.y), over_vt(vt.z));
     const double vt_sig = dvvc.x * tv.x + dvvc.y * tv.y + dvvc.z * tv.z;
     xi = dt * vt_sig;
     if (less_bits(cns_1 * normal, fabs(xi))) xi = 0.0;
-    const double xi_dot = nonzero_bits(xi) || !nonzero_bits(dt) ? div_rn(xi, dt) : xi;
+    const double xi_dot = nonzero_bits(xi) || !nonzero_bits(dt) ? quot<CALL>(xi, dt) : xi;
     fsdt = 1.0e12 * mass_t * xi + 2.0e6 * mass_t * xi_dot;
   }
   if (positive_bits(vt_mag)) {
@@ -290,11 +326,11 @@ __device__ __forceinline__ bool contact_law(V3 dvvc, V3 n, double comp, double k
     // a warp whose lanes take different branches executes three divisions, not seven; every
     // lane still evaluates exactly its own branch's operations.
     const bool coulomb = less_bits(mu * normal, fabs(fsdt)) || (xi0 && !nonzero_bits(xi));
-    const double q1 = div_by(coulomb ? 0.8 * mu * normal : fsdt * vt.x, vt_div);   // af  | f_x term
-    const double q2 = div_rn(coulomb ? mass_t : fsdt * vt.y, coulomb ? q1 : vt_mag);   // t0 | f_y
-    const double q3 = div_rn(coulomb ? dt : fsdt * vt.z, coulomb ? q2 : vt_mag);   // dt/t0 | f_z
+    const double q1 = over_vt(coulomb ? 0.8 * mu * normal : fsdt * vt.x);   // af  | f_x term
+    const double q2 = quot<CALL>(coulomb ? mass_t : fsdt * vt.y, coulomb ? q1 : vt_mag);   // t0 | f_y
+    const double q3 = quot<CALL>(coulomb ? dt : fsdt * vt.z, coulomb ? q2 : vt_mag);   // dt/t0 | f_z
     if (coulomb) {
-      const double af = div_rn(q1, 1.0 + q3 * q3);
+      const double af = quot<CALL>(q1, 1.0 + q3 * q3);
       f.x += af * vt.x;
       f.y += af * vt.y;
       f.z += af * vt.z;
@@ -381,10 +417,11 @@ __device__ __forceinline__ void wall_input(const Sph &o, V3 rrc, V3 n, double co
 }
 
 // The contact law on a prepared contact: force fs and its torque term about the clump centre r.
+template <bool CALL = false>
 __device__ __forceinline__ bool apply_law(const ContactIn &ci, V3 r, const Consts &c, V3 &fs, V3 &tq) {
   const bool on = kFast ? contact_law_fast(ci.dvvc, ci.n, ci.comp, ci.km, ci.gm, ci.mass_t, ci.mu, ci.cns, c.dt,
                                            c.inv_dt, ci.xi0, ci.gate, c.variant == AF3D_FRICTION_DEV, fs)
-                        : contact_law(ci.dvvc, ci.n, ci.comp, ci.km, ci.gm, ci.mass_t, ci.mu, ci.cns, c.dt,
+                        : contact_law<CALL>(ci.dvvc, ci.n, ci.comp, ci.km, ci.gm, ci.mass_t, ci.mu, ci.cns, c.dt,
                                       ci.xi0, ci.gate, fs);
   if (!on) return false;
   tq = torque_term(ci.rrc, r, fs);
@@ -542,9 +579,10 @@ __device__ __forceinline__ bool bnd_input(int routine, const Sph &o, const Const
 }
 
 // The force of routine `routine` on one sphere and its torque term (false: no force).
+template <bool CALL = false>
 __device__ __forceinline__ bool bnd_sphere(int routine, const Sph &o, const Consts &c, V3 &fs, V3 &tq) {
   ContactIn ci;
-  return bnd_input(routine, o, c, ci) && apply_law(ci, o.r, c, fs, tq);
+  return bnd_input(routine, o, c, ci) && apply_law<CALL>(ci, o.r, c, fs, tq);
 }
 
 // One boundary routine over the four spheres of a clump, with the reference's removed-clump
@@ -658,6 +696,7 @@ __device__ __forceinline__ bool spheres_overlap(const V3 &s1, double rad_1, cons
   return less_bits(dist2, sep2);
 }
 
+template <bool CALL = false>
 __device__ __forceinline__ bool pair_input(const V3 &rrl, const V3 &vvl, const V3 &wwl, const V3 &s1,
                                            double rad_1, double massl, const NbrRec &m, int sm,
                                            const Consts &c, bool xi0, ContactIn &ci) {
@@ -685,9 +724,8 @@ __device__ __forceinline__ bool pair_input(const V3 &rrl, const V3 &vvl, const V
     }
     ci.n = mk(d.x * inv, d.y * inv, d.z * inv);
   } else {
-    dist = sqrt_rn(dist2);
-    const Divisor by = divisor_of(dist);
-    ci.n = mk(div_by(d.x, by), div_by(d.y, by), div_by(d.z, by));
+    dist = root<CALL>(dist2);
+    ci.n = div3<CALL>(d, dist);
   }
   ci.rrc = mk(s1.x + rad_1 * ci.n.x, s1.y + rad_1 * ci.n.y, s1.z + rad_1 * ci.n.z);
   V3 vl = point_velocity(vvl, wwl, ci.rrc, rrl);
@@ -741,9 +779,10 @@ __device__ __forceinline__ double plus_signed_zero(double q, float a, float b) {
 }
 
 // |v| of the drag from v2 = |v|^2 (dev: the device friction law, see the header comment).
+template <bool CALL = false>
 __device__ __forceinline__ double speed_of(double v2, bool dev) {
   if (kFast && dev) return v2 == 0.0 ? 0.0 : v2 * rsqrt(v2);   // NaN stays NaN
-  return sqrt_rn(v2);
+  return root<CALL>(v2);
 }
 
 // get_accel.cu:21-75 for one clump; R rows Rx, Ry, Rz.  `adrag0` = DRAG*rad*rad/m (the same
@@ -752,21 +791,22 @@ __device__ __forceinline__ double speed_of(double v2, bool dev) {
 // i.e. signed zeros; they are formed from the sign bits instead of two divisions-by-I and four
 // multiplications, which gives the same bits for finite angular velocities.
 // (fast mode: im = 1/m and iI = 1/I.x, formed once at import, replace the divisions)
+template <bool CALL = false>
 __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 Ry, V3 Rz, double m,
                                               double adrag0, V3 I, V3 &a, V3 &al, double im, double iI,
                                               bool dev) {
   const double v2 = v.x * v.x + v.y * v.y + v.z * v.z;
-  double vmag = speed_of(v2, dev);
+  double vmag = speed_of<CALL>(v2, dev);
   double adrag = adrag0 * vmag;
   if (kFast) {
     a.x = f.x * im - adrag * v.x;
     a.y = f.y * im - adrag * v.y;
     a.z = f.z * im - adrag * v.z - kGRAV;
   } else {
-    const Divisor by = divisor_of(m);
-    a.x = div_by(f.x, by) - adrag * v.x;
-    a.y = div_by(f.y, by) - adrag * v.y;
-    a.z = div_by(f.z, by) - adrag * v.z - kGRAV;
+    const V3 q = div3<CALL>(f, m);
+    a.x = q.x - adrag * v.x;
+    a.y = q.y - adrag * v.y;
+    a.z = q.z - adrag * v.z - kGRAV;
   }
   V3 wb, tb, ab;
   const bool isotropic =
@@ -789,8 +829,7 @@ __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 
   if (!kFast && isotropic) {
     // Only the signs of the body-frame spin are needed, and only where a quotient is zero
     // (a clump without contacts): taken in FP32 where they are certain.
-    const Divisor by = divisor_of(I.x);
-    ab = mk(div_by(tb.x, by), div_by(tb.y, by), div_by(tb.z, by));
+    ab = div3<CALL>(tb, I.x);
     const float wx = truncated_f(w.x), wy = truncated_f(w.y), wz = truncated_f(w.z);
     const float r[9] = {truncated_f(Rx.x), truncated_f(Ry.x), truncated_f(Rz.x), truncated_f(Rx.y), truncated_f(Ry.y),
                         truncated_f(Rz.y), truncated_f(Rx.z), truncated_f(Ry.z), truncated_f(Rz.z)};
@@ -821,10 +860,10 @@ __device__ __forceinline__ void get_accel_one(V3 f, V3 t, V3 v, V3 w, V3 Rx, V3 
       ab.y = tb.y * iI + signed_zero_product(wb.z, wb.x);
       ab.z = tb.z * iI + signed_zero_product(wb.x, wb.y);
     } else {
-      const Divisor by = divisor_of(I.x);
-      ab.x = div_by(tb.x, by) + signed_zero_product(wb.y, wb.z);
-      ab.y = div_by(tb.y, by) + signed_zero_product(wb.z, wb.x);
-      ab.z = div_by(tb.z, by) + signed_zero_product(wb.x, wb.y);
+      const V3 q = div3<CALL>(tb, I.x);
+      ab.x = q.x + signed_zero_product(wb.y, wb.z);
+      ab.y = q.y + signed_zero_product(wb.z, wb.x);
+      ab.z = q.z + signed_zero_product(wb.x, wb.y);
     }
   } else {
     double Cxy = (I.x - I.y) / I.z;

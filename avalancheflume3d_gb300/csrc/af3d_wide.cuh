@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
         if (it < kBndItem) continue;
         const long os = bbase + sh.owner[i];
         const int at = sh.place[i];
-        sh.flag[at] = (unsigned char)bnd_contact(it, nbr + os, constants_of(os), &sh.res[0][at], kBatch);
+        sh.flag[at] = (unsigned char)bnd_contact<>(it, nbr + os, constants_of(os), &sh.res[0][at], kBatch);
       }
       __syncthreads();
       const int e1 = base + nitems < b0 + bn ? base + nitems - b0 : bn;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
                     plus_signed_zero(ab.z, sb[0], sb[1]));
           }
           const double v2s = v.x * v.x + v.y * v.y + v.z * v.z;
-          const double adrag = adrag0 * speed_of(v2s, dev);
+          const double adrag = adrag0 * speed_of<false>(v2s, dev);
           const double vi = comp(v, i);
           if (kFast) ai = Fi * im - adrag * vi;
           else ai = div_by(Fi, divisor_of(mass)) - adrag * vi;
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kWideThreads, 4)
             place_row(comp(r1, i), mk(Rr[0], Rr[1], Rr[2]), pos, c4);
           }
         } else {
-          const Rows t = turn_rows(dO, mk(sh.col[0][lane], sh.col[1][lane], sh.col[2][lane]),
+          const Rows t = turn_rows<>(dO, mk(sh.col[0][lane], sh.col[1][lane], sh.col[2][lane]),
                                    mk(sh.col[3][lane], sh.col[4][lane], sh.col[5][lane]),
                                    mk(sh.col[6][lane], sh.col[7][lane], sh.col[8][lane]));
           const V3 row = i == 0 ? t.x : i == 1 ? t.y : t.z;
