@@ -268,8 +268,8 @@ __device__ __forceinline__ void for_slots_around(float4 c, const CellAt &at, con
         end[q] = __ldg(row + b.x1 + 1);
       }
     }
-#pragma unroll
-    for (int q = 0; q < 4; q++)
+#pragma unroll 1
+    for (int q = 0; q < 4; q++)   // (one copy of f's code)
 #pragma unroll 1
       for (; k[q] < end[q]; k[q]++) f(order ? __ldg(&order[k[q]]) : k[q]);
   }
