@@ -273,8 +273,8 @@ constexpr long kWideClumps = AF3D_WIDE_CLUMPS;
 
 // Per-clump item lists of one force pass, from the list phase to the force phase of the force
 // kernel: entry e of slot s at items[e * n + s] (an item is a boundary (routine, sphere) or a
-// particle (partner slot, sph_id) contact).  With cnt, the pass also records each clump's list
-// layout there (pack_list_counts), which lets the adjoint reverse the pass from the same lists,
+// particle (partner slot, sph_id) contact).  With cnt, the pass leaves the items with a force alone and
+// records each clump's list layout there (pack_list_counts), from which the adjoint reverses the pass,
 // and with ovf sets *ovf when any clump's lists overflowed (its contacts then ran by the
 // per-clump walk, which needs the pass's cell structure).
 constexpr int kListCap = 32;

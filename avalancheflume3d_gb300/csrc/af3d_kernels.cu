@@ -1009,17 +1009,17 @@ __device__ __noinline__ int bnd_contact(unsigned it, const NbrRec *me, const Con
 
 // UNIFORM: every clump of the launch belongs to one flume, whose constants `c` are (a
 // reference to) a kernel parameter.  lc: the clump's list layout (pre boundary items, particle
-// items, the rest boundary items).
-template <int NB, bool UNIFORM>
+// items, the rest boundary items).  RECORD: a pass that keeps its lists (`record`) leaves only the items
+// with a force in them, and `listed` and lc say so: the adjoint has nothing to reverse at the others.
+template <int NB, bool UNIFORM, bool RECORD>
 __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, long s, bool act, bool aval,
                                               const Consts &c, const DevScalars *d, const int *__restrict__ flume,
                                               const NbrRec *__restrict__ nbr,
                                               const CullRec *__restrict__ cull,
                                               const int *__restrict__ start,
                                               const int *__restrict__ order, const long long *__restrict__ id,
-                                              const NearLists &near, const Margins &m, const unsigned *items,
-                                              int listed, ListCounts lc, long n,
-                                              V3 &F, V3 &T) {
+                                              const NearLists &near, const Margins &m, unsigned *items, bool record,
+                                              int &listed, ListCounts &lc, long n, V3 &F, V3 &T) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pre0 = aval ? R_HOP0 : 1, pre1 = aval ? R_WALLS : 0;         // fill: none before
   const int post0 = aval ? R_FLUME : R_HOP0, post1 = aval ? R_FLUME : R_HOP2;
@@ -1057,6 +1057,8 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
     bq.flag[jb] = (unsigned char)r;
   };
   int active = 0;
+  int kept = 0;
+  ListCounts kc = {0, 0};
   // Owners add their items' terms in list order.
   auto gather = [&](int b0, int bn) {
     if (nitems <= 0) return;
@@ -1068,6 +1070,12 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
       T.x += bq.res[3][e]; T.y += bq.res[4][e]; T.z += bq.res[5][e];
       F.x += bq.res[0][e]; F.y += bq.res[1][e]; F.z += bq.res[2][e];
       active += fl == 2;   // sphere-sphere contacts only
+      if (RECORD && record) {   // (never past the entries that are still to be laid out)
+        const int at = e + b0 - base;
+        items[n * kept++ + s] = items[(long)at * n + s];
+        kc.pre += at < lc.pre;
+        kc.pair += fl == 2;
+      }
     }
   };
   // A block whose items fit one batch takes them in kind order: every particle item of the
@@ -1108,6 +1116,10 @@ __device__ __forceinline__ int block_contacts(BlockQueue<NB> &bq, long bbase, lo
     __syncthreads();
     gather(b0, bn);
     __syncthreads();
+  }
+  if (RECORD && record && nitems > 0) {
+    listed = kept;
+    lc = kc;
   }
   if (slow) {
     const SlowSums r = slow_contacts(s, pre0, pre1, post0, post1, c, d, flume, nbr, cull, start, order, id, near, m, n,
@@ -1306,9 +1318,11 @@ __device__ __forceinline__ void fused_body(const Consts &c, Planes P, Planes out
     T = r.T;
   }
   const long bbase = s0 + blockIdx.x * (long)blockDim.x;
-  const int active = block_contacts<NB, UNIFORM>(sh.bq, bbase, sv, valid && !removed, aval, c, d, flume, nbr, cull,
-                                                 cells.start, order, id, near, P.m, lists.items, valid ? listed : 0, lc,
-                                                 n, F, T);
+  if (!valid) listed = 0;
+  const int active =
+      block_contacts<NB, UNIFORM, WRITE_FT>(sh.bq, bbase, sv, valid && !removed, aval, c, d, flume, nbr, cull,
+                                            cells.start, order, id, near, P.m, lists.items, lists.cnt != nullptr,
+                                            listed, lc, n, F, T);
   if (la.nbr) __syncthreads();   // the force phase's shared memory is free for the record staging
   if (valid) {
     if (lists.cnt) lists.cnt[s] = pack_list_counts(listed, lc.pre, lc.pair);

@@ -103,12 +103,12 @@ __global__ void __launch_bounds__(kWideThreads, 4)
     const bool kind_order = total <= kBatch;
     if (w == 2 && valid) {
       if (slow || (act && info < 0)) atomicAdd(&d->overflows, 1ull);
-      if (lists.cnt) lists.cnt[s] = pack_list_counts(slow ? -1 : nitems, npre, npair);
       if (lists.ovf && slow) *lists.ovf = 1;
       if (counted) cells.occ[cull[s].key] = 0;
     }
     double Fi = 0.0, Ti = 0.0;   // warps 0..2: this component of the sums
     int active = 0;              // warp 3: sphere-sphere contacts
+    int kept = 0, kept_pre = 0;  // ... and the recorded items, those with a force (block_contacts)
     if (valid && removed && aval && w < 3) {
       const SlowSums r = removed_contacts(&me, (double)cull[sv].c.w, c);
       Fi = comp(r.F, w);
@@ -184,6 +184,11 @@ __global__ void __launch_bounds__(kWideThreads, 4)
           Fi += sh.res[w][e];
         } else {
           active += k == 2;
+          if (lists.cnt) {
+            const int at = e + b0 - base;
+            col[n * kept++] = col[(long)at * n];
+            kept_pre += at < npre;
+          }
         }
       }
       __syncthreads();
@@ -201,7 +206,10 @@ __global__ void __launch_bounds__(kWideThreads, 4)
         active = r.active;
       }
     }
-    if (w == 3) warp_count(d, active);
+    if (w == 3) {
+      warp_count(d, active);
+      if (lists.cnt && valid) lists.cnt[s] = pack_list_counts(slow ? -1 : kept, kept_pre, slow ? 0 : active);
+    }
 
     // get_accel and finish_Verlet, one component a warp (i = w)
     const int i = w, i1 = w == 2 ? 0 : w + 1, i2 = w == 0 ? 2 : w - 1;
