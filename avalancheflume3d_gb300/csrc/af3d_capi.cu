@@ -122,6 +122,7 @@ struct af3d_ctx {
   int phase = AF3D_PHASE_AVALANCHE;
   int variant = AF3D_FRICTION_HST;
   int fp_mode = AF3D_FP_EXACT;
+  int sms = 0;
   int force_shape = 0;       // index into kForceShapeBlock / kForceShapeMinb
   double obj_length = 0.0;   // objective of af3d_adjoint: 0 deposit centroid, > 0 runout length scale
   long cc = 0;                        // steps done in the current phase
@@ -388,10 +389,12 @@ void forces_for(af3d_ctx *c, bool write_ft, Planes out, bool warm = false, bool 
     uni = &kc;
   }
   LookAhead la{};
-  if (look) la = LookAhead{c->nbr_next, c->cull_next, next_builds, look && !c->taping};
-  auto run = c->fp_mode == AF3D_FP_FAST ? fast::launch_lists_forces : launch_lists_forces;
+  if (look) la = LookAhead{c->nbr_next, c->cull_next, next_builds, !c->taping};
+  const bool fast = c->fp_mode == AF3D_FP_FAST;
+  const bool wide = c->n <= wide_clumps(c->sms, fast && c->variant == AF3D_FRICTION_DEV);
+  auto run = fast ? fast::launch_lists_forces : launch_lists_forces;
   run(c->L(), c->cur, out, c->d, c->fl_cur, c->nbr, c->cull, c->cells, c->built_order, c->id_cur, c->near, c->lists,
-      c->ntags, write_ft, counted, uni, warm, la, s0, count, c->force_shape);
+      c->ntags, write_ft, counted, wide, uni, warm, la, s0, count, c->force_shape);
   c->launches++;
 }
 
@@ -642,6 +645,7 @@ af3d_status af3d_create_ensemble(int nflumes, const af3d_system_par *sys, const 
   cudaError_t e = cudaGetDevice(&c->device);
   int sms = 0;
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  c->sms = sms;
   c->force_shape = force_shape_for(c->n, sms);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
@@ -736,7 +740,8 @@ af3d_status af3d_destroy(af3d_ctx *c) {
   drop_graphs(c);
   for (void *p : {(void *)c->plane_mem[0], (void *)c->plane_mem[1], (void *)c->id_cur, (void *)c->id_alt,
                   (void *)c->fl_cur, (void *)c->fl_alt, (void *)c->flume_of_id, (void *)c->nbr,
-                  (void *)c->cull, (void *)c->lists.items, (void *)c->nbr_next, (void *)c->cull_next, (void *)c->cells.key, (void *)c->cells.rank_tmp, (void *)c->cells.tmp_slot,
+                  (void *)c->cull, (void *)c->lists.items, (void *)c->nbr_next, (void *)c->cull_next,
+                  (void *)c->cells.key, (void *)c->cells.rank_tmp, (void *)c->cells.tmp_slot,
                   (void *)c->cells.perm, (void *)c->cells.csort, (void *)c->cells.count, (void *)c->cells.start,
                   (void *)c->cells.tile_count, (void *)c->cells.occ, (void *)c->cells.occ_next, (void *)c->near.items,
                   (void *)c->near.info, (void *)c->near.bnd, (void *)c->near.rem, (void *)c->near.loose,

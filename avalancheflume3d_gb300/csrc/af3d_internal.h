@@ -262,14 +262,17 @@ constexpr long kForceAlign = 384;
 static_assert(kForceAlign % 128 == 0 && kForceAlign % 96 == 0 && kForceAlign % 64 == 0 && kForceAlign % 192 == 0,
               "a multiple of every shape's block");
 
-// Up to this many clumps a force pass runs in blocks of 32 clumps on 128 threads whatever the shape
-// (af3d_wide.cuh).  The line lies where its blocks fill the 152 SMs once (four an SM, 19,456 clumps);
-// us a step of a dense bed, wide against the shapes: 16,384 clumps fast 31 and 44, exact 42 and 58;
-// 20,000 45 and 46, 62 and 65; 24,576 50 and 48, 72 and 66.
-#ifndef AF3D_WIDE_CLUMPS
-#define AF3D_WIDE_CLUMPS 20480
-#endif
-constexpr long kWideClumps = AF3D_WIDE_CLUMPS;
+// Up to how many clumps a force pass runs in blocks of 32 clumps on 128 threads whatever the shape
+// (af3d_wide.cuh): four such blocks an SM are one wave, 19,456 clumps on 152 SMs, and a few blocks more
+// cost less than the shapes do, up to a nineteenth of a wave (20,480 clumps); under the fast mode's device
+// law, whose rotation three of its warps each form whole, just the wave.  us a step of a dense bed, wide and the
+// shapes: fast 16,384 clumps 23.0 and 31.7, 19,456 24.4 and 34.0, 20,480 34.0 and 34.8, 21,000 34.9 and
+// 35.0, 22,000 35.9 and 34.6; exact 20,480 44.8 and 49.2, 22,000 48.6 and 49.1, 24,320 51.6 and 49.7; fast with
+// the device law 19,456 31.2 and 31.8, 20,011 42.6 and 37.8.
+inline long wide_clumps(int sms, bool fast_device_law) {
+  const long wave = 4L * 32 * sms;
+  return fast_device_law ? wave : wave + wave / 19;
+}
 
 // Per-clump item lists of one force pass, from the list phase to the force phase of the force
 // kernel: entry e of slot s at items[e * n + s] (an item is a boundary (routine, sphere) or a
@@ -374,11 +377,12 @@ void launch_build_lists (const Launch &L, Margins m, DevScalars *d, const int *f
 // them (walls, contacts, bed, get_accel, finish_Verlet).  order: that of the last built lists.
 // warm: the step's predicted state was made by the previous pass's look-ahead (records, RN
 // planes) and is committed to the planes here; look: this pass runs the next step's predictor.
-// counted: this step's buckets were counted in cells.occ, which the pass zeroes.
+// counted: this step's buckets were counted in cells.occ, which the pass zeroes.  wide: in blocks of 32
+// clumps on four warps (wide_clumps), else in blocks of `shape`.
 void launch_lists_forces (const Launch &L, Planes cur, Planes out, DevScalars *d, const int *flume,
                           const NbrRec *nbr, const CullRec *cull, Cells cells, const int *order,
                           const long long *id, NearLists near, ContactLists lists, long ntags, bool write_ft,
-                          bool counted, const Consts *uniform = nullptr, bool warm = false,
+                          bool counted, bool wide, const Consts *uniform = nullptr, bool warm = false,
                           LookAhead look = LookAhead{}, long s0 = 0, long count = -1, int shape = 0);
 void launch_boundary (const Launch &L, Planes cur, DevScalars *d, const int *flume, int routine);
 void launch_part (const Launch &L, Planes cur, DevScalars *d, const int *flume, const NbrRec *nbr,
@@ -442,7 +446,7 @@ void launch_predict (const Launch &L, Planes cur, DevScalars *d, bool predict, b
 void launch_lists_forces (const Launch &L, Planes cur, Planes out, DevScalars *d, const int *flume,
                           const NbrRec *nbr, const CullRec *cull, Cells cells, const int *order,
                           const long long *id, NearLists near, ContactLists lists, long ntags, bool write_ft,
-                          bool counted, const Consts *uniform = nullptr, bool warm = false,
+                          bool counted, bool wide, const Consts *uniform = nullptr, bool warm = false,
                           LookAhead look = LookAhead{}, long s0 = 0, long count = -1, int shape = 0);
 }  // namespace fast
 

@@ -526,8 +526,8 @@ __device__ __forceinline__ long bucket_key(V3 r, const DevFlume &fl, DevScalars 
 // A clump's place in a step that keeps its near lists: counted in its cell for the capacity check
 // of cells.cu:96-102 (at most ntags - 1 clumps), and its motion since the previous step's record
 // (old) against its allowance: with none left it is away at tick `tick` (true, for its record).
-__device__ __forceinline__ bool keep_place(long s, const int4 *old, const CullRec &cr, const DevFlume &fl, DevScalars *d,
-                                           int *occ, long ntags, const NearLists &near,
+__device__ __forceinline__ bool keep_place(long s, const int4 *old, const CullRec &cr, const DevFlume &fl,
+                                           DevScalars *d, int *occ, long ntags, const NearLists &near,
                                            const int *__restrict__ start, const int *__restrict__ order,
                                            const Margins &m, int tick, long n) {
   if (ntags > 0 && cr.key < d->ncell_total && atomicAdd(&occ[cr.key], 1) + 1 >= ntags)
@@ -548,7 +548,8 @@ __device__ __forceinline__ bool keep_place(long s, const int4 *old, const CullRe
 // the clump's neighbour records at its own slot (steps that keep the slot order).  count_only: the
 // step does not sort but keeps its near lists (keep_place; with RECORDS).
 template <bool PREDICT, bool KEYS, bool RECORDS>
-__global__ void __launch_bounds__(kBlock) k_predict(const __grid_constant__ Planes P, DevScalars *d, bool t_prev, Cells cells,
+__global__ void __launch_bounds__(kBlock) k_predict(const __grid_constant__ Planes P, DevScalars *d, bool t_prev,
+                                                    Cells cells,
                                                     const long long *__restrict__ id,
                                                     const int *__restrict__ flume, long ntags,
                                                     const __grid_constant__ NearLists near,
@@ -1723,8 +1724,8 @@ void launch_build_records(const Launch &L, Planes cur, NbrRec *nbr, CullRec *cul
 // memory (the block's own entries, visible to its threads after the barrier).
 template <int NB, int MINB, bool WRITE_FT, bool UNIFORM>
 __global__ void __launch_bounds__(NB, MINB)
-    k_lists_forces(const __grid_constant__ Planes P, const __grid_constant__ Planes out, DevScalars *d, const int *__restrict__ flume, const NbrRec *__restrict__ nbr,
-                   const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
+    k_lists_forces(const __grid_constant__ Planes P, const __grid_constant__ Planes out, DevScalars *d,
+                   const int *__restrict__ flume, const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
                    const int *__restrict__ order, const long long *__restrict__ id,
                    const __grid_constant__ NearLists near, ContactLists lists, long ntags, bool counted,
                    const __grid_constant__ Consts kc, bool warm, const __grid_constant__ LookAhead la, long s0,
@@ -1753,7 +1754,7 @@ __global__ void __launch_bounds__(NB, MINB)
 
 void launch_lists_forces(const Launch &L, Planes cur, Planes out, DevScalars *d, const int *flume,
                          const NbrRec *nbr, const CullRec *cull, Cells cells, const int *order, const long long *id,
-                         NearLists near, ContactLists lists, long ntags, bool write_ft, bool counted,
+                         NearLists near, ContactLists lists, long ntags, bool write_ft, bool counted, bool wide,
                          const Consts *uniform, bool warm, LookAhead look, long s0, long count, int shape) {
   // slots [s0, s0 + count) of L.n (count < 0: to the end); s0 a multiple of the shape's block,
   // so the launch's blocks are those of the whole pass
@@ -1762,13 +1763,13 @@ void launch_lists_forces(const Launch &L, Planes cur, Planes out, DevScalars *d,
   static_assert(kForceShapes == 4 && kForceShapeBlock[0] == 128 && kForceShapeBlock[1] == 96 &&
                     kForceShapeBlock[2] == 64 && kForceShapeBlock[3] == 192, "the instantiated shapes");
   const Consts kc = uniform ? *uniform : Consts{};
-  if (L.n <= kWideClumps) {
-    auto wide = [&](auto kernel) {
-      kernel<<<grid_for(m, kWide), kWideThreads, 0, L.st>>>(cur, out, d, flume, nbr, cull, cells, order, id, near, lists,
-                                                           ntags, write_ft, counted, kc, warm, look, s0, L.n);
+  if (wide) {
+    auto run = [&](auto kernel) {
+      kernel<<<grid_for(m, kWide), kWideThreads, 0, L.st>>>(cur, out, d, flume, nbr, cull, cells, order, id, near,
+                                                           lists, ntags, write_ft, counted, kc, warm, look, s0, L.n);
     };
-    if (uniform) wide(k_forces_wide<true>);
-    else wide(k_forces_wide<false>);
+    if (uniform) run(k_forces_wide<true>);
+    else run(k_forces_wide<false>);
     return;
   }
   auto run = [&](auto kernel, int nb) {

@@ -30,7 +30,8 @@ struct NearShared {
 // the partners with smaller ids.  Bound by the latency of its chain of loads and tests, so it is
 // split over four warps: a whole clump per thread took 47 us at 8,192 clumps, 49 at 32,768 and
 // about 200 for 100,003 in four parts; so it is 31, 38 and 75 (in one launch).
-__global__ void __launch_bounds__(kNearBlock) k_build_lists(const __grid_constant__ Margins m, DevScalars *d, const int *__restrict__ flume,
+__global__ void __launch_bounds__(kNearBlock) k_build_lists(const __grid_constant__ Margins m, DevScalars *d,
+                                                            const int *__restrict__ flume,
                                                             const CullRec *__restrict__ cull,
                                                             const int *__restrict__ start,
                                                             const int *__restrict__ order,

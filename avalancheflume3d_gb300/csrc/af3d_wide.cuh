@@ -1,6 +1,6 @@
 // af3d_wide.cuh -- the force pass of small clump counts: 32 clumps on a block of 128 threads.
 //
-// Up to kWideClumps clumps k_lists_forces leaves most of the chip idle (2,048 clumps are 64 warps on
+// Up to about 20,000 clumps (wide_clumps) k_lists_forces leaves most of the chip idle (2,048 clumps are 64 warps on
 // 608 sub-partitions) and a pass takes as long as one warp's chain of instructions: an FP64
 // instruction every 64 cycles, ~400 of them, and as many cycles again in integer work and loads.
 // Here a block's four warps share its 32 clumps (lane = clump): warp 0 tests the near pairs while
@@ -49,8 +49,8 @@ __device__ __noinline__ Accel get_accel_whole(V3 f, V3 t, V3 v, V3 w, Rows R, do
 
 template <bool UNIFORM>
 __global__ void __launch_bounds__(kWideThreads, 4)
-    k_forces_wide(const __grid_constant__ Planes P, const __grid_constant__ Planes out, DevScalars *d, const int *__restrict__ flume, const NbrRec *__restrict__ nbr,
-                  const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
+    k_forces_wide(const __grid_constant__ Planes P, const __grid_constant__ Planes out, DevScalars *d,
+                  const int *__restrict__ flume, const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
                   const int *__restrict__ order, const long long *__restrict__ id,
                   const __grid_constant__ NearLists near, ContactLists lists, long ntags, bool write_ft, bool counted,
                   const __grid_constant__ Consts kc, bool warm, const __grid_constant__ LookAhead la, long s0, long n) {
@@ -77,7 +77,9 @@ __global__ void __launch_bounds__(kWideThreads, 4)
       sh.npair[lane] = np;
     } else if (w == 1) {
       unsigned b = 0u;
-      if (act) b = touching(search ? 0x0FFFFFFFu : near.bnd[sv], me, __int_as_float(cull[sv].s[0].w) * unit_power(-P.m.qs), c);
+      if (act)
+        b = touching(search ? 0x0FFFFFFFu : near.bnd[sv], me,
+                     __int_as_float(cull[sv].s[0].w) * unit_power(-P.m.qs), c);
       sh.bnd[lane] = b;
     }
     __syncthreads();
@@ -134,7 +136,9 @@ __global__ void __launch_bounds__(kWideThreads, 4)
       };
       if (w == 0 && !slow)
         for (int e = npair - 1; e >= 0; e--)   // (a search left its items in the column: the last first)
-          lay(search ? col[(long)(e + (lists.cnt && b0 > 0 ? npre : 0)) * n] : list[(long)(sh.pl.cand[e][lane] & 63u) * n], npre + e, pb + e);
+          lay(search ? col[(long)(e + (lists.cnt && b0 > 0 ? npre : 0)) * n]
+                     : list[(long)(sh.pl.cand[e][lane] & 63u) * n],
+              npre + e, pb + e);
       __syncthreads();   // (the recorded column's head may hold a search's items until here)
       if (w == 1 && !slow) {
         int e = 0, j = ptotal + (base - pb);

@@ -272,8 +272,9 @@ af3d_status af3d_autotune (af3d_ctx *ctx, long steps_per_trial, long *resort_eve
 /* The fused force kernel's block (no counterpart in the reference): 64, 96, 128 or 192 threads,
    one clump per thread, the block's clumps pooling their contact items; each runs at the
    resident blocks per SM that measured fastest for it (10, 6, 5 and 3).  Results do not depend
-   on it, and up to 20,480 clumps the steps run in a shape of their own.  A new context starts with the block of 64, 96 and 128 whose last wave is fullest for
-   its clump count on the current device; af3d_set_force_block overrides it. */
+   on it, and up to 20,480 clumps (on 152 SMs; 19,456 in fast mode with the device friction law) the
+   steps run in a shape of their own.  A new context starts with the block of 64, 96 and 128 whose last
+   wave is fullest for its clump count on the current device; af3d_set_force_block overrides it. */
 af3d_status af3d_set_force_block (af3d_ctx *ctx, int block);
 af3d_status af3d_get_force_block (af3d_ctx *ctx, int *block);
 /* Autotuner over both shape parameters (no counterpart in the reference): af3d_autotune (the
