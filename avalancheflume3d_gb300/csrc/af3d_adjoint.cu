@@ -17,7 +17,9 @@
 // sum do not depend on the order of its terms.
 //
 // Compiled with -fmad=false like the exact step kernels (the forward re-evaluation must take
-// the forward's branches).
+// the forward's branches).  The derivative itself takes products with reciprocals of one unit in the
+// last place where the formulas have quotients: 1/|v_t| and 1/(1 + r^2) of the law, 1/|d| of a pair, 1/m,
+// 1/I and the drag's 1/|v|.
 #include "af3d_adjoint.cuh"
 #include "af3d_cellwalk.cuh"
 

@@ -2,7 +2,9 @@
 //
 // These kernels recompute only the rotation update of the step they reverse, to form its
 // derivative: no branch depends on a recomputed value, so they are compiled with contracted
-// multiply-adds (-fmad=true), unlike the contact re-evaluation in af3d_adjoint.cu.
+// multiply-adds (-fmad=true), unlike the contact re-evaluation in af3d_adjoint.cu, and with
+// reciprocals of one unit in the last place for 1/|dO| and the column norms, radius (1/sqrt 2) for radius /
+// sqrt 2.
 #include "af3d_adjoint.cuh"
 
 namespace af3d {
