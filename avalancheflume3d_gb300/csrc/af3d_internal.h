@@ -177,7 +177,8 @@ struct Consts {
 };
 
 // The constants of a flume from its parameters (the same values the device loads).
-__host__ __device__ inline Consts make_consts(const af3d_system_par &s, const af3d_funnel &fun, double tant, int phase, int variant,
+__host__ __device__ inline Consts make_consts(const af3d_system_par &s, const af3d_funnel &fun, double tant, int phase,
+                                              int variant,
                           const double *tp) {
   Consts c;
   c.dt = s.dt; c.hdt = s.hdt;
@@ -327,7 +328,8 @@ struct NearLists {
 // RN planes, and it is counted in the next step's buckets: for the sort (build: the next step
 // sorts and builds lists) or for the cells' capacity alone.  The pass's last block advances the
 // clock.  The records carry r, v, w and the sphere centres from step to step and the RN planes the
-// rotation: a pass with `keep` stores 240 B per clump less (262,144 clumps: a step 171 -> 167 us, 582,320 in 64 flumes 358 -> 346).
+// rotation: a pass with `keep` stores 240 B per clump less (262,144 clumps: a step 171 -> 167 us, 582,320
+// in 64 flumes 358 -> 346).
 // nbr == null: none.
 struct LookAhead {
   NbrRec *nbr;

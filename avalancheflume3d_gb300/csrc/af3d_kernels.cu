@@ -895,7 +895,7 @@ __device__ __noinline__ int search_items(long s, const DevScalars *d, const int 
                                           const int *__restrict__ start, const int *__restrict__ order,
                                           const long long *__restrict__ id, const NearLists &near, const Margins &m,
                                           long n, unsigned *col, int nitems) {
-  unsigned long long keys[kListCap];
+  unsigned long long keys[kListCap] = {};
   unsigned items[kListCap];
   const int room = kListCap - nitems;
   int found = 0;
@@ -1725,7 +1725,8 @@ void launch_build_records(const Launch &L, Planes cur, NbrRec *nbr, CullRec *cul
 template <int NB, int MINB, bool WRITE_FT, bool UNIFORM>
 __global__ void __launch_bounds__(NB, MINB)
     k_lists_forces(const __grid_constant__ Planes P, const __grid_constant__ Planes out, DevScalars *d,
-                   const int *__restrict__ flume, const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
+                   const int *__restrict__ flume, const NbrRec *__restrict__ nbr,
+                   const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
                    const int *__restrict__ order, const long long *__restrict__ id,
                    const __grid_constant__ NearLists near, ContactLists lists, long ntags, bool counted,
                    const __grid_constant__ Consts kc, bool warm, const __grid_constant__ LookAhead la, long s0,

@@ -75,8 +75,9 @@ __device__ __forceinline__ V3 mk(double x, double y, double z) {
 // CALL: the exact mode's force kernel of large counts calls them.  Its some thirty integer-pipe quotients
 // and roots inlined made it 818 KB of code (663 KB so), and blocks that drift out of phase in a long launch
 // then wait for instructions: 64 flumes of 32,768 clumps, device friction law, 4207 us a step inlined,
-// 3532 called (3789 with the hardware's); 262,144 clumps 8.28 and 8.18 ms a 20-step call.  Elsewhere a
-// call costs up to 1.5 % (9,973 clumps 3.35 -> 3.41 ms a 100-step call), and the fast mode forms fewer.
+// 3488 called (3790 with the hardware's); one flume of 262,144 clumps 8.27 and 8.14 ms a 20-step call, of
+// 32,768 clumps, whose launches are short, 80.9 and 82.3 us a step.  Elsewhere a call costs up to 1.5 %
+// (9,973 clumps 3.35 -> 3.41 ms a 100-step call), and the fast mode forms fewer.
 static __device__ __noinline__ V3 div3_called(V3 a, double b) {
   const Divisor by = divisor_of(b);
   return mk(div_by(a.x, by), div_by(a.y, by), div_by(a.z, by));

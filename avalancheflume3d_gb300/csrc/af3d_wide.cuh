@@ -50,7 +50,8 @@ __device__ __noinline__ Accel get_accel_whole(V3 f, V3 t, V3 v, V3 w, Rows R, do
 template <bool UNIFORM>
 __global__ void __launch_bounds__(kWideThreads, 4)
     k_forces_wide(const __grid_constant__ Planes P, const __grid_constant__ Planes out, DevScalars *d,
-                  const int *__restrict__ flume, const NbrRec *__restrict__ nbr, const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
+                  const int *__restrict__ flume, const NbrRec *__restrict__ nbr,
+                  const CullRec *__restrict__ cull, const __grid_constant__ Cells cells,
                   const int *__restrict__ order, const long long *__restrict__ id,
                   const __grid_constant__ NearLists near, ContactLists lists, long ntags, bool write_ft, bool counted,
                   const __grid_constant__ Consts kc, bool warm, const __grid_constant__ LookAhead la, long s0, long n) {

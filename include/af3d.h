@@ -200,7 +200,7 @@ af3d_status af3d_step (af3d_ctx *ctx, long k);
 
 /* Same steps as af3d_step, enqueued without graphs and with CUDA events between the kernels on
    the context stream; adds the milliseconds of each phase to ms[AF3D_NPROF]:
-   0 time advance, 1 init_Verlet + cell keys, 2 cell sort and near lists (one step in 16),
+   0 time advance, 1 init_Verlet + cell keys, 2 cell sort and near lists (one step in 16, 8, 4 or 2),
    3 permutation + neighbour records, 4 force kernel (contacts, walls, bed, get_accel,
    finish_Verlet, the next step's init_Verlet), 5 re-grid. */
 enum { AF3D_NPROF = 6 };
